@@ -165,7 +165,74 @@ col2im_kernel(const bf16* __restrict__ dcol, bf16* __restrict__ dx, const GeepsC
   }
 }
 
-// ---------------- per-channel reductions over a [P][C] (pitch ld) bf16 matrix ----------------
+// ---------------- per-channel work on a [P][C] (pitch ld) bf16 matrix ----------------
+// How a block's threads cover the matrix: thread = (pixel row r, 8-channel slot), so a thread keeps its slot for every
+// pixel it visits: per-channel constants are loaded once, sums stay in registers, and no item costs an integer
+// division (bn_apply spent most of its 77 us on a 32 x 56 x 56 x 192 tensor there and on reloading its six
+// constants per channel; forward + backward of that layer 198 -> 158 us, the 49-kernel Inception block 334 -> 269 us).
+// A row of threads reads whole contiguous pixels.  gridDim.y splits C above 2048 channels.
+struct SlotMap {
+  int cvb, rows, row, slot, c;     // slots per block, pixel rows per block, this thread's row / slot / first channel
+  bool on;
+  long long p0, step;              // first pixel, pixels between two of this thread
+  __device__ __forceinline__ explicit SlotMap(int C) {
+    const int cv = C >> 3;
+    cvb = (cv + (int)gridDim.y - 1) / (int)gridDim.y;
+    rows = (int)blockDim.x / cvb;
+    row = (int)threadIdx.x / cvb;
+    slot = (int)threadIdx.x - row * cvb;
+    const int gslot = (int)blockIdx.y * cvb + slot;
+    c = gslot * 8;
+    on = row < rows && gslot < cv;
+    p0 = (long long)blockIdx.x * rows + row;
+    step = (long long)gridDim.x * rows;
+  }
+};
+struct SlotGrid { dim3 grid; int threads; size_t smem; };
+// Launch shape: 256-ish threads as rows x slots, about `per_thread` pixels a thread (one batch of loads in flight),
+// at most `per_sm` blocks per SM.  smem: the block's partial sums, nq floats per channel and pixel row.
+inline SlotGrid slot_grid(long long P, int C, int per_thread, int per_sm, int nq) {
+  const int cv = C / 8 < 1 ? 1 : C / 8;
+  SlotGrid g;
+  const int chunks = (cv + 255) / 256;
+  const int cvb = (cv + chunks - 1) / chunks;
+  const int rows = cvb >= 256 ? 1 : 256 / cvb;
+  g.threads = (rows * cvb + 31) / 32 * 32;
+  const int rows_used = g.threads / cvb;        // as SlotMap computes it
+  long long want = (P + (long long)rows_used * per_thread - 1) / ((long long)rows_used * per_thread);
+  const long long cap = (long long)geeps_sm_count() * per_sm / chunks;
+  if (want > cap) want = cap;
+  if (want < 1) want = 1;
+  g.grid = dim3((unsigned)want, (unsigned)chunks, 1);
+  g.smem = (size_t)rows_used * cvb * 8 * nq * sizeof(float);
+  return g;
+}
+// Sum the threads' partial sums over the block's pixel rows and add them to out[channel] (+ out[C + channel]).  The
+// rows meet in shared memory as plain stores: float atomics on shared memory are compare-and-swap loops, and 16 of
+// them per thread were most of the 12 us a reduction of a 6272 x 160 matrix took.
+template <int NQ>
+__device__ __forceinline__ void slot_sums(const SlotMap& m, const float (&a0)[8], const float (&a1)[8], float* out, int C,
+                                          float scale, float* part) {
+  const int width = m.cvb * 8;
+  if (m.row < m.rows) {
+    float* d = part + (size_t)m.row * width * NQ + m.slot * 8;
+    *reinterpret_cast<float4*>(d) = make_float4(a0[0], a0[1], a0[2], a0[3]);
+    *reinterpret_cast<float4*>(d + 4) = make_float4(a0[4], a0[5], a0[6], a0[7]);
+    if (NQ == 2) {
+      *reinterpret_cast<float4*>(d + width) = make_float4(a1[0], a1[1], a1[2], a1[3]);
+      *reinterpret_cast<float4*>(d + width + 4) = make_float4(a1[4], a1[5], a1[6], a1[7]);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < width * NQ; i += blockDim.x) {
+    float v = 0.f;
+    for (int r = 0; r < m.rows; ++r) v += part[(size_t)r * width * NQ + i];
+    const int q = NQ == 2 && i >= width ? 1 : 0;
+    const int ch = (int)blockIdx.y * width + i - q * width;
+    if (ch < C) atomicAdd(out + (size_t)q * C + ch, v * scale);
+  }
+}
+
 // MODE 0: out[c] += sum x, out[C+c] += sum x^2                  (BN forward statistics)
 // MODE 1: out[c] += sum dy', out[C+c] += sum dy' * xhat          (BN backward; dy' = dy masked by y>0 if relu)
 // MODE 2: out[c] += scale * sum x                                (bias gradient)
@@ -174,52 +241,59 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
                                                     const bf16* __restrict__ y, const float* __restrict__ mean_rstd,
                                                     float* __restrict__ out, long long P, int C, long long ldx,
                                                     long long lddy, int relu, float scale) {
-  extern __shared__ float sacc[];  // [2*C]
-  for (int i = threadIdx.x; i < 2 * C; i += blockDim.x) sacc[i] = 0.f;
-  __syncthreads();
-  const int cv = C >> 3;
-  const long long nthreads = (long long)gridDim.x * blockDim.x;
-  const long long groups = nthreads / cv;  // pixel lanes: each owns one 8-channel slot
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid < groups * cv) {
-    const int c = (int)(tid % cv) * 8;
-    float a0[8], a1[8];
+  extern __shared__ __align__(16) float sacc[];  // [rows][(1 or 2) * 8 * slots]
+  const SlotMap m(C);
+  float a0[8], a1[8], mu[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) { a0[e] = 0.f; a1[e] = 0.f; }
-    float mu[8], rs[8];
+  for (int e = 0; e < 8; ++e) { a0[e] = 0.f; a1[e] = 0.f; mu[e] = 0.f; }
+  if (m.on) {
     if (MODE == 1) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { mu[e] = mean_rstd[c + e]; rs[e] = mean_rstd[C + c + e]; }
+      for (int e = 0; e < 8; ++e) mu[e] = mean_rstd[m.c + e];
     }
-    for (long long p = tid / cv; p < P; p += groups) {
-      if (MODE == 0 || MODE == 2) {
-        Bf8 v = ld8(x + p * ldx + c);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) { float f = bf(v.v[e]); a0[e] += f; if (MODE == 0) a1[e] += f * f; }
-      } else {
-        Bf8 xv = ld8(x + p * ldx + c), dv = ld8(dy + p * lddy + c), yv;
-        if (relu) yv = ld8(y + p * lddy + c);
+    auto add = [&](const Bf8& xv, const Bf8& dv, const Bf8& yv) {
+      if (MODE == 1) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           float d = bf(dv.v[e]);
           if (relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
           a0[e] += d;
-          a1[e] += d * (bf(xv.v[e]) - mu[e]) * rs[e];
+          a1[e] += d * (bf(xv.v[e]) - mu[e]);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { const float f = bf(xv.v[e]); a0[e] += f; if (MODE == 0) a1[e] += f * f; }
+      }
+    };
+    constexpr int U = 4;              // pixels whose loads are in flight together
+    long long p = m.p0;
+    for (; p + (U - 1) * m.step < P; p += U * m.step) {
+      Bf8 xv[U], dv[U], yv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        xv[u] = ld8(x + (p + u * m.step) * ldx + m.c);
+        if (MODE == 1) {
+          dv[u] = ld8(dy + (p + u * m.step) * lddy + m.c);
+          if (relu) yv[u] = ld8(y + (p + u * m.step) * lddy + m.c);
         }
       }
-    }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      atomicAdd(&sacc[c + e], a0[e]);
-      if (MODE != 2) atomicAdd(&sacc[C + c + e], a1[e]);
+      for (int u = 0; u < U; ++u) add(xv[u], dv[u], yv[u]);
+    }
+    for (; p < P; p += m.step) {
+      Bf8 xv = ld8(x + p * ldx + m.c), dv, yv;
+      if (MODE == 1) {
+        dv = ld8(dy + p * lddy + m.c);
+        if (relu) yv = ld8(y + p * lddy + m.c);
+      }
+      add(xv, dv, yv);
+    }
+    if (MODE == 1) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a1[e] *= mean_rstd[C + m.c + e];
     }
   }
-  __syncthreads();
-  const int nout = MODE == 2 ? C : 2 * C;
-  for (int i = threadIdx.x; i < nout; i += blockDim.x) {
-    const float v = sacc[i];
-    if (v != 0.f) atomicAdd(out + i, MODE == 2 ? v * scale : v);
-  }
+  slot_sums<MODE == 2 ? 1 : 2>(m, a0, a1, out, C, MODE == 2 ? scale : 1.f, sacc);
 }
 template <int MODE>
 __global__ void __launch_bounds__(256)
@@ -256,25 +330,46 @@ __global__ void bn_finalize_kernel(const float* __restrict__ sums, float* __rest
   }
 }
 
+// y = (x - m) * k + b, k = gamma / std, through ReLU where asked: the pixel loop of both normalisation kernels
+__device__ __forceinline__ void bn_apply_pixels(const SlotMap& s, const bf16* __restrict__ x, bf16* __restrict__ y,
+                                                const float (&m)[8], const float (&k)[8], const float (&b)[8], long long P,
+                                                long long ldx, long long ldy, int relu) {
+  auto one = [&](const Bf8& v) {
+    Bf8 o;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float f = fmaf(bf(v.v[e]) - m[e], k[e], b[e]);
+      if (relu) f = fmaxf(f, 0.f);
+      o.v[e] = __float2bfloat16(f);
+    }
+    return o;
+  };
+  constexpr int U = 4;
+  long long p = s.p0;
+  for (; p + (U - 1) * s.step < P; p += U * s.step) {
+    Bf8 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = ld8(x + (p + u * s.step) * ldx + s.c);
+#pragma unroll
+    for (int u = 0; u < U; ++u) st8(y + (p + u * s.step) * ldy + s.c, one(v[u]));
+  }
+  for (; p < P; p += s.step) st8(y + p * ldy + s.c, one(ld8(x + p * ldx + s.c)));
+}
+
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ mean_rstd,
                 const float* __restrict__ gamma, const float* __restrict__ beta, long long P, int C,
                 long long ldx, long long ldy, int relu) {
-  const int cv = C >> 3;
-  const long long total = P * cv;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const int c = (int)(i % cv) * 8;
-    const long long p = i / cv;
-    Bf8 v = ld8(x + p * ldx + c), o;
+  const SlotMap s(C);
+  if (!s.on) return;
+  float m[8], k[8], b[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float f = (bf(v.v[e]) - mean_rstd[c + e]) * mean_rstd[C + c + e] * gamma[c + e] + beta[c + e];
-      if (relu) f = fmaxf(f, 0.f);
-      o.v[e] = __float2bfloat16(f);
-    }
-    st8(y + p * ldy + c, o);
+  for (int e = 0; e < 8; ++e) {
+    m[e] = mean_rstd[s.c + e];
+    k[e] = mean_rstd[C + s.c + e] * gamma[s.c + e];
+    b[e] = beta[s.c + e];
   }
+  bn_apply_pixels(s, x, y, m, k, b, P, ldx, ldy, relu);
 }
 
 // Normalisation with the statistics finalised inside: every thread derives mean and 1/std of its eight channels from
@@ -287,37 +382,28 @@ __device__ __forceinline__ void bn_apply_fused_body(const bf16* __restrict__ x, 
                                                     const float* __restrict__ gamma, const float* __restrict__ beta,
                                                     float* zero_after, long long P, int C, long long ldx, long long ldy,
                                                     int relu, float inv_count, float eps, float momentum) {
-  const int cv = C >> 3;
-  const long long total = P * cv;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const int c = (int)(i % cv) * 8;
-    const long long p = i / cv;
-    float m[8], r[8];
+  const SlotMap s(C);
+  if (!s.on) return;
+  float m[8], k[8], b[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      m[e] = sums[c + e] * inv_count;
-      const float var = fmaxf(sums[C + c + e] * inv_count - m[e] * m[e], 0.f);
-      r[e] = rsqrtf(var + eps);
-      if (p == 0) {
-        mean_rstd[c + e] = m[e];
-        mean_rstd[C + c + e] = r[e];
-        if (running_mean) {
-          running_mean[c + e] = (1.f - momentum) * running_mean[c + e] + momentum * m[e];
-          running_var[c + e] = (1.f - momentum) * running_var[c + e] + momentum * var;
-        }
-        if (zero_after) { zero_after[c + e] = 0.f; zero_after[C + c + e] = 0.f; }
+  for (int e = 0; e < 8; ++e) {
+    const int c = s.c + e;
+    m[e] = __ldcg(sums + c) * inv_count;
+    const float var = fmaxf(__ldcg(sums + C + c) * inv_count - m[e] * m[e], 0.f);
+    const float r = rsqrtf(var + eps);
+    k[e] = r * gamma[c];
+    b[e] = beta[c];
+    if (s.p0 == 0 && P > 0) {
+      mean_rstd[c] = m[e];
+      mean_rstd[C + c] = r;
+      if (running_mean) {
+        running_mean[c] = (1.f - momentum) * running_mean[c] + momentum * m[e];
+        running_var[c] = (1.f - momentum) * running_var[c] + momentum * var;
       }
+      if (zero_after) { zero_after[c] = 0.f; zero_after[C + c] = 0.f; }
     }
-    Bf8 v = ld8(x + p * ldx + c), o;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float f = (bf(v.v[e]) - m[e]) * r[e] * gamma[c + e] + beta[c + e];
-      if (relu) f = fmaxf(f, 0.f);
-      o.v[e] = __float2bfloat16(f);
-    }
-    st8(y + p * ldy + c, o);
   }
+  bn_apply_pixels(s, x, y, m, k, b, P, ldx, ldy, relu);
 }
 __global__ void __launch_bounds__(256)
 bn_apply_fused_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ sums,
@@ -335,31 +421,52 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
                                                  const float* sums, float* dgamma, float* dbeta, long long P, int C,
                                                  long long ldx, long long lddy, long long lddx, int relu,
                                                  float grad_scale, float* zero_after) {
-  const int cv = C >> 3;
-  const long long total = P * cv;
-  const long long stride = (long long)gridDim.x * blockDim.x;
+  const SlotMap s(C);
+  if (!s.on) return;
   const float invP = 1.f / (float)P;
-  const long long tid0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid0 < C) {
-    if (dbeta) dbeta[tid0] = sums[tid0] * grad_scale;
-    if (dgamma) dgamma[tid0] = sums[C + tid0] * grad_scale;
-    // the scratch of this layer's next forward reduction (nobody reads it during the backward pass)
-    if (zero_after) { zero_after[tid0] = 0.f; zero_after[C + tid0] = 0.f; }
+  float m[8], k[8], c0[8], c1[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int c = s.c + e;
+    const float rs = mean_rstd[C + c], s0 = __ldcg(sums + c), s1 = __ldcg(sums + C + c);
+    m[e] = mean_rstd[c];
+    k[e] = gamma[c] * rs;
+    c0[e] = s0 * invP;
+    c1[e] = rs * (s1 * invP);
+    if (s.p0 == 0) {
+      if (dbeta) dbeta[c] = s0 * grad_scale;
+      if (dgamma) dgamma[c] = s1 * grad_scale;
+      // the scratch of this layer's next forward reduction (nobody reads it during the backward pass)
+      if (zero_after) { zero_after[c] = 0.f; zero_after[C + c] = 0.f; }
+    }
   }
-  for (long long i = tid0; i < total; i += stride) {
-    const int c = (int)(i % cv) * 8;
-    const long long p = i / cv;
-    Bf8 xv = ld8(x + p * ldx + c), dv = ld8(dy + p * lddy + c), yv, o;
-    if (relu) yv = ld8(y + p * lddy + c);
+  auto one = [&](const Bf8& xv, const Bf8& dv, const Bf8& yv) {
+    Bf8 o;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       float d = bf(dv.v[e]);
       if (relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
-      const float rs = mean_rstd[C + c + e];
-      const float xhat = (bf(xv.v[e]) - mean_rstd[c + e]) * rs;
-      o.v[e] = __float2bfloat16(gamma[c + e] * rs * (d - sums[c + e] * invP - xhat * sums[C + c + e] * invP));
+      o.v[e] = __float2bfloat16(k[e] * (d - c0[e] - (bf(xv.v[e]) - m[e]) * c1[e]));
     }
-    st8(dx + p * lddx + c, o);
+    return o;
+  };
+  constexpr int U = 4;
+  long long p = s.p0;
+  for (; p + (U - 1) * s.step < P; p += U * s.step) {
+    Bf8 xv[U], dv[U], yv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      xv[u] = ld8(x + (p + u * s.step) * ldx + s.c);
+      dv[u] = ld8(dy + (p + u * s.step) * lddy + s.c);
+      if (relu) yv[u] = ld8(y + (p + u * s.step) * lddy + s.c);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) st8(dx + (p + u * s.step) * lddx + s.c, one(xv[u], dv[u], yv[u]));
+  }
+  for (; p < P; p += s.step) {
+    Bf8 xv = ld8(x + p * ldx + s.c), dv = ld8(dy + p * lddy + s.c), yv;
+    if (relu) yv = ld8(y + p * lddy + s.c);
+    st8(dx + p * lddx + s.c, one(xv, dv, yv));
   }
 }
 __global__ void __launch_bounds__(256)
@@ -400,11 +507,11 @@ bn_forward_coop_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, float* 
                        const float* __restrict__ beta, float* zero_after, int* bar, long long P, int C, long long ldx,
                        long long ldy, int relu, float inv_count, float eps, float momentum) {
   channel_reduce_body<0>(x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
-  if (bn_grid_barrier(bar, (int)gridDim.x))
+  if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
     bn_apply_fused_body(x, y, sums, mean_rstd, running_mean, running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                         inv_count, eps, momentum);
   else if (threadIdx.x == 0) { bar[2] = 1; mean_rstd[0] = __int_as_float(0x7fc00000); }
-  bn_grid_done(bar, (int)gridDim.x);
+  bn_grid_done(bar, (int)(gridDim.x * gridDim.y));
 }
 __global__ void __launch_bounds__(256)
 bn_backward_coop_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
@@ -412,11 +519,11 @@ bn_backward_coop_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
                         float* dgamma, float* dbeta, float* zero_after, int* bar, long long P, int C, long long ldx,
                         long long lddy, long long lddx, int relu, float grad_scale) {
   channel_reduce_body<1>(x, dy, y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  if (bn_grid_barrier(bar, (int)gridDim.x))
+  if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
     bn_backward_body(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
                      zero_after);
   else if (threadIdx.x == 0) { bar[2] = 1; mean_rstd[0] = __int_as_float(0x7fc00000); }
-  bn_grid_done(bar, (int)gridDim.x);
+  bn_grid_done(bar, (int)(gridDim.x * gridDim.y));
 }
 
 // ---------------- ReLU backward / dropout ----------------
@@ -467,25 +574,17 @@ f32_to_bf16_2d_kernel(const float* __restrict__ src, bf16* __restrict__ dst, lon
   }
 }
 // ReLU backward fused with the per-channel sums of its result (the bias gradient of the layer whose output y is):
-// dx = y > 0 ? dy : 0, out[c] += sum over pixels of dx.  Every thread keeps one 8-channel slot and strides over
-// the pixels, as in channel_reduce_kernel.
+// dx = y > 0 ? dy : 0, out[c] += sum over pixels of dx.
 __global__ void __launch_bounds__(256)
 relu_backward_colsum_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ y, bf16* __restrict__ dx,
                             float* __restrict__ out, long long P, int C, long long lddy, long long ldy, long long lddx) {
-  extern __shared__ float sacc[];  // [C]
-  for (int i = threadIdx.x; i < C; i += blockDim.x) sacc[i] = 0.f;
-  __syncthreads();
-  const int cv = C >> 3;
-  const long long nthreads = (long long)gridDim.x * blockDim.x;
-  const long long groups = nthreads / cv;
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid < groups * cv) {
-    const int c = (int)(tid % cv) * 8;
-    float a[8];
+  extern __shared__ __align__(16) float sacc[];  // [rows][8 * slots]
+  const SlotMap m(C);
+  float a[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) a[e] = 0.f;
-    for (long long p = tid / cv; p < P; p += groups) {
-      const Bf8 d = ld8(dy + p * lddy + c), v = ld8(y + p * ldy + c);
+  for (int e = 0; e < 8; ++e) a[e] = 0.f;
+  if (m.on) {
+    auto one = [&](const Bf8& d, const Bf8& v) {
       Bf8 o;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
@@ -493,13 +592,23 @@ relu_backward_colsum_kernel(const bf16* __restrict__ dy, const bf16* __restrict_
         o.v[e] = on ? d.v[e] : __float2bfloat16(0.f);
         a[e] += on ? bf(d.v[e]) : 0.f;
       }
-      st8(dx + p * lddx + c, o);
-    }
+      return o;
+    };
+    constexpr int U = 4;
+    long long p = m.p0;
+    for (; p + (U - 1) * m.step < P; p += U * m.step) {
+      Bf8 d[U], v[U];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) atomicAdd(&sacc[c + e], a[e]);
+      for (int u = 0; u < U; ++u) {
+        d[u] = ld8(dy + (p + u * m.step) * lddy + m.c);
+        v[u] = ld8(y + (p + u * m.step) * ldy + m.c);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) st8(dx + (p + u * m.step) * lddx + m.c, one(d[u], v[u]));
+    }
+    for (; p < P; p += m.step) st8(dx + p * lddx + m.c, one(ld8(dy + p * lddy + m.c), ld8(y + p * ldy + m.c)));
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < C; i += blockDim.x) atomicAdd(out + i, sacc[i]);
+  slot_sums<1>(m, a, a, out, C, 1.f, sacc);
 }
 // dst += src over 2-D views (sum of branch gradients)
 __global__ void __launch_bounds__(256)
@@ -1318,13 +1427,10 @@ int geeps_col2im(const void* dcol, void* dx, const GeepsConvGeom* g, int accumul
   return CK();
 }
 
-static int reduce_grid(long long P, int C) {
-  long long want = (P * (C / 8) + 255) / 256;
-  if (want > geeps_sm_count() * 4) want = geeps_sm_count() * 4;
-  long long min_blocks = ((long long)(C / 8) + 255) / 256;
-  if (want < min_blocks) want = min_blocks;
-  return (int)(want < 1 ? 1 : want);
-}
+// reductions: one batch of four pixels per thread where that leaves SMs idle, at most four blocks per SM beyond
+static SlotGrid reduce_grid(long long P, int C, int nq = 2) { return slot_grid(P, C, 4, 4, nq); }
+// element-wise passes with per-channel constants: up to eight blocks per SM
+static SlotGrid apply_grid(long long P, int C) { return slot_grid(P, C, 4, 8, 0); }
 
 int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* beta, float* sums,
                      float* mean_rstd, float* running_mean, float* running_var, long long P, int C,
@@ -1332,11 +1438,12 @@ int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* be
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
-  channel_reduce_kernel<0><<<reduce_grid(P, C), 256, 2 * C * sizeof(float), st>>>(
+  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  channel_reduce_kernel<0><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   bn_finalize_kernel<<<(C + 127) / 128, 128, 0, st>>>(sums, mean_rstd, running_mean, running_var, C,
                                                       1.f / (float)P, eps, momentum);
-  bn_apply_kernel<<<grid_1d(P * (C / 8)), 256, 0, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
+  bn_apply_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
                                                         ldy, relu);
   return CK();
 }
@@ -1347,9 +1454,10 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
-  channel_reduce_kernel<1><<<reduce_grid(P, C), 256, 2 * C * sizeof(float), st>>>(
+  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  channel_reduce_kernel<1><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  bn_backward_kernel<<<grid_1d(P * (C / 8)), 256, 0, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
+  bn_backward_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
                                                            (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
                                                            ldx, lddy, lddx, relu, grad_scale, nullptr);
   return CK();
@@ -1360,11 +1468,7 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
 // finalisation launch: 2 launches per direction instead of 4 and 3.
 // grid of a single-launch BatchNorm kernel: enough blocks for the reduction, never more than can be resident at
 // once beside other kernels (the blocks wait for one another at the grid barrier)
-static int bn_coop_grid(long long P, int C) {
-  int g = reduce_grid(P, C);
-  const int cap = geeps_sm_count();
-  return g > cap ? cap : g;
-}
+static SlotGrid bn_coop_grid(long long P, int C) { return slot_grid(P, C, 4, 1, 2); }
 static bool bn_coop_enabled() {
   static int v = -1;
   // off by default: with at most one block per SM and a grid barrier the single launch is slower than two full-width
@@ -1384,13 +1488,14 @@ int geeps_bn_forward_fused(const void* x, void* y, const float* gamma, const flo
     float inv_count = 1.f / (float)P;
     void* args[] = {&xx, &yy, &sums, &mean_rstd, &running_mean, &running_var, &gamma, &beta, &zero_after, &barrier,
                     &P, &C, &ldx, &ldy, &relu, &inv_count, &eps, &momentum};
-    cudaError_t e = cudaLaunchCooperativeKernel((void*)bn_forward_coop_kernel, dim3(bn_coop_grid(P, C)), dim3(256), args,
-                                                2 * C * sizeof(float), st);
+    const SlotGrid cg = bn_coop_grid(P, C);
+    cudaError_t e = cudaLaunchCooperativeKernel((void*)bn_forward_coop_kernel, cg.grid, dim3(cg.threads), args, cg.smem, st);
     return e == cudaSuccess ? CK() : (int)e;
   }
-  channel_reduce_kernel<0><<<reduce_grid(P, C), 256, 2 * C * sizeof(float), st>>>(
+  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  channel_reduce_kernel<0><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
-  bn_apply_fused_kernel<<<grid_1d(P * (C / 8)), 256, 0, st>>>((const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
+  bn_apply_fused_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
                                                               running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                                                               1.f / (float)P, eps, momentum);
   return CK();
@@ -1406,13 +1511,14 @@ int geeps_bn_backward_fused(const void* x, const void* dy, const void* y, void* 
     bf16* dxx = (bf16*)dx;
     void* args[] = {&xx, &dd, &yy, &dxx, &mean_rstd, &gamma, &sums, &dgamma, &dbeta, &zero_after, &barrier,
                     &P, &C, &ldx, &lddy, &lddx, &relu, &grad_scale};
-    cudaError_t e = cudaLaunchCooperativeKernel((void*)bn_backward_coop_kernel, dim3(bn_coop_grid(P, C)), dim3(256),
-                                                args, 2 * C * sizeof(float), st);
+    const SlotGrid cg = bn_coop_grid(P, C);
+    cudaError_t e = cudaLaunchCooperativeKernel((void*)bn_backward_coop_kernel, cg.grid, dim3(cg.threads), args, cg.smem, st);
     return e == cudaSuccess ? CK() : (int)e;
   }
-  channel_reduce_kernel<1><<<reduce_grid(P, C), 256, 2 * C * sizeof(float), st>>>(
+  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  channel_reduce_kernel<1><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  bn_backward_kernel<<<grid_1d(P * (C / 8)), 256, 0, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
+  bn_backward_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
                                                            (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
                                                            ldx, lddy, lddx, relu, grad_scale, zero_after);
   return CK();
@@ -1426,7 +1532,8 @@ int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, f
     return CK();
   }
   if (zero_first) cudaMemsetAsync(out, 0, sizeof(float) * C, st);
-  channel_reduce_kernel<2><<<reduce_grid(P, C), 256, 2 * C * sizeof(float), st>>>(
+  const SlotGrid rg = reduce_grid(P, C, 1);
+  channel_reduce_kernel<2><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, nullptr, nullptr, nullptr, out, P, C, ldx, 0, 0, scale);
   return CK();
 }
@@ -1453,12 +1560,8 @@ int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* c
   if (C % 8 || lddy % 8 || ldy % 8 || lddx % 8 || C > 8192) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(colsum, 0, sizeof(float) * C, st);
-  // enough CTAs that every pixel lane has work, a whole number of channel slots per grid
-  long long want = (P * (C / 8) + 255) / 256;
-  if (want > geeps_sm_count() * 8) want = geeps_sm_count() * 8;
-  const long long min_blocks = ((long long)(C / 8) + 255) / 256;
-  if (want < min_blocks) want = min_blocks;
-  relu_backward_colsum_kernel<<<(int)(want < 1 ? 1 : want), 256, C * sizeof(float), st>>>(
+  const SlotGrid rg = slot_grid(P, C, 4, 8, 1);
+  relu_backward_colsum_kernel<<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)dy, (const bf16*)y, (bf16*)dx, colsum, P, C, lddy, ldy, lddx);
   return CK();
 }
@@ -1646,11 +1749,12 @@ int geeps_bn_forward_noalloc(const void* x, void* y, const float* gamma, const f
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);   // the array keeps the last call's sums
   if (e != cudaSuccess) return (int)e;
-  channel_reduce_kernel<0><<<reduce_grid(P, C), 256, 2 * C * sizeof(float), st>>>(
+  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  channel_reduce_kernel<0><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   bn_finalize_kernel<<<(C + 127) / 128, 128, 0, st>>>(sums, mean_rstd, running_mean, running_var, C,
                                                       1.f / (float)P, eps, momentum);
-  bn_apply_kernel<<<grid_1d(P * (C / 8)), 256, 0, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
+  bn_apply_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
                                                         ldy, relu);
   return CK();
 }

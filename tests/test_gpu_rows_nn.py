@@ -378,3 +378,39 @@ def test_linear_with_the_k_range_split_over_the_sms_matches_fp32(relu, fp32_out,
     dx_ref = (dyb.float() * mask) @ w.float()
     assert ((dx.float() - dx_ref).norm() / dx_ref.norm()).item() < 1e-2
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("P,Cc", [(1, 8), (3, 24), (777, 64), (129, 104), (1000, 1600), (37, 2056), (6, 4096)])
+def test_channel_kernels_at_the_edges_of_their_thread_map(P, Cc):
+    """One row to more rows than a batch of loads, slots that do not divide a block, C split over two block columns."""
+    torch.manual_seed(P + Cc)
+    x, dy = torch.randn(P, Cc, device=DEV).to(BF), torch.randn(P, Cc, device=DEV).to(BF)
+    x64, dy64 = x.double(), dy.double()
+    eps = 2.0 ** -8                                 # half an ulp of bf16, doubled
+    total = torch.empty(Cc, device=DEV)
+    F.colsum(x, total, scale=0.5)
+    assert torch.allclose(total.double(), 0.5 * x64.sum(0), atol=1e-5 * P ** 0.5 * 4, rtol=1e-5)
+    dx = torch.empty_like(dy)
+    F.relu_backward_colsum(dy, x, dx, total)
+    ref = torch.where(x64 > 0, dy64, torch.zeros_like(dy64))
+    assert torch.equal(dx.double(), ref)
+    assert torch.allclose(total.double(), ref.sum(0), atol=1e-5 * P ** 0.5 * 4, rtol=1e-5)
+    if P < 3:
+        return
+    g, b = torch.rand(Cc, device=DEV) + 0.5, torch.randn(Cc, device=DEV)
+    sums, sums_b, stat = torch.zeros(2 * Cc, device=DEV), torch.ones(2 * Cc, device=DEV), torch.empty(2 * Cc, device=DEV)
+    rm, rv = torch.zeros(Cc, device=DEV), torch.ones(Cc, device=DEV)
+    y = torch.empty_like(x)
+    F.bn_forward_fused(x, y, g, b, sums, stat, rm, rv, zero_after=sums_b, relu=True)
+    xr, gr, br = (t.double().requires_grad_(True) for t in (x, g, b))
+    yr = torch.relu(TF.batch_norm(xr, None, None, gr, br, training=True, eps=1e-5))
+    # E[x^2] - mean^2 in fp32: a few 1e-7 of the variance, before bf16 rounding
+    assert torch.allclose(y.double(), yr, atol=1e-4, rtol=eps)
+    assert torch.allclose(rm.double(), 0.1 * x64.mean(0), atol=1e-6) and sums_b.abs().max().item() == 0
+    yr.backward(torch.where(y.double() > 0, dy64, torch.zeros_like(dy64)))
+    dg, db = torch.empty(Cc, device=DEV), torch.empty(Cc, device=DEV)
+    F.bn_backward_fused(x, dy, y, dx, stat, g, sums_b, dg, db, zero_after=sums, relu=True)
+    scale = xr.grad.abs().max().item()
+    assert torch.allclose(dx.double(), xr.grad, atol=1e-4 * scale, rtol=eps)
+    assert torch.allclose(dg.double(), gr.grad, atol=1e-4 * P ** 0.5, rtol=1e-4)
+    assert torch.allclose(db.double(), br.grad, atol=1e-5 * P ** 0.5 * 4, rtol=1e-5) and sums.abs().max().item() == 0
