@@ -16,6 +16,10 @@
 // Every mbarrier wait is bounded; on expiry the CTA records TIMEOUT in `status`, stops
 // issuing work, frees its TMEM and returns.
 //
+// Outputs with too few tiles for the machine (batch-sized M) split K over the CTAs of a thread-block cluster: every CTA
+// accumulates one K slice of the same tile, leaves it in its shared memory as fp32, and each CTA of the cluster then
+// sums its share of the rows over distributed shared memory in slice order (no workspace, no atomics, bit-reproducible).
+//
 // The reference has no GEMM kernel of its own: it only carries cuBLAS wrappers
 // (src/common/gpu-util/math_functions_cuda.cu:14-60) that the parameter server never calls.
 #include <cuda.h>
@@ -43,6 +47,7 @@ struct GemmDev {
   int bn;           // tile width: multiple of 32 (64 for an MN-major B), <= 256
   int tmem_cols;    // power of two >= 2 * bn: two accumulators, so the epilogue of a tile overlaps the next main loop
   int m_tiles, n_tiles;
+  int cluster;      // > 1: K slices of one tile per cluster of this many CTAs (split_k is then the same number)
   int tma_store;    // 1: epilogue stages 128-byte-wide slabs in swizzled smem and stores them with TMA
 };
 
@@ -57,7 +62,25 @@ struct SmemCtl {
 
 // Persistent kernel: one CTA per SM walks the tile list t = blockIdx.x, blockIdx.x + gridDim.x, ...
 // Consecutive CTAs take consecutive M tiles of the same N tile, so the B tile they share stays in L2.
-template <bool A_MN, bool B_MN>
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t smem_addr, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+// byte offset of the 16-byte piece `q` of row `r` in a [128][bn] fp32 tile; the XOR keeps a column of rows (how the
+// accumulator comes out of TMEM, one row per lane) off a single bank
+__device__ __forceinline__ uint32_t part_off(int r, int q, int bn) { return (uint32_t)(r * bn * 4 + ((q ^ (r & 7)) << 4)); }
+
+template <bool A_MN, bool B_MN, bool CL>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const GemmDev d) {
@@ -67,7 +90,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* cslab = tiles + (size_t)d.stages * STAGE_BYTES;          // 2 x C_SLAB_BYTES, 1024-byte aligned
-  SmemCtl* ctl = (SmemCtl*)(cslab + 2 * C_SLAB_BYTES);
+  SmemCtl* ctl = (SmemCtl*)(cslab + (CL ? 0 : 2 * C_SLAB_BYTES));   // a cluster stages its tile in the operand ring
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = d.stages;
@@ -75,6 +98,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int tiles_mn = d.m_tiles * d.n_tiles;
   const int num_tiles = tiles_mn * d.split_k;
   const int acc_stride = d.tmem_cols >> 1;
+  // work items t, t + t_step, ...; a cluster CTA has one: K slice (rank) of tile blockIdx.x / cluster
+  const int t_first = CL ? (int)(blockIdx.x % d.cluster) * tiles_mn + (int)(blockIdx.x / d.cluster) : (int)blockIdx.x;
+  const int t_step = CL ? num_tiles : (int)gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) { tc05::mbar_init(&ctl->full[s], 1); tc05::mbar_init(&ctl->empty[s], 1); }
@@ -103,7 +129,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = t_first; t < num_tiles && ok; t += t_step) {
         const int mn = t % tiles_mn, z = t / tiles_mn;
         const int m0 = (mn % d.m_tiles) * BM, n0 = (mn / d.m_tiles) * BN;
         const int kt_begin = z * kt_per, kt_end = min(d.kt_total, kt_begin + kt_per);
@@ -140,7 +166,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       uint32_t tile_i = 0, ph = 0;
       int s = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_i) {
+      for (int t = t_first; t < num_tiles && ok; t += t_step, ++tile_i) {
         const int z = t / tiles_mn;
         const int kt_begin = z * kt_per, kt_end = min(d.kt_total, kt_begin + kt_per);
         const uint32_t acc = tile_i & 1u, acc_ph = (tile_i >> 1) & 1u;
@@ -174,7 +200,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // ---------------- epilogue: TMEM -> registers -> global ----------------
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     uint32_t tile_i = 0, slab_i = 0;
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tile_i) {
+    for (int t = t_first; t < num_tiles; t += t_step, ++tile_i) {
       const int mn = t % tiles_mn, z = t / tiles_mn;
       const int m0 = (mn % d.m_tiles) * BM, n0 = (mn / d.m_tiles) * BN;
       const int kt_begin = z * kt_per, kt_end = min(d.kt_total, kt_begin + kt_per);
@@ -186,7 +212,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const float bias_m = (d.bias_mode == 2 && row < d.M) ? d.bias[row] : 0.f;
       const bool add_bias = (d.split_k == 1) || (z == 0);
       const bool has_k = kt_end > kt_begin;
-      if (d.tma_store) {
+      if (CL) {
+        // the commit behind tmem_full covers every MMA of the slice: the operand stages are free to hold the partial tile
+        const int r = q * 32 + lane;
+#pragma unroll 1
+        for (int c = 0; c < BN; c += 32) {
+          uint32_t v[32];
+          tc05::tmem_ld_32x32(tacc + (uint32_t)c, v);
+          tc05::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(tiles + part_off(r, (c >> 2) + j, BN)) =
+                make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        }
+      } else if (d.tma_store) {
         // 128-byte-wide slabs (64 bf16 or 32 fp32 columns) go through swizzled smem and leave with one
         // TMA store (or reduce-add for split-K) each: coalesced, asynchronous, clipped at the matrix edge
         const int cols_per_slab = d.out_fp32 ? 32 : 64;
@@ -340,7 +379,61 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   }
 
-  if (d.tma_store && threadIdx.x == 64) tc05::bulk_wait<0>();   // all TMA stores of this CTA have landed
+  if (CL) {
+    __syncwarp();
+    cluster_sync_all();
+    // this CTA finishes 128 / cluster rows of the tile, eight columns per thread and step
+    const int rank = (int)(blockIdx.x % d.cluster), mn = (int)(blockIdx.x / d.cluster);
+    const int m0 = (mn % d.m_tiles) * BM, n0 = (mn / d.m_tiles) * BN;
+    const int rows = BM / d.cluster, oct = BN >> 3;
+    const uint32_t part = tc05::smem_u32(tiles);
+    for (int i = threadIdx.x; i < rows * oct; i += blockDim.x) {
+      const int rr = i / oct, o = i - rr * oct;
+      const int r = rank * rows + rr;
+      const long long row = (long long)m0 + r, col0 = (long long)n0 + o * 8;
+      if (row >= d.M || col0 >= d.N) continue;
+      const uint32_t o0 = part_off(r, 2 * o, BN), o1 = part_off(r, 2 * o + 1, BN);
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = 0.f;
+      for (int z = 0; z < d.cluster; ++z) {
+        const uint32_t base = cluster_addr(part, z);
+        const float4 a = ld_cluster_f4(base + o0), b = ld_cluster_f4(base + o1);
+        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+        v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+      }
+      const int nc = (int)min((long long)8, d.N - col0);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        float x = d.alpha * v[e];
+        if (d.bias_mode == 1 && e < nc) x += __ldg(d.bias + col0 + e);
+        else if (d.bias_mode == 2) x += __ldg(d.bias + row);
+        v[e] = d.relu ? fmaxf(x, 0.f) : x;
+      }
+      if (d.out_fp32) {
+        float* out = (float*)d.C + row * d.ldc + col0;
+        if (nc == 8 && (((uintptr_t)out) & 15) == 0) {
+          st_f4(out, make_float4(v[0], v[1], v[2], v[3]));
+          st_f4(out + 4, make_float4(v[4], v[5], v[6], v[7]));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) if (e < nc) out[e] = v[e];
+        }
+      } else {
+        __nv_bfloat16* out = (__nv_bfloat16*)d.C + row * d.ldc + col0;
+        if (nc == 8 && (((uintptr_t)out) & 15) == 0) {
+          *reinterpret_cast<uint4*>(out) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
+                                                      pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) if (e < nc) out[e] = __float2bfloat16(v[e]);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();      // nobody leaves while a peer still reads its partial tile
+  }
+  if (!CL && d.tma_store && threadIdx.x == 64) tc05::bulk_wait<0>();   // all TMA stores of this CTA have landed
   tc05::fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0 && ctl->abort_flag)
@@ -384,23 +477,70 @@ bool make_map(CUtensorMap* map, const void* base, long long inner, long long out
   return r == CUDA_SUCCESS;
 }
 
-template <bool A_MN, bool B_MN>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmDev& d, int grid,
-           cudaStream_t st) {
+template <bool A_MN, bool B_MN, bool CL>
+int launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmDev& d, int grid,
+                  cudaStream_t st) {
   const int stage_bytes = A_STAGE_BYTES + d.bn * BK * 2;
-  const size_t smem = (size_t)d.stages * stage_bytes + 2 * C_SLAB_BYTES + sizeof(SmemCtl) + 1024;
+  const size_t smem = (size_t)d.stages * stage_bytes + (CL ? 0 : 2 * C_SLAB_BYTES) + sizeof(SmemCtl) + 1024;
   static bool attr_set = false;  // per instantiation
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<A_MN, B_MN, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          220 * 1024);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  gemm_tc_kernel<A_MN, B_MN><<<grid, 192, smem, st>>>(ta, tb, tc, d);
-  return (int)cudaGetLastError();
+  if (!CL) {
+    gemm_tc_kernel<A_MN, B_MN, CL><<<grid, 192, smem, st>>>(ta, tb, tc, d);
+    return (int)cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(192);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)d.cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_kernel<A_MN, B_MN, CL>, ta, tb, tc, d);
+}
+template <bool A_MN, bool B_MN>
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmDev& d, int grid,
+           cudaStream_t st) {
+  return d.cluster > 1 ? launch_kernel<A_MN, B_MN, true>(ta, tb, tc, d, grid, st)
+                       : launch_kernel<A_MN, B_MN, false>(ta, tb, tc, d, grid, st);
 }
 
 int round_up(long long v, int m) { return (int)((v + m - 1) / m * m); }
+
+// Tile width and K slices (cluster size) for an output that 256-wide tiles would not spread over every SM.  Such a
+// product is bound by the operand bytes its CTAs pull through L2 (about 75 bytes per ns and SM here), so the choice is
+// the one with the least traffic on the busiest SM: rounds x k tiles per CTA x (A rows + B rows) x 128 bytes, plus
+// kTileOver per round (fill, drain) and, for a cluster, the exchange of its partial tile.  Narrow tiles spread an
+// output but re-read A once per tile; a cluster keeps the tile wide and cuts K instead.
+struct TileChoice { int bn, cluster; };
+TileChoice choose_tiles(const GeepsGemmParams* p, int unit, int kt, int sms, bool cluster_ok) {
+  constexpr double kTileOver = 150e3, kClusterOver = 150e3;
+  const long long m_tiles = (p->M + BM - 1) / BM;
+  const double a_rows = p->M < BM ? (double)p->M : (double)BM;
+  TileChoice best = {unit > 64 ? unit : 64, 1};
+  double best_cost = 1e300;
+  for (int bn = 64; bn <= 256; bn += unit) {
+    const long long tiles = m_tiles * ((p->N + bn - 1) / bn);
+    for (int cs = 1; cs <= (cluster_ok ? 8 : 1); cs *= 2) {
+      const int per = (kt + cs - 1) / cs;
+      if (cs > 1 && (per < 4 || (long long)(cs - 1) * per >= kt)) continue;    // every slice needs k tiles
+      const long long slots = cs <= 2 ? sms : sms / 18 * 16;                   // whole clusters per GPC
+      const long long rounds = (tiles * cs + slots - 1) / slots;
+      double cost = rounds * (per * (a_rows + bn) * 128.0 + kTileOver);
+      if (cs > 1) cost += rounds * (kClusterOver + a_rows * bn * 8.0);
+      if (cost < best_cost * 0.98) { best_cost = cost; best = {bn, cs}; }
+    }
+  }
+  return best;
+}
 
 }  // namespace
 
@@ -429,16 +569,18 @@ int geeps_gemm_bf16(const GeepsGemmParams* p, void* stream) {
   // TMA-store epilogue: C 16-byte aligned with a 16-byte-multiple pitch, no read-modify-write of C
   const int esz = p->out_fp32 ? 4 : 2;
   const bool tma_c = (((uintptr_t)p->C & 15) == 0) && ((p->ldc * esz) % 16 == 0) && p->beta == 0.f;
-  int bn = p->block_n;
+  int bn = p->block_n, cluster = 1;
   if (bn <= 0 || bn > 256 || bn % unit) {
     const long long nt = (p->N + 255) / 256;
     bn = round_up((p->N + nt - 1) / nt, unit);
     // ... but enough tiles to occupy every SM when the problem allows it
     const bool can_split = p->split_k == 0 && p->out_fp32 && !p->relu && kt_total >= 16;
-    while (!can_split && bn > 64 && (long long)m_tiles * ((p->N + bn - 1) / bn) < kSMs) {
-      const int smaller = round_up(bn / 2, unit);
-      if (smaller >= bn) break;
-      bn = smaller;
+    if (!can_split && (long long)m_tiles * ((p->N + bn - 1) / bn) < kSMs && p->N > 64) {
+      // a bf16 slab is 64 columns wide (see below): several tiles have widths that are multiples of it
+      const int step = tma_c && !p->out_fp32 ? 64 : unit;
+      const bool cluster_ok = p->split_k <= 1 && p->beta == 0.f && p->K > 0;
+      const TileChoice c = choose_tiles(p, step, kt_total, kSMs, cluster_ok);
+      if (c.cluster > 1 || c.bn < bn) { bn = c.bn; cluster = c.cluster; }
     }
   }
   if (bn > 256) bn = 256;
@@ -480,24 +622,26 @@ int geeps_gemm_bf16(const GeepsGemmParams* p, void* stream) {
     const int per = (d.kt_total + d.split_k - 1) / d.split_k;
     d.split_k = (d.kt_total + per - 1) / per;
   }
-  if (d.split_k > 1) {
+  d.cluster = cluster;
+  if (cluster > 1) d.split_k = cluster;
+  if (d.split_k > 1 && cluster == 1) {
     // partial sums are accumulated with atomics: bring C to beta*C (or zero) first
     int e = geeps_scale_matrix_f32((float*)p->C, p->M, p->N, p->ldc, p->beta, stream);
     if (e) return e;
     d.beta = 0.f;
   }
-  d.tma_store = tma_c ? 1 : 0;
+  d.tma_store = tma_c && cluster == 1 ? 1 : 0;
   CUtensorMap tc;
-  if (tma_c) {
+  if (d.tma_store) {
     if (!make_map(&tc, p->C, p->N, p->M, p->ldc, p->out_fp32 ? 32 : 64, BM, p->out_fp32 != 0)) d.tma_store = 0;
   }
   if (!d.tma_store) tc = ta;   // unused by the kernel
   const int stage_bytes = A_STAGE_BYTES + bn * BK * 2;
-  d.stages = (200 * 1024 - 2 * C_SLAB_BYTES) / stage_bytes;
+  d.stages = (200 * 1024 - (cluster > 1 ? 0 : 2 * C_SLAB_BYTES)) / stage_bytes;
   if (d.stages > MAX_STAGES) d.stages = MAX_STAGES;
   if (d.stages < 2) d.stages = 2;
   const long long num_tiles = (long long)m_tiles * n_tiles * d.split_k;
-  const int grid = (int)(num_tiles < kSMs ? num_tiles : kSMs);
+  const int grid = (int)(num_tiles < kSMs || cluster > 1 ? num_tiles : kSMs);
   cudaStream_t st = (cudaStream_t)stream;
   if (!p->a_mn_major && !p->b_mn_major) return launch<false, false>(ta, tb, tc, d, grid, st);
   if (p->a_mn_major && !p->b_mn_major) return launch<true, false>(ta, tb, tc, d, grid, st);

@@ -123,3 +123,31 @@ def test_gemm_auto_dispatch_uses_pairs_for_large_products():
     F.gemm(a, b, out)
     ref = _ref(a, b, False, False)
     assert ((out.float() - ref).norm() / ref.norm()).item() < 5e-3
+
+
+@pytest.mark.parametrize("M,N,K,b_mn,fp32", [(256, 1000, 4096, False, False), (5, 4096, 1096, False, True),
+                                             (32, 1024, 21841, True, False), (129, 200, 328, True, True),
+                                             (256, 512, 520, False, False), (100, 72, 2056, False, True)])
+def test_gemm_cluster_split_k(M, N, K, b_mn, fp32):
+    """Few output tiles, long K: slices of one tile on the CTAs of a cluster (uneven last slice, ragged M and N, column
+    slices that end on odd widths), bias and ReLU applied once; the same bits on every run."""
+    dev = torch.device("cuda:0")
+    torch.manual_seed(M + N + K)
+    kp = (K + 7) // 8 * 8
+    a = _mk(M, kp, False, dev)[:, :K]
+    b = _mk(N, K, b_mn, dev, pad=8 if b_mn else kp - K)
+    bias = torch.randn(N, device=dev)
+    wide = torch.zeros((M, N + 16), dtype=torch.float32 if fp32 else torch.bfloat16, device=dev)
+    out = wide[:, 8:8 + N]
+    st = L.new_status(dev)
+    F.gemm(a, b, out, b_mn=b_mn, bias=bias, relu=True, alpha=0.5, status=st, impl="tc")
+    torch.cuda.synchronize()
+    assert L.read_status(st)["code"] == 0
+    A, B = a.double(), (b.double().t() if b_mn else b.double())
+    ref = torch.relu(0.5 * (A @ B.t()) + bias)
+    # fp32 sums of K products of size 1/4: K^0.5 * 2^-24 * a few, then the rounding of the output type
+    assert torch.allclose(out.double(), ref, atol=2e-6 * K ** 0.5 * 4, rtol=2.0 ** -8 if not fp32 else 1e-5)
+    assert wide[:, :8].abs().max().item() == 0 and wide[:, 8 + N:].abs().max().item() == 0
+    again = torch.empty_like(wide)[:, 8:8 + N]
+    F.gemm(a, b, again, b_mn=b_mn, bias=bias, relu=True, alpha=0.5, impl="tc")
+    assert torch.equal(out, again)
