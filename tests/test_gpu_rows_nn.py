@@ -414,3 +414,21 @@ def test_channel_kernels_at_the_edges_of_their_thread_map(P, Cc):
     assert torch.allclose(dx.double(), xr.grad, atol=1e-4 * scale, rtol=eps)
     assert torch.allclose(dg.double(), gr.grad, atol=1e-4 * P ** 0.5, rtol=1e-4)
     assert torch.allclose(db.double(), br.grad, atol=1e-5 * P ** 0.5 * 4, rtol=1e-5) and sums.abs().max().item() == 0
+
+
+@pytest.mark.parametrize("Cc,pad", [(1, 7), (127, 1), (1000, 0), (1001, 7), (8199, 0), (24576, 0), (30001, 7)])
+def test_softmax_rows_in_registers_and_past_them(Cc, pad):
+    """Aligned rows (pitch a multiple of 8) and unaligned ones, one thread's worth of classes to rows that are read again."""
+    torch.manual_seed(Cc)
+    B = 5
+    logits = (torch.randn(B, Cc + pad, device=DEV) * 4)[:, :Cc]
+    labels = torch.randint(0, Cc, (B,), device=DEV)
+    wide = torch.full((B, Cc + pad), 3.0, dtype=BF, device=DEV)
+    loss = torch.empty(1, device=DEV)
+    F.softmax_ce(logits, labels, loss, wide[:, :Cc], loss_scale=1.0 / B, grad_scale=1.0 / B)
+    lr = logits.double().clone().requires_grad_(True)
+    ref = TF.cross_entropy(lr, labels)
+    ref.backward()
+    assert abs(loss.item() - ref.item()) < 1e-5 * max(1, abs(ref.item()))
+    assert torch.allclose(wide[:, :Cc].double(), lr.grad, atol=1e-7, rtol=2.0 ** -7)
+    assert pad == 0 or (wide[:, Cc:] == 3.0).all()
