@@ -432,3 +432,34 @@ def test_softmax_rows_in_registers_and_past_them(Cc, pad):
     assert abs(loss.item() - ref.item()) < 1e-5 * max(1, abs(ref.item()))
     assert torch.allclose(wide[:, :Cc].double(), lr.grad, atol=1e-7, rtol=2.0 ** -7)
     assert pad == 0 or (wide[:, Cc:] == 3.0).all()
+
+
+@pytest.mark.parametrize("H,Cc,pad", [(3, 8, 0), (14, 32, 1), (7, 64, 0), (18, 72, 0), (9, 104, 1), (8, 144, 0), (11, 232, 0),
+                                      (6, 264, 1), (5, 512, 0), (5, 520, 0)])
+@pytest.mark.parametrize("alpha", [1e-4, 0.5])
+def test_lrn_maxpool_backward_over_channel_counts(H, Cc, pad, alpha):
+    """Every lane / vector split of the register kernel (the last size takes the general one), odd and even sizes with
+    and without padding; alpha 0.5 leaves the range of the polynomials."""
+    torch.manual_seed(H * Cc)
+    B, size, beta, kk = 2, 5, 0.75, 1.0
+    x = torch.relu(torch.randn(B, H, H, Cc, device=DEV) * 3).to(BF)
+    g = F.pool_geom(x.shape, 3, 2, pad, Cc, Cc)
+    p = torch.empty(B, g.OH, g.OW, Cc, dtype=BF, device=DEV)
+    arg = torch.empty(B, g.OH, g.OW, Cc, dtype=torch.uint8, device=DEV)
+    F.lrn_maxpool_forward(x, p, arg, g, size, alpha, beta, kk)
+    dp = torch.randn_like(p)
+    dx, cs = torch.empty_like(x), torch.empty(Cc, device=DEV)
+    F.lrn_maxpool_backward(x, dp, arg, dx, g, size, alpha, beta, kk, relu_mask=True, colsum=cs)
+    # the pooling gradient by the kernel's own window codes, then autograd through the normalisation
+    n = torch.arange(g.OH, device=DEV) * 2 - pad
+    rows = n.view(1, -1, 1, 1) + arg.long() // 3
+    cols = n.view(1, 1, -1, 1) + arg.long() % 3
+    flat = ((torch.arange(B, device=DEV).view(-1, 1, 1, 1) * H + rows) * H + cols) * Cc + torch.arange(Cc, device=DEV)
+    dy = torch.zeros(x.numel(), dtype=torch.float64, device=DEV).scatter_add_(0, flat.view(-1), dp.double().view(-1))
+    xr = x.double().permute(0, 3, 1, 2).requires_grad_(True)
+    TF.local_response_norm(xr, size, alpha=alpha, beta=beta, k=kk).backward(dy.view(B, H, H, Cc).permute(0, 3, 1, 2))
+    ref = torch.where(x > 0, xr.grad.permute(0, 2, 3, 1), torch.zeros((), dtype=torch.float64, device=DEV))
+    # bf16 result of two bf16-rounded terms (a and the ratios, five of which meet in a window)
+    err = (dx.double() - ref).norm() / ref.norm()
+    assert err.item() < 3 * 2.0 ** -9, err.item()
+    assert torch.allclose(cs.double(), ref.sum((0, 1, 2)), atol=0.02 * (B * H * H) ** 0.5, rtol=1e-2)
