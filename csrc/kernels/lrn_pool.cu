@@ -94,97 +94,7 @@ struct ItemWalk {
   }
 };
 
-// ---------------- forward ----------------
-// grid = B * ceil(OH / RO); one CTA produces RO pooled rows from the (RO-1)*stride + K input rows under them.
-// The input is read from global memory (one 16-byte and two 8-byte loads per 8 outputs), normalised once per
-// element into shared memory ([n_in][W][C] bf16), and pooled from there.
-// K3S2: 3 x 3 windows with stride 2 (window size and stride are then constants of the pooling loops)
-template <int HALF, bool K3S2>
-__global__ void __launch_bounds__(512)
-lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uint8_t* __restrict__ argmax,
-                           const GeepsPoolGeom g, const LrnCoef cf, int RO) {
-  extern __shared__ __align__(16) uint8_t lp_smem[];
-  const int C = g.C, cv = C >> 3, W = g.W;
-  const int PK = K3S2 ? 3 : g.K, PS = K3S2 ? 2 : g.stride;
-  const int row_elems = W * C;
-  bf16* ys = reinterpret_cast<bf16*>(lp_smem);
-  const int oh_blocks = (g.OH + RO - 1) / RO;
-  const int b = blockIdx.x / oh_blocks, oh0 = (blockIdx.x - b * oh_blocks) * RO;
-  const int n_out = min(RO, g.OH - oh0);
-  const int ih_base = oh0 * PS - g.pad;                    // input row of shared-memory row 0 (may be < 0)
-  const int r_lo = max(0, -ih_base);
-  const int r_hi = min((n_out - 1) * PS + PK, g.H - ih_base);   // rows [r_lo, r_hi) exist
-  const int tid = threadIdx.x, nt = blockDim.x;
-  {
-    const bf16* xbase = x + ((long long)b * g.H + ih_base + r_lo) * row_elems;
-    bf16* ybase = ys + (size_t)r_lo * row_elems;
-    const int nrows = r_hi - r_lo;
-    for (ItemWalk it(tid, nt, W, cv); it.r < nrows; it.next(W, cv)) {
-      const int c = it.cvi * 8;
-      const int pix = it.r * row_elems + it.w * C;          // offsets inside a block of a few rows: 32 bits
-      float v[16], t[16], ws[8], o[8];
-      load16(xbase + pix, c, C, v);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) t[j] = v[j] * v[j];
-      window8<HALF>(t, ws);
-      if (max8(ws) <= cf.w_max) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = v[4 + e] * fmaf(ws[e], fmaf(ws[e], fmaf(ws[e], cf.p3, cf.p2), cf.p1), cf.p0);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = v[4 + e] * __powf(cf.k * fmaf(cf.es, ws[e], 1.f), -cf.beta);
-      }
-      *reinterpret_cast<uint4*>(ybase + pix + c) = pack8(o);
-    }
-  }
-  __syncthreads();
-  for (ItemWalk it(tid, nt, g.OW, cv); it.r < n_out; it.next(g.OW, cv)) {
-    const int oh = oh0 + it.r, ow = it.w, c = it.cvi * 8;
-    const int ih0 = oh * PS - g.pad;
-    const int kh_lo = max(0, -ih0), kh_hi = min(PK, g.H - ih0);
-    const int iw0 = ow * PS - g.pad;
-    const int kw_lo = max(0, -iw0), kw_hi = min(PK, W - iw0);
-    // packed: best value and window code per 16-bit lane; strict > keeps the first maximum
-    const uint32_t neg = 0xff7fff7fu;                 // two bf16 lowest finite values
-    __nv_bfloat162 best[4];
-    uint32_t arg[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { best[j] = *reinterpret_cast<const __nv_bfloat162*>(&neg); arg[j] = 0x00ff00ffu; }
-    for (int kh = kh_lo; kh < kh_hi; ++kh) {
-      const bf16* yr = ys + (ih0 + kh - ih_base) * row_elems + c;
-      for (int kw = kw_lo; kw < kw_hi; ++kw) {
-        const uint4 v = *reinterpret_cast<const uint4*>(yr + (iw0 + kw) * C);
-        const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
-        const uint32_t code1 = (uint32_t)(kh * PK + kw);
-        const uint32_t code = code1 | (code1 << 16);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const __nv_bfloat162 x2 = *reinterpret_cast<const __nv_bfloat162*>(&vv[j]);
-          const uint32_t gt = __hgt2_mask(x2, best[j]);
-          best[j] = __hmax2(best[j], x2);
-          arg[j] = (arg[j] & ~gt) | (code & gt);
-        }
-      }
-    }
-    const long long opix = ((long long)b * g.OH + oh) * g.OW + ow;
-    *reinterpret_cast<uint4*>(p + opix * g.ldy + c) =
-        make_uint4(*reinterpret_cast<const uint32_t*>(&best[0]), *reinterpret_cast<const uint32_t*>(&best[1]),
-                   *reinterpret_cast<const uint32_t*>(&best[2]), *reinterpret_cast<const uint32_t*>(&best[3]));
-    uint2 pk;      // 16-bit lanes -> bytes
-    pk.x = __byte_perm(arg[0], arg[1], 0x6420);
-    pk.y = __byte_perm(arg[2], arg[3], 0x6420);
-    *reinterpret_cast<uint2*>(argmax + opix * C + c) = pk;
-  }
-}
-
-// ---------------- backward, 3 x 3 windows with stride 2, window of 5 channels ----------------
-// The general kernel below spends 79 instructions per element: three passes over shared memory, the halo channels of
-// every 8-channel vector unpacked and squared again, window loops whose trip counts differ inside a warp.  Here LP lanes
-// share one pixel and a lane holds NV vectors of 8 channels (vector lane + LP * j, so loads stay coalesced); x, the
-// scaled gradient and the ratio stay in registers, a halo channel pair comes from the neighbouring lane by shuffle, and
-// nothing goes through shared memory.  A warp takes pixels of one column parity at a time, so all its lanes visit the
-// same number of windows (1 or 2 per direction).  fp32 arithmetic runs on register pairs (fma.rn.f32x2).
-// 256 x 55 x 55 x 96: 245 -> 173 us; still bound by instruction issue.
+// ---- fp32 on register pairs (one instruction for two products or sums) ----
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   unsigned long long r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
@@ -215,6 +125,130 @@ __device__ __forceinline__ void window5(const float2 (&t)[6], float2 (&w)[4]) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) w[k] = make_float2(q[k] + t[k + 2].x, t[k].y + q[k + 1]);
 }
+
+// ---------------- forward ----------------
+// grid = B * ceil(OH / RO); one CTA produces RO pooled rows from the (RO-1)*stride + K input rows under them.
+// The input is read from global memory (one 16-byte and two 8-byte loads per 8 outputs), normalised once per
+// element into shared memory ([n_in][W][C] bf16), and pooled from there.
+// K3S2: 3 x 3 windows with stride 2 (window size and stride are then constants of the pooling loops)
+template <int HALF, bool K3S2>
+__global__ void __launch_bounds__(512)
+lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uint8_t* __restrict__ argmax,
+                           const GeepsPoolGeom g, const LrnCoef cf, int RO) {
+  extern __shared__ __align__(16) uint8_t lp_smem[];
+  const int C = g.C, cv = C >> 3, W = g.W;
+  const int PK = K3S2 ? 3 : g.K, PS = K3S2 ? 2 : g.stride;
+  const int row_elems = W * C;
+  bf16* ys = reinterpret_cast<bf16*>(lp_smem);
+  const int oh_blocks = (g.OH + RO - 1) / RO;
+  const int b = blockIdx.x / oh_blocks, oh0 = (blockIdx.x - b * oh_blocks) * RO;
+  const int n_out = min(RO, g.OH - oh0);
+  const int ih_base = oh0 * PS - g.pad;                    // input row of shared-memory row 0 (may be < 0)
+  const int r_lo = max(0, -ih_base);
+  const int r_hi = min((n_out - 1) * PS + PK, g.H - ih_base);   // rows [r_lo, r_hi) exist
+  const int tid = threadIdx.x, nt = blockDim.x;
+  {
+    const bf16* xbase = x + ((long long)b * g.H + ih_base + r_lo) * row_elems;
+    bf16* ybase = ys + (size_t)r_lo * row_elems;
+    const int nrows = r_hi - r_lo;
+    for (ItemWalk it(tid, nt, W, cv); it.r < nrows; it.next(W, cv)) {
+      const int c = it.cvi * 8;
+      const int pix = it.r * row_elems + it.w * C;          // offsets inside a block of a few rows: 32 bits
+      if (HALF == 2) {
+        // pairs of channels: half the fp32 instructions, and a halo of one word per side instead of two
+        const bf16* px = xbase + pix + c;
+        const uint32_t before = c > 0 ? *reinterpret_cast<const uint32_t*>(px - 2) : 0u;
+        const uint4 xv = *reinterpret_cast<const uint4*>(px);
+        const uint32_t after = c + 8 < C ? *reinterpret_cast<const uint32_t*>(px + 8) : 0u;
+        const float2 v[6] = {unpack2(before), unpack2(xv.x), unpack2(xv.y), unpack2(xv.z), unpack2(xv.w), unpack2(after)};
+        float2 t[6], ws[4], o[4];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) t[k] = mul2(v[k], v[k]);
+        window5(t, ws);
+        const float top = fmaxf(fmaxf(fmaxf(ws[0].x, ws[0].y), fmaxf(ws[1].x, ws[1].y)),
+                                fmaxf(fmaxf(ws[2].x, ws[2].y), fmaxf(ws[3].x, ws[3].y)));
+        if (top <= cf.w_max) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            o[k] = mul2(v[k + 1], fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.p3), both(cf.p2)), both(cf.p1)), both(cf.p0)));
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            o[k] = make_float2(v[k + 1].x * __powf(cf.k * fmaf(cf.es, ws[k].x, 1.f), -cf.beta),
+                               v[k + 1].y * __powf(cf.k * fmaf(cf.es, ws[k].y, 1.f), -cf.beta));
+        }
+        *reinterpret_cast<uint4*>(ybase + pix + c) =
+            make_uint4(pack_bf16x2(o[0].x, o[0].y), pack_bf16x2(o[1].x, o[1].y), pack_bf16x2(o[2].x, o[2].y),
+                       pack_bf16x2(o[3].x, o[3].y));
+        continue;
+      }
+      float v[16], t[16], ws[8], o[8];
+      load16(xbase + pix, c, C, v);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) t[j] = v[j] * v[j];
+      window8<HALF>(t, ws);
+      if (max8(ws) <= cf.w_max) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = v[4 + e] * fmaf(ws[e], fmaf(ws[e], fmaf(ws[e], cf.p3, cf.p2), cf.p1), cf.p0);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = v[4 + e] * __powf(cf.k * fmaf(cf.es, ws[e], 1.f), -cf.beta);
+      }
+      *reinterpret_cast<uint4*>(ybase + pix + c) = pack8(o);
+    }
+  }
+  __syncthreads();
+  for (ItemWalk it(tid, nt, g.OW, cv); it.r < n_out; it.next(g.OW, cv)) {
+    const int oh = oh0 + it.r, ow = it.w, c = it.cvi * 8;
+    const int ih0 = oh * PS - g.pad;
+    const int kh_lo = max(0, -ih0), kh_hi = min(PK, g.H - ih0);
+    const int iw0 = ow * PS - g.pad;
+    const int kw_lo = max(0, -iw0), kw_hi = min(PK, W - iw0);
+    // packed: best value and window code per 16-bit lane; strict > keeps the first maximum
+    const uint32_t neg = 0xff7fff7fu;                 // two bf16 lowest finite values
+    __nv_bfloat162 best[4];
+    uint32_t arg[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { best[j] = *reinterpret_cast<const __nv_bfloat162*>(&neg); arg[j] = 0x00ff00ffu; }
+    auto visit = [&](const bf16* yv, uint32_t code1) {
+      const uint4 v = *reinterpret_cast<const uint4*>(yv);
+      const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
+      const uint32_t code = code1 | (code1 << 16);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __nv_bfloat162 x2 = *reinterpret_cast<const __nv_bfloat162*>(&vv[j]);
+        const uint32_t gt = __hgt2_mask(x2, best[j]);
+        best[j] = __hmax2(best[j], x2);
+        arg[j] = (arg[j] & ~gt) | (code & gt);
+      }
+    };
+    const bf16* y0 = ys + (ih0 - ih_base) * row_elems + iw0 * C + c;
+    if (K3S2 && kh_hi - kh_lo == 3 && kw_hi - kw_lo == 3) {      // a whole 3 x 3 window: no loop counters, constant codes
+#pragma unroll
+      for (int t = 0; t < 9; ++t) visit(y0 + (t / 3) * row_elems + (t % 3) * C, (uint32_t)t);
+    } else {
+      for (int kh = kh_lo; kh < kh_hi; ++kh)
+        for (int kw = kw_lo; kw < kw_hi; ++kw) visit(y0 + kh * row_elems + kw * C, (uint32_t)(kh * PK + kw));
+    }
+    const long long opix = ((long long)b * g.OH + oh) * g.OW + ow;
+    *reinterpret_cast<uint4*>(p + opix * g.ldy + c) =
+        make_uint4(*reinterpret_cast<const uint32_t*>(&best[0]), *reinterpret_cast<const uint32_t*>(&best[1]),
+                   *reinterpret_cast<const uint32_t*>(&best[2]), *reinterpret_cast<const uint32_t*>(&best[3]));
+    uint2 pk;      // 16-bit lanes -> bytes
+    pk.x = __byte_perm(arg[0], arg[1], 0x6420);
+    pk.y = __byte_perm(arg[2], arg[3], 0x6420);
+    *reinterpret_cast<uint2*>(argmax + opix * C + c) = pk;
+  }
+}
+
+// ---------------- backward, 3 x 3 windows with stride 2, window of 5 channels ----------------
+// The general kernel below spends 79 instructions per element: three passes over shared memory, the halo channels of
+// every 8-channel vector unpacked and squared again, window loops whose trip counts differ inside a warp.  Here LP lanes
+// share one pixel and a lane holds NV vectors of 8 channels (vector lane + LP * j, so loads stay coalesced); x, the
+// scaled gradient and the ratio stay in registers, a halo channel pair comes from the neighbouring lane by shuffle, and
+// nothing goes through shared memory.  A warp takes pixels of one column parity at a time, so all its lanes visit the
+// same number of windows (1 or 2 per direction).  fp32 arithmetic runs on register pairs (fma.rn.f32x2).
+// 256 x 55 x 55 x 96: 245 -> 173 us; still bound by instruction issue.
 // The 32-bit word (two channels) before / after vector j of this lane: the neighbouring lane's, or across the wrap of
 // the vector order the last (first) lane's vector j - 1 (j + 1); zero outside the pixel.
 template <int LP, int NV>
