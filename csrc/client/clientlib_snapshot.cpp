@@ -177,11 +177,14 @@ bool ClientLib::load_snapshot(const std::string& dir) {
       const TableArena& ta = fabric_.tables[t];
       if (!ta.pull) {
         cudaMemcpy(fabric_.base + ta.cache_off, full.data(), full.size() * sizeof(RowData), cudaMemcpyHostToDevice);
+        // a copy from pageable memory may return once it is staged: its own stream has to drain before another reads it
+        cudaStreamSynchronize(nullptr);
         if (config_.bf16_compute_cache)
           geeps_f32_to_bf16(reinterpret_cast<const float*>(fabric_.base + ta.cache_off), fabric_.base + ta.cache16_off,
                             (long long)(full.size() * ROW_DATA_SIZE), default_stream_);
       }
       if (own.count) cudaMemcpy(fabric_.base + ta.master_off, mine.data(), own.count * sizeof(RowData), cudaMemcpyHostToDevice);
+      cudaStreamSynchronize(nullptr);
       if (ta.pull && config_.bf16_compute_cache && own.count)   // uncached table: the shard's bf16 copy of its rows
         geeps_f32_to_bf16(reinterpret_cast<const float*>(fabric_.base + ta.master_off), fabric_.base + ta.master16_off,
                           (long long)(own.count * ROW_DATA_SIZE), default_stream_);
@@ -191,6 +194,7 @@ bool ClientLib::load_snapshot(const std::string& dir) {
       flags[16] = snap_clock;                                                              // global clock stamp
       for (int i = 0; i < 8; ++i) flags[24 + i] = snap_clock;                              // publish-begin stamps
       cudaMemcpy(fabric_.base + ta.flags_off, flags.data(), 128, cudaMemcpyHostToDevice);
+      cudaStreamSynchronize(nullptr);
       ct.waited_floor = snap_clock;
       ct.waited_by_stream.clear();
       cudaStreamSynchronize((cudaStream_t)default_stream_);
