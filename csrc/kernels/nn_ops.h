@@ -75,6 +75,8 @@ int geeps_relu_backward_2d(const void* dy, const void* y, void* dx, long long P,
 // dst[P][C] (bf16) = src[P][C] (fp32), optionally through ReLU; row pitches in elements
 int geeps_f32_to_bf16_2d(const float* src, void* dst, long long P, int C, long long lds, long long ldd, int relu,
                          void* stream);
+int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s2, long long P, int C, long long ldd,
+                        long long ld0, long long ld1, long long ld2, void* stream);   // dst += s0 (+ s1 (+ s2)), null: absent
 int geeps_add_bf16_2d(void* dst, const void* src, long long P, int C, long long ldd, long long lds, void* stream);
 int geeps_dropout(const void* x, void* y, long long n, float p, unsigned long long seed, void* stream);
 // the same with the seed taken as seed + *step_ref when the kernel runs (a device-resident step counter: the launch

@@ -132,8 +132,8 @@ class Concat(Layer):
             grads[i] = g.view(-1, self.in_shape[-1])
         self._run_branches(run)
         total = grads[0]
-        for g2 in grads[1:]:
-            F.add_2d(total, g2)
+        for i in range(1, len(grads), 3):
+            F.add_2d_n(total, grads[i:i + 3])
         return total
 
 

@@ -281,6 +281,15 @@ def add_2d(dst2d, src2d) -> None:
                                   C.c_longlong(_ld(src2d)), stream_ptr())
 
 
+def add_2d_n(dst2d, srcs) -> None:
+    """dst += the sum of up to three sources, added in fp32 and rounded once."""
+    P, Cc = dst2d.shape
+    assert 1 <= len(srcs) <= 3 and all(t.shape == dst2d.shape and t.dtype == bf16 for t in srcs)
+    t = list(srcs) + [None] * (3 - len(srcs))
+    launch(lib().geeps_add_bf16_2d_n, "add_bf16_2d_n", ptr(dst2d), ptr(t[0]), ptr(t[1]), ptr(t[2]), C.c_longlong(P), Cc,
+           C.c_longlong(_ld(dst2d)), *(C.c_longlong(_ld(u) if u is not None else 0) for u in t), stream_ptr())
+
+
 def f32_to_bf16_2d(src2d, dst2d, relu: bool = False) -> None:
     """dst (bf16) = src (fp32), optionally through ReLU; both may be column slices of wider matrices."""
     P, Cc = src2d.shape

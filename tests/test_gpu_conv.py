@@ -285,3 +285,34 @@ def test_uint8_data_transformer_matches_torch(layout, mode):
         y2 = inp.forward(x)
         xc = (x[:, :, (Hin - H) // 2:(Hin - H) // 2 + H, (Win - W) // 2:(Win - W) // 2 + W].float() - m) * scale
         assert torch.equal(y2, ref.forward(xc.contiguous()))
+
+
+@pytest.mark.parametrize("B,H,W,cpad", [(1, 11, 11, 64), (3, 30, 37, 48), (2, 227, 227, 64), (2, 45, 62, 56)])
+@pytest.mark.parametrize("mirror", [0, 1])
+def test_space_to_depth_of_8_and_16_bit_sources(B, H, W, cpad, mirror):
+    """Rows that start on any byte, ragged right and lower edges, pixels of several rows in one warp, and a source whose
+    size is not a whole number of words (the per-element kernel)."""
+    from geeps_b200.ops import functional as F
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(H * W)
+    Hs, Ws = -(-H // 4), -(-W // 4)
+
+    def ref(v):                                            # v: [B, 3, H, W] in the output's values
+        p = torch.zeros(B, 3, Hs * 4, Ws * 4, device=dev)
+        p[:, :, :H, :W] = v
+        p = p.view(B, 3, Hs, 4, Ws, 4).permute(0, 2, 4, 3, 5, 1).reshape(B, Hs, Ws, 48)
+        return torch.nn.functional.pad(p, (0, cpad - 48)).to(torch.bfloat16)
+
+    y = torch.full((B, Hs, Ws, cpad), 9.0, dtype=torch.bfloat16, device=dev)
+    if not mirror:
+        x = torch.randn(B, 3, H, W, device=dev, generator=gen).to(torch.bfloat16)
+        F.nchw_to_s2d_bf16(x, y, 4)
+        assert torch.equal(y, ref(x.float()))
+    for ho, wo in ((0, 0), (2, 3), (5, 6)):
+        x = torch.randint(0, 256, (B, 3, H + 5, W + 6), device=dev, generator=gen, dtype=torch.uint8)
+        aug = torch.tensor([[ho, wo, mirror]] * B, dtype=torch.int32, device=dev)
+        mean, scale = (104.0, 117.0, 123.0), 1.0 / 58.0
+        F.u8_transform(x, y.fill_(9.0), (H, W), 4, aug, mean, scale)
+        v = x[:, :, ho:ho + H, wo:wo + W].float()
+        v = (v.flip(3) if mirror else v) - torch.tensor(mean, device=dev).view(3, 1, 1)
+        assert torch.equal(y, ref(v * torch.tensor(scale, device=dev)))

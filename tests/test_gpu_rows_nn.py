@@ -463,3 +463,14 @@ def test_lrn_maxpool_backward_over_channel_counts(H, Cc, pad, alpha):
     err = (dx.double() - ref).norm() / ref.norm()
     assert err.item() < 3 * 2.0 ** -9, err.item()
     assert torch.allclose(cs.double(), ref.sum((0, 1, 2)), atol=0.02 * (B * H * H) ** 0.5, rtol=1e-2)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3])
+def test_branch_gradients_are_added_in_one_pass(n):
+    torch.manual_seed(n)
+    dst = torch.randn(333, 88, device=DEV).to(BF)
+    srcs = [torch.randn(333, 96 + 8 * i, device=DEV).to(BF)[:, 8:96] for i in range(n)]
+    ref = dst.double() + sum(t.double() for t in srcs)
+    F.add_2d_n(dst, srcs)
+    # one rounding to bf16 of an fp32 sum
+    assert torch.allclose(dst.double(), ref, atol=1e-6, rtol=2.0 ** -8)
