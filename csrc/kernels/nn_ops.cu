@@ -169,7 +169,7 @@ col2im_kernel(const bf16* __restrict__ dcol, bf16* __restrict__ dx, const GeepsC
 // How a block's threads cover the matrix: thread = (pixel row r, 8-channel slot), so a thread keeps its slot for every
 // pixel it visits: per-channel constants are loaded once, sums stay in registers, and no item costs an integer
 // division (bn_apply spent most of its 77 us on a 32 x 56 x 56 x 192 tensor there and on reloading its six
-// constants per channel; forward + backward of that layer 198 -> 158 us, the 49-kernel Inception block 334 -> 269 us).
+// constants per channel).
 // A row of threads reads whole contiguous pixels.  gridDim.y splits C above 2048 channels.
 struct SlotMap {
   int cvb, rows, row, slot, c;     // slots per block, pixel rows per block, this thread's row / slot / first channel
@@ -233,6 +233,29 @@ __device__ __forceinline__ void slot_sums(const SlotMap& m, const float (&a0)[8]
   }
 }
 
+// Per-channel constants of a block's slots meet in shared memory ([n][8 * slots]): computed or loaded once per block with
+// coalesced reads, then eight consecutive ones per thread.  Read from global memory by every thread (32 bytes apart per
+// lane) they were 39 of the 52 us of a 32 x 56 x 56 x 192 normalisation.
+template <int N, typename Fn>
+__device__ __forceinline__ void slot_consts(const SlotMap& s, int C, float* sh, float (&v)[N][8], Fn fn) {
+  const int width = s.cvb * 8, c0 = (int)blockIdx.y * width;
+  for (int i = threadIdx.x; i < width && c0 + i < C; i += blockDim.x) {
+    float o[N];
+    fn(c0 + i, o);
+#pragma unroll
+    for (int n = 0; n < N; ++n) sh[n * width + i] = o[n];
+  }
+  __syncthreads();
+  if (s.on) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const float4 a = *reinterpret_cast<const float4*>(sh + n * width + s.slot * 8);
+      const float4 b = *reinterpret_cast<const float4*>(sh + n * width + s.slot * 8 + 4);
+      v[n][0] = a.x; v[n][1] = a.y; v[n][2] = a.z; v[n][3] = a.w; v[n][4] = b.x; v[n][5] = b.y; v[n][6] = b.z; v[n][7] = b.w;
+    }
+  }
+}
+
 // MODE 0: out[c] += sum x, out[C+c] += sum x^2                  (BN forward statistics)
 // MODE 1: out[c] += sum dy', out[C+c] += sum dy' * xhat          (BN backward; dy' = dy masked by y>0 if relu)
 // MODE 2: out[c] += scale * sum x                                (bias gradient)
@@ -243,14 +266,14 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
                                                     long long lddy, int relu, float scale) {
   extern __shared__ __align__(16) float sacc[];  // [rows][(1 or 2) * 8 * slots]
   const SlotMap m(C);
-  float a0[8], a1[8], mu[8];
+  float a0[8], a1[8], mr[2][8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) { a0[e] = 0.f; a1[e] = 0.f; mu[e] = 0.f; }
+  for (int e = 0; e < 8; ++e) { a0[e] = 0.f; a1[e] = 0.f; }
+  if (MODE == 1) {
+    slot_consts(m, C, sacc, mr, [&](int c, float (&o)[2]) { o[0] = mean_rstd[c]; o[1] = mean_rstd[C + c]; });
+    __syncthreads();              // the partial sums go to the same shared memory
+  }
   if (m.on) {
-    if (MODE == 1) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) mu[e] = mean_rstd[m.c + e];
-    }
     auto add = [&](const Bf8& xv, const Bf8& dv, const Bf8& yv) {
       if (MODE == 1) {
 #pragma unroll
@@ -258,7 +281,7 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
           float d = bf(dv.v[e]);
           if (relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
           a0[e] += d;
-          a1[e] += d * (bf(xv.v[e]) - mu[e]);
+          a1[e] += d * (bf(xv.v[e]) - mr[0][e]);
         }
       } else {
 #pragma unroll
@@ -290,7 +313,7 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
     }
     if (MODE == 1) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) a1[e] *= mean_rstd[C + m.c + e];
+      for (int e = 0; e < 8; ++e) a1[e] *= mr[1][e];
     }
   }
   slot_sums<MODE == 2 ? 1 : 2>(m, a0, a1, out, C, MODE == 2 ? scale : 1.f, sacc);
@@ -332,13 +355,13 @@ __global__ void bn_finalize_kernel(const float* __restrict__ sums, float* __rest
 
 // y = (x - m) * k + b, k = gamma / std, through ReLU where asked: the pixel loop of both normalisation kernels
 __device__ __forceinline__ void bn_apply_pixels(const SlotMap& s, const bf16* __restrict__ x, bf16* __restrict__ y,
-                                                const float (&m)[8], const float (&k)[8], const float (&b)[8], long long P,
+                                                const float (&mkb)[3][8], long long P,
                                                 long long ldx, long long ldy, int relu) {
   auto one = [&](const Bf8& v) {
     Bf8 o;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      float f = fmaf(bf(v.v[e]) - m[e], k[e], b[e]);
+      float f = fmaf(bf(v.v[e]) - mkb[0][e], mkb[1][e], mkb[2][e]);
       if (relu) f = fmaxf(f, 0.f);
       o.v[e] = __float2bfloat16(f);
     }
@@ -360,20 +383,16 @@ __global__ void __launch_bounds__(256)
 bn_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ mean_rstd,
                 const float* __restrict__ gamma, const float* __restrict__ beta, long long P, int C,
                 long long ldx, long long ldy, int relu) {
+  extern __shared__ __align__(16) float sacc[];
   const SlotMap s(C);
+  float mkb[3][8];
+  slot_consts(s, C, sacc, mkb, [&](int c, float (&o)[3]) { o[0] = mean_rstd[c]; o[1] = mean_rstd[C + c] * gamma[c]; o[2] = beta[c]; });
   if (!s.on) return;
-  float m[8], k[8], b[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    m[e] = mean_rstd[s.c + e];
-    k[e] = mean_rstd[C + s.c + e] * gamma[s.c + e];
-    b[e] = beta[s.c + e];
-  }
-  bn_apply_pixels(s, x, y, m, k, b, P, ldx, ldy, relu);
+  bn_apply_pixels(s, x, y, mkb, P, ldx, ldy, relu);
 }
 
-// Normalisation with the statistics finalised inside: every thread derives mean and 1/std of its eight channels from
-// the channel sums (no separate finalisation launch); the threads of the first pixel also store mean / rstd for the
+// Normalisation with the statistics finalised inside: every block derives mean and 1/std of its channels from
+// the channel sums (no separate finalisation launch); the blocks of the first pixels also store mean / rstd for the
 // backward pass, update the running statistics and zero `zero_after` (2 C floats: the scratch of the NEXT reduction
 // of this layer, e.g. the backward one, so that no memset node sits in front of it).
 __device__ __forceinline__ void bn_apply_fused_body(const bf16* __restrict__ x, bf16* __restrict__ y,
@@ -382,28 +401,26 @@ __device__ __forceinline__ void bn_apply_fused_body(const bf16* __restrict__ x, 
                                                     const float* __restrict__ gamma, const float* __restrict__ beta,
                                                     float* zero_after, long long P, int C, long long ldx, long long ldy,
                                                     int relu, float inv_count, float eps, float momentum) {
+  extern __shared__ __align__(16) float sacc[];
   const SlotMap s(C);
-  if (!s.on) return;
-  float m[8], k[8], b[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int c = s.c + e;
-    m[e] = __ldcg(sums + c) * inv_count;
-    const float var = fmaxf(__ldcg(sums + C + c) * inv_count - m[e] * m[e], 0.f);
+  float mkb[3][8];
+  slot_consts(s, C, sacc, mkb, [&](int c, float (&o)[3]) {
+    const float m = sums[c] * inv_count;
+    const float var = fmaxf(sums[C + c] * inv_count - m * m, 0.f);
     const float r = rsqrtf(var + eps);
-    k[e] = r * gamma[c];
-    b[e] = beta[c];
-    if (s.p0 == 0 && P > 0) {
-      mean_rstd[c] = m[e];
+    o[0] = m; o[1] = r * gamma[c]; o[2] = beta[c];
+    if (blockIdx.x == 0 && P > 0) {
+      mean_rstd[c] = m;
       mean_rstd[C + c] = r;
       if (running_mean) {
-        running_mean[c] = (1.f - momentum) * running_mean[c] + momentum * m[e];
+        running_mean[c] = (1.f - momentum) * running_mean[c] + momentum * m;
         running_var[c] = (1.f - momentum) * running_var[c] + momentum * var;
       }
       if (zero_after) { zero_after[c] = 0.f; zero_after[C + c] = 0.f; }
     }
-  }
-  bn_apply_pixels(s, x, y, m, k, b, P, ldx, ldy, relu);
+  });
+  if (!s.on) return;
+  bn_apply_pixels(s, x, y, mkb, P, ldx, ldy, relu);
 }
 __global__ void __launch_bounds__(256)
 bn_apply_fused_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ sums,
@@ -421,32 +438,28 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
                                                  const float* sums, float* dgamma, float* dbeta, long long P, int C,
                                                  long long ldx, long long lddy, long long lddx, int relu,
                                                  float grad_scale, float* zero_after) {
+  extern __shared__ __align__(16) float sacc[];
   const SlotMap s(C);
-  if (!s.on) return;
   const float invP = 1.f / (float)P;
-  float m[8], k[8], c0[8], c1[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int c = s.c + e;
-    const float rs = mean_rstd[C + c], s0 = __ldcg(sums + c), s1 = __ldcg(sums + C + c);
-    m[e] = mean_rstd[c];
-    k[e] = gamma[c] * rs;
-    c0[e] = s0 * invP;
-    c1[e] = rs * (s1 * invP);
-    if (s.p0 == 0) {
+  float q[4][8];                    // mean, gamma / std, sum_dy / P, sum_dy_xhat / (P std)
+  slot_consts(s, C, sacc, q, [&](int c, float (&o)[4]) {
+    const float rs = mean_rstd[C + c], s0 = sums[c], s1 = sums[C + c];
+    o[0] = mean_rstd[c]; o[1] = gamma[c] * rs; o[2] = s0 * invP; o[3] = rs * (s1 * invP);
+    if (blockIdx.x == 0) {
       if (dbeta) dbeta[c] = s0 * grad_scale;
       if (dgamma) dgamma[c] = s1 * grad_scale;
       // the scratch of this layer's next forward reduction (nobody reads it during the backward pass)
       if (zero_after) { zero_after[c] = 0.f; zero_after[C + c] = 0.f; }
     }
-  }
+  });
+  if (!s.on) return;
   auto one = [&](const Bf8& xv, const Bf8& dv, const Bf8& yv) {
     Bf8 o;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       float d = bf(dv.v[e]);
       if (relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
-      o.v[e] = __float2bfloat16(k[e] * (d - c0[e] - (bf(xv.v[e]) - m[e]) * c1[e]));
+      o.v[e] = __float2bfloat16(q[1][e] * (d - q[2][e] - (bf(xv.v[e]) - q[0][e]) * q[3][e]));
     }
     return o;
   };
@@ -1579,7 +1592,11 @@ int geeps_col2im(const void* dcol, void* dx, const GeepsConvGeom* g, int accumul
 // reductions: one batch of four pixels per thread where that leaves SMs idle, at most four blocks per SM beyond
 static SlotGrid reduce_grid(long long P, int C, int nq = 2) { return slot_grid(P, C, 4, 4, nq); }
 // element-wise passes with per-channel constants: up to eight blocks per SM
-static SlotGrid apply_grid(long long P, int C) { return slot_grid(P, C, 4, 8, 0); }
+static SlotGrid apply_grid(long long P, int C) {
+  SlotGrid g = slot_grid(P, C, 4, 8, 0);
+  g.smem = ((size_t)(C / 8) + g.grid.y - 1) / g.grid.y * 8 * 4 * sizeof(float);      // four constants per channel
+  return g;
+}
 
 int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* beta, float* sums,
                      float* mean_rstd, float* running_mean, float* running_var, long long P, int C,
@@ -1592,7 +1609,7 @@ int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* be
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   bn_finalize_kernel<<<(C + 127) / 128, 128, 0, st>>>(sums, mean_rstd, running_mean, running_var, C,
                                                       1.f / (float)P, eps, momentum);
-  bn_apply_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
+  bn_apply_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
                                                         ldy, relu);
   return CK();
 }
@@ -1606,7 +1623,7 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
   channel_reduce_kernel<1><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  bn_backward_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
+  bn_backward_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
                                                            (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
                                                            ldx, lddy, lddx, relu, grad_scale, nullptr);
   return CK();
@@ -1617,7 +1634,12 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
 // finalisation launch: 2 launches per direction instead of 4 and 3.
 // grid of a single-launch BatchNorm kernel: enough blocks for the reduction, never more than can be resident at
 // once beside other kernels (the blocks wait for one another at the grid barrier)
-static SlotGrid bn_coop_grid(long long P, int C) { return slot_grid(P, C, 4, 1, 2); }
+static SlotGrid bn_coop_grid(long long P, int C) {
+  SlotGrid g = slot_grid(P, C, 4, 1, 2);
+  const size_t consts = apply_grid(P, C).smem;
+  if (g.smem < consts) g.smem = consts;
+  return g;
+}
 static bool bn_coop_enabled() {
   static int v = -1;
   // off by default: with at most one block per SM and a grid barrier the single launch is slower than two full-width
@@ -1644,7 +1666,7 @@ int geeps_bn_forward_fused(const void* x, void* y, const float* gamma, const flo
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
   channel_reduce_kernel<0><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
-  bn_apply_fused_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
+  bn_apply_fused_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
                                                               running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                                                               1.f / (float)P, eps, momentum);
   return CK();
@@ -1667,7 +1689,7 @@ int geeps_bn_backward_fused(const void* x, const void* dy, const void* y, void* 
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
   channel_reduce_kernel<1><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  bn_backward_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
+  bn_backward_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
                                                            (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
                                                            ldx, lddy, lddx, relu, grad_scale, zero_after);
   return CK();
@@ -1922,7 +1944,7 @@ int geeps_bn_forward_noalloc(const void* x, void* y, const float* gamma, const f
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   bn_finalize_kernel<<<(C + 127) / 128, 128, 0, st>>>(sums, mean_rstd, running_mean, running_var, C,
                                                       1.f / (float)P, eps, momentum);
-  bn_apply_kernel<<<ag.grid, ag.threads, 0, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
+  bn_apply_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
                                                         ldy, relu);
   return CK();
 }
