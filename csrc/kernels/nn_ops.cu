@@ -259,27 +259,31 @@ __device__ __forceinline__ void slot_consts(const SlotMap& s, int C, float* sh, 
 // MODE 0: out[c] += sum x, out[C+c] += sum x^2                  (BN forward statistics)
 // MODE 1: out[c] += sum dy', out[C+c] += sum dy' * xhat          (BN backward; dy' = dy masked by y>0 if relu)
 // MODE 2: out[c] += scale * sum x                                (bias gradient)
+// MODE 3: as 1, dy' = dy where the forward pass left a bit (y then points to the bit bytes, one per 8-channel vector)
 template <int MODE>
 __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, const bf16* __restrict__ dy,
                                                     const bf16* __restrict__ y, const float* __restrict__ mean_rstd,
                                                     float* __restrict__ out, long long P, int C, long long ldx,
                                                     long long lddy, int relu, float scale) {
   extern __shared__ __align__(16) float sacc[];  // [rows][(1 or 2) * 8 * slots]
+  constexpr bool BWD = MODE == 1 || MODE == 3;
+  const uint8_t* bits = reinterpret_cast<const uint8_t*>(y);
+  const long long cv = C >> 3;
   const SlotMap m(C);
   float a0[8], a1[8], mr[2][8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) { a0[e] = 0.f; a1[e] = 0.f; }
-  if (MODE == 1) {
+  if (BWD) {
     slot_consts(m, C, sacc, mr, [&](int c, float (&o)[2]) { o[0] = mean_rstd[c]; o[1] = mean_rstd[C + c]; });
     __syncthreads();              // the partial sums go to the same shared memory
   }
   if (m.on) {
-    auto add = [&](const Bf8& xv, const Bf8& dv, const Bf8& yv) {
-      if (MODE == 1) {
+    auto add = [&](const Bf8& xv, const Bf8& dv, const Bf8& yv, uint32_t on) {
+      if (BWD) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           float d = bf(dv.v[e]);
-          if (relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
+          if (MODE == 3 ? !(on >> e & 1u) : relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
           a0[e] += d;
           a1[e] += d * (bf(xv.v[e]) - mr[0][e]);
         }
@@ -292,26 +296,27 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
     long long p = m.p0;
     for (; p + (U - 1) * m.step < P; p += U * m.step) {
       Bf8 xv[U], dv[U], yv[U];
+      uint32_t on[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         xv[u] = ld8(x + (p + u * m.step) * ldx + m.c);
+        on[u] = 0u;
+        if (BWD) dv[u] = ld8(dy + (p + u * m.step) * lddy + m.c);
+        if (MODE == 3) on[u] = bits[(p + u * m.step) * cv + (m.c >> 3)];
         if (MODE == 1) {
-          dv[u] = ld8(dy + (p + u * m.step) * lddy + m.c);
           if (relu) yv[u] = ld8(y + (p + u * m.step) * lddy + m.c);
         }
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) add(xv[u], dv[u], yv[u]);
+      for (int u = 0; u < U; ++u) add(xv[u], dv[u], yv[u], on[u]);
     }
     for (; p < P; p += m.step) {
       Bf8 xv = ld8(x + p * ldx + m.c), dv, yv;
-      if (MODE == 1) {
-        dv = ld8(dy + p * lddy + m.c);
-        if (relu) yv = ld8(y + p * lddy + m.c);
-      }
-      add(xv, dv, yv);
+      if (BWD) dv = ld8(dy + p * lddy + m.c);
+      if (MODE == 1 && relu) yv = ld8(y + p * lddy + m.c);
+      add(xv, dv, yv, MODE == 3 ? bits[p * cv + (m.c >> 3)] : 0u);
     }
-    if (MODE == 1) {
+    if (BWD) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) a1[e] *= mr[1][e];
     }
@@ -353,10 +358,17 @@ __global__ void bn_finalize_kernel(const float* __restrict__ sums, float* __rest
   }
 }
 
-// y = (x - m) * k + b, k = gamma / std, through ReLU where asked: the pixel loop of both normalisation kernels
+// y = (x - m) * k + b, k = gamma / std, through ReLU where asked: the pixel loop of both normalisation kernels.
+// bits (optional): one byte per 8-channel vector with bit e set where y[e] > 0, all that the ReLU backward needs of y.
 __device__ __forceinline__ void bn_apply_pixels(const SlotMap& s, const bf16* __restrict__ x, bf16* __restrict__ y,
                                                 const float (&mkb)[3][8], long long P,
-                                                long long ldx, long long ldy, int relu) {
+                                                long long ldx, long long ldy, int relu, uint8_t* bits, int cv) {
+  auto mark = [&](long long p, const Bf8& o) {
+    uint32_t on = 0u;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) on |= bf(o.v[e]) > 0.f ? 1u << e : 0u;
+    bits[p * cv + (s.c >> 3)] = (uint8_t)on;
+  };
   auto one = [&](const Bf8& v) {
     Bf8 o;
 #pragma unroll
@@ -374,9 +386,17 @@ __device__ __forceinline__ void bn_apply_pixels(const SlotMap& s, const bf16* __
 #pragma unroll
     for (int u = 0; u < U; ++u) v[u] = ld8(x + (p + u * s.step) * ldx + s.c);
 #pragma unroll
-    for (int u = 0; u < U; ++u) st8(y + (p + u * s.step) * ldy + s.c, one(v[u]));
+    for (int u = 0; u < U; ++u) {
+      const Bf8 o = one(v[u]);
+      st8(y + (p + u * s.step) * ldy + s.c, o);
+      if (bits) mark(p + u * s.step, o);
+    }
   }
-  for (; p < P; p += s.step) st8(y + p * ldy + s.c, one(ld8(x + p * ldx + s.c)));
+  for (; p < P; p += s.step) {
+    const Bf8 o = one(ld8(x + p * ldx + s.c));
+    st8(y + p * ldy + s.c, o);
+    if (bits) mark(p, o);
+  }
 }
 
 __global__ void __launch_bounds__(256)
@@ -388,7 +408,7 @@ bn_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* _
   float mkb[3][8];
   slot_consts(s, C, sacc, mkb, [&](int c, float (&o)[3]) { o[0] = mean_rstd[c]; o[1] = mean_rstd[C + c] * gamma[c]; o[2] = beta[c]; });
   if (!s.on) return;
-  bn_apply_pixels(s, x, y, mkb, P, ldx, ldy, relu);
+  bn_apply_pixels(s, x, y, mkb, P, ldx, ldy, relu, nullptr, 0);
 }
 
 // Normalisation with the statistics finalised inside: every block derives mean and 1/std of its channels from
@@ -400,7 +420,7 @@ __device__ __forceinline__ void bn_apply_fused_body(const bf16* __restrict__ x, 
                                                     float* running_mean, float* running_var,
                                                     const float* __restrict__ gamma, const float* __restrict__ beta,
                                                     float* zero_after, long long P, int C, long long ldx, long long ldy,
-                                                    int relu, float inv_count, float eps, float momentum) {
+                                                    int relu, float inv_count, float eps, float momentum, uint8_t* bits) {
   extern __shared__ __align__(16) float sacc[];
   const SlotMap s(C);
   float mkb[3][8];
@@ -420,18 +440,19 @@ __device__ __forceinline__ void bn_apply_fused_body(const bf16* __restrict__ x, 
     }
   });
   if (!s.on) return;
-  bn_apply_pixels(s, x, y, mkb, P, ldx, ldy, relu);
+  bn_apply_pixels(s, x, y, mkb, P, ldx, ldy, relu, bits, C >> 3);
 }
 __global__ void __launch_bounds__(256)
 bn_apply_fused_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ sums,
                       float* __restrict__ mean_rstd, float* running_mean, float* running_var,
                       const float* __restrict__ gamma, const float* __restrict__ beta, float* zero_after, long long P,
-                      int C, long long ldx, long long ldy, int relu, float inv_count, float eps, float momentum) {
+                      int C, long long ldx, long long ldy, int relu, float inv_count, float eps, float momentum, uint8_t* bits) {
   bn_apply_fused_body(x, y, sums, mean_rstd, running_mean, running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
-                      inv_count, eps, momentum);
+                      inv_count, eps, momentum, bits);
 }
 
 // dx = gamma * rstd * (dy' - sum_dy/P - xhat * sum_dy_xhat/P); also emits dgamma, dbeta (scaled).
+template <bool BITS>
 __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, const bf16* __restrict__ dy,
                                                  const bf16* __restrict__ y, bf16* __restrict__ dx,
                                                  const float* mean_rstd, const float* __restrict__ gamma,
@@ -439,6 +460,8 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
                                                  long long ldx, long long lddy, long long lddx, int relu,
                                                  float grad_scale, float* zero_after) {
   extern __shared__ __align__(16) float sacc[];
+  const uint8_t* bits = reinterpret_cast<const uint8_t*>(y);
+  const long long cv = C >> 3;
   const SlotMap s(C);
   const float invP = 1.f / (float)P;
   float q[4][8];                    // mean, gamma / std, sum_dy / P, sum_dy_xhat / (P std)
@@ -453,12 +476,12 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
     }
   });
   if (!s.on) return;
-  auto one = [&](const Bf8& xv, const Bf8& dv, const Bf8& yv) {
+  auto one = [&](const Bf8& xv, const Bf8& dv, const Bf8& yv, uint32_t on) {
     Bf8 o;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       float d = bf(dv.v[e]);
-      if (relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
+      if (BITS ? !(on >> e & 1u) : relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
       o.v[e] = __float2bfloat16(q[1][e] * (d - q[2][e] - (bf(xv.v[e]) - q[0][e]) * q[3][e]));
     }
     return o;
@@ -467,27 +490,30 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
   long long p = s.p0;
   for (; p + (U - 1) * s.step < P; p += U * s.step) {
     Bf8 xv[U], dv[U], yv[U];
+    uint32_t on[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       xv[u] = ld8(x + (p + u * s.step) * ldx + s.c);
       dv[u] = ld8(dy + (p + u * s.step) * lddy + s.c);
-      if (relu) yv[u] = ld8(y + (p + u * s.step) * lddy + s.c);
+      on[u] = BITS ? bits[(p + u * s.step) * cv + (s.c >> 3)] : 0u;
+      if (!BITS && relu) yv[u] = ld8(y + (p + u * s.step) * lddy + s.c);
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) st8(dx + (p + u * s.step) * lddx + s.c, one(xv[u], dv[u], yv[u]));
+    for (int u = 0; u < U; ++u) st8(dx + (p + u * s.step) * lddx + s.c, one(xv[u], dv[u], yv[u], on[u]));
   }
   for (; p < P; p += s.step) {
     Bf8 xv = ld8(x + p * ldx + s.c), dv = ld8(dy + p * lddy + s.c), yv;
-    if (relu) yv = ld8(y + p * lddy + s.c);
-    st8(dx + p * lddx + s.c, one(xv, dv, yv));
+    if (!BITS && relu) yv = ld8(y + p * lddy + s.c);
+    st8(dx + p * lddx + s.c, one(xv, dv, yv, BITS ? bits[p * cv + (s.c >> 3)] : 0u));
   }
 }
+template <bool BITS>
 __global__ void __launch_bounds__(256)
 bn_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                    bf16* __restrict__ dx, const float* __restrict__ mean_rstd, const float* __restrict__ gamma,
                    const float* __restrict__ sums, float* dgamma, float* dbeta, long long P, int C,
                    long long ldx, long long lddy, long long lddx, int relu, float grad_scale, float* zero_after) {
-  bn_backward_body(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
+  bn_backward_body<BITS>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
                    zero_after);
 }
 
@@ -522,7 +548,7 @@ bn_forward_coop_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, float* 
   channel_reduce_body<0>(x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
     bn_apply_fused_body(x, y, sums, mean_rstd, running_mean, running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
-                        inv_count, eps, momentum);
+                        inv_count, eps, momentum, nullptr);
   else if (threadIdx.x == 0) { bar[2] = 1; mean_rstd[0] = __int_as_float(0x7fc00000); }
   bn_grid_done(bar, (int)(gridDim.x * gridDim.y));
 }
@@ -533,8 +559,8 @@ bn_backward_coop_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
                         long long lddy, long long lddx, int relu, float grad_scale) {
   channel_reduce_body<1>(x, dy, y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
   if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
-    bn_backward_body(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
-                     zero_after);
+    bn_backward_body<false>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
+                            zero_after);
   else if (threadIdx.x == 0) { bar[2] = 1; mean_rstd[0] = __int_as_float(0x7fc00000); }
   bn_grid_done(bar, (int)(gridDim.x * gridDim.y));
 }
@@ -1623,7 +1649,7 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
   channel_reduce_kernel<1><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  bn_backward_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
+  bn_backward_kernel<false><<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
                                                            (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
                                                            ldx, lddy, lddx, relu, grad_scale, nullptr);
   return CK();
@@ -1652,6 +1678,13 @@ int geeps_bn_forward_fused(const void* x, void* y, const float* gamma, const flo
                            float* mean_rstd, float* running_mean, float* running_var, float* zero_after, int* barrier,
                            long long P, int C, long long ldx, long long ldy, float eps, float momentum, int relu,
                            void* stream) {
+  return geeps_bn_forward_fused_bits(x, y, gamma, beta, sums, mean_rstd, running_mean, running_var, zero_after, barrier,
+                                     nullptr, P, C, ldx, ldy, eps, momentum, relu, stream);
+}
+int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, const float* beta, float* sums,
+                                float* mean_rstd, float* running_mean, float* running_var, float* zero_after,
+                                int* barrier, unsigned char* bits, long long P, int C, long long ldx, long long ldy,
+                                float eps, float momentum, int relu, void* stream) {
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   if (barrier != nullptr && bn_coop_enabled()) {
@@ -1668,13 +1701,20 @@ int geeps_bn_forward_fused(const void* x, void* y, const float* gamma, const flo
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   bn_apply_fused_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
                                                               running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
-                                                              1.f / (float)P, eps, momentum);
+                                                              1.f / (float)P, eps, momentum, bits);
   return CK();
 }
 int geeps_bn_backward_fused(const void* x, const void* dy, const void* y, void* dx, float* mean_rstd,
                             const float* gamma, float* sums, float* dgamma, float* dbeta, float* zero_after,
                             int* barrier, long long P, int C, long long ldx, long long lddy, long long lddx, int relu,
                             float grad_scale, void* stream) {
+  return geeps_bn_backward_fused_bits(x, dy, y, nullptr, dx, mean_rstd, gamma, sums, dgamma, dbeta, zero_after, barrier, P,
+                                      C, ldx, lddy, lddx, relu, grad_scale, stream);
+}
+int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, const unsigned char* bits, void* dx,
+                                 float* mean_rstd, const float* gamma, float* sums, float* dgamma, float* dbeta,
+                                 float* zero_after, int* barrier, long long P, int C, long long ldx, long long lddy,
+                                 long long lddx, int relu, float grad_scale, void* stream) {
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   if (barrier != nullptr && bn_coop_enabled()) {
@@ -1687,9 +1727,17 @@ int geeps_bn_backward_fused(const void* x, const void* dy, const void* y, void* 
     return e == cudaSuccess ? CK() : (int)e;
   }
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  if (bits != nullptr && relu) {
+    channel_reduce_kernel<3><<<rg.grid, rg.threads, rg.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)bits,
+                                                                   mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
+    bn_backward_kernel<true><<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
+                                                             mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx,
+                                                             relu, grad_scale, zero_after);
+    return CK();
+  }
   channel_reduce_kernel<1><<<rg.grid, rg.threads, rg.smem, st>>>(
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  bn_backward_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
+  bn_backward_kernel<false><<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
                                                            (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
                                                            ldx, lddy, lddx, relu, grad_scale, zero_after);
   return CK();

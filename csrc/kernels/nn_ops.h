@@ -55,6 +55,15 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
 // `barrier` (4 ints, zero at first use, private to this layer and direction) - ONE cooperative launch whose blocks meet
 // at a bounded grid barrier between the reduction and the normalisation, when GEEPS_BN_COOP=1 (measured slower than the
 // two launches, so it is off by default).
+// the fused pair with the ReLU mask kept as bits ([P][C / 8] bytes, written forward, read backward in the place of y)
+int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, const float* beta, float* sums,
+                                float* mean_rstd, float* running_mean, float* running_var, float* zero_after,
+                                int* barrier, unsigned char* bits, long long P, int C, long long ldx, long long ldy,
+                                float eps, float momentum, int relu, void* stream);
+int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, const unsigned char* bits, void* dx,
+                                 float* mean_rstd, const float* gamma, float* sums, float* dgamma, float* dbeta,
+                                 float* zero_after, int* barrier, long long P, int C, long long ldx, long long lddy,
+                                 long long lddx, int relu, float grad_scale, void* stream);
 int geeps_bn_forward_fused(const void* x, void* y, const float* gamma, const float* beta, float* sums,
                            float* mean_rstd, float* running_mean, float* running_var, float* zero_after, int* barrier,
                            long long P, int C, long long ldx, long long ldy, float eps, float momentum, int relu,

@@ -467,6 +467,9 @@ class BatchNorm(Layer):
         self.running_var = torch.ones(self.C, device=device)
         self.y = torch.empty(self.P, self.C, dtype=BF, device=device)
         self.dx = torch.empty(self.P, self.C, dtype=BF, device=device)
+        # where the output passed the ReLU, one bit per element: the backward pass reads these instead of y, twice
+        self.bits = torch.empty(self.P, self.C // 8, dtype=torch.uint8, device=device) if self.relu and self.C % 8 == 0 else None
+        self._bits_valid = False
         self.out_shape = in_shape
         return in_shape
 
@@ -479,14 +482,14 @@ class BatchNorm(Layer):
 
     def forward(self, x):
         self.x = x if x.dim() == 2 else x.view(self.P, self.C)
+        self._bits_valid = self.bits is not None and self._clean_f
         if not self._clean_f:       # two forward passes in a row (no backward in between zeroed the scratch)
             F.bn_forward(self.x, self.y, self.p32["gamma"], self.p32["beta"], self.sums, self.mean_rstd,
                          self.running_mean, self.running_var, eps=self.eps, momentum=self.momentum, relu=self.relu)
             return self.y
         F.bn_forward_fused(self.x, self.y, self.p32["gamma"], self.p32["beta"], self.sums, self.mean_rstd,
                            self.running_mean, self.running_var, zero_after=self.sums_b, barrier=self.bar[0:4],
-                           eps=self.eps,
-                           momentum=self.momentum, relu=self.relu)
+                           eps=self.eps, momentum=self.momentum, relu=self.relu, bits=self.bits)
         self._clean_f, self._clean_b = False, True
         return self.y
 
@@ -499,7 +502,7 @@ class BatchNorm(Layer):
             return self.dx
         F.bn_backward_fused(self.x, dy, self.y, self.dx, self.mean_rstd, self.p32["gamma"], self.sums_b,
                             self.g32["gamma"], self.g32["beta"], zero_after=self.sums, barrier=self.bar[4:8],
-                            relu=self.relu)
+                            relu=self.relu, bits=self.bits if self._bits_valid else None)
         self._clean_b, self._clean_f = False, True
         return self.dx
 

@@ -474,3 +474,24 @@ def test_branch_gradients_are_added_in_one_pass(n):
     F.add_2d_n(dst, srcs)
     # one rounding to bf16 of an fp32 sum
     assert torch.allclose(dst.double(), ref, atol=1e-6, rtol=2.0 ** -8)
+
+
+@pytest.mark.parametrize("P,Cc", [(5, 8), (777, 104), (64, 2056)])
+def test_batchnorm_backward_from_mask_bits_equals_the_one_from_the_output(P, Cc):
+    torch.manual_seed(P)
+    x, dy = torch.randn(P, Cc, device=DEV).to(BF), torch.randn(P, Cc, device=DEV).to(BF)
+    g, b = torch.rand(Cc, device=DEV) + 0.5, torch.randn(Cc, device=DEV)
+    y, stat = torch.empty_like(x), torch.empty(2 * Cc, device=DEV)
+    bits = torch.full((P, Cc // 8), 0xa5, dtype=torch.uint8, device=DEV)
+    rm, rv = torch.zeros(Cc, device=DEV), torch.ones(Cc, device=DEV)
+    F.bn_forward_fused(x, y, g, b, torch.zeros(2 * Cc, device=DEV), stat, rm, rv, relu=True, bits=bits)
+    want = (y.view(P, Cc // 8, 8) > 0).long() << torch.arange(8, device=DEV)
+    assert torch.equal(bits.long(), want.sum(2))
+    got = []
+    for m in (None, bits):
+        dx, dg, db = torch.empty_like(x), torch.empty(Cc, device=DEV), torch.empty(Cc, device=DEV)
+        F.bn_backward_fused(x, dy, y, dx, stat, g, torch.zeros(2 * Cc, device=DEV), dg, db, relu=True, bits=m)
+        got.append((dx, dg, db))
+    # the sums of the blocks meet in any order: last digits of fp32, and the bf16 rounding they may tip
+    assert torch.allclose(got[0][0].float(), got[1][0].float(), atol=1e-5, rtol=2.0 ** -7)
+    assert torch.allclose(got[0][1], got[1][1], atol=1e-4, rtol=1e-4) and torch.allclose(got[0][2], got[1][2], atol=1e-4, rtol=1e-4)
