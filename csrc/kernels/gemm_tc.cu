@@ -578,7 +578,12 @@ int geeps_gemm_bf16(const GeepsGemmParams* p, void* stream) {
     if (!can_split && (long long)m_tiles * ((p->N + bn - 1) / bn) < kSMs && p->N > 64) {
       // a bf16 slab is 64 columns wide (see below): several tiles have widths that are multiples of it
       const int step = tma_c && !p->out_fp32 ? 64 : unit;
-      const bool cluster_ok = p->split_k <= 1 && p->beta == 0.f && p->K > 0;
+      // Clusters only for a long K over very few tiles (the data gradient of a wide classifier: 32 x 1024, K = 21841,
+      // 16 tiles: 76 -> 31 us).  Elsewhere they give less (256 x 4096, K = 9216: 40 -> 32 us) and every product would
+      // add its K slices in another order: in a deep network with near-ties in its pooling windows that changes which
+      // element a later step's maximum picks, so ordinary layers keep one running sum over K.
+      const bool cluster_ok = p->split_k <= 1 && p->beta == 0.f && kt_total >= 128 &&
+                              (long long)m_tiles * ((p->N + 63) / 64) <= kSMs / 8;
       const TileChoice c = choose_tiles(p, step, kt_total, kSMs, cluster_ok);
       if (c.cluster > 1 || c.bn < bn) { bn = c.bn; cluster = c.cluster; }
     }
