@@ -115,15 +115,20 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 }
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 unpack2(uint32_t w) { return make_float2(bf_lo(w), bf_hi(w)); }
-// sums over five neighbouring entries: t holds entries c-2 .. c+9 as pairs, w the sums around c .. c+7
+// sums over five neighbouring entries: t holds entries c-2 .. c+9 as pairs, w the sums around c .. c+7 (sliding, the
+// same operations as window8: both kernels of a direction give the same bits)
 __device__ __forceinline__ void window5(const float2 (&t)[6], float2 (&w)[4]) {
-  float p[6], q[5];
+  const float v[12] = {t[0].x, t[0].y, t[1].x, t[1].y, t[2].x, t[2].y, t[3].x, t[3].y, t[4].x, t[4].y, t[5].x, t[5].y};
+  float acc = v[0];
 #pragma unroll
-  for (int k = 0; k < 6; ++k) p[k] = t[k].x + t[k].y;
+  for (int i = 1; i < 5; ++i) acc += v[i];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) q[k] = p[k] + p[k + 1];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) w[k] = make_float2(q[k] + t[k + 2].x, t[k].y + q[k + 1]);
+  for (int k = 0; k < 4; ++k) {
+    w[k].x = acc;
+    acc += v[2 * k + 5] - v[2 * k];
+    w[k].y = acc;
+    if (k < 3) acc += v[2 * k + 6] - v[2 * k + 1];
+  }
 }
 
 // ---------------- forward ----------------
