@@ -542,6 +542,78 @@ TileChoice choose_tiles(const GeepsGemmParams* p, int unit, int kt, int sms, boo
   return best;
 }
 
+// TMA-store epilogue: C 16-byte aligned with a 16-byte-multiple pitch, no read-modify-write of C
+bool tma_c_ok(const GeepsGemmParams* p) {
+  return (((uintptr_t)p->C & 15) == 0) && ((p->ldc * (p->out_fp32 ? 4 : 2)) % 16 == 0) && p->beta == 0.f;
+}
+
+// How a product is cut: tile width, K slices, and whether the slices of a tile share a cluster.
+struct GemmPlan { int bn, split_k, cluster; };
+// Calls that may cut K into slices which meet in fp32 atomics (split_k 0, plain fp32 output).
+bool auto_split(const GeepsGemmParams* p, int kt) { return p->split_k == 0 && p->out_fp32 && !p->relu && kt >= 8; }
+GemmPlan plan_gemm(const GeepsGemmParams* p, int sms) {
+  const long long m_tiles = (p->M + BM - 1) / BM;
+  const int unit = p->b_mn_major ? 64 : 32;
+  const int kt = (int)((p->K + BK - 1) / BK);
+  const bool tma_c = tma_c_ok(p);
+  GemmPlan g = {p->block_n, 1, 1};
+  if (g.bn <= 0 || g.bn > 256 || g.bn % unit) {
+    // as few N tiles as possible with little padding ...
+    const long long nt = (p->N + 255) / 256;
+    g.bn = round_up((p->N + nt - 1) / nt, unit);
+    // ... but enough tiles to occupy every SM when the problem allows it
+    auto tiles = [&] { return m_tiles * ((p->N + g.bn - 1) / g.bn); };
+    if (auto_split(p, kt)) {
+      // A long K is split below and keeps its wide tiles.  A short one (K < 1024) is spread by narrow tiles first: every
+      // K slice costs a clearing pass and a read-modify-write of the output, so the cost of choose_tiles, which knows
+      // only operand bytes, does not hold here (1000 x 4096, K = 512: two slices 20.2 us, narrow tiles 10.9 us;
+      // 439 x 4162, K = 632: 15.0 and 10.9 us).
+      while (kt < 16 && g.bn > 64 && tiles() < sms) {
+        const int narrow = round_up(g.bn / 2, unit);
+        if (narrow >= g.bn) break;
+        g.bn = narrow;
+      }
+    } else if (tiles() < sms && p->N > 64) {
+      // a bf16 slab is 64 columns wide (see below): several tiles have widths that are multiples of it
+      const int step = tma_c && !p->out_fp32 ? 64 : unit;
+      // Clusters only for a long K over very few tiles (the data gradient of a wide classifier: 32 x 1024, K = 21841,
+      // 16 tiles: 76 -> 31 us).  Elsewhere they give less (256 x 4096, K = 9216: 40 -> 32 us) and every product would
+      // add its K slices in another order: in a deep network with near-ties in its pooling windows that changes which
+      // element a later step's maximum picks, so ordinary layers keep one running sum over K.
+      const bool cluster_ok = p->split_k <= 1 && p->beta == 0.f && kt >= 128 &&
+                              m_tiles * ((p->N + 63) / 64) <= sms / 8;
+      const TileChoice c = choose_tiles(p, step, kt, sms, cluster_ok);
+      if (c.cluster > 1 || c.bn < g.bn) { g.bn = c.bn; g.cluster = c.cluster; }
+    }
+  }
+  if (g.bn > 256) g.bn = 256;
+  // a bf16 slab is 64 columns wide: with several N tiles the tile width must be a multiple of it
+  if (tma_c && !p->out_fp32 && (g.bn % 64) && (p->N + g.bn - 1) / g.bn > 1) g.bn = round_up(g.bn, 64);
+  if (g.cluster > 1) { g.split_k = g.cluster; return g; }
+  int split = p->split_k;
+  if (split == 0) {  // auto: occupy the SMs about twice over when the output has few tiles
+    split = 1;
+    const long long tiles = m_tiles * ((p->N + g.bn - 1) / g.bn);
+    if (auto_split(p, kt) && tiles < sms) {
+      const long long want = (2 * sms) / tiles;   // at most two full waves: one work item more would add a third round
+      const long long cap = kt / 4;
+      split = (int)(want < cap ? want : cap);
+    }
+  }
+  g.split_k = split < 1 ? 1 : (split > kt ? kt : split);
+  if (g.split_k > 1) {
+    // every k-slice must be non-empty, otherwise its tile would never be completed by an MMA commit
+    const int per = (kt + g.split_k - 1) / g.split_k;
+    g.split_k = (kt + per - 1) / per;
+  }
+  return g;
+}
+// large K-major products go to CTA pairs (half the B traffic per SM) when 256-row tiles can fill the machine
+bool takes_pairs(const GeepsGemmParams* p, int sms) {
+  return p->block_n == 0 && p->split_k <= 1 && geeps_gemm_pair_supported(p) &&
+         ((p->M + 255) / 256) * ((p->N + 255) / 256) >= sms / 2;
+}
+
 }  // namespace
 
 extern "C" {
@@ -555,42 +627,27 @@ int geeps_gemm_tc_supported(const GeepsGemmParams* p) {
   return 1;
 }
 
+int geeps_gemm_plan(const GeepsGemmParams* p, GeepsGemmPlan* out) {
+  if (!geeps_gemm_tc_supported(p)) return 0;
+  const int sms = geeps_sm_count();
+  const GemmPlan g = plan_gemm(p, sms);
+  out->pair = takes_pairs(p, sms) ? 1 : 0;
+  out->block_n = g.bn;
+  out->split_k = g.split_k;
+  out->cluster = g.cluster;
+  out->tiles = (p->M + BM - 1) / BM * ((p->N + g.bn - 1) / g.bn);
+  return 1;
+}
+
 int geeps_gemm_bf16(const GeepsGemmParams* p, void* stream) {
   if (!geeps_gemm_tc_supported(p)) return (int)cudaErrorInvalidValue;
   const int kSMs = geeps_sm_count();
-  // large K-major products go to CTA pairs (half the B traffic per SM) when 256-row tiles can fill the machine
-  if (p->block_n == 0 && p->split_k <= 1 && geeps_gemm_pair_supported(p) &&
-      ((p->M + 255) / 256) * ((p->N + 255) / 256) >= kSMs / 2)
-    return geeps_gemm_bf16_pair(p, stream);
+  if (takes_pairs(p, kSMs)) return geeps_gemm_bf16_pair(p, stream);
+  const GemmPlan plan = plan_gemm(p, kSMs);
+  const int bn = plan.bn, cluster = plan.cluster;
   const int m_tiles = (int)((p->M + BM - 1) / BM);
-  const int unit = p->b_mn_major ? 64 : 32;
   const int kt_total = (int)((p->K + BK - 1) / BK);
-  // tile width: as few N tiles as possible with little padding ...
-  // TMA-store epilogue: C 16-byte aligned with a 16-byte-multiple pitch, no read-modify-write of C
-  const int esz = p->out_fp32 ? 4 : 2;
-  const bool tma_c = (((uintptr_t)p->C & 15) == 0) && ((p->ldc * esz) % 16 == 0) && p->beta == 0.f;
-  int bn = p->block_n, cluster = 1;
-  if (bn <= 0 || bn > 256 || bn % unit) {
-    const long long nt = (p->N + 255) / 256;
-    bn = round_up((p->N + nt - 1) / nt, unit);
-    // ... but enough tiles to occupy every SM when the problem allows it
-    const bool can_split = p->split_k == 0 && p->out_fp32 && !p->relu && kt_total >= 16;
-    if (!can_split && (long long)m_tiles * ((p->N + bn - 1) / bn) < kSMs && p->N > 64) {
-      // a bf16 slab is 64 columns wide (see below): several tiles have widths that are multiples of it
-      const int step = tma_c && !p->out_fp32 ? 64 : unit;
-      // Clusters only for a long K over very few tiles (the data gradient of a wide classifier: 32 x 1024, K = 21841,
-      // 16 tiles: 76 -> 31 us).  Elsewhere they give less (256 x 4096, K = 9216: 40 -> 32 us) and every product would
-      // add its K slices in another order: in a deep network with near-ties in its pooling windows that changes which
-      // element a later step's maximum picks, so ordinary layers keep one running sum over K.
-      const bool cluster_ok = p->split_k <= 1 && p->beta == 0.f && kt_total >= 128 &&
-                              (long long)m_tiles * ((p->N + 63) / 64) <= kSMs / 8;
-      const TileChoice c = choose_tiles(p, step, kt_total, kSMs, cluster_ok);
-      if (c.cluster > 1 || c.bn < bn) { bn = c.bn; cluster = c.cluster; }
-    }
-  }
-  if (bn > 256) bn = 256;
-  // a bf16 slab is 64 columns wide: with several N tiles the tile width must be a multiple of it
-  if (tma_c && !p->out_fp32 && (bn % 64) && (p->N + bn - 1) / bn > 1) bn = round_up(bn, 64);
+  const bool tma_c = tma_c_ok(p);
   const long long n_tiles = (p->N + bn - 1) / bn;
   CUtensorMap ta, tb;
   bool ok = p->a_mn_major ? make_map(&ta, p->A, p->M, p->K, p->lda, 64, BK)
@@ -610,25 +667,8 @@ int geeps_gemm_bf16(const GeepsGemmParams* p, void* stream) {
   int tmem_cols = 32;
   while (tmem_cols < 2 * bn) tmem_cols <<= 1;
   d.tmem_cols = tmem_cols;
-  int split = p->split_k;
-  if (split == 0) {  // auto: occupy the SMs about twice over when the output has few tiles
-    split = 1;
-    const long long tiles = (long long)m_tiles * n_tiles;
-    if (p->out_fp32 && !p->relu && tiles < kSMs && d.kt_total >= 8) {
-      long long want = (2 * kSMs) / tiles;   // at most two full waves: one work item more would add a third round
-      long long cap = d.kt_total / 4;
-      split = (int)(want < cap ? want : cap);
-      if (split < 1) split = 1;
-    }
-  }
-  d.split_k = split < 1 ? 1 : (split > d.kt_total ? d.kt_total : split);
-  if (d.split_k > 1) {
-    // every k-slice must be non-empty, otherwise its tile would never be completed by an MMA commit
-    const int per = (d.kt_total + d.split_k - 1) / d.split_k;
-    d.split_k = (d.kt_total + per - 1) / per;
-  }
+  d.split_k = plan.split_k;
   d.cluster = cluster;
-  if (cluster > 1) d.split_k = cluster;
   if (d.split_k > 1 && cluster == 1) {
     // partial sums are accumulated with atomics: bring C to beta*C (or zero) first
     int e = geeps_scale_matrix_f32((float*)p->C, p->M, p->N, p->ldc, p->beta, stream);

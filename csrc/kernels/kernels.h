@@ -142,6 +142,11 @@ int geeps_gemm_tc_supported(const GeepsGemmParams* p);             // 1 if the t
 // CTA-pair variant (tcgen05 cta_group::2, 256-row tiles): K-major A and B, no split-K, beta == 0, M >= 256
 int geeps_gemm_bf16_pair(const GeepsGemmParams* p, void* stream);
 int geeps_gemm_pair_supported(const GeepsGemmParams* p);
+// How geeps_gemm_bf16 would cut this product on the current device (host arithmetic only): CTA pairs or not, tile width,
+// output tiles, K slices, and the CTAs of a cluster that hold the slices of one tile (1: slices meet in atomics).
+// Returns 0 if the tcgen05 path does not accept p.
+typedef struct GeepsGemmPlan { int pair, block_n, split_k, cluster; long long tiles; } GeepsGemmPlan;
+int geeps_gemm_plan(const GeepsGemmParams* p, GeepsGemmPlan* out);
 // C[m][n] = beta * C[m][n] (exactly 0 when beta == 0) over an M x N view with pitch ldc
 int geeps_scale_matrix_f32(float* c, long long M, long long N, long long ldc, float beta, void* stream);
 

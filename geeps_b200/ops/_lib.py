@@ -36,6 +36,10 @@ class ConvTcParams(C.Structure):
     ]
 
 
+class GemmPlan(C.Structure):
+    _fields_ = [("pair", C.c_int), ("block_n", C.c_int), ("split_k", C.c_int), ("cluster", C.c_int), ("tiles", C.c_longlong)]
+
+
 class HaloPlanInfo(C.Structure):
     _fields_ = [
         ("ok", C.c_int), ("routed", C.c_int),
