@@ -988,11 +988,14 @@ __device__ __forceinline__ void xform_image(const XformDev& t, long long b, int&
 // ---- S = 4, C = 3 space-to-depth, 8- and 16-bit sources ----
 // Two lanes make one output pixel (two image rows of four columns each): a lane fetches the four columns of a colour as
 // the one to three aligned 32-bit words that cover them, converts them in registers and builds three 16-byte pieces of
-// the pixel; a warp's 16 pixels meet in shared memory and leave as one contiguous run.  (One element per load and one
-// 2-byte shared-memory store per value, 32 pixels of one output row per block, took 62 us for 256 images of 8 bits and
-// left a tenth of the lanes without a pixel; this takes 47 us.  Bound by instruction issue and the 106 MB written.)
+// the pixel; a warp's 16 pixels meet in shared memory and leave as one contiguous run.  256 images of 8 bits, cropped to
+// 227 x 227: one element per load and 2-byte shared-memory stores, 32 pixels of one output row per block, 59 us; this
+// 34 us, of which the 106 MB written are 16.  Bound by instruction issue.
+// An 8-bit source may start and end inside a word (a batch slice, odd image sizes): the lanes whose words could reach past
+// it fetch by elements, every other lane by words (by elements throughout: 423 us).
 struct U8Quads {
   XformDev t;
+  const uint8_t* end;       // one past the source
   int h_off, w_off, mirror;
   __device__ __forceinline__ void image(long long b) { xform_image(t, b, h_off, w_off, mirror); }
   __device__ __forceinline__ int height() const { return t.H; }
@@ -1007,10 +1010,17 @@ struct U8Quads {
   __device__ __forceinline__ uint32_t one(long long b, int c, int h, int w) const {
     return bits(value(__ldg(row(b, c, h) + (mirror ? t.W - 1 - w : w)), c));
   }
-  // columns w .. w + 3 as two packed words; the words that hold them lie inside the tensor (the second is read only
-  // when it holds one of them)
+  __device__ __forceinline__ const uint8_t* quad_at(long long b, int c, int h, int w) const {
+    return row(b, c, h) + (mirror ? t.W - 4 - w : w);
+  }
+  // are all words around columns w .. w + 3 of rows h .. h1, every colour, inside the source?
+  __device__ __forceinline__ bool inside(long long b, int h, int h1, int w) const {
+    const uint8_t* first = quad_at(b, 0, h, w);
+    return first - ((uintptr_t)first & 3) >= t.x && end - quad_at(b, 2, h1, w) >= 8;
+  }
+  // columns w .. w + 3 as two packed words (the second word is read only when it holds one of the columns)
   __device__ __forceinline__ uint2 quad(long long b, int c, int h, int w) const {
-    const uint8_t* p = row(b, c, h) + (mirror ? t.W - 4 - w : w);
+    const uint8_t* p = quad_at(b, c, h, w);
     const uint32_t sh = (uint32_t)((uintptr_t)p & 3) * 8;
     const uint32_t* q = reinterpret_cast<const uint32_t*>((uintptr_t)p & ~(uintptr_t)3);
     const uint32_t lo = __ldg(q), hi = sh ? __ldg(q + 1) : 0u;
@@ -1029,6 +1039,7 @@ struct Bf16Quads {
   __device__ __forceinline__ uint32_t one(long long b, int c, int h, int w) const {
     return (uint32_t)__bfloat16_as_ushort(x[((b * 3 + c) * H + h) * (long long)W + w]);
   }
+  __device__ __forceinline__ bool inside(long long, int, int, int) const { return true; }   // whole words: see the launch
   __device__ __forceinline__ uint2 quad(long long b, int c, int h, int w) const {
     const bf16* p = x + ((b * 3 + c) * H + h) * (long long)W + w;
     const bool odd = ((uintptr_t)p & 2) != 0;
@@ -1042,7 +1053,7 @@ __global__ void __launch_bounds__(256)
 s2d43_quad_kernel(Src src, bf16* __restrict__ y, unsigned npix, int Hs, int Ws, int Cpad) {
   __shared__ uint4 tile[8][16 * 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane & 1, px = lane >> 1;
-  const unsigned base = (blockIdx.x * 8u + warp) * 16u;
+  const unsigned base = (blockIdx.x * (blockDim.x >> 5) + warp) * 16u;
   if (base >= npix) return;                       // whole warps: nothing below meets another warp
   const unsigned pix = base + px;
   const int per_pix = Cpad >> 3;
@@ -1053,30 +1064,48 @@ s2d43_quad_kernel(Src src, bf16* __restrict__ y, unsigned npix, int Hs, int Ws, 
     const unsigned row = pix / (unsigned)Ws, b = row / (unsigned)Hs;
     const int w = (int)(pix - row * Ws) * 4, h0 = (int)(row - b * Hs) * 4 + half * 2;
     src.image(b);
+    unsigned long long q[2][3];          // four columns of 16 bits
+    const int last = src.height() - 1, wq = min(w, src.width() - 4);
+    // All fetches of a lane are in flight together, then masked.  (A branch per colour that fetched the one to three
+    // columns of a ragged right edge waited for each: 256 images 45 us, 35 us without; one image 4.9 and 2.5 us.)
+    if (wq >= 0 && src.inside(b, min(h0, last), min(h0 + 1, last), wq)) {
+      const int shift = (w - wq) * 16;   // past the right edge: the last four columns, shifted
+#pragma unroll
+      for (int d = 0; d < 2; ++d)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const uint2 v = src.quad(b, c, min(h0 + d, last), wq);
+          q[d][c] = shift < 64 ? ((unsigned long long)v.y << 32 | v.x) >> shift : 0ull;
+        }
+    } else {
+      const int n = src.width() - w;
+      const unsigned long long keep = n >= 4 ? ~0ull : (n > 0 ? (1ull << (16 * n)) - 1 : 0ull);
+#pragma unroll
+      for (int d = 0; d < 2; ++d)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          unsigned long long v = 0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            v |= (unsigned long long)src.one(b, c, min(h0 + d, last), min(w + k, src.width() - 1)) << (16 * k);
+          q[d][c] = v & keep;
+        }
+    }
+    // interleave: column-major, colour fastest
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
-      const int h = h0 + d;
-      uint2 q[3];
+      uint32_t lo[3], hi[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        q[c] = make_uint2(0u, 0u);
-        if (h >= src.height()) continue;
-        if (w + 4 <= src.width()) {
-          q[c] = src.quad(b, c, h, w);
-        } else {
-          const int n = src.width() - w;          // ragged right edge: up to three columns
-          if (n > 0) q[c].x = src.one(b, c, h, w);
-          if (n > 1) q[c].x |= src.one(b, c, h, w + 1) << 16;
-          if (n > 2) q[c].y = src.one(b, c, h, w + 2);
-        }
+        lo[c] = h0 + d <= last ? (uint32_t)q[d][c] : 0u;
+        hi[c] = h0 + d <= last ? (uint32_t)(q[d][c] >> 32) : 0u;
       }
-      // interleave: column-major, colour fastest
-      o[6 * d + 0] = __byte_perm(q[0].x, q[1].x, 0x5410);
-      o[6 * d + 1] = __byte_perm(q[2].x, q[0].x, 0x7610);
-      o[6 * d + 2] = __byte_perm(q[1].x, q[2].x, 0x7632);
-      o[6 * d + 3] = __byte_perm(q[0].y, q[1].y, 0x5410);
-      o[6 * d + 4] = __byte_perm(q[2].y, q[0].y, 0x7610);
-      o[6 * d + 5] = __byte_perm(q[1].y, q[2].y, 0x7632);
+      o[6 * d + 0] = __byte_perm(lo[0], lo[1], 0x5410);
+      o[6 * d + 1] = __byte_perm(lo[2], lo[0], 0x7610);
+      o[6 * d + 2] = __byte_perm(lo[1], lo[2], 0x7632);
+      o[6 * d + 3] = __byte_perm(hi[0], hi[1], 0x5410);
+      o[6 * d + 4] = __byte_perm(hi[2], hi[0], 0x7610);
+      o[6 * d + 5] = __byte_perm(hi[1], hi[2], 0x7632);
     }
   }
   // pieces of a pixel XOR-ed with the pixel number: the 16-byte stores spread over the banks
@@ -1093,10 +1122,18 @@ s2d43_quad_kernel(Src src, bf16* __restrict__ y, unsigned npix, int Hs, int Ws, 
     dst[i] = tile[warp][p * 8 + (k ^ (p & 7))];
   }
 }
-// The word loads need a 4-byte aligned source that ends on a word; everything else takes the per-element kernels.
-inline bool s2d43_quads_ok(const void* x, long long src_bytes, const void* y, long long npix, int Cpad) {
-  return ((uintptr_t)x & 3) == 0 && src_bytes % 4 == 0 && ((uintptr_t)y & 15) == 0 && Cpad % 8 == 0 && Cpad >= 48 &&
-         Cpad <= 64 && npix > 0 && npix < 0x7fffff00LL;
+// what the kernel asks of the output and of the pixel count (its indexes are 32 bits wide)
+inline bool s2d43_quads_ok(const void* y, long long npix, int Cpad) {
+  return ((uintptr_t)y & 15) == 0 && Cpad % 8 == 0 && Cpad >= 48 && Cpad <= 64 && npix > 0 && npix < 0x7fffff00LL;
+}
+// Eight warps a block, fewer where that would leave SMs without a block (one image of 227 x 227: 26 blocks of eight).
+template <typename Src>
+void launch_s2d43_quads(const Src& src, void* y, long long npix, int Hs, int Ws, int Cpad, cudaStream_t st) {
+  const long long warps = (npix + 15) / 16;
+  long long per_block = warps / (2 * geeps_sm_count());
+  per_block = per_block < 1 ? 1 : (per_block > 8 ? 8 : per_block);
+  s2d43_quad_kernel<<<(unsigned)((warps + per_block - 1) / per_block), (unsigned)(32 * per_block), 0, st>>>(
+      src, (bf16*)y, (unsigned)npix, Hs, Ws, Cpad);
 }
 
 // any S >= 1 (S = 1: plain NHWC) and C <= 4: one thread per output element
@@ -1555,9 +1592,8 @@ static int nchw_to_s2d_launch(const T* x, void* y, int B, int C, int H, int W, i
                               cudaStream_t st) {
   if constexpr (sizeof(T) == 2) {
     const long long npix = (long long)B * Hs * Ws;
-    if (S == 4 && C == 3 && s2d43_quads_ok(x, (long long)B * 3 * H * W * 2, y, npix, Cpad)) {
-      Bf16Quads q{(const bf16*)x, H, W};
-      s2d43_quad_kernel<<<(unsigned)((npix + 127) / 128), 256, 0, st>>>(q, (bf16*)y, (unsigned)npix, Hs, Ws, Cpad);
+    if (S == 4 && C == 3 && s2d43_quads_ok(y, npix, Cpad) && ((uintptr_t)x & 3) == 0 && (long long)B * 3 * H * W % 2 == 0) {
+      launch_s2d43_quads(Bf16Quads{(const bf16*)x, H, W}, y, npix, Hs, Ws, Cpad, st);
       return CK();
     }
   }
@@ -1608,10 +1644,11 @@ int geeps_u8_transform_bf16(const GeepsU8Transform* p, void* stream) {
   t.scale = p->scale;
   cudaStream_t st = (cudaStream_t)stream;
   const long long npix = (long long)p->B * p->Hs * p->Ws;
-  if (S == 4 && p->C == 3 && s2d43_quads_ok(p->x, (long long)p->B * 3 * p->Hin * p->Win, p->y, npix, p->Cpad)) {
+  if (S == 4 && p->C == 3 && s2d43_quads_ok(p->y, npix, p->Cpad)) {
     U8Quads q;
     q.t = t;
-    s2d43_quad_kernel<<<(unsigned)((npix + 127) / 128), 256, 0, st>>>(q, (bf16*)p->y, (unsigned)npix, p->Hs, p->Ws, p->Cpad);
+    q.end = p->x + (long long)p->B * 3 * p->Hin * p->Win;
+    launch_s2d43_quads(q, p->y, npix, p->Hs, p->Ws, p->Cpad, st);
   } else {
     u8_xform_generic_kernel<<<grid_1d((long long)p->B * p->Hs * p->Ws * p->Cpad), 256, 0, st>>>(t, (bf16*)p->y, p->B, p->C,
                                                                                               S, p->Hs, p->Ws, p->Cpad);

@@ -291,7 +291,7 @@ def test_uint8_data_transformer_matches_torch(layout, mode):
 @pytest.mark.parametrize("mirror", [0, 1])
 def test_space_to_depth_of_8_and_16_bit_sources(B, H, W, cpad, mirror):
     """Rows that start on any byte, ragged right and lower edges, pixels of several rows in one warp, and a source whose
-    size is not a whole number of words (the per-element kernel)."""
+    size is not a whole number of words (16-bit: the kernel by elements; 8-bit: first and last words by bytes)."""
     from geeps_b200.ops import functional as F
     dev = torch.device("cuda:0")
     gen = torch.Generator(device=dev).manual_seed(H * W)
@@ -316,3 +316,53 @@ def test_space_to_depth_of_8_and_16_bit_sources(B, H, W, cpad, mirror):
         v = x[:, :, ho:ho + H, wo:wo + W].float()
         v = (v.flip(3) if mirror else v) - torch.tensor(mean, device=dev).view(3, 1, 1)
         assert torch.equal(y, ref(v * torch.tensor(scale, device=dev)))
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 4, 4), (2, 3, 2), (1, 5, 7), (2, 11, 13), (2, 6, 9), (3, 227, 227)])
+@pytest.mark.parametrize("off", [0, 1, 2, 3])
+def test_8_bit_sources_on_any_byte(B, H, W, off):
+    """A source that starts and ends on any byte, taken whole (the first and the last quad reach the tensor's ends), as
+    it is and mirrored; the bytes around it are another buffer's."""
+    from geeps_b200.ops import functional as F
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(B * H * W + off)
+    n = B * 3 * H * W
+    buf = torch.randint(0, 256, (n + 8,), device=dev, generator=gen, dtype=torch.uint8)
+    x = buf[off:off + n].view(B, 3, H, W)
+    Hs, Ws = -(-H // 4), -(-W // 4)
+    for mirror in (0, 1):
+        y = torch.full((B, Hs, Ws, 64), 9.0, dtype=torch.bfloat16, device=dev)
+        aug = torch.tensor([[0, 0, mirror]] * B, dtype=torch.int32, device=dev)
+        F.u8_transform(x, y, (H, W), 4, aug, (104.0, 117.0, 123.0), 1.0 / 58.0)
+        v = x.flip(3) if mirror else x
+        v = (v.float() - torch.tensor((104.0, 117.0, 123.0), device=dev).view(3, 1, 1)) * torch.tensor(1.0 / 58.0, device=dev)
+        p = torch.zeros(B, 3, Hs * 4, Ws * 4, device=dev)
+        p[:, :, :H, :W] = v
+        p = p.view(B, 3, Hs, 4, Ws, 4).permute(0, 2, 4, 3, 5, 1).reshape(B, Hs, Ws, 48)
+        assert torch.equal(y, torch.nn.functional.pad(p, (0, 16)).to(torch.bfloat16))
+
+
+def test_8_bit_sources_on_any_byte_take_the_fast_kernel():
+    """A source off a word boundary costs about what an aligned one does (by elements it cost seven times as much)."""
+    from geeps_b200.ops import functional as F
+    dev = torch.device("cuda:0")
+    B, H = 128, 227
+    n = B * 3 * H * H
+    buf = torch.zeros(n + 8, dtype=torch.uint8, device=dev)
+    y = torch.empty(B, 57, 57, 64, dtype=torch.bfloat16, device=dev)
+    aug = torch.zeros(B, 3, dtype=torch.int32, device=dev)
+
+    def ms(off):
+        x = buf[off:off + n].view(B, 3, H, H)
+        best = 1e9
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                F.u8_transform(x, y, (H, H), 4, aug, (104.0, 117.0, 123.0), 1.0 / 58.0)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+    aligned = ms(0)
+    assert ms(1) < 2.5 * aligned and ms(2) < 2.5 * aligned
