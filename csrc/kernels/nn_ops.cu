@@ -17,6 +17,7 @@ __device__ __forceinline__ float bf(const bf16 v) { return __bfloat162float(v); 
 
 struct alignas(16) Bf8 { bf16 v[8]; };
 __device__ __forceinline__ Bf8 ld8(const bf16* p) { Bf8 r; *reinterpret_cast<uint4*>(&r) = *reinterpret_cast<const uint4*>(p); return r; }
+__device__ __forceinline__ Bf8 zero8() { Bf8 r; *reinterpret_cast<uint4*>(&r) = make_uint4(0u, 0u, 0u, 0u); return r; }
 __device__ __forceinline__ void st8(bf16* p, const Bf8& r) { *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(&r); }
 
 // t = q * stride exactly?  Strides 1 and 2 (every layer of the supported nets but conv1) avoid the divider.
@@ -32,6 +33,22 @@ inline dim3 pool_block(int cv) {
   int bx = cv < 1 ? 1 : (cv > 256 ? 256 : cv);
   int by = 256 / bx;
   return dim3(bx, by < 1 ? 1 : by, 1);
+}
+
+// Average pooling: up to 256 threads as (8-channel vectors of a pixel) x (pixels of a row, in even shares where it takes
+// several blocks) x (rows, where two or more fit and `group` allows it).
+struct PoolGrid { dim3 grid, block; };
+inline PoolGrid avgpool_grid(int cv, int width, long long rows, bool group) {
+  const int bx = cv < 1 ? 1 : (cv > 256 ? 256 : cv), room = 256 / bx;
+  const int parts = (width + room - 1) / room;
+  const int by = (width + parts - 1) / parts;
+  long long bz = group ? 256 / (bx * by) : 1;
+  bz = bz > 64 ? 64 : (bz > rows ? rows : bz);
+  if (bz < 1) bz = 1;
+  PoolGrid g;
+  g.block = dim3((unsigned)bx, (unsigned)by, (unsigned)bz);
+  g.grid = dim3((unsigned)((rows + bz - 1) / bz), (unsigned)parts, 1);
+  return g;
 }
 
 inline int grid_1d(long long n, int block = 256, int cap = 0) {
@@ -1355,13 +1372,24 @@ __device__ __forceinline__ int avg_area(int o, int stride, int pad, int K, int s
   const int e = min(s + K, size + pad);
   return e - s;
 }
-// Block and thread map of the max pooling kernels: a block stays in one row of the tensor it writes, threadIdx.x the
-// 8-channel vectors of a pixel, threadIdx.y (and blockIdx.y) the pixels, so nothing is divided to find coordinates and only the windows that cover
-// a pixel are visited (a 64-bit division chain per vector was most of the 14 and 17.5 us on 32 x 14 x 14 x 576).
+// threadIdx.x is the 8-channel vector of a pixel and threadIdx.y (with blockIdx.y) the pixel, so nothing is divided to
+// find columns and only the windows that cover a pixel are visited (a 64-bit division chain per vector: 14 and 17.5 us on
+// 32 x 14 x 14 x 576, this 10 and 15).  A block stays in one row, whose coordinates and window rows are then the same for
+// all its threads (forward 17.5 us on 32 x 56 x 56 x 64, 21 with a row per thread).  ROWS: several rows per block, on
+// threadIdx.z, where a row has work for 128 threads or fewer and at most three windows (taps) per direction cover a pixel;
+// the loads of a window row are in flight together.  512 x 5 x 5 x 24, forward and backward: one row per 256 threads 8.1
+// and 10.8 us, one row per block of its size 4.5 and 5.7, this 2.8 and 3.4.  (Larger windows, such as the global pooling
+// at the end of a network, are bound by the taps of a thread: 100 x 8 x 8 x 336, one row 9.2 us, grouped 9.9.)
+template <bool ROWS>
+__device__ __forceinline__ unsigned pool_row() { return ROWS ? blockIdx.x * blockDim.z + threadIdx.z : blockIdx.x; }
+
+template <bool ROWS>
 __global__ void __launch_bounds__(256)
 avgpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const GeepsPoolGeom g) {
   const int cv = g.C >> 3;
-  const int oh = blockIdx.x % g.OH, b = blockIdx.x / g.OH;
+  const unsigned row = pool_row<ROWS>();
+  if (ROWS && row >= (unsigned)g.B * (unsigned)g.OH) return;
+  const int oh = row % g.OH, b = row / g.OH;
   const int ih0 = oh * g.stride - g.pad;
   const int kh_lo = max(0, -ih0), kh_hi = min(g.K, g.H - ih0);
   const int area_h = avg_area(oh, g.stride, g.pad, g.K, g.H);
@@ -1377,11 +1405,21 @@ avgpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const G
       for (int e = 0; e < 8; ++e) acc[e] = 0.f;
       for (int kh = kh_lo; kh < kh_hi; ++kh) {
         const bf16* xr = x + (((long long)b * g.H + ih0 + kh) * g.W + iw0) * g.ldx + c;
-#pragma unroll 3
-        for (int kw = kw_lo; kw < kw_hi; ++kw) {
-          const Bf8 v = ld8(xr + (long long)kw * g.ldx);
+        if (ROWS) {
+          Bf8 v[3];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) acc[e] += bf(v.v[e]);
+          for (int kw = 0; kw < 3; ++kw) v[kw] = kw >= kw_lo && kw < kw_hi ? ld8(xr + (long long)kw * g.ldx) : zero8();
+#pragma unroll
+          for (int kw = 0; kw < 3; ++kw)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] += bf(v[kw].v[e]);
+        } else {
+#pragma unroll 3
+          for (int kw = kw_lo; kw < kw_hi; ++kw) {
+            const Bf8 v = ld8(xr + (long long)kw * g.ldx);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] += bf(v.v[e]);
+          }
         }
       }
       Bf8 o;
@@ -1391,14 +1429,18 @@ avgpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const G
     }
   }
 }
+template <bool ROWS>
 __global__ void __launch_bounds__(256)
 avgpool_backward_kernel(const bf16* __restrict__ dy, bf16* __restrict__ dx, const GeepsPoolGeom g, int accumulate) {
   const int cv = g.C >> 3;
-  const int ih = blockIdx.x % g.H, b = blockIdx.x / g.H;
+  const unsigned row = pool_row<ROWS>();
+  if (ROWS && row >= (unsigned)g.B * (unsigned)g.H) return;
+  const int ih = row % g.H, b = row / g.H;
   const int th = ih + g.pad;
   // oh * stride <= th <= oh * stride + K - 1
   const int oh_lo = max(0, (th - g.K + g.stride) / g.stride), oh_hi = min(g.OH - 1, th / g.stride);
   bf16* drow = dx + ((long long)b * g.H + ih) * g.W * g.ldx;
+  const float inv_full = __frcp_rn((float)(g.K * g.K));
   for (int iw = blockIdx.y * blockDim.y + threadIdx.y; iw < g.W; iw += blockDim.y * gridDim.y) {
     const int tw = iw + g.pad;
     const int ow_lo = max(0, (tw - g.K + g.stride) / g.stride), ow_hi = min(g.OW - 1, tw / g.stride);
@@ -1410,12 +1452,25 @@ avgpool_backward_kernel(const bf16* __restrict__ dy, bf16* __restrict__ dx, cons
       for (int oh = oh_hi; oh >= oh_lo; --oh) {             // the order of the window rows and columns
         const int area_h = avg_area(oh, g.stride, g.pad, g.K, g.H);
         const bf16* src = dy + (((long long)b * g.OH + oh) * g.OW) * g.ldy + c;
-#pragma unroll 3
-        for (int ow = ow_hi; ow >= ow_lo; --ow) {
-          const float inv = __frcp_rn((float)(area_h * avg_area(ow, g.stride, g.pad, g.K, g.W)));
-          const Bf8 d = ld8(src + (long long)ow * g.ldy);
+        if (ROWS) {
+          Bf8 d[3];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) acc[e] += bf(d.v[e]) * inv;
+          for (int i = 0; i < 3; ++i) d[i] = ow_hi - i >= ow_lo ? ld8(src + (long long)(ow_hi - i) * g.ldy) : zero8();
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const int area = area_h * avg_area(ow_hi - i, g.stride, g.pad, g.K, g.W);
+            const float inv = area == g.K * g.K ? inv_full : ow_hi - i >= ow_lo ? __frcp_rn((float)area) : 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] += bf(d[i].v[e]) * inv;
+          }
+        } else {
+#pragma unroll 3
+          for (int ow = ow_hi; ow >= ow_lo; --ow) {
+            const float inv = __frcp_rn((float)(area_h * avg_area(ow, g.stride, g.pad, g.K, g.W)));
+            const Bf8 d = ld8(src + (long long)ow * g.ldy);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] += bf(d.v[e]) * inv;
+          }
         }
       }
       bf16* dst = drow + (long long)iw * g.ldx + c;
@@ -1958,16 +2013,28 @@ int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const G
       (const bf16*)dy, (const uint8_t*)argmax, (bf16*)dx, *g, accumulate);
   return CK();
 }
+int geeps_avgpool_blocks(int C, int width, long long rows, int group, int* out) {
+  const PoolGrid g = avgpool_grid(C / 8, width, rows, group != 0);
+  const unsigned v[5] = {g.grid.x, g.grid.y, g.block.x, g.block.y, g.block.z};
+  for (int i = 0; i < 5; ++i) out[i] = (int)v[i];
+  return 0;
+}
 int geeps_avgpool_forward(const void* x, void* y, const GeepsPoolGeom* g, void* stream) {
   if (g->C % 8 || g->ldx % 8 || g->ldy % 8) return (int)cudaErrorInvalidValue;
-  const dim3 blk = pool_block(g->C / 8);
-  avgpool_forward_kernel<<<dim3(g->B * g->OH, (g->OW + blk.y - 1) / blk.y), blk, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, *g);
+  const PoolGrid pg = avgpool_grid(g->C / 8, g->OW, (long long)g->B * g->OH, g->K <= 3);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (pg.block.z == 1) avgpool_forward_kernel<false><<<pg.grid, pg.block, 0, st>>>((const bf16*)x, (bf16*)y, *g);
+  else avgpool_forward_kernel<true><<<pg.grid, pg.block, 0, st>>>((const bf16*)x, (bf16*)y, *g);
   return CK();
 }
 int geeps_avgpool_backward(const void* dy, void* dx, const GeepsPoolGeom* g, int accumulate, void* stream) {
   if (g->C % 8 || g->ldx % 8 || g->ldy % 8) return (int)cudaErrorInvalidValue;
-  const dim3 blk = pool_block(g->C / 8);
-  avgpool_backward_kernel<<<dim3(g->B * g->H, (g->W + blk.y - 1) / blk.y), blk, 0, (cudaStream_t)stream>>>((const bf16*)dy, (bf16*)dx, *g, accumulate);
+  const PoolGrid pg = avgpool_grid(g->C / 8, g->W, (long long)g->B * g->H, g->K <= 3 * g->stride);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (pg.block.z == 1)
+    avgpool_backward_kernel<false><<<pg.grid, pg.block, 0, st>>>((const bf16*)dy, (bf16*)dx, *g, accumulate);
+  else
+    avgpool_backward_kernel<true><<<pg.grid, pg.block, 0, st>>>((const bf16*)dy, (bf16*)dx, *g, accumulate);
   return CK();
 }
 

@@ -112,6 +112,9 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
 int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream);
 int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const GeepsPoolGeom* g, int accumulate,
                            void* stream);
+// launch shape of the average pooling kernels (host arithmetic only): grid x, y, block x (vectors), y (pixels), z (rows);
+// group: at most three windows per direction cover a pixel
+int geeps_avgpool_blocks(int C, int width, long long rows, int group, int* out);
 int geeps_avgpool_forward(const void* x, void* y, const GeepsPoolGeom* g, void* stream);
 int geeps_avgpool_backward(const void* dy, void* dx, const GeepsPoolGeom* g, int accumulate, void* stream);
 int geeps_softmax_ce(const float* logits, const long long* labels, float* loss_sum, float* per_sample,

@@ -495,3 +495,25 @@ def test_batchnorm_backward_from_mask_bits_equals_the_one_from_the_output(P, Cc)
     # the sums of the blocks meet in any order: last digits of fp32, and the bf16 rounding they may tip
     assert torch.allclose(got[0][0].float(), got[1][0].float(), atol=1e-5, rtol=2.0 ** -7)
     assert torch.allclose(got[0][1], got[1][1], atol=1e-4, rtol=1e-4) and torch.allclose(got[0][2], got[1][2], atol=1e-4, rtol=1e-4)
+
+
+@pytest.mark.parametrize("B,H,W,Cc,k,stride,pad", [(40, 5, 5, 24, 3, 1, 1), (3, 1, 1, 8, 1, 1, 0), (5, 4, 4, 8, 2, 2, 0),
+                                                   (2, 9, 257, 8, 3, 2, 1), (2, 3, 130, 16, 3, 1, 1), (1, 5, 3, 2056, 3, 1, 1), (3, 9, 9, 16, 5, 1, 2),
+                                                   (2, 7, 7, 1024, 7, 1, 0), (4, 8, 8, 40, 5, 2, 2)])
+def test_average_pooling_over_launch_shapes(B, H, W, Cc, k, stride, pad):
+    """Several rows in a block (with a ragged last block), rows in even shares over two blocks, more vectors than threads;
+    windows of up to three taps per direction and more."""
+    torch.manual_seed(H * W + Cc)
+    x = torch.randn(B, H, W, Cc, device=DEV).to(BF)
+    g = F.pool_geom(x.shape, k, stride, pad, Cc, Cc, ceil_mode=False)
+    y = torch.empty(B, g.OH, g.OW, Cc, dtype=BF, device=DEV)
+    F.avgpool_forward(x, y, g)
+    dy = torch.randn_like(y)
+    dx = torch.empty_like(x)
+    F.avgpool_backward(dy, dx, g)
+    xr = x.double().permute(0, 3, 1, 2).contiguous().requires_grad_(True)      # NCHW-contiguous reference
+    ref = TF.avg_pool2d(xr, k, stride, pad)
+    ref.backward(dy.double().permute(0, 3, 1, 2).contiguous())
+    # one rounding to bf16 of fp32 sums of at most 9 terms
+    assert torch.allclose(y.double(), ref.detach().permute(0, 2, 3, 1), atol=1e-5, rtol=2.0 ** -8)
+    assert torch.allclose(dx.double(), xr.grad.permute(0, 2, 3, 1), atol=1e-5, rtol=2.0 ** -8)

@@ -1,0 +1,20 @@
+"""Launch shapes of the element-wise and pooling kernels (host arithmetic only, no GPU)."""
+import ctypes as C
+import itertools
+
+from geeps_b200.ops import _lib as L
+
+
+def test_average_pooling_blocks_cover_the_rows_and_are_full():
+    for Cc, width, rows, group in itertools.product((8, 24, 96, 576, 1024, 2048, 2056), (1, 2, 4, 5, 7, 13, 14, 56, 224, 257, 513),
+                                                    (1, 2, 5, 64, 448, 2560), (0, 1)):
+        out = (C.c_int * 5)()
+        L.lib().geeps_avgpool_blocks(Cc, width, C.c_longlong(rows), group, out)
+        gx, gy, bx, by, bz = out
+        assert bx == min(Cc // 8, 256) and bx * by * bz <= 256 and 1 <= bz <= (64 if group else 1)
+        assert gx * bz >= rows and (gx - 1) * bz < rows              # every row once, no empty block
+        assert gy * by >= width and (gy - 1) * by < width            # every pixel once, no empty block
+        # threads that have a pixel, of all in the launched warps, where there is work for more than one block
+        if rows * width * bx >= 512 and (group or width * bx >= 16):
+            launched = gx * gy * -(-bx * by * bz // 32) * 32
+            assert rows * width * bx >= 0.5 * launched, (Cc, width, rows, list(out))
