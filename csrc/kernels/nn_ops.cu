@@ -37,8 +37,10 @@ inline dim3 pool_block(int cv) {
 
 // Average pooling: up to 256 threads as (8-channel vectors of a pixel) x (pixels of a row, in even shares where it takes
 // several blocks) x (rows, where two or more fit and `group` allows it).
+// No rows or no pixels: an empty grid, nothing to launch.
 struct PoolGrid { dim3 grid, block; };
 inline PoolGrid avgpool_grid(int cv, int width, long long rows, bool group) {
+  if (rows <= 0 || width <= 0) return {dim3(0, 0, 0), dim3(0, 0, 0)};
   const int bx = cv < 1 ? 1 : (cv > 256 ? 256 : cv), room = 256 / bx;
   const int parts = (width + room - 1) / room;
   const int by = (width + parts - 1) / parts;
@@ -47,7 +49,7 @@ inline PoolGrid avgpool_grid(int cv, int width, long long rows, bool group) {
   if (bz < 1) bz = 1;
   PoolGrid g;
   g.block = dim3((unsigned)bx, (unsigned)by, (unsigned)bz);
-  g.grid = dim3((unsigned)((rows + bz - 1) / bz), (unsigned)parts, 1);
+  g.grid = dim3((unsigned)((rows + bz - 1) / bz), (unsigned)(parts > 65535 ? 65535 : parts), 1);   // the kernels stride over y
   return g;
 }
 
@@ -2023,6 +2025,7 @@ int geeps_avgpool_forward(const void* x, void* y, const GeepsPoolGeom* g, void* 
   if (g->C % 8 || g->ldx % 8 || g->ldy % 8) return (int)cudaErrorInvalidValue;
   const PoolGrid pg = avgpool_grid(g->C / 8, g->OW, (long long)g->B * g->OH, g->K <= 3);
   cudaStream_t st = (cudaStream_t)stream;
+  if (pg.grid.x == 0) return 0;
   if (pg.block.z == 1) avgpool_forward_kernel<false><<<pg.grid, pg.block, 0, st>>>((const bf16*)x, (bf16*)y, *g);
   else avgpool_forward_kernel<true><<<pg.grid, pg.block, 0, st>>>((const bf16*)x, (bf16*)y, *g);
   return CK();
@@ -2031,6 +2034,7 @@ int geeps_avgpool_backward(const void* dy, void* dx, const GeepsPoolGeom* g, int
   if (g->C % 8 || g->ldx % 8 || g->ldy % 8) return (int)cudaErrorInvalidValue;
   const PoolGrid pg = avgpool_grid(g->C / 8, g->W, (long long)g->B * g->H, g->K <= 3 * g->stride);
   cudaStream_t st = (cudaStream_t)stream;
+  if (pg.grid.x == 0) return 0;
   if (pg.block.z == 1)
     avgpool_backward_kernel<false><<<pg.grid, pg.block, 0, st>>>((const bf16*)dy, (bf16*)dx, *g, accumulate);
   else

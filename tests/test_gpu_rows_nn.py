@@ -517,3 +517,18 @@ def test_average_pooling_over_launch_shapes(B, H, W, Cc, k, stride, pad):
     # one rounding to bf16 of fp32 sums of at most 9 terms
     assert torch.allclose(y.double(), ref.detach().permute(0, 2, 3, 1), atol=1e-5, rtol=2.0 ** -8)
     assert torch.allclose(dx.double(), xr.grad.permute(0, 2, 3, 1), atol=1e-5, rtol=2.0 ** -8)
+
+
+def test_average_pooling_of_an_empty_batch_and_of_very_wide_rows():
+    x = torch.empty(0, 6, 6, 16, dtype=BF, device=DEV)
+    g = F.pool_geom(x.shape, 3, 1, 1, 16, 16)
+    y = torch.empty(0, g.OH, g.OW, 16, dtype=BF, device=DEV)
+    F.avgpool_forward(x, y, g)
+    F.avgpool_backward(y, x, g)
+    W = 65540                                                        # more pixels in a row than the grid's second dimension
+    x = torch.randn(1, 1, W, 2048, device=DEV).to(BF)
+    g = F.pool_geom(x.shape, 1, 1, 0, 2048, 2048)
+    y, dx = torch.empty_like(x), torch.empty_like(x)
+    F.avgpool_forward(x, y, g)
+    F.avgpool_backward(y, dx, g)
+    assert torch.equal(y, x) and torch.equal(dx, x)

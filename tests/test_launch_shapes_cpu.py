@@ -18,3 +18,12 @@ def test_average_pooling_blocks_cover_the_rows_and_are_full():
         if rows * width * bx >= 512 and (group or width * bx >= 16):
             launched = gx * gy * -(-bx * by * bz // 32) * 32
             assert rows * width * bx >= 0.5 * launched, (Cc, width, rows, list(out))
+
+
+def test_average_pooling_of_nothing_and_of_very_wide_rows():
+    out = (C.c_int * 5)()
+    for Cc, width, rows in ((64, 7, 0), (64, 0, 7), (0, 7, 7)):
+        L.lib().geeps_avgpool_blocks(Cc, width, C.c_longlong(rows), 1, out)
+        assert (out[0] == 0) == (width * rows == 0)
+    L.lib().geeps_avgpool_blocks(2048, 70000, C.c_longlong(3), 1, out)
+    assert list(out) == [3, 65535, 256, 1, 1]                        # the second grid dimension has 16 bits
