@@ -189,40 +189,50 @@ col2im_kernel(const bf16* __restrict__ dcol, bf16* __restrict__ dx, const GeepsC
 // pixel it visits: per-channel constants are loaded once, sums stay in registers, and no item costs an integer
 // division (bn_apply spent most of its 77 us on a 32 x 56 x 56 x 192 tensor there and on reloading its six
 // constants per channel).
-// A row of threads reads whole contiguous pixels.  gridDim.y splits C above 2048 channels.
+// A row of threads reads whole contiguous pixels.  Above 1024 channels the blocks of gridDim.x share the channels, 512 or
+// fewer each, neighbouring blocks the same pixels.
 struct SlotMap {
   int cvb, rows, row, slot, c;     // slots per block, pixel rows per block, this thread's row / slot / first channel
   bool on;
   long long p0, step;              // first pixel, pixels between two of this thread
   __device__ __forceinline__ explicit SlotMap(int C) {
     const int cv = C >> 3;
-    cvb = (cv + (int)gridDim.y - 1) / (int)gridDim.y;
+    cvb = (cv + (int)gridDim.x - 1) / (int)gridDim.x;
     rows = (int)blockDim.x / cvb;
     row = (int)threadIdx.x / cvb;
     slot = (int)threadIdx.x - row * cvb;
-    const int gslot = (int)blockIdx.y * cvb + slot;
+    const int gslot = (int)blockIdx.x * cvb + slot;
     c = gslot * 8;
     on = row < rows && gslot < cv;
-    p0 = (long long)blockIdx.x * rows + row;
-    step = (long long)gridDim.x * rows;
+    p0 = (long long)blockIdx.y * rows + row;
+    step = (long long)gridDim.y * rows;
   }
 };
 struct SlotGrid { dim3 grid; int threads; size_t smem; };
-// Launch shape: 256-ish threads as rows x slots, about `per_thread` pixels a thread (one batch of loads in flight),
-// at most `per_sm` blocks per SM.  smem: the block's partial sums, nq floats per channel and pixel row.
+// Launch shape: 256-ish threads as rows x slots, about `per_thread` pixels a thread (one batch of loads in flight), one
+// pixel where more would leave seven SMs in eight without a block, at most `per_sm` blocks per SM.  smem: the block's
+// partial sums, nq floats per channel and pixel row.
+// At most 64 slots a block above 128: a block then has four rows or more, whose sums meet before they go to memory, and
+// nearly all of its threads a slot (one row of 161 slots leaves 31 of 192 idle).  Against one row of up to 256 slots:
+// column sums of 100352 x 1032 55 -> 39 us, ReLU mask + sums of 20000 x 1288 42 -> 32 us, BatchNorm backward of 32 x 4096
+// 12.5 -> 6.1 us, of 3000 x 2056 35 -> 22 us; up to 128 slots a block lie between the two.  (Mask + sums of
+// 100352 x 1032 109 -> 114 us, bound by DRAM.)
 inline SlotGrid slot_grid(long long P, int C, int per_thread, int per_sm, int nq) {
   const int cv = C / 8 < 1 ? 1 : C / 8;
   SlotGrid g;
-  const int chunks = (cv + 255) / 256;
+  const int chunks = cv <= 128 ? 1 : (cv + 63) / 64;                // block columns
   const int cvb = (cv + chunks - 1) / chunks;
-  const int rows = cvb >= 256 ? 1 : 256 / cvb;
+  const int rows = 256 / cvb;
   g.threads = (rows * cvb + 31) / 32 * 32;
   const int rows_used = g.threads / cvb;        // as SlotMap computes it
-  long long want = (P + (long long)rows_used * per_thread - 1) / ((long long)rows_used * per_thread);
+  const long long one_each = (P + rows_used - 1) / rows_used;      // blocks at one pixel a thread
+  const long long fill = geeps_sm_count() / chunks;
+  long long want = (one_each + per_thread - 1) / per_thread;
+  if (want * 8 < fill) want = one_each < fill ? one_each : fill;
   const long long cap = (long long)geeps_sm_count() * per_sm / chunks;
   if (want > cap) want = cap;
   if (want < 1) want = 1;
-  g.grid = dim3((unsigned)want, (unsigned)chunks, 1);
+  g.grid = dim3((unsigned)chunks, (unsigned)want, 1);
   g.smem = (size_t)rows_used * cvb * 8 * nq * sizeof(float);
   return g;
 }
@@ -247,7 +257,7 @@ __device__ __forceinline__ void slot_sums(const SlotMap& m, const float (&a0)[8]
     float v = 0.f;
     for (int r = 0; r < m.rows; ++r) v += part[(size_t)r * width * NQ + i];
     const int q = NQ == 2 && i >= width ? 1 : 0;
-    const int ch = (int)blockIdx.y * width + i - q * width;
+    const int ch = (int)blockIdx.x * width + i - q * width;
     if (ch < C) atomicAdd(out + (size_t)q * C + ch, v * scale);
   }
 }
@@ -257,7 +267,7 @@ __device__ __forceinline__ void slot_sums(const SlotMap& m, const float (&a0)[8]
 // lane) they were 39 of the 52 us of a 32 x 56 x 56 x 192 normalisation.
 template <int N, typename Fn>
 __device__ __forceinline__ void slot_consts(const SlotMap& s, int C, float* sh, float (&v)[N][8], Fn fn) {
-  const int width = s.cvb * 8, c0 = (int)blockIdx.y * width;
+  const int width = s.cvb * 8, c0 = (int)blockIdx.x * width;
   for (int i = threadIdx.x; i < width && c0 + i < C; i += blockDim.x) {
     float o[N];
     fn(c0 + i, o);
@@ -311,7 +321,9 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
         for (int e = 0; e < 8; ++e) { const float f = bf(xv.v[e]); a0[e] += f; if (MODE == 0) a1[e] += f * f; }
       }
     };
-    constexpr int U = 4;              // pixels whose loads are in flight together
+    // pixels whose loads are in flight together; two where there are three tensors to load: four took 153 registers, one
+    // block per SM (BatchNorm backward of 100352 x 192 by its output 73 us, 56 now)
+    constexpr int U = MODE == 1 ? 2 : 4;
     long long p = m.p0;
     for (; p + (U - 1) * m.step < P; p += U * m.step) {
       Bf8 xv[U], dv[U], yv[U];
@@ -343,7 +355,7 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
   slot_sums<MODE == 2 ? 1 : 2>(m, a0, a1, out, C, MODE == 2 ? scale : 1.f, sacc);
 }
 template <int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 channel_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                       const float* __restrict__ mean_rstd, float* __restrict__ out, long long P, int C,
                       long long ldx, long long lddy, int relu, float scale) {
@@ -448,7 +460,7 @@ __device__ __forceinline__ void bn_apply_fused_body(const bf16* __restrict__ x, 
     const float var = fmaxf(sums[C + c] * inv_count - m * m, 0.f);
     const float r = rsqrtf(var + eps);
     o[0] = m; o[1] = r * gamma[c]; o[2] = beta[c];
-    if (blockIdx.x == 0 && P > 0) {
+    if (blockIdx.y == 0 && P > 0) {
       mean_rstd[c] = m;
       mean_rstd[C + c] = r;
       if (running_mean) {
@@ -487,7 +499,7 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
   slot_consts(s, C, sacc, q, [&](int c, float (&o)[4]) {
     const float rs = mean_rstd[C + c], s0 = sums[c], s1 = sums[C + c];
     o[0] = mean_rstd[c]; o[1] = gamma[c] * rs; o[2] = s0 * invP; o[3] = rs * (s1 * invP);
-    if (blockIdx.x == 0) {
+    if (blockIdx.y == 0) {
       if (dbeta) dbeta[c] = s0 * grad_scale;
       if (dgamma) dgamma[c] = s1 * grad_scale;
       // the scratch of this layer's next forward reduction (nobody reads it during the backward pass)
@@ -505,7 +517,7 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
     }
     return o;
   };
-  constexpr int U = 4;
+  constexpr int U = BITS ? 4 : 2;
   long long p = s.p0;
   for (; p + (U - 1) * s.step < P; p += U * s.step) {
     Bf8 xv[U], dv[U], yv[U];
@@ -527,7 +539,7 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
   }
 }
 template <bool BITS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 bn_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                    bf16* __restrict__ dx, const float* __restrict__ mean_rstd, const float* __restrict__ gamma,
                    const float* __restrict__ sums, float* dgamma, float* dbeta, long long P, int C,
@@ -1747,7 +1759,7 @@ static SlotGrid reduce_grid(long long P, int C, int nq = 2) { return slot_grid(P
 // element-wise passes with per-channel constants: up to eight blocks per SM
 static SlotGrid apply_grid(long long P, int C) {
   SlotGrid g = slot_grid(P, C, 4, 8, 0);
-  g.smem = ((size_t)(C / 8) + g.grid.y - 1) / g.grid.y * 8 * 4 * sizeof(float);      // four constants per channel
+  g.smem = ((size_t)(C / 8) + g.grid.x - 1) / g.grid.x * 8 * 4 * sizeof(float);      // four constants per channel
   return g;
 }
 
@@ -2014,6 +2026,11 @@ int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const G
   maxpool_backward_kernel<<<g->B * g->H, pool_block(g->C / 8), 0, (cudaStream_t)stream>>>(
       (const bf16*)dy, (const uint8_t*)argmax, (bf16*)dx, *g, accumulate);
   return CK();
+}
+int geeps_channel_blocks(long long P, int C, int* out) {
+  const SlotGrid g = slot_grid(P, C, 4, 4, 2);
+  out[0] = (int)g.grid.x; out[1] = (int)g.grid.y; out[2] = g.threads; out[3] = (int)g.smem;
+  return 0;
 }
 int geeps_avgpool_blocks(int C, int width, long long rows, int group, int* out) {
   const PoolGrid g = avgpool_grid(C / 8, width, rows, group != 0);

@@ -112,6 +112,9 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
 int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream);
 int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const GeepsPoolGeom* g, int accumulate,
                            void* stream);
+// launch shape of a reduction over P pixels of C channels (host arithmetic only): channel shares, pixel shares, threads a
+// block, bytes of shared memory
+int geeps_channel_blocks(long long P, int C, int* out);
 // launch shape of the average pooling kernels (host arithmetic only): grid x, y, block x (vectors), y (pixels), z (rows);
 // group: at most three windows per direction cover a pixel
 int geeps_avgpool_blocks(int C, int width, long long rows, int group, int* out);

@@ -380,9 +380,10 @@ def test_linear_with_the_k_range_split_over_the_sms_matches_fp32(relu, fp32_out,
     torch.cuda.synchronize()
 
 
-@pytest.mark.parametrize("P,Cc", [(1, 8), (3, 24), (777, 64), (129, 104), (1000, 1600), (37, 2056), (6, 4096)])
+@pytest.mark.parametrize("P,Cc", [(1, 8), (3, 24), (777, 64), (129, 104), (1000, 1600), (37, 2056), (6, 4096),
+                                  (1, 1032), (90, 1024), (9, 1032), (50, 2048), (2500, 1288)])
 def test_channel_kernels_at_the_edges_of_their_thread_map(P, Cc):
-    """One row to more rows than a batch of loads, slots that do not divide a block, C split over two block columns."""
+    """One row to more rows than a batch of loads, slots that do not divide a block, C split over several block columns."""
     torch.manual_seed(P + Cc)
     x, dy = torch.randn(P, Cc, device=DEV).to(BF), torch.randn(P, Cc, device=DEV).to(BF)
     x64, dy64 = x.double(), dy.double()

@@ -27,3 +27,20 @@ def test_average_pooling_of_nothing_and_of_very_wide_rows():
         assert (out[0] == 0) == (width * rows == 0)
     L.lib().geeps_avgpool_blocks(2048, 70000, C.c_longlong(3), 1, out)
     assert list(out) == [3, 65535, 256, 1, 1]                        # the second grid dimension has 16 bits
+
+
+def test_channel_blocks_cover_the_matrix_and_spread_few_pixels():
+    for P, Cc in itertools.product((1, 3, 8, 32, 49, 100, 392, 1568, 20000, 100352, 1000000),
+                                   (8, 24, 64, 192, 576, 1000, 1024, 1032, 1288, 1536, 2040, 2048, 2056, 4096, 8192)):
+        out = (C.c_int * 4)()
+        L.lib().geeps_channel_blocks(C.c_longlong(P), Cc, out)
+        cols, blocks, threads, smem = out
+        cv = Cc // 8
+        cvb = -(-cv // cols)                          # slots of a block, as the kernels compute them
+        rows = threads // cvb
+        assert threads % 32 == 0 and threads <= 256 and rows >= 1 and (cols - 1) * cvb < cv
+        assert smem == rows * cvb * 8 * 2 * 4 <= 32 * 1024
+        assert cols * blocks <= 148 * 4
+        assert rows * cv >= 0.75 * cols * threads, (P, Cc, list(out))         # threads with a slot
+        # few pixels: an eighth of the SMs at least, or a block for every batch of rows
+        assert cols * blocks >= min(148 // 8, cols * -(-P // rows)), (P, Cc, list(out))
