@@ -682,23 +682,28 @@ relu_backward_colsum_kernel(const bf16* __restrict__ dy, const bf16* __restrict_
 }
 // dst += the sum of N sources over 2-D views (branch gradients): one pass and one rounding for up to three of them
 struct AddSrc { const bf16* p[3]; long long ld[3]; };
-template <int N>
+// One vector per thread and step over the whole matrix; a dense one (every pitch equal to C) needs no coordinates.  Bound
+// by memory.  One source of 6272 x 576: a 64-bit division per vector 4.2 us, a thread that keeps its channels (and its
+// pixels one after the other) 5.1, this 3.7, pitched 4.1; three sources 5.1 -> 3.7 us.
+template <int N, bool DENSE>
 __global__ void __launch_bounds__(256)
-add_2d_kernel(bf16* __restrict__ dst, const AddSrc src, long long P, int C, long long ldd) {
-  const SlotMap m(C);
-  if (!m.on) return;
-  for (long long p = m.p0; p < P; p += m.step) {
-    Bf8 a = ld8(dst + p * ldd + m.c), v[N], o;
+add_2d_kernel(bf16* __restrict__ dst, const AddSrc src, long long total, int cv, long long ldd) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    // a pixel number of 32 bits is found by a 32-bit division
+    const long long p = DENSE ? 0 : (total <= 0xffffffffLL ? (long long)((unsigned)i / (unsigned)cv) : i / cv);
+    const long long c = (i - p * cv) * 8;
+    Bf8 a = ld8(dst + p * ldd + c), v[N], o;
 #pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = ld8(src.p[i] + p * src.ld[i] + m.c);
+    for (int n = 0; n < N; ++n) v[n] = ld8(src.p[n] + p * src.ld[n] + c);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       float f = bf(a.v[e]);
 #pragma unroll
-      for (int i = 0; i < N; ++i) f += bf(v[i].v[e]);
+      for (int n = 0; n < N; ++n) f += bf(v[n].v[e]);
       o.v[e] = __float2bfloat16(f);
     }
-    st8(dst + p * ldd + m.c, o);
+    st8(dst + p * ldd + c, o);
   }
 }
 
@@ -1935,11 +1940,14 @@ int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s
   if (C % 8 || ldd % 8 || ld0 % 8 || (n > 1 && ld1 % 8) || (n > 2 && ld2 % 8) || !s0 || (s2 && !s1))
     return (int)cudaErrorInvalidValue;
   const AddSrc src = {{(const bf16*)s0, (const bf16*)s1, (const bf16*)s2}, {ld0, ld1, ld2}};
-  const SlotGrid g = slot_grid(P, C, 1, 16, 0);
+  const long long total = P * (C / 8);
+  const bool dense = ldd == C && ld0 == C && (n < 2 || ld1 == C) && (n < 3 || ld2 == C);
+  const int grid = grid_1d(total);
   cudaStream_t st = (cudaStream_t)stream;
-  if (n == 3) add_2d_kernel<3><<<g.grid, g.threads, 0, st>>>((bf16*)dst, src, P, C, ldd);
-  else if (n == 2) add_2d_kernel<2><<<g.grid, g.threads, 0, st>>>((bf16*)dst, src, P, C, ldd);
-  else add_2d_kernel<1><<<g.grid, g.threads, 0, st>>>((bf16*)dst, src, P, C, ldd);
+#define ADD_2D(N, DENSE) add_2d_kernel<N, DENSE><<<grid, 256, 0, st>>>((bf16*)dst, src, total, C / 8, ldd)
+  if (dense) { if (n == 3) ADD_2D(3, true); else if (n == 2) ADD_2D(2, true); else ADD_2D(1, true); }
+  else { if (n == 3) ADD_2D(3, false); else if (n == 2) ADD_2D(2, false); else ADD_2D(1, false); }
+#undef ADD_2D
   return CK();
 }
 int geeps_add_bf16_2d(void* dst, const void* src, long long P, int C, long long ldd, long long lds, void* stream) {

@@ -533,3 +533,17 @@ def test_average_pooling_of_an_empty_batch_and_of_very_wide_rows():
     F.avgpool_forward(x, y, g)
     F.avgpool_backward(y, dx, g)
     assert torch.equal(y, x) and torch.equal(dx, x)
+
+
+@pytest.mark.parametrize("P,Cc", [(1, 8), (5, 24), (300, 1032), (2000, 2056)])
+@pytest.mark.parametrize("pitched", [(False, False), (True, False), (False, True), (True, True)])
+def test_sums_of_dense_and_pitched_matrices(P, Cc, pitched):
+    torch.manual_seed(P)
+    full = [torch.randn(P, Cc + (16 if p else 0), device=DEV).to(BF) for p in (*pitched, False)]
+    dst, s0, s1 = (t[:, 8:8 + Cc] if t.shape[1] > Cc else t for t in full)
+    edges = full[0].clone()
+    ref = (dst.double() + s0.double() + s1.double()).to(BF).double()
+    F.add_2d_n(dst, [s0, s1])
+    assert torch.allclose(dst.double(), ref, atol=0, rtol=2.0 ** -7)      # fp32 sum: at most the other neighbour
+    if pitched[0]:
+        assert torch.equal(full[0][:, :8], edges[:, :8]) and torch.equal(full[0][:, 8 + Cc:], edges[:, 8 + Cc:])
