@@ -606,6 +606,17 @@ bool lp_shape_ok(const GeepsPoolGeom* g, int size) {
 constexpr size_t kLpMaxSmem = 200 * 1024;
 constexpr size_t kLpTwoPerSm = 112 * 1024;    // two CTAs of this size share one SM's shared memory
 
+// Lanes per pixel and 8-channel vectors per lane of the register kernel.  Two thirds of the vector slots are used at every
+// channel count (64 x 55 x 55 x 264, 33 vectors: 206 us on 32 x 2 slots, 150 on 16 x 3; x 8, one vector, without column
+// sums: 19.7 us on 4 x 1, 6.4 on 1 x 1; x 40: 31 us on 4 x 2, 21.5 on 2 x 3; the general kernel takes 177, 14.0 and 30),
+// but where that leaves an SM fewer than eight warps more lanes share a pixel (2 x 27 x 27 x 40: 9.8 us on 2 x 3, 8.3 on 4 x 2).
+struct LrnLanes { int lp, nv; };
+LrnLanes lrn_lanes(int cv, long long pixels) {
+  int lp = cv <= 1 ? 1 : cv == 2 || cv == 5 || cv == 6 ? 2 : cv <= 12 ? 4 : cv <= 24 ? 8 : cv <= 48 ? 16 : 32;
+  if (pixels * lp / 32 < 8LL * geeps_sm_count()) lp = cv <= 12 ? 4 : cv <= 24 ? 8 : cv <= 32 ? 16 : 32;
+  return {lp, (cv + lp - 1) / lp};
+}
+
 int lp_env(const char* name, int dflt) {
   const char* e = getenv(name);
   return e ? atoi(e) : dflt;
@@ -635,6 +646,13 @@ int geeps_lrn_maxpool_supported(const GeepsPoolGeom* g, int size) {
   if (lp_fwd_smem(g) > kLpMaxSmem) return 0;
   while (R > 1 && lp_bwd_smem(g, R, lp_bwd_max_oh(g, R)) > kLpTwoPerSm) R >>= 1;
   return lp_bwd_smem(g, R, lp_bwd_max_oh(g, R)) <= kLpMaxSmem ? 1 : 0;
+}
+
+int geeps_lrn_lanes(int C, long long pixels, int* lanes, int* vectors) {
+  const LrnLanes l = lrn_lanes(C / 8, pixels);
+  *lanes = l.lp;
+  *vectors = l.nv;
+  return 0;
 }
 
 int geeps_lrn_maxpool_forward(const void* x, void* p, void* argmax, const GeepsPoolGeom* g, int size, float alpha,
@@ -688,7 +706,8 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
   // the register kernel covers the usual pair (5 channels, 3 x 3 stride 2) up to 512 channels; its item count is 32 bits
   const int cv = g->C / 8;
   if (k3s2 && size == 5 && cv <= 64 && (long long)g->B * g->H * (g->W + 64) < 0x7fffffffLL) {
-    const int lp = cv <= 12 ? 4 : cv <= 24 ? 8 : cv <= 32 ? 16 : 32, nv = (cv + lp - 1) / lp;
+    const LrnLanes ln = lrn_lanes(cv, (long long)g->B * g->H * g->W);
+    const int lp = ln.lp, nv = ln.nv;
     const int ppw = 32 / lp, strips = ((g->W + 1) / 2 + ppw - 1) / ppw;
     long long blocks = ((long long)g->B * g->H * 2 * strips + 7) / 8;
     const long long cap = (long long)geeps_sm_count() * 2;
@@ -696,9 +715,11 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
 #define LP_LANES(LP, NV)                                                                                           \
   lrn_maxpool_backward_lanes_kernel<LP, NV><<<(int)blocks, 256, sizeof(float) * g->C, st>>>(                         \
       (const bf16*)x, (const bf16*)dp, (const uint8_t*)argmax, (bf16*)dx, *g, cf, coef, relu_mask, colsum)
-    if (lp == 4) { if (nv == 1) LP_LANES(4, 1); else if (nv == 2) LP_LANES(4, 2); else LP_LANES(4, 3); }
+    if (lp == 1) LP_LANES(1, 1);
+    else if (lp == 2) { if (nv == 1) LP_LANES(2, 1); else LP_LANES(2, 3); }
+    else if (lp == 4) { if (nv == 1) LP_LANES(4, 1); else if (nv == 2) LP_LANES(4, 2); else LP_LANES(4, 3); }
     else if (lp == 8) { if (nv == 2) LP_LANES(8, 2); else LP_LANES(8, 3); }
-    else if (lp == 16) LP_LANES(16, 2);
+    else if (lp == 16) { if (nv == 2) LP_LANES(16, 2); else LP_LANES(16, 3); }
     else LP_LANES(32, 2);
 #undef LP_LANES
     return (int)cudaGetLastError();

@@ -104,6 +104,8 @@ int geeps_copy_f32(float* dst, const float* src, long long n, void* stream);
 // Forward keeps only the pooled tensor and the window codes; backward recomputes the normalisation from x and
 // delivers dx (gradient w.r.t. the LRN input) with an optional ReLU mask (x <= 0 -> 0) and, in colsum (C floats
 // or NULL), the per-channel sums of dx.
+// lanes per pixel and 8-channel vectors per lane of the backward register kernel (host arithmetic only)
+int geeps_lrn_lanes(int C, long long pixels, int* lanes, int* vectors);
 int geeps_lrn_maxpool_supported(const GeepsPoolGeom* g, int size);
 int geeps_lrn_maxpool_forward(const void* x, void* p, void* argmax, const GeepsPoolGeom* g, int size, float alpha,
                               float beta, float k, void* stream);

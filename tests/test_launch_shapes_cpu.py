@@ -44,3 +44,14 @@ def test_channel_blocks_cover_the_matrix_and_spread_few_pixels():
         assert rows * cv >= 0.75 * cols * threads, (P, Cc, list(out))         # threads with a slot
         # few pixels: an eighth of the SMs at least, or a block for every batch of rows
         assert cols * blocks >= min(148 // 8, cols * -(-P // rows)), (P, Cc, list(out))
+
+
+def test_lrn_backward_lanes_fit_the_channels():
+    for cv, pixels in itertools.product(range(1, 65), (1, 700, 40000, 200000)):
+        lp, nv = C.c_int(), C.c_int()
+        L.lib().geeps_lrn_lanes(cv * 8, C.c_longlong(pixels), C.byref(lp), C.byref(nv))
+        lp, nv = lp.value, nv.value
+        # the splits that the kernel is compiled for
+        assert (lp, nv) in ((1, 1), (2, 1), (2, 3), (4, 1), (4, 2), (4, 3), (8, 2), (8, 3), (16, 2), (16, 3), (32, 2))
+        assert lp * nv >= cv
+        assert pixels < 40000 or 3 * cv >= 2 * lp * nv, (cv, lp, nv)
