@@ -127,19 +127,13 @@ int geeps_softmax_ce(const float* logits, const long long* labels, float* loss_s
                      int zero_loss, int* status, void* stream);
 
 // ---- allocation-free BatchNorm forward (no counterpart in the reference, which has no layer kernels) ----
-// Same result as geeps_bn_forward, but the 2*C floats of reduction scratch come from a fixed device
-// array inside the library (GEEPS_BN_NOALLOC_MAX_CHANNELS channels, 32 KB per GPU, held until exit)
-// instead of from the caller.  It is meant for callers that cannot allocate: code under the parameter
-// server's fully planned GPU budget, and hosts without a device allocator that must keep cudaMalloc's
-// device-wide synchronisation out of their step loop.  The call itself never calls cudaMalloc / cudaFree
-// or any allocating library routine.
+// Same result as geeps_bn_forward without its 2*C floats of scratch: the sums are formed in mean_rstd and finalised in
+// place.  It is meant for callers that cannot allocate: code under the parameter server's fully planned GPU budget, and
+// hosts without a device allocator that must keep cudaMalloc's device-wide synchronisation out of their step loop.
+// The call never calls cudaMalloc / cudaFree or any allocating library routine, and calls share no memory: they may
+// overlap on several streams and be captured.
 //  * C must be a multiple of 8 and <= GEEPS_BN_NOALLOC_MAX_CHANNELS; a larger C is rejected with
 //    GEEPS_ERR_NOALLOC_TOO_LARGE (and a message on stderr) without launching anything.
-//  * The first call on each device looks up the array's device address (cudaGetSymbolAddress, with that
-//    device current); make that first call before any stream capture begins.
-//  * All calls share the one array, which keeps the previous call's contents; the part in use is cleared
-//    on `stream` first.  Calls whose kernels may overlap on the GPU race on it: keep them on one stream
-//    or order them with events.
 #define GEEPS_BN_NOALLOC_MAX_CHANNELS 4096
 #define GEEPS_ERR_NOALLOC_TOO_LARGE (-2)
 int geeps_bn_noalloc_max_channels(void);

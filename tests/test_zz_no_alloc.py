@@ -3,10 +3,9 @@
 Some users of the library cannot hand a kernel scratch memory: code that runs inside the parameter
 server's fully planned GPU budget has no allocator once the clocks are running, and a host program
 that links the library without a device allocator of its own does not want cudaMalloc (which
-synchronises the whole device) inside its step loop.  For them the entry point takes its reduction
-scratch from a fixed array inside the library.  This test calls it through the exported C symbol
-and checks it against the ordinary entry point, twice in a row, because the built-in array keeps
-the previous call's contents and must be cleared by the call itself.
+synchronises the whole device) inside its step loop.  For them the entry point forms its sums in the
+buffer that receives mean and 1/std.  This test calls it through the exported C symbol and checks it
+against the ordinary entry point, twice in a row and on several streams at once.
 
 The file name sorts last on purpose: a run that stops at the first failure has then already run
 every other test.
@@ -46,8 +45,7 @@ def test_bn_forward_noalloc_matches_plain_entry_point_twice():
     dev = torch.device("cuda:0")
     torch.manual_seed(7)
     stream = torch.cuda.current_stream().cuda_stream or 1   # 0x1 = CUDA's legacy default stream
-    # two calls in a row with different widths: the second one reuses (part of) the array the first one
-    # filled, so stale sums would show up as wrong statistics
+    # two calls in a row with different widths
     for call, (P, Cc, relu) in enumerate([(4000, 96, True), (2500, 48, False)]):
         x = (torch.randn(P, Cc, device=dev) * (call + 1.5) + call).to(torch.bfloat16)
         gamma = torch.rand(Cc, device=dev) + 0.5
@@ -80,3 +78,28 @@ def test_bn_forward_noalloc_rejects_too_many_channels():
     assert rc == -2                          # GEEPS_ERR_NOALLOC_TOO_LARGE, nothing launched
     torch.cuda.synchronize()
     assert mr.abs().sum().item() == 0
+
+
+def test_bn_forward_noalloc_calls_on_several_streams_do_not_meet():
+    """Four streams, each with its own data and widths, all in flight together: every call's statistics are its own."""
+    noalloc, _, _ = _sym()
+    dev = torch.device("cuda:0")
+    torch.manual_seed(11)
+    shapes = [(60000, 96), (40000, 96), (50000, 192), (30000, 64)]
+    work = []
+    for i, (P, Cc) in enumerate(shapes):
+        x = (torch.randn(P, Cc, device=dev) * (i + 1) + 3 * i).to(torch.bfloat16)
+        work.append((torch.cuda.Stream(), x, torch.empty_like(x), torch.ones(Cc, device=dev), torch.zeros(Cc, device=dev),
+                     [torch.empty(2 * Cc, device=dev) for _ in range(10)]))
+    torch.cuda.synchronize()
+    for k in range(10):
+        for st, x, y, g, b, mrs in work:
+            assert _call_noalloc(noalloc, x, y, g, b, mrs[k], False, st.cuda_stream) == 0
+    torch.cuda.synchronize()
+    for _, x, y, g, b, mrs in work:
+        mean, var = x.double().mean(0), x.double().var(0, unbiased=False)
+        for mr in mrs:
+            Cc = x.shape[1]
+            # E[x^2] - mean^2 in fp32: a few 1e-7 of E[x^2], which is up to 7 times the variance here
+            assert torch.allclose(mr[:Cc].double(), mean, atol=1e-4, rtol=1e-5)
+            assert torch.allclose(mr[Cc:].double(), (var + 1e-5).rsqrt(), rtol=1e-4)
