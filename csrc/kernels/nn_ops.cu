@@ -576,23 +576,24 @@ __global__ void __launch_bounds__(256)
 bn_forward_coop_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, float* sums, float* mean_rstd,
                        float* running_mean, float* running_var, const float* __restrict__ gamma,
                        const float* __restrict__ beta, float* zero_after, int* bar, long long P, int C, long long ldx,
-                       long long ldy, int relu, float inv_count, float eps, float momentum) {
+                       long long ldy, int relu, float inv_count, float eps, float momentum, uint8_t* bits) {
   channel_reduce_body<0>(x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
     bn_apply_fused_body(x, y, sums, mean_rstd, running_mean, running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
-                        inv_count, eps, momentum, nullptr);
+                        inv_count, eps, momentum, bits);
   else if (threadIdx.x == 0) { bar[2] = 1; mean_rstd[0] = __int_as_float(0x7fc00000); }
   bn_grid_done(bar, (int)(gridDim.x * gridDim.y));
 }
+template <bool BITS>      // y points to the mask bits
 __global__ void __launch_bounds__(256)
 bn_backward_coop_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                         bf16* __restrict__ dx, float* mean_rstd, const float* __restrict__ gamma, float* sums,
                         float* dgamma, float* dbeta, float* zero_after, int* bar, long long P, int C, long long ldx,
                         long long lddy, long long lddx, int relu, float grad_scale) {
-  channel_reduce_body<1>(x, dy, y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
+  channel_reduce_body<BITS ? 3 : 1>(x, dy, y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
   if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
-    bn_backward_body<false>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
-                            zero_after);
+    bn_backward_body<BITS>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
+                           zero_after);
   else if (threadIdx.x == 0) { bar[2] = 1; mean_rstd[0] = __int_as_float(0x7fc00000); }
   bn_grid_done(bar, (int)(gridDim.x * gridDim.y));
 }
@@ -1836,7 +1837,7 @@ int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, cons
     const bf16* xx = (const bf16*)x; bf16* yy = (bf16*)y;
     float inv_count = 1.f / (float)P;
     void* args[] = {&xx, &yy, &sums, &mean_rstd, &running_mean, &running_var, &gamma, &beta, &zero_after, &barrier,
-                    &P, &C, &ldx, &ldy, &relu, &inv_count, &eps, &momentum};
+                    &P, &C, &ldx, &ldy, &relu, &inv_count, &eps, &momentum, &bits};
     const SlotGrid cg = bn_coop_grid(P, C);
     cudaError_t e = cudaLaunchCooperativeKernel((void*)bn_forward_coop_kernel, cg.grid, dim3(cg.threads), args, cg.smem, st);
     return e == cudaSuccess ? CK() : (int)e;
@@ -1863,12 +1864,14 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   if (barrier != nullptr && bn_coop_enabled()) {
-    const bf16* xx = (const bf16*)x; const bf16* dd = (const bf16*)dy; const bf16* yy = (const bf16*)y;
+    const bool by_bits = bits != nullptr && relu;
+    const bf16* xx = (const bf16*)x; const bf16* dd = (const bf16*)dy; const bf16* yy = (const bf16*)(by_bits ? bits : y);
     bf16* dxx = (bf16*)dx;
     void* args[] = {&xx, &dd, &yy, &dxx, &mean_rstd, &gamma, &sums, &dgamma, &dbeta, &zero_after, &barrier,
                     &P, &C, &ldx, &lddy, &lddx, &relu, &grad_scale};
     const SlotGrid cg = bn_coop_grid(P, C);
-    cudaError_t e = cudaLaunchCooperativeKernel((void*)bn_backward_coop_kernel, cg.grid, dim3(cg.threads), args, cg.smem, st);
+    void* kernel = by_bits ? (void*)bn_backward_coop_kernel<true> : (void*)bn_backward_coop_kernel<false>;
+    cudaError_t e = cudaLaunchCooperativeKernel(kernel, cg.grid, dim3(cg.threads), args, cg.smem, st);
     return e == cudaSuccess ? CK() : (int)e;
   }
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);

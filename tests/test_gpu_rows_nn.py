@@ -549,3 +549,40 @@ def test_sums_of_dense_and_pitched_matrices(P, Cc, pitched):
     assert torch.allclose(dst.double(), ref, atol=0, rtol=2.0 ** -7)      # fp32 sum: at most the other neighbour
     if pitched[0]:
         assert torch.equal(full[0][:, :8], edges[:, :8]) and torch.equal(full[0][:, 8 + Cc:], edges[:, 8 + Cc:])
+
+
+_COOP = """
+import torch
+from geeps_b200.ops import functional as F
+BF, dev = torch.bfloat16, torch.device("cuda:0")
+for P, C in ((5, 8), (777, 104), (64, 2056), (3000, 192)):
+    torch.manual_seed(P)
+    x, dy = torch.randn(P, C, device=dev).to(BF), torch.randn(P, C, device=dev).to(BF)
+    g, b = torch.rand(C, device=dev) + 0.5, torch.randn(C, device=dev)
+    z = lambda: torch.zeros(2 * C, device=dev)
+    got = []
+    for bar in (torch.zeros(8, dtype=torch.int32, device=dev), None):
+        y, stat, rm, rv = torch.empty_like(x), z(), torch.zeros(C, device=dev), torch.ones(C, device=dev)
+        bits = torch.full((P, C // 8), 0xa5, dtype=torch.uint8, device=dev)
+        dx, dg, db = torch.empty_like(x), torch.empty(C, device=dev), torch.empty(C, device=dev)
+        F.bn_forward_fused(x, y, g, b, z(), stat, rm, rv, barrier=bar[:4] if bar is not None else None, relu=True, bits=bits)
+        want = ((y.view(P, C // 8, 8) > 0).long() << torch.arange(8, device=dev)).sum(2)
+        assert torch.equal(bits.long(), want), (P, C, bar is None)
+        F.bn_backward_fused(x, dy, torch.ones_like(y), dx, stat, g, z(), dg, db, barrier=bar[4:] if bar is not None else None,
+                            relu=True, bits=bits)
+        got.append((y, stat, dx, dg, db))
+    for u, v in zip(*got):      # sums of blocks meet in any order
+        assert torch.allclose(u.float(), v.float(), atol=1e-4, rtol=2.0 ** -7), (P, C)
+print("ok")
+"""
+
+
+def test_batchnorm_in_one_launch_keeps_and_reads_the_mask_bits():
+    """GEEPS_BN_COOP=1 (read once per process): one cooperative launch per direction writes the same mask, and its backward
+    pass reads it in the place of y."""
+    import os
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", _COOP], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, GEEPS_BN_COOP="1"), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stderr[-2000:]
