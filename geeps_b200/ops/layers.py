@@ -87,6 +87,9 @@ class Layer:
         raise NotImplementedError
 
     # ---- hooks for activations managed by the parameter server's memory plan ----
+    def hold_no_extras(self) -> None:
+        """Give back buffers that only save a second read of the output: they are outside the plan and its budget."""
+
     def out_numel(self) -> int:
         n = 1
         for s_ in self.out_shape:
@@ -479,6 +482,9 @@ class BatchNorm(Layer):
 
     def bind_output(self, y2d):
         self.y = y2d
+
+    def hold_no_extras(self):
+        self.bits, self._bits_valid = None, False      # the backward pass reads y, which the plan has fetched back
 
     def forward(self, x):
         self.x = x if x.dim() == 2 else x.view(self.P, self.C)

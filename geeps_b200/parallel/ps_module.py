@@ -94,6 +94,8 @@ class PSModule:
                 if isinstance(l, (Linear, Dropout)) or nbytes < (1 << 20):
                     continue
                 nrows = (nbytes + 511) // 512
+                for sub in (l.sublayers() if hasattr(l, "sublayers") else [l]):
+                    sub.hold_no_extras()
                 self.managed[i] = {"rows": range(1_000_000 * (i + 1), 1_000_000 * (i + 1) + nrows), "nrows": nrows}
         direct16 = ps_config.transport == TRANSPORT_NVLINK and ps_config.bf16_compute_cache
         # uncached (pull) tables

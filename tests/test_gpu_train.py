@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 from geeps_b200.models.alexnet import alexnet
 from geeps_b200.models.inception_bn import inception_bn_small
-from geeps_b200.ops.layers import Conv2d, Linear, Pool, LRN, Input
+from geeps_b200.ops.layers import BatchNorm, Conv2d, Linear, Pool, LRN, Input
 from geeps_b200.models.net import Net
 from geeps_b200.parallel.ps_module import PSModule
 from geeps_b200.utils.config import (DEVICE_CUDA, TABLE_ADDITIVE, TABLE_SGD_MOMENTUM, TRANSPORT_NVLINK, TRANSPORT_TCP,
@@ -129,6 +129,10 @@ def test_managed_activations_match_unmanaged(frac):
             x = torch.randn(B, 3, 32, 32, device=dev, generator=gen)
             y = torch.randint(0, 10, (B,), device=dev, generator=gen)
             losses[managed] = [mod.step(x, y).item() for _ in range(5)]
+            # a managed output is all that its layers keep of it: nothing beside it outside the plan's budget
+            held = [l.bits is not None for i, (top, _) in enumerate(mod.groups) if i in mod.managed or not managed
+                    for l in (top.sublayers() if hasattr(top, "sublayers") else [top]) if isinstance(l, BatchNorm)]
+            assert held and all(h != managed for h in held)
             if managed:
                 st = mod.ps.get_stats()["client"]
                 assert len(mod.managed) > 0
