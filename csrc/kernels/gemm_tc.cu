@@ -60,8 +60,6 @@ struct SmemCtl {
   int abort_flag;
 };
 
-// Persistent kernel: one CTA per SM walks the tile list t = blockIdx.x, blockIdx.x + gridDim.x, ...
-// Consecutive CTAs take consecutive M tiles of the same N tile, so the B tile they share stays in L2.
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -69,6 +67,11 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t smem_addr, int rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
+}
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
 }
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   float4 v;
@@ -80,6 +83,9 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
 // accumulator comes out of TMEM, one row per lane) off a single bank
 __device__ __forceinline__ uint32_t part_off(int r, int q, int bn) { return (uint32_t)(r * bn * 4 + ((q ^ (r & 7)) << 4)); }
 
+// Persistent kernel: one CTA per SM walks the tile list t = blockIdx.x, blockIdx.x + gridDim.x, ...
+// Consecutive CTAs take consecutive M tiles of the same N tile, so the B tile they share stays in L2.
+// CL: a cluster of d.cluster CTAs per tile, one K slice each.
 template <bool A_MN, bool B_MN, bool CL>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -387,7 +393,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int m0 = (mn % d.m_tiles) * BM, n0 = (mn / d.m_tiles) * BN;
     const int rows = BM / d.cluster, oct = BN >> 3;
     const uint32_t part = tc05::smem_u32(tiles);
-    for (int i = threadIdx.x; i < rows * oct; i += blockDim.x) {
+    // a CTA that gave up left no partial tile: nobody stores (the status word names it), as without a cluster
+    const uint32_t gave_up = ld_cluster_u32(cluster_addr(tc05::smem_u32(&ctl->abort_flag), lane % d.cluster));
+    const int todo = __any_sync(0xffffffffu, gave_up != 0u) ? 0 : rows * oct;
+    for (int i = threadIdx.x; i < todo; i += blockDim.x) {
       const int rr = i / oct, o = i - rr * oct;
       const int r = rank * rows + rr;
       const long long row = (long long)m0 + r, col0 = (long long)n0 + o * 8;
