@@ -133,8 +133,8 @@ __device__ __forceinline__ void window5(const float2 (&t)[6], float2 (&w)[4]) {
 
 // ---------------- forward ----------------
 // grid = B * ceil(OH / RO); one CTA produces RO pooled rows from the (RO-1)*stride + K input rows under them.
-// The input is read from global memory (one 16-byte and two 8-byte loads per 8 outputs), normalised once per
-// element into shared memory ([n_in][W][C] bf16), and pooled from there.
+// The input is read from global memory (one 16-byte load per 8 outputs and two of 4 bytes for the neighbours, 8 bytes for
+// a window of 3 or 7 channels), normalised once per element into shared memory ([n_in][W][C] bf16), and pooled from there.
 // K3S2: 3 x 3 windows with stride 2 (window size and stride are then constants of the pooling loops)
 template <int HALF, bool K3S2>
 __global__ void __launch_bounds__(512)
@@ -159,7 +159,7 @@ lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uin
     for (ItemWalk it(tid, nt, W, cv); it.r < nrows; it.next(W, cv)) {
       const int c = it.cvi * 8;
       const int pix = it.r * row_elems + it.w * C;          // offsets inside a block of a few rows: 32 bits
-      if (HALF == 2) {
+      if constexpr (HALF == 2) {
         // pairs of channels: half the fp32 instructions, and a halo of one word per side instead of two
         const bf16* px = xbase + pix + c;
         const uint32_t before = c > 0 ? *reinterpret_cast<const uint32_t*>(px - 2) : 0u;
@@ -185,21 +185,21 @@ lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uin
         *reinterpret_cast<uint4*>(ybase + pix + c) =
             make_uint4(pack_bf16x2(o[0].x, o[0].y), pack_bf16x2(o[1].x, o[1].y), pack_bf16x2(o[2].x, o[2].y),
                        pack_bf16x2(o[3].x, o[3].y));
-        continue;
-      }
-      float v[16], t[16], ws[8], o[8];
-      load16(xbase + pix, c, C, v);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) t[j] = v[j] * v[j];
-      window8<HALF>(t, ws);
-      if (max8(ws) <= cf.w_max) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = v[4 + e] * fmaf(ws[e], fmaf(ws[e], fmaf(ws[e], cf.p3, cf.p2), cf.p1), cf.p0);
       } else {
+        float v[16], t[16], ws[8], o[8];
+        load16(xbase + pix, c, C, v);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = v[4 + e] * __powf(cf.k * fmaf(cf.es, ws[e], 1.f), -cf.beta);
+        for (int j = 0; j < 16; ++j) t[j] = v[j] * v[j];
+        window8<HALF>(t, ws);
+        if (max8(ws) <= cf.w_max) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] = v[4 + e] * fmaf(ws[e], fmaf(ws[e], fmaf(ws[e], cf.p3, cf.p2), cf.p1), cf.p0);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] = v[4 + e] * __powf(cf.k * fmaf(cf.es, ws[e], 1.f), -cf.beta);
+        }
+        *reinterpret_cast<uint4*>(ybase + pix + c) = pack8(o);
       }
-      *reinterpret_cast<uint4*>(ybase + pix + c) = pack8(o);
     }
   }
   __syncthreads();

@@ -1820,13 +1820,6 @@ static bool bn_coop_enabled() {
   return v != 0;
 }
 
-int geeps_bn_forward_fused(const void* x, void* y, const float* gamma, const float* beta, float* sums,
-                           float* mean_rstd, float* running_mean, float* running_var, float* zero_after, int* barrier,
-                           long long P, int C, long long ldx, long long ldy, float eps, float momentum, int relu,
-                           void* stream) {
-  return geeps_bn_forward_fused_bits(x, y, gamma, beta, sums, mean_rstd, running_mean, running_var, zero_after, barrier,
-                                     nullptr, P, C, ldx, ldy, eps, momentum, relu, stream);
-}
 int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, const float* beta, float* sums,
                                 float* mean_rstd, float* running_mean, float* running_var, float* zero_after,
                                 int* barrier, unsigned char* bits, long long P, int C, long long ldx, long long ldy,
@@ -1849,13 +1842,6 @@ int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, cons
                                                               running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                                                               1.f / (float)P, eps, momentum, bits);
   return CK();
-}
-int geeps_bn_backward_fused(const void* x, const void* dy, const void* y, void* dx, float* mean_rstd,
-                            const float* gamma, float* sums, float* dgamma, float* dbeta, float* zero_after,
-                            int* barrier, long long P, int C, long long ldx, long long lddy, long long lddx, int relu,
-                            float grad_scale, void* stream) {
-  return geeps_bn_backward_fused_bits(x, dy, y, nullptr, dx, mean_rstd, gamma, sums, dgamma, dbeta, zero_after, barrier, P,
-                                      C, ldx, lddy, lddx, relu, grad_scale, stream);
 }
 int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, const unsigned char* bits, void* dx,
                                  float* mean_rstd, const float* gamma, float* sums, float* dgamma, float* dbeta,
@@ -1953,9 +1939,6 @@ int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s
   else { if (n == 3) ADD_2D(3, false); else if (n == 2) ADD_2D(2, false); else ADD_2D(1, false); }
 #undef ADD_2D
   return CK();
-}
-int geeps_add_bf16_2d(void* dst, const void* src, long long P, int C, long long ldd, long long lds, void* stream) {
-  return geeps_add_bf16_2d_n(dst, src, nullptr, nullptr, P, C, ldd, lds, 0, 0, stream);
 }
 
 int geeps_dropout(const void* x, void* y, long long n, float p, unsigned long long seed, void* stream) {

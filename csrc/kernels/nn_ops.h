@@ -55,7 +55,7 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
 // `barrier` (4 ints, zero at first use, private to this layer and direction) - ONE cooperative launch whose blocks meet
 // at a bounded grid barrier between the reduction and the normalisation, when GEEPS_BN_COOP=1 (measured slower than the
 // two launches, so it is off by default).
-// the fused pair with the ReLU mask kept as bits ([P][C / 8] bytes, written forward, read backward in the place of y)
+// bits (or NULL): the ReLU mask, [P][C / 8] bytes, written forward and read backward in the place of y.
 int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, const float* beta, float* sums,
                                 float* mean_rstd, float* running_mean, float* running_var, float* zero_after,
                                 int* barrier, unsigned char* bits, long long P, int C, long long ldx, long long ldy,
@@ -64,14 +64,6 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
                                  float* mean_rstd, const float* gamma, float* sums, float* dgamma, float* dbeta,
                                  float* zero_after, int* barrier, long long P, int C, long long ldx, long long lddy,
                                  long long lddx, int relu, float grad_scale, void* stream);
-int geeps_bn_forward_fused(const void* x, void* y, const float* gamma, const float* beta, float* sums,
-                           float* mean_rstd, float* running_mean, float* running_var, float* zero_after, int* barrier,
-                           long long P, int C, long long ldx, long long ldy, float eps, float momentum, int relu,
-                           void* stream);
-int geeps_bn_backward_fused(const void* x, const void* dy, const void* y, void* dx, float* mean_rstd,
-                            const float* gamma, float* sums, float* dgamma, float* dbeta, float* zero_after,
-                            int* barrier, long long P, int C, long long ldx, long long lddy, long long lddx, int relu,
-                            float grad_scale, void* stream);
 // out[c] (+)= scale * sum_p x[p][c]
 // dx = y > 0 ? dy : 0 and colsum[c] = sum over the P pixels of dx (C % 8 == 0, C <= 8192), one pass
 int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* colsum, long long P, int C,
@@ -86,7 +78,6 @@ int geeps_f32_to_bf16_2d(const float* src, void* dst, long long P, int C, long l
                          void* stream);
 int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s2, long long P, int C, long long ldd,
                         long long ld0, long long ld1, long long ld2, void* stream);   // dst += s0 (+ s1 (+ s2)), null: absent
-int geeps_add_bf16_2d(void* dst, const void* src, long long P, int C, long long ldd, long long lds, void* stream);
 int geeps_dropout(const void* x, void* y, long long n, float p, unsigned long long seed, void* stream);
 // the same with the seed taken as seed + *step_ref when the kernel runs (a device-resident step counter: the launch
 // arguments stay the same from step to step, so the launch can sit in a replayed CUDA graph)

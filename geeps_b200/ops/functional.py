@@ -279,9 +279,7 @@ def new_event() -> int:
 
 
 def add_2d(dst2d, src2d) -> None:
-    P, Cc = dst2d.shape
-    launch(lib().geeps_add_bf16_2d, "add_bf16_2d", ptr(dst2d), ptr(src2d), C.c_longlong(P), Cc, C.c_longlong(_ld(dst2d)),
-                                  C.c_longlong(_ld(src2d)), stream_ptr())
+    add_2d_n(dst2d, [src2d])
 
 
 def add_2d_n(dst2d, srcs) -> None:
