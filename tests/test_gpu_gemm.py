@@ -1,4 +1,6 @@
 """tcgen05 GEMM vs a plain PyTorch fp32 reference of the same product."""
+import ctypes
+
 import pytest
 import torch
 
@@ -125,12 +127,14 @@ def test_gemm_auto_dispatch_uses_pairs_for_large_products():
     assert ((out.float() - ref).norm() / ref.norm()).item() < 5e-3
 
 
-@pytest.mark.parametrize("M,N,K,b_mn,fp32", [(256, 512, 8200, False, False), (5, 1000, 8264, False, True),
-                                             (32, 1024, 21841, True, False), (129, 200, 8328, True, True),
-                                             (256, 1000, 4096, False, False), (100, 72, 16392, False, True)])
-def test_gemm_cluster_split_k(M, N, K, b_mn, fp32):
+@pytest.mark.parametrize("M,N,K,b_mn,fp32,cluster", [(256, 512, 8200, False, False, True), (5, 1000, 8264, False, True, True),
+                                                     (32, 1024, 21841, True, False, True), (129, 200, 8328, True, True, True),
+                                                     (256, 1000, 4096, False, False, False), (100, 72, 16392, False, True, True),
+                                                     (1, 200, 8192, False, False, True), (257, 330, 8129, False, False, True)])
+def test_gemm_cluster_split_k(M, N, K, b_mn, fp32, cluster):
     """Few output tiles, long K: slices of one tile on the CTAs of a cluster (uneven last slice, ragged M and N, column
-    slices that end on odd widths), bias and ReLU applied once; the same bits on every run."""
+    slices that end on odd widths), bias and ReLU applied once; the same bits on every run.  One product takes narrow tiles
+    without a cluster."""
     dev = torch.device("cuda:0")
     torch.manual_seed(M + N + K)
     kp = (K + 7) // 8 * 8
@@ -140,6 +144,11 @@ def test_gemm_cluster_split_k(M, N, K, b_mn, fp32):
     wide = torch.zeros((M, N + 16), dtype=torch.float32 if fp32 else torch.bfloat16, device=dev)
     out = wide[:, 8:8 + N]
     st = L.new_status(dev)
+    p, plan = L.GemmParams(), L.GemmPlan()
+    p.A, p.B, p.C, p.bias, p.bias_mode = a.data_ptr(), b.data_ptr(), out.data_ptr(), bias.data_ptr(), 1
+    p.M, p.N, p.K, p.lda, p.ldb, p.ldc = M, N, K, a.stride(0), b.stride(0), out.stride(0)
+    p.alpha, p.b_mn_major, p.out_fp32, p.relu, p.split_k = 0.5, int(b_mn), int(fp32), 1, 1
+    assert L.lib().geeps_gemm_plan(ctypes.byref(p), ctypes.byref(plan)) == 1 and (plan.cluster > 1) == cluster
     F.gemm(a, b, out, b_mn=b_mn, bias=bias, relu=True, alpha=0.5, status=st, impl="tc")
     torch.cuda.synchronize()
     assert L.read_status(st)["code"] == 0

@@ -417,9 +417,12 @@ def test_channel_kernels_at_the_edges_of_their_thread_map(P, Cc):
     assert torch.allclose(db.double(), br.grad, atol=1e-5 * P ** 0.5 * 4, rtol=1e-5) and sums.abs().max().item() == 0
 
 
-@pytest.mark.parametrize("Cc,pad", [(1, 7), (127, 1), (1000, 0), (1001, 7), (8199, 0), (24576, 0), (30001, 7)])
+@pytest.mark.parametrize("Cc,pad", [(1, 7), (127, 1), (1000, 0), (1001, 7), (8199, 0), (24576, 0), (30001, 7),
+                                    (4095, 1), (4095, 0), (4096, 0), (4096, 1), (4097, 7), (4097, 0), (6000, 0), (6001, 2),
+                                    (24577, 7), (24577, 0), (30001, 2)])
 def test_softmax_rows_in_registers_and_past_them(Cc, pad):
-    """Aligned rows (pitch a multiple of 8) and unaligned ones, one thread's worth of classes to rows that are read again."""
+    """Aligned rows (pitch a multiple of 8) and unaligned ones, on both sides of 4096 classes (fewer: the narrow kernel),
+    blocks of fewer than 1024 threads, rows that are read again (more than 24576 classes)."""
     torch.manual_seed(Cc)
     B = 5
     logits = (torch.randn(B, Cc + pad, device=DEV) * 4)[:, :Cc]
