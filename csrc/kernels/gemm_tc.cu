@@ -525,9 +525,10 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
 int round_up(long long v, int m) { return (int)((v + m - 1) / m * m); }
 
 // Tile width and K slices (cluster size) for an output that 256-wide tiles would not spread over every SM.  Such a
-// product is bound by the operand bytes its CTAs pull through L2 (about 75 bytes per ns and SM here), so the choice is
-// the one with the least traffic on the busiest SM: rounds x k tiles per CTA x (A rows + B rows) x 128 bytes, plus
-// kTileOver per round (fill, drain) and, for a cluster, the exchange of its partial tile.  Narrow tiles spread an
+// product is bound by the operand bytes its CTAs pull through L2 (75 to 90 bytes per ns and SM: 256 x 4096, K = 9216 takes
+// 43, 51 and 80 us on widths 64, 128 and 256), so the choice is the one with the least traffic on the busiest SM: rounds x
+// k tiles per CTA x (A rows + B rows) x 128 bytes, plus kTileOver (2 us of that traffic) per round (fill, drain) and, for a
+// cluster, the exchange of its partial tile.  Narrow tiles spread an
 // output but re-read A once per tile; a cluster keeps the tile wide and cuts K instead.
 struct TileChoice { int bn, cluster; };
 TileChoice choose_tiles(const GeepsGemmParams* p, int unit, int kt, int sms, bool cluster_ok) {
@@ -585,10 +586,12 @@ GemmPlan plan_gemm(const GeepsGemmParams* p, int sms) {
     } else if (tiles() < sms && p->N > 64) {
       // a bf16 slab is 64 columns wide (see below): several tiles have widths that are multiples of it
       const int step = tma_c && !p->out_fp32 ? 64 : unit;
-      // Clusters only for a long K over very few tiles (the data gradient of a wide classifier: 32 x 1024, K = 21841,
-      // 16 tiles: 76 -> 31 us).  Elsewhere they give less (256 x 4096, K = 9216: 40 -> 32 us) and every product would
-      // add its K slices in another order: in a deep network with near-ties in its pooling windows that changes which
-      // element a later step's maximum picks, so ordinary layers keep one running sum over K.
+      // Clusters only for K above 8128 over at most sms / 8 narrow tiles: the data gradient of a wide classifier, 32 x 1024,
+      // K = 21841, 16 tiles: 80 us without a cluster, 37 on 64 x 8 (31 on 64 x 4).  The line is drawn by the order of the
+      // sums, not by speed: a cluster adds its K slices in another order than one running sum, and in a deep network with
+      // near-ties in its pooling windows that changes which element a later step's maximum picks, so ordinary layers
+      // keep one sum.  What that leaves (tile width x cluster, L2 flushed): 256 x 4096, K = 9216: 45 us on 64 x 1, 53 on
+      // 128 x 1, 41 on 128 x 2; 32 rows: 43 on 64 x 1, 31 on 128 x 4; 256 x 1000, K = 4096: 24.5 on 64 x 1, 16.5 on 64 x 4.
       const bool cluster_ok = p->split_k <= 1 && p->beta == 0.f && kt >= 128 &&
                               m_tiles * ((p->N + 63) / 64) <= sms / 8;
       const TileChoice c = choose_tiles(p, step, kt, sms, cluster_ok);

@@ -2059,7 +2059,10 @@ int geeps_softmax_ce(const float* logits, const long long* labels, float* loss_s
                      int zero_loss, int* status, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if (zero_loss && loss_sum) cudaMemsetAsync(loss_sum, 0, sizeof(float), st);
-  if (C < 4096) {     // 16 values per thread at most: nothing for wider blocks to gain (the wide kernel: 54 -> 8 us at 21841)
+  // Narrow rows keep the order in which 256 threads have always summed them.  The register kernel takes the same time up to
+  // 1000 classes and less from there (32 x 2000 8.5 -> 6.5 us, 32 x 4000 10.5 -> 7.0, 256 x 4000 10.6 -> 8.7; rows off a
+  // 16-byte boundary 8.5, 8.5 and 10.6), 32 x 6000 12.6 -> 8.5, 32 x 21841 54 -> 8.
+  if (C < 4096) {
     softmax_ce_small_kernel<<<B, 256, 0, st>>>(logits, labels, loss_sum, per_sample, (bf16*)dlogits, C, ldl, ldd, loss_scale,
                                                grad_scale, status);
     return CK();
