@@ -22,6 +22,7 @@
 #include <cuda.h>
 #include <mutex>
 #include <stdio.h>
+#include <string.h>
 
 #include "kernels.h"
 #include "tc05.cuh"
@@ -39,6 +40,16 @@ constexpr int C_SLAB_BYTES = BM * 128;
 
 enum { MODE_FWD = 0, MODE_DGRAD = 1, MODE_WGRAD = 2 };
 
+// One parity class of a data gradient (see geeps_conv_tc): pixels (s i + a, s j + b) of dX with the sub-filter of the
+// taps that reach them.  A stride-1 layer is one class.
+struct DgradDev {
+  int t0;                         // first tile of the class
+  int wt, ht, m_tiles;            // pixel boxes along W, along H, in all
+  int KW, kt_total;               // taps per row of the sub-filter; its taps x channel chunks
+  int pad_w, pad_h, tap0;         // dY offset of sub-filter tap (0, 0) and its place in the whole filter
+};
+constexpr int MAX_CLS = 4;        // classes per launch: all of a stride-2 layer
+
 struct ConvDev {
   const float* bias; int* status;
   int taps, KW, pad, cchunks;     // k-tile (fwd, dgrad) or N panel (wgrad) = (tap, 64-channel chunk)
@@ -50,11 +61,17 @@ struct ConvDev {
   int ch_valid;                   // wgrad: channels per tap (cg)
   int narrow;                     // fwd / dgrad: result leaves in 32-channel (64-byte) slabs, see the host code
   int stride;                     // fwd / wgrad: pixel stride of the layer (the X boxes are loaded with this element stride)
-  int pad_w, pad_h;               // dgrad: dY offset of tap (0, 0); equal to pad for a stride-1 layer
-  int tap0, tap_dw, tap_dh;       // dgrad: weight tap of loop position (kh, kw) = tap0 + kh * tap_dh + kw * tap_dw
-                                  // (a strided layer's data gradient runs one parity class of dX at a time, each
-                                  // with the sub-filter of the taps that reach it)
+  int n_cls, tap_dw, tap_dh;      // dgrad: weight tap of loop position (kh, kw) = tap0 + kh * tap_dh + kw * tap_dw
+  DgradDev cls[MAX_CLS];          // dgrad: tiles are ordered by class
 };
+
+struct OutMaps { CUtensorMap m[MAX_CLS]; };     // dgrad: the view of each class; else m[0]
+
+__device__ __forceinline__ int dgrad_class(const ConvDev& d, int t) {
+  int c = 0;
+  while (c + 1 < d.n_cls && t >= d.cls[c + 1].t0) ++c;
+  return c;
+}
 
 struct SmemCtl {
   uint64_t full[MAX_STAGES];
@@ -66,13 +83,13 @@ struct SmemCtl {
 };
 
 struct Box { int w0, h0, b0; };
-__device__ __forceinline__ Box decode_box(const ConvDev& d, int i) {
+__device__ __forceinline__ Box decode_box(const ConvDev& d, int i, int wt, int ht) {
   Box b;
-  const int wi = i % d.wt;
-  const int r = i / d.wt;
+  const int wi = i % wt;
+  const int r = i / wt;
   b.w0 = wi * d.bw;
-  b.h0 = (r % d.ht) * d.bh;
-  b.b0 = (r / d.ht) * d.bnb;
+  b.h0 = (r % ht) * d.bh;
+  b.b0 = (r / ht) * d.bnb;
   return b;
 }
 
@@ -81,7 +98,7 @@ __device__ __forceinline__ Box decode_box(const ConvDev& d, int i) {
 template <int MODE>
 __global__ void __launch_bounds__(192, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               const __grid_constant__ CUtensorMap tmC, const ConvDev d) {
+               const __grid_constant__ OutMaps tmC, const ConvDev d) {
   constexpr bool A_MN = MODE == MODE_WGRAD;
   constexpr bool B_MN = MODE != MODE_FWD;
   extern __shared__ uint8_t smem_raw[];
@@ -136,18 +153,26 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const uint32_t tx_bytes = MODE == MODE_WGRAD ? (uint32_t)((2 + BN / 64) * d.rows * 128)
                                                    : (uint32_t)(d.rows * 128 + BN * 128);
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const int mn = t % tiles_mn, z = t / tiles_mn;
-        const int mi = mn % d.m_tiles, ni = mn / d.m_tiles;
-        const int kt_begin = z * kt_per, kt_end = min(d.kt_total, kt_begin + kt_per);
+        const DgradDev& q = d.cls[MODE == MODE_DGRAD ? dgrad_class(d, t) : 0];
+        const int tq = MODE == MODE_DGRAD ? t - q.t0 : t;
+        const int mn = MODE == MODE_DGRAD ? tq : tq % tiles_mn, z = MODE == MODE_DGRAD ? 0 : tq / tiles_mn;
+        const int mts = MODE == MODE_DGRAD ? q.m_tiles : d.m_tiles;
+        const int mi = mn % mts, ni = mn / mts;
+        const int kt_begin = z * kt_per, kt_end = MODE == MODE_DGRAD ? q.kt_total : min(d.kt_total, kt_begin + kt_per);
+        const int KW = MODE == MODE_DGRAD ? q.KW : d.KW;
         Box mb = {0, 0, 0};
-        if (MODE != MODE_WGRAD) mb = decode_box(d, mi);
+        if (MODE == MODE_FWD) mb = decode_box(d, mi, d.wt, d.ht);
+        if (MODE == MODE_DGRAD) {      // of dY: where tap (0, 0) reads
+          mb = decode_box(d, mi, q.wt, q.ht);
+          mb.w0 += q.pad_w; mb.h0 += q.pad_h;
+        }
         // fwd / dgrad: k-tile = (kh, kw, channel chunk), starting at 0 (no split)
-        int kh = 0, kw = 0, cc = 0, tap = 0, wtap = d.tap0;
+        int kh = 0, kw = 0, cc = 0, tap = 0, wtap = MODE == MODE_DGRAD ? q.tap0 : 0;
         // wgrad: k-tile = pixel box; the N panels of this tile are fixed
         Box kb = {0, 0, 0};
         int pc[4] = {0, 0, 0, 0}, pdw[4] = {0, 0, 0, 0}, pdh[4] = {0, 0, 0, 0};
         if (MODE == MODE_WGRAD) {
-          kb = decode_box(d, kt_begin);
+          kb = decode_box(d, kt_begin, d.wt, d.ht);
           for (int j = 0; j < BN / 64; ++j) {
             const int panel = ni * (BN / 64) + j;
             const bool valid = panel * 64 < d.n_valid;
@@ -169,7 +194,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             tc05::tma_load_4d(sa, &tmA, bar, cc * 64, mb.w0 * d.stride + kw - d.pad, mb.h0 * d.stride + kh - d.pad, mb.b0);
             tc05::tma_load_3d(sb, &tmB, bar, cc * 64, tap, ni * BN);
           } else if (MODE == MODE_DGRAD) {
-            tc05::tma_load_4d(sa, &tmA, bar, cc * 64, mb.w0 + d.pad_w - kw, mb.h0 + d.pad_h - kh, mb.b0);
+            tc05::tma_load_4d(sa, &tmA, bar, cc * 64, mb.w0 - kw, mb.h0 - kh, mb.b0);
             for (int h = 0; h < BN / 64; ++h)
               tc05::tma_load_3d(sb + h * PANEL_BYTES, &tmB, bar, ni * BN + 64 * h, wtap, cc * 64);
           } else {
@@ -187,7 +212,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
           } else if (++cc == d.cchunks) {
             cc = 0; ++tap; wtap += d.tap_dw;
-            if (++kw == d.KW) { kw = 0; ++kh; wtap += d.tap_dh - d.KW * d.tap_dw; }
+            if (++kw == KW) { kw = 0; ++kh; wtap += d.tap_dh - KW * d.tap_dw; }
           }
           if (++s == S) { s = 0; ph ^= 1u; }
         }
@@ -202,8 +227,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int s = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_i) {
-        const int z = t / tiles_mn;
-        const int kt_begin = z * kt_per, kt_end = min(d.kt_total, kt_begin + kt_per);
+        const int z = MODE == MODE_DGRAD ? 0 : t / tiles_mn;
+        const int kt_begin = z * kt_per;
+        const int kt_end = MODE == MODE_DGRAD ? d.cls[dgrad_class(d, t)].kt_total : min(d.kt_total, kt_begin + kt_per);
         const uint32_t acc = tile_i & 1u, acc_ph = (tile_i >> 1) & 1u;
         if (!tc05::mbar_wait_warp(&ctl->tmem_empty[acc], acc_ph ^ 1u, abort_flag, WAIT_BUDGET_NS)) { ok = false; break; }
         tc05::fence_after_sync();
@@ -242,15 +268,19 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t rsw = narrow ? (uint32_t)((rloc >> 1) & 3) : (uint32_t)(rloc & 7);
     const bool relu = d.relu != 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tile_i) {
-      const int mn = t % tiles_mn;
-      const int mi = mn % d.m_tiles, ni = mn / d.m_tiles;
+      const int cl = MODE == MODE_DGRAD ? dgrad_class(d, t) : 0;
+      const DgradDev& cq = d.cls[cl];
+      const int mn = MODE == MODE_DGRAD ? t - cq.t0 : t % tiles_mn;
+      const int mts = MODE == MODE_DGRAD ? cq.m_tiles : d.m_tiles;
+      const int mi = mn % mts, ni = mn / mts;
       const int n0 = ni * BN;
       const uint32_t acc = tile_i & 1u, acc_ph = (tile_i >> 1) & 1u;
       if (!tc05::mbar_wait(&ctl->tmem_full[acc], acc_ph, abort_flag, WAIT_BUDGET_NS)) break;
       tc05::fence_after_sync();
       const uint32_t tacc = tmem + acc * (uint32_t)acc_stride + ((uint32_t)(q * 32) << 16);
       Box mb = {0, 0, 0};
-      if (MODE != MODE_WGRAD) mb = decode_box(d, mi);
+      if (MODE == MODE_FWD) mb = decode_box(d, mi, d.wt, d.ht);
+      if (MODE == MODE_DGRAD) mb = decode_box(d, mi, cq.wt, cq.ht);
 #pragma unroll 1
       for (int c = 0; c < BN; c += cols_per_slab) {
         if (n0 + c >= d.n_valid) break;
@@ -300,11 +330,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int tap = panel / d.cchunks, cc = panel - tap * d.cchunks;
             const int x = cc * 64 + (c & 32);
             if (x < d.ch_valid) {       // never start a store past the extent
-              if (d.split_k > 1) tc05::tma_reduce_add_3d(&tmC, slab, x, tap, mi * BM);
-              else tc05::tma_store_3d(&tmC, slab, x, tap, mi * BM);
+              if (d.split_k > 1) tc05::tma_reduce_add_3d(&tmC.m[0], slab, x, tap, mi * BM);
+              else tc05::tma_store_3d(&tmC.m[0], slab, x, tap, mi * BM);
             }
           } else {
-            tc05::tma_store_4d(&tmC, slab, n0 + c, mb.w0, mb.h0, mb.b0);
+            tc05::tma_store_4d(&tmC.m[cl], slab, n0 + c, mb.w0, mb.h0, mb.b0);
           }
           tc05::bulk_commit();
         }
@@ -413,7 +443,7 @@ int narrow_store(int channels, long long pitch) {
 }
 
 template <int MODE>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const ConvDev& d, int grid,
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tc, const ConvDev& d, int grid,
            cudaStream_t st) {
   const int stage_bytes = A_STAGE_BYTES + d.bn * BK * 2;
   const size_t smem = (size_t)d.stages * stage_bytes + 2 * C_SLAB_BYTES + sizeof(SmemCtl) + 1024;
@@ -450,9 +480,9 @@ int geeps_conv_tc_supported(const GeepsConvTcParams* p) {
 }  // extern "C"
 
 namespace {
-// one parity class (a, b) of a strided layer's data gradient, or {s = 1}: the whole problem
-struct DgradClass { int s, a, b; };
-int conv_tc_run(const GeepsConvTcParams* p, DgradClass cls, void* stream);
+// parity classes (a, b) that one launch of a data gradient covers; s = 1: the whole problem, one class
+struct DgradClasses { int s, n, a[MAX_CLS], b[MAX_CLS]; };
+int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* stream);
 }  // namespace
 
 extern "C" {
@@ -465,22 +495,39 @@ int geeps_conv_tc(const GeepsConvTcParams* p, void* stream) {
   if (p->mode == MODE_DGRAD && p->stride > 1) {
     // dX[s i + a, s j + b] = sum over u, v of dY[i + oh0 - u, j + ow0 - v] * W[kh0 + s u, kw0 + s v]: s * s
     // stride-1 problems over dense views of dX, each with its sub-filter
-    for (int a = 0; a < p->stride; ++a)
-      for (int b = 0; b < p->stride; ++b) {
-        if (a >= p->H || b >= p->W) continue;
-        const int e = conv_tc_run(p, DgradClass{p->stride, a, b}, stream);
-        if (e) return e;
+    // (100 x 32 x 32 pixels, 80 -> 80 channels, stride 2: four launches of 8 - 12 us one after the other 32.3 us, one launch
+    // 19.5).  Classes with more taps come first: few large tiles left over at the end would wait for one another
+    const int sd = p->stride;
+    DgradClasses all{sd, 0, {}, {}};
+    auto taps = [&](int a, int b) {
+      const int kh0 = (a + p->pad) % sd, kw0 = (b + p->pad) % sd;
+      return ((p->KH - kh0 + sd - 1) / sd) * ((p->KW - kw0 + sd - 1) / sd);
+    };
+    int order[64], n = 0;
+    for (int a = 0; a < sd && a < p->H; ++a)
+      for (int b = 0; b < sd && b < p->W; ++b) order[n++] = a * sd + b;
+    for (int i = 1; i < n; ++i)       // insertion sort, stable: at most 8 x 8 classes
+      for (int j = i; j > 0 && taps(order[j] / sd, order[j] % sd) > taps(order[j - 1] / sd, order[j - 1] % sd); --j) {
+        const int o = order[j]; order[j] = order[j - 1]; order[j - 1] = o;
       }
+    for (int i = 0; i < n; ++i) {
+      all.a[all.n] = order[i] / sd; all.b[all.n] = order[i] % sd;
+      if (++all.n == MAX_CLS || i + 1 == n) {
+        const int e = conv_tc_run(p, all, stream);
+        if (e) return e;
+        all.n = 0;
+      }
+    }
     return 0;
   }
-  return conv_tc_run(p, DgradClass{1, 0, 0}, stream);
+  return conv_tc_run(p, DgradClasses{1, 1, {0}, {0}}, stream);
 }
 
 }  // extern "C"
 
 namespace {
 
-int conv_tc_run(const GeepsConvTcParams* p, DgradClass cls, void* stream) {
+int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* stream) {
   const int kSMs = geeps_sm_count();
   cudaStream_t st = (cudaStream_t)stream;
   ConvDev d;
@@ -493,29 +540,41 @@ int conv_tc_run(const GeepsConvTcParams* p, DgradClass cls, void* stream) {
   d.ch_valid = p->cg;
   d.narrow = 0;
   d.stride = p->stride > 1 ? p->stride : 1;
-  d.pad_w = d.pad_h = p->pad;
-  d.tap0 = 0; d.tap_dw = 1; d.tap_dh = p->KW;
-  CUtensorMap ta, tb, tc;
+  d.n_cls = cls.n;
+  d.tap_dw = cls.s; d.tap_dh = cls.s * p->KW;
+  memset(d.cls, 0, sizeof(d.cls));
+  CUtensorMap ta, tb;
+  OutMaps tc;
+  memset(&tc, 0, sizeof(tc));
   bool ok = true;
   const long long wdims[3] = {p->cg, d.taps, p->og};
   if (p->mode == MODE_FWD || p->mode == MODE_DGRAD) {
     const bool fwd = p->mode == MODE_FWD;
     // rows of the tile: pixels of the output (fwd) or of the input gradient (dgrad)
-    int GW = fwd ? p->OW : p->W, GH = fwd ? p->OH : p->H;
-    if (cls.s > 1) {
-      const int sd = cls.s;
-      GW = (p->W - cls.b + sd - 1) / sd; GH = (p->H - cls.a + sd - 1) / sd;
-      const int kh0 = (cls.a + p->pad) % sd, kw0 = (cls.b + p->pad) % sd;
-      const int khs = (p->KH - kh0 + sd - 1) / sd, kws = (p->KW - kw0 + sd - 1) / sd;    // >= 1: KH, KW >= s
-      d.pad_h = (cls.a + p->pad - kh0) / sd; d.pad_w = (cls.b + p->pad - kw0) / sd;
-      d.tap0 = kh0 * p->KW + kw0; d.tap_dw = sd; d.tap_dh = sd * p->KW;
-      d.KW = kws; d.taps = khs * kws;
-      d.stride = 1;
-    }
+    // (the classes share one box, which the largest class is cut into)
+    const int GW = fwd ? p->OW : (p->W + cls.s - 1) / cls.s, GH = fwd ? p->OH : (p->H + cls.s - 1) / cls.s;
+    if (!fwd) d.stride = 1;
     pick_box(GW, GH, p->B, BM, &d.bw, &d.bh, &d.bnb);
     d.rows = d.bw * d.bh * d.bnb;
     d.wt = (GW + d.bw - 1) / d.bw; d.ht = (GH + d.bh - 1) / d.bh;
-    d.m_tiles = d.wt * d.ht * ((p->B + d.bnb - 1) / d.bnb);
+    const int bt = (p->B + d.bnb - 1) / d.bnb;
+    d.m_tiles = d.wt * d.ht * bt;
+    int CW[MAX_CLS], CH[MAX_CLS];
+    if (!fwd) {
+      d.m_tiles = 0;
+      for (int i = 0; i < cls.n; ++i) {
+        DgradDev& q = d.cls[i];
+        const int kh0 = (cls.a[i] + p->pad) % cls.s, kw0 = (cls.b[i] + p->pad) % cls.s;
+        const int khs = (p->KH - kh0 + cls.s - 1) / cls.s, kws = (p->KW - kw0 + cls.s - 1) / cls.s;   // >= 1: KH, KW >= s
+        CW[i] = (p->W - cls.b[i] + cls.s - 1) / cls.s; CH[i] = (p->H - cls.a[i] + cls.s - 1) / cls.s;
+        q.wt = (CW[i] + d.bw - 1) / d.bw; q.ht = (CH[i] + d.bh - 1) / d.bh;
+        q.m_tiles = q.wt * q.ht * bt;
+        q.pad_h = (cls.a[i] + p->pad - kh0) / cls.s; q.pad_w = (cls.b[i] + p->pad - kw0) / cls.s;
+        q.tap0 = kh0 * p->KW + kw0;
+        q.KW = kws; q.kt_total = khs * kws;            // times the channel chunks, below
+        d.m_tiles += q.m_tiles;
+      }
+    }
     const int kch = fwd ? p->cg : p->og;          // reduced channels
     const int nch = fwd ? p->og : p->cg;          // produced channels
     d.cchunks = (kch + 63) / 64;
@@ -536,23 +595,26 @@ int conv_tc_run(const GeepsConvTcParams* p, DgradClass cls, void* stream) {
     }
     d.bn = bn;
     d.n_tiles = (nch + bn - 1) / bn;
+    for (int i = 0, t0 = 0; !fwd && i < cls.n; ++i) {
+      d.cls[i].kt_total *= d.cchunks;
+      d.cls[i].t0 = t0;
+      t0 += d.cls[i].m_tiles * d.n_tiles;
+    }
     const long long wst[2] = {(long long)p->cg * 2, p->ldw * 2};
     if (fwd) {
       ok = make_act_map(&ta, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, d.bw, d.bh, d.bnb, false, d.stride);
       const int wbox[3] = {64, 1, bn};
       ok = ok && make_map(&tb, p->w, 3, wdims, wst, wbox, false);
       d.narrow = narrow_store(p->og, p->y_pitch);
-      ok = ok && make_act_map(&tc, p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, d.bw, d.bh, d.bnb, d.narrow != 0);
+      ok = ok && make_act_map(&tc.m[0], p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, d.bw, d.bh, d.bnb, d.narrow != 0);
     } else {
       ok = make_act_map(&ta, p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, d.bw, d.bh, d.bnb);
       const int wbox[3] = {64, 1, 64};
       ok = ok && make_map(&tb, p->w, 3, wdims, wst, wbox, false);
       d.narrow = narrow_store(p->cg, p->x_pitch);
-      if (cls.s > 1)
-        ok = ok && make_act_view(&tc, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, cls.s, cls.a, cls.b, GW, GH, d.bw,
-                                 d.bh, d.bnb, d.narrow != 0);
-      else
-        ok = ok && make_act_map(&tc, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, d.bw, d.bh, d.bnb, d.narrow != 0);
+      for (int i = 0; i < cls.n; ++i)
+        ok = ok && make_act_view(&tc.m[i], p->x, p->cg, p->W, p->H, p->B, p->x_pitch, cls.s, cls.a[i], cls.b[i], CW[i], CH[i],
+                                 d.bw, d.bh, d.bnb, d.narrow != 0);
     }
   } else {
     // reduction over output pixels in boxes of up to 64
@@ -579,7 +641,7 @@ int conv_tc_run(const GeepsConvTcParams* p, DgradClass cls, void* stream) {
     ok = ok && make_act_map(&tb, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, d.bw, d.bh, d.bnb, false, d.stride);
     const long long wst[2] = {(long long)p->cg * 4, p->ldw * 4};
     const int wbox[3] = {32, 1, BM};
-    ok = ok && make_map(&tc, p->w, 3, wdims, wst, wbox, true);
+    ok = ok && make_map(&tc.m[0], p->w, 3, wdims, wst, wbox, true);
     int split = p->split_k;
     const long long tiles = (long long)d.m_tiles * d.n_tiles;
     if (split <= 0) {

@@ -80,7 +80,9 @@ STRIDED = [
     (4, 28, 28, 64, 96, 3, 1, 2),        # Inception down-sampling branch
     (2, 64, 64, 8, 64, 7, 3, 2),         # first layer of the 22K net (3 channels padded to 8), scaled down
     (3, 17, 17, 32, 32, 3, 0, 2),        # no padding, odd size
-    (2, 23, 23, 16, 48, 5, 2, 3),        # stride 3
+    (2, 23, 23, 16, 48, 5, 2, 3),        # stride 3: nine classes, three launches of the data gradient
+    (20, 32, 32, 80, 80, 3, 1, 2),       # more tiles than SMs over the four classes
+    (2, 1, 9, 16, 16, 3, 1, 2),          # one image row: the classes of odd rows are empty
 ]
 
 
