@@ -29,8 +29,10 @@
 // a 4-D TMA store (64 channels, PW, rows, 1) writes the slab to the NHWC tensor, clipping the dropped columns, the
 // rows past the image and the channels past the layer's extent.  A tile is two store blocks of Rb image rows; the
 // pitch PW is padded until a block has a multiple of 8 positions, which makes the swizzled chunk offsets of a
-// thread's channel constants; each block has its own pair of slabs; eight epilogue warps (two per TMEM lane quarter,
-// alternate column groups) share the conversion.
+// thread's channel constants; eight epilogue warps (two per TMEM lane quarter, alternate column groups) share the
+// conversion.  Both blocks leave through one pair of slabs, one after the other: the epilogue has time to wait for a slab
+// to be read, the main loop none to wait for its weights (16 KB per tap and chunk out of L2), and the 32 KB of a second
+// pair are two more weight stages: conv2 forward per group with 3 stages 66.6 us, with 5 60.4; conv1 with 4 99, with 6 96.
 //
 // conv_tc() routes a forward / data-gradient call here when the geometry wastes little (see
 // geeps_conv_halo_applicable); GEEPS_HALO_CONV=0 keeps every call on the box kernel.  Bounded waits and TMEM
@@ -106,7 +108,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   uint8_t* tiles_x = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles_w = tiles_x + (size_t)d.stages_x * d.x_stage_bytes;
   uint8_t* cslab = tiles_w + (size_t)d.stages_w * W_STAGE_BYTES;
-  SmemCtl* ctl = (SmemCtl*)(cslab + 4 * C_SLAB_BYTES);          // two sets (one per store block) of two slabs
+  SmemCtl* ctl = (SmemCtl*)(cslab + 2 * C_SLAB_BYTES);          // one slab per 64 channels
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = d.m_tiles * d.n_images * d.row_tiles;
 
@@ -227,7 +229,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     // ---------------- epilogue: TMEM (channel lanes) -> bf16 [position][channel] slab -> TMA store ----------------
     const int q4 = warp & 3;                       // TMEM lane quarter this warp may access
     const int sub = (warp - 2) >> 2;               // which of the quarter's two warps
-    const int half = q4 >> 1;                      // which 64-channel slab of a set
+    const int half = q4 >> 1;                      // which 64-channel slab
     const int chin = (q4 & 1) * 32 + lane;         // channel inside the slab
     const uint32_t chunk = (uint32_t)(chin >> 3), within = (uint32_t)((chin & 7) * 2);
     // Slab rows are positions (128 bytes, 128-byte swizzle: 16-byte chunk ^ row % 8).  A block has a multiple of
@@ -236,7 +238,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     uint32_t cb[8];
 #pragma unroll
     for (int jj = 0; jj < 8; ++jj) cb[jj] = ((chunk ^ (uint32_t)jj) << 4) + within;
-    const uint32_t slab_base = tc05::smem_u32(cslab) + (uint32_t)(half * C_SLAB_BYTES);     // set p adds p * 2 slabs
+    const uint32_t slab_base = tc05::smem_u32(cslab) + (uint32_t)(half * C_SLAB_BYTES);
     const bool storer = lane == 0 && (q4 & 1) == 0 && sub == 0;          // one thread per slab issues its stores
     const float floor_v = d.relu ? 0.f : -INFINITY;
     uint32_t tile_i = 0;
@@ -255,10 +257,8 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       tc05::fence_after_sync();
       const uint32_t tacc = tmem + acc * (uint32_t)ACC_COLS + ((uint32_t)(q4 * 32) << 16);
       for (int p = 0; p < q.nb; ++p) {
-        const uint32_t slab = slab_base + (uint32_t)(p * 2 * C_SLAB_BYTES);
-        // block p of the previous tile was stored out of this slab: that store must have read it (the one store
-        // issued since, out of the other set, may still be reading)
-        if (storer) tc05::bulk_wait_read<1>();
+        // the previous block was stored out of this slab: that store must have read it
+        if (storer) tc05::bulk_wait_read<0>();
         tc05::named_bar_sync(1, 32 * kEpilogueWarps);
         if (slab_valid) {
           const int c_begin = p * d.split, c_end = c_begin + d.split;
@@ -268,7 +268,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             tc05::tmem_ld_32x32(tacc + (uint32_t)g, r);
             tc05::tmem_ld_wait();
             const int row0 = g - c_begin;              // slab row of element 0: a multiple of 8, negative for a first
-            const uint32_t rbase = slab + (uint32_t)(row0 * 128);     // group that starts in the previous block
+            const uint32_t rbase = slab_base + (uint32_t)(row0 * 128);     // group that starts in the previous block
             if (row0 >= 0 && row0 + 32 <= d.split) {
 #pragma unroll
               for (int e = 0; e < 32; ++e) {
@@ -292,7 +292,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (storer && slab_valid) {
           // box (64 channels, PW, Rb, 1): columns past the image width, rows past its height and channels past
           // the extent are clipped by TMA
-          tc05::tma_store_4d_addr(&tmC, slab, q.mi * BM + half * 64, 0, q.y0 + p * d.Rb, q.b);
+          tc05::tma_store_4d_addr(&tmC, slab_base, q.mi * BM + half * 64, 0, q.y0 + p * d.Rb, q.b);
           tc05::bulk_commit();
         }
       }
@@ -407,11 +407,11 @@ HaloPlan plan_halo(const GeepsConvTcParams* p) {
   const int over = d.ncols2 - 2 * d.split + p->KW;     // rows an MMA may read past the halo tile
   d.x_stage_bytes = round_up((long long)(NR * d.PW + over) * 128, 1024);
   d.stages_x = 2;
-  const long long budget = 224 * 1024 - 4 * C_SLAB_BYTES - (long long)d.stages_x * d.x_stage_bytes;
+  const long long budget = 224 * 1024 - 2 * C_SLAB_BYTES - (long long)d.stages_x * d.x_stage_bytes;
   d.stages_w = (int)(budget / W_STAGE_BYTES);
   if (d.stages_w > MAX_W_STAGES) d.stages_w = MAX_W_STAGES;
   if (d.stages_w < 3) return hp;
-  hp.smem = (size_t)d.stages_x * d.x_stage_bytes + (size_t)d.stages_w * W_STAGE_BYTES + 4 * C_SLAB_BYTES + sizeof(SmemCtl) + 1024;
+  hp.smem = (size_t)d.stages_x * d.x_stage_bytes + (size_t)d.stages_w * W_STAGE_BYTES + 2 * C_SLAB_BYTES + sizeof(SmemCtl) + 1024;
   // share of the issued MMA work that lands in real outputs: positions x channels
   const double pos = (double)GH * GW / ((double)d.row_tiles * d.ncols2);
   const double chn = (double)nch / ((double)d.m_tiles * BM);
