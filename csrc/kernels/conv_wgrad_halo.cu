@@ -308,9 +308,12 @@ WgPlan plan_wgrad(const GeepsConvTcParams* p) {
   int tc = 32;
   while (tc < d.TY * d.KW * 64) tc <<= 1;
   d.tmem_cols = tc;
-  // slices of the positions: at most two items per SM (one more would add a third round for a few SMs)
+  // slices of the positions: one item per SM, so that accumulators are drained once (nothing covers that: they take most
+  // of TMEM) and every part of dW is added to half as often: conv2 per group 74.2 us, with two items 77.8.  Items of
+  // several filter rows have more to drain and do better with two, the first drained while other SMs multiply (conv1: 105
+  // us, with one 109)
   const long long base_items = (long long)d.m_tiles * d.cchunks * d.passes;
-  long long split = (2LL * geeps_sm_count()) / base_items;
+  long long split = ((d.TY > 1 ? 2LL : 1LL) * geeps_sm_count()) / base_items;
   if (split > d.n_blocks) split = d.n_blocks;
   if (split < 1) split = 1;
   const int per = (int)((d.n_blocks + split - 1) / split);
