@@ -107,6 +107,7 @@ conv_dgrad_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   __syncthreads();
   tc05::fence_after_sync();
   const uint32_t tmem = ctl->tmem_base;
+  geeps_pdl_wait();          // everything above touches this CTA's own memory only
   volatile int* abort_flag = &ctl->abort_flag;
 
   if (warp == 0) {
@@ -139,6 +140,7 @@ conv_dgrad_rows_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         }
       }
     }
+    geeps_pdl_trigger();       // every operand is on its way: the rest of this CTA is its last products and stores
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     const bool leader = tc05::elect_one();
@@ -366,7 +368,7 @@ int geeps_conv_dgrad_rows(const GeepsConvTcParams* p, void* stream) {
   const long long num_tiles = (long long)d.n_images * (d.pairs + d.single);
   const int sms = geeps_sm_count();
   const int grid = (int)(num_tiles < sms ? num_tiles : sms);
-  conv_dgrad_rows_kernel<<<grid, kThreads, rp.smem, (cudaStream_t)stream>>>(tx, tw, tc, d);
+  geeps_launch(conv_dgrad_rows_kernel, grid, kThreads, rp.smem, (cudaStream_t)stream, tx, tw, tc, d);
   return (int)cudaGetLastError();
 }
 

@@ -135,6 +135,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   __syncthreads();
   tc05::fence_after_sync();
   const uint32_t tmem = ctl->tmem_base;
+  geeps_pdl_wait();          // everything above touches this CTA's own memory only
   volatile int* abort_flag = &ctl->abort_flag;
   const int NR = 2 * d.Rb + d.KH - 1;
   const uint32_t x_tx = (uint32_t)(NR * d.PW * 128);
@@ -173,6 +174,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         }
       }
     }
+    geeps_pdl_trigger();       // every operand is on its way: the rest of this CTA is its last products and stores
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     const bool leader = tc05::elect_one();
@@ -357,7 +359,7 @@ int launch(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tc, 
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  conv_halo_kernel<MODE><<<grid, kThreads, smem, st>>>(tx, tw, tc, d);
+  geeps_launch(conv_halo_kernel<MODE>, grid, kThreads, smem, st, tx, tw, tc, d);
   return (int)cudaGetLastError();
 }
 

@@ -137,6 +137,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __syncthreads();
   tc05::fence_after_sync();
   const uint32_t tmem = ctl->tmem_base;
+  geeps_pdl_wait();          // everything above touches this CTA's own memory only
   volatile int* abort_flag = &ctl->abort_flag;
 
   if (warp == 0) {
@@ -218,6 +219,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
       }
     }
+    geeps_pdl_trigger();       // every operand is on its way: the rest of this CTA is its last products and stores
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     {
@@ -453,7 +455,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tc, cons
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  conv_tc_kernel<MODE><<<grid, 192, smem, st>>>(ta, tb, tc, d);
+  geeps_launch(conv_tc_kernel<MODE>, grid, 192, smem, st, ta, tb, tc, d);
   return (int)cudaGetLastError();
 }
 

@@ -104,6 +104,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_con
   __syncthreads();
   tc05::fence_after_sync();
   const uint32_t tmem = ctl->tmem_base;
+  geeps_pdl_wait();          // everything above touches this CTA's own memory only
   volatile int* abort_flag = &ctl->abort_flag;
 
   if (warp == 0) {
@@ -132,6 +133,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap tmY, const __grid_con
         if (++rt == d.row_tiles) { rt = 0; ++b; }
       }
     }
+    geeps_pdl_trigger();       // every operand is on its way: the rest of this CTA is its last products and stores
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     const bool leader = tc05::elect_one();
@@ -393,7 +395,7 @@ int geeps_conv_wgrad_halo(const GeepsConvTcParams* p, void* stream) {
   const long long items = (long long)d.m_tiles * d.cchunks * d.passes * d.split;
   const int sms = geeps_sm_count();
   const int grid = (int)(items < sms ? items : sms);
-  conv_wgrad_halo_kernel<<<grid, 192, wp.smem, (cudaStream_t)stream>>>(ty, tx, tw, d);
+  geeps_launch(conv_wgrad_halo_kernel, grid, 192, wp.smem, (cudaStream_t)stream, ty, tx, tw, d);
   return (int)cudaGetLastError();
 }
 

@@ -9,6 +9,7 @@ namespace {
 
 __global__ void __launch_bounds__(256)
 gemm_simt_kernel(const GeepsGemmParams p) {
+  geeps_pdl_enter();
   __shared__ float As[16][64 + 1];
   __shared__ float Bs[16][64 + 1];
   const __nv_bfloat16* A = (const __nv_bfloat16*)p.A;
@@ -66,6 +67,7 @@ gemm_simt_kernel(const GeepsGemmParams p) {
 }
 
 __global__ void scale_matrix_kernel(float* c, long long M, long long N, long long ldc, float beta) {
+  geeps_pdl_enter();
   const long long total = M * N;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -81,7 +83,7 @@ extern "C" {
 int geeps_gemm_bf16_simt(const GeepsGemmParams* p, void* stream) {
   if (p->M <= 0 || p->N <= 0 || p->K <= 0) return (int)cudaErrorInvalidValue;
   dim3 grid((unsigned)((p->M + 63) / 64), (unsigned)((p->N + 63) / 64));
-  gemm_simt_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(*p);
+  geeps_launch(gemm_simt_kernel, grid, 256, 0, (cudaStream_t)stream, *p);
   return (int)cudaGetLastError();
 }
 
@@ -90,7 +92,7 @@ int geeps_scale_matrix_f32(float* c, long long M, long long N, long long ldc, fl
   if (total <= 0) return 0;
   long long blocks = (total + 255) / 256;
   if (blocks > geeps_sm_count() * 8) blocks = geeps_sm_count() * 8;
-  scale_matrix_kernel<<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(c, M, N, ldc, beta);
+  geeps_launch(scale_matrix_kernel, (int)blocks, 256, 0, (cudaStream_t)stream, c, M, N, ldc, beta);
   return (int)cudaGetLastError();
 }
 

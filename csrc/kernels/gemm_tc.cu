@@ -122,6 +122,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __syncthreads();
   tc05::fence_after_sync();
   const uint32_t tmem = ctl->tmem_base;
+  geeps_pdl_wait();          // everything above touches this CTA's own memory only
   volatile int* abort_flag = &ctl->abort_flag;
 
   if (warp == 0) {
@@ -164,6 +165,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
       }
     }
+    geeps_pdl_trigger();       // every operand is on its way: the rest of this CTA is its last products and stores
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     {
@@ -499,7 +501,7 @@ int launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
     attr_set = true;
   }
   if (!CL) {
-    gemm_tc_kernel<A_MN, B_MN, CL><<<grid, 192, smem, st>>>(ta, tb, tc, d);
+    geeps_launch(gemm_tc_kernel<A_MN, B_MN, CL>, grid, 192, smem, st, ta, tb, tc, d);
     return (int)cudaGetLastError();
   }
   cudaLaunchConfig_t cfg = {};
@@ -507,12 +509,14 @@ int launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)d.cluster;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return (int)cudaLaunchKernelEx(&cfg, gemm_tc_kernel<A_MN, B_MN, CL>, ta, tb, tc, d);
 }
 template <bool A_MN, bool B_MN>

@@ -84,6 +84,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc05::cluster_sync();            // the peer's barriers are initialised before anything signals them
   tc05::fence_after_sync();
   const uint32_t tmem = ctl->tmem_base;
+  geeps_pdl_wait();          // everything above touches this CTA's own memory only
   volatile int* abort_flag = &ctl->abort_flag;
 
   if (warp == 0) {
@@ -307,7 +308,7 @@ int geeps_gemm_bf16_pair(const GeepsGemmParams* p, void* stream) {
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  gemm_pair_kernel<<<2 * pairs, 192, smem, (cudaStream_t)stream>>>(ta, tb, tc, d);
+  geeps_launch(gemm_pair_kernel, 2 * pairs, 192, smem, (cudaStream_t)stream, ta, tb, tc, d);
   return (int)cudaGetLastError();
 }
 

@@ -140,6 +140,7 @@ template <int HALF, bool K3S2>
 __global__ void __launch_bounds__(512)
 lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uint8_t* __restrict__ argmax,
                            const GeepsPoolGeom g, const LrnCoef cf, int RO) {
+  geeps_pdl_enter();
   extern __shared__ __align__(16) uint8_t lp_smem[];
   const int C = g.C, cv = C >> 3, W = g.W;
   const int PK = K3S2 ? 3 : g.K, PS = K3S2 ? 2 : g.stride;
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(256, 2)
 lrn_maxpool_backward_lanes_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dp,
                                   const uint8_t* __restrict__ argmax, bf16* __restrict__ dx, const GeepsPoolGeom g,
                                   const LrnCoef cf, float coef, int relu_mask, float* __restrict__ colsum) {
+  geeps_pdl_enter();
   extern __shared__ __align__(16) uint8_t lp_smem[];
   float* cs_sh = reinterpret_cast<float*>(lp_smem);      // [C]
   constexpr int PPW = 32 / LP;                           // pixels of a warp
@@ -436,6 +438,7 @@ __global__ void __launch_bounds__(512, 2)
 lrn_maxpool_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dp, const uint8_t* __restrict__ argmax,
                             bf16* __restrict__ dx, const GeepsPoolGeom g, int R, int max_oh, const LrnCoef cf, float coef,
                             int relu_mask, float* __restrict__ colsum) {
+  geeps_pdl_enter();
   extern __shared__ __align__(16) uint8_t lp_smem[];
   const int C = g.C, cv = C >> 3, W = g.W, OW = g.OW;
   const int PK = K3S2 ? 3 : g.K, PS = K3S2 ? 2 : g.stride;
@@ -674,7 +677,7 @@ int geeps_lrn_maxpool_forward(const void* x, void* p, void* argmax, const GeepsP
       if (e != cudaSuccess) return (int)e;                                                                         \
       attr_set = true;                                                                                             \
     }                                                                                                              \
-    lrn_maxpool_forward_kernel<HALF, K3S2><<<grid, block, smem, st>>>((const bf16*)x, (bf16*)p, (uint8_t*)argmax,   \
+    geeps_launch(lrn_maxpool_forward_kernel<HALF, K3S2>, grid, block, smem, st, (const bf16*)x, (bf16*)p, (uint8_t*)argmax,   \
                                                                        *g, cf, RO);                                \
   } while (0)
   const bool k3s2 = g->K == 3 && g->stride == 2;
@@ -713,7 +716,7 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
     const long long cap = (long long)geeps_sm_count() * 2;
     if (blocks > cap) blocks = cap;
 #define LP_LANES(LP, NV)                                                                                           \
-  lrn_maxpool_backward_lanes_kernel<LP, NV><<<(int)blocks, 256, sizeof(float) * g->C, st>>>(                         \
+  geeps_launch(lrn_maxpool_backward_lanes_kernel<LP, NV>, (int)blocks, 256, sizeof(float) * g->C, st,                          \
       (const bf16*)x, (const bf16*)dp, (const uint8_t*)argmax, (bf16*)dx, *g, cf, coef, relu_mask, colsum)
     if (lp == 1) LP_LANES(1, 1);
     else if (lp == 2) { if (nv == 1) LP_LANES(2, 1); else LP_LANES(2, 3); }
@@ -733,7 +736,7 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
       if (e != cudaSuccess) return (int)e;                                                                         \
       attr_set = true;                                                                                             \
     }                                                                                                              \
-    lrn_maxpool_backward_kernel<HALF, K3S2><<<grid, block, smem, st>>>((const bf16*)x, (const bf16*)dp,             \
+    geeps_launch(lrn_maxpool_backward_kernel<HALF, K3S2>, grid, block, smem, st, (const bf16*)x, (const bf16*)dp,             \
                                                                  (const uint8_t*)argmax, (bf16*)dx, *g, R, max_oh,  \
                                                                  cf, coef, relu_mask, colsum);                     \
   } while (0)

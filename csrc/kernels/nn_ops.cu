@@ -69,6 +69,7 @@ __device__ __forceinline__ float in_val(const bf16* p) { return __bfloat162float
 template <typename T>
 __global__ void __launch_bounds__(256)
 nchw_f32_to_nhwc_bf16_kernel(const T* __restrict__ x, bf16* __restrict__ y, int B, int C, int H, int W, int Cpad) {
+  geeps_pdl_enter();
   const long long total = (long long)B * H * W * Cpad;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -88,6 +89,7 @@ nchw_f32_to_nhwc_bf16_kernel(const T* __restrict__ x, bf16* __restrict__ y, int 
 template <int VEC>
 __global__ void __launch_bounds__(256)
 im2col_kernel(const bf16* __restrict__ x, bf16* __restrict__ col, const GeepsConvGeom g) {
+  geeps_pdl_enter();
   const int cv = g.Cg / VEC;
   const int per_kh = g.KW * cv;
   const int per_row = g.KH * per_kh;
@@ -125,6 +127,7 @@ im2col_kernel(const bf16* __restrict__ x, bf16* __restrict__ col, const GeepsCon
 
 // Zero the pad columns [Kd, ldcol) of the patch matrix once (TMA reads them as K).
 __global__ void zero_col_pad_kernel(bf16* col, long long rows, int kd, int ldcol) {
+  geeps_pdl_enter();
   const int padw = ldcol - kd;
   const long long total = rows * padw;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -137,6 +140,7 @@ __global__ void zero_col_pad_kernel(bf16* col, long long rows, int kd, int ldcol
 template <int VEC>
 __global__ void __launch_bounds__(256)
 col2im_kernel(const bf16* __restrict__ dcol, bf16* __restrict__ dx, const GeepsConvGeom g, int accumulate) {
+  geeps_pdl_enter();
   const int cv = g.Cg / VEC;
   const long long total = (long long)g.B * g.H * g.W * cv;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -359,12 +363,14 @@ __global__ void __launch_bounds__(256, 2)
 channel_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                       const float* __restrict__ mean_rstd, float* __restrict__ out, long long P, int C,
                       long long ldx, long long lddy, int relu, float scale) {
+  geeps_pdl_enter();
   channel_reduce_body<MODE>(x, dy, y, mean_rstd, out, P, C, ldx, lddy, relu, scale);
 }
 
 // any C, any pitch: one thread per column (small P: FC bias gradients with odd widths)
 __global__ void colsum_simple_kernel(const bf16* __restrict__ x, float* __restrict__ out, long long P, int C,
                                      long long ldx, float scale, int accumulate) {
+  geeps_pdl_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   float a = 0.f;
@@ -377,6 +383,7 @@ __global__ void colsum_simple_kernel(const bf16* __restrict__ x, float* __restri
 __global__ void bn_finalize_kernel(const float* sums, float* mean_rstd,
                                    float* running_mean, float* running_var, int C, float inv_count, float eps,
                                    float momentum) {
+  geeps_pdl_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const float m = sums[c] * inv_count;
@@ -435,6 +442,7 @@ __global__ void __launch_bounds__(256)
 bn_apply_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ mean_rstd,
                 const float* __restrict__ gamma, const float* __restrict__ beta, long long P, int C,
                 long long ldx, long long ldy, int relu) {
+  geeps_pdl_enter();
   extern __shared__ __align__(16) float sacc[];
   const SlotMap s(C);
   float mkb[3][8];
@@ -479,6 +487,7 @@ bn_apply_fused_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const fl
                       float* __restrict__ mean_rstd, float* running_mean, float* running_var,
                       const float* __restrict__ gamma, const float* __restrict__ beta, float* zero_after, long long P,
                       int C, long long ldx, long long ldy, int relu, float inv_count, float eps, float momentum, uint8_t* bits) {
+  geeps_pdl_enter();
   bn_apply_fused_body(x, y, sums, mean_rstd, running_mean, running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                       inv_count, eps, momentum, bits);
 }
@@ -545,6 +554,7 @@ bn_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, cons
                    bf16* __restrict__ dx, const float* __restrict__ mean_rstd, const float* __restrict__ gamma,
                    const float* __restrict__ sums, float* dgamma, float* dbeta, long long P, int C,
                    long long ldx, long long lddy, long long lddx, int relu, float grad_scale, float* zero_after) {
+  geeps_pdl_enter();
   bn_backward_body<BITS>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
                    zero_after);
 }
@@ -577,6 +587,7 @@ bn_forward_coop_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, float* 
                        float* running_mean, float* running_var, const float* __restrict__ gamma,
                        const float* __restrict__ beta, float* zero_after, int* bar, long long P, int C, long long ldx,
                        long long ldy, int relu, float inv_count, float eps, float momentum, uint8_t* bits) {
+  geeps_pdl_enter();
   channel_reduce_body<0>(x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
     bn_apply_fused_body(x, y, sums, mean_rstd, running_mean, running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
@@ -590,6 +601,7 @@ bn_backward_coop_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
                         bf16* __restrict__ dx, float* mean_rstd, const float* __restrict__ gamma, float* sums,
                         float* dgamma, float* dbeta, float* zero_after, int* bar, long long P, int C, long long ldx,
                         long long lddy, long long lddx, int relu, float grad_scale) {
+  geeps_pdl_enter();
   channel_reduce_body<BITS ? 3 : 1>(x, dy, y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
   if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
     bn_backward_body<BITS>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
@@ -601,6 +613,7 @@ bn_backward_coop_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
 // ---------------- ReLU backward / dropout ----------------
 __global__ void __launch_bounds__(256)
 relu_backward_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ y, bf16* __restrict__ dx, long long n8) {
+  geeps_pdl_enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += stride) {
     Bf8 d = ld8(dy + i * 8), v = ld8(y + i * 8), o;
@@ -614,6 +627,7 @@ relu_backward_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ y, bf
 __global__ void __launch_bounds__(256)
 relu_backward_2d_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ y, bf16* __restrict__ dx, long long P,
                         int C, long long lddy, long long ldy, long long lddx) {
+  geeps_pdl_enter();
   const int cv = C >> 3;
   const long long total = P * cv;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -631,6 +645,7 @@ relu_backward_2d_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ y,
 __global__ void __launch_bounds__(256)
 f32_to_bf16_2d_kernel(const float* __restrict__ src, bf16* __restrict__ dst, long long P, int C, long long lds,
                       long long ldd, int relu) {
+  geeps_pdl_enter();
   const int cv = C >> 3;
   const long long total = P * cv;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -650,6 +665,7 @@ f32_to_bf16_2d_kernel(const float* __restrict__ src, bf16* __restrict__ dst, lon
 __global__ void __launch_bounds__(256)
 relu_backward_colsum_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ y, bf16* __restrict__ dx,
                             float* __restrict__ out, long long P, int C, long long lddy, long long ldy, long long lddx) {
+  geeps_pdl_enter();
   extern __shared__ __align__(16) float sacc[];  // [rows][8 * slots]
   const SlotMap m(C);
   float a[8];
@@ -690,6 +706,7 @@ struct AddSrc { const bf16* p[3]; long long ld[3]; };
 template <int N, bool DENSE>
 __global__ void __launch_bounds__(256)
 add_2d_kernel(bf16* __restrict__ dst, const AddSrc src, long long total, int cv, long long ldd) {
+  geeps_pdl_enter();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     // a pixel number of 32 bits is found by a 32-bit division
@@ -719,6 +736,7 @@ __device__ __forceinline__ uint32_t mix32(uint64_t z) {
 __global__ void __launch_bounds__(256)
 dropout_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long long n, float p, unsigned long long seed,
                const int* __restrict__ step_ref) {
+  geeps_pdl_enter();
   if (step_ref != nullptr) seed += (unsigned long long)(long long)*step_ref;
   const float inv = 1.f / (1.f - p);
   const uint32_t thresh = (uint32_t)(p * 4294967296.0);
@@ -734,6 +752,7 @@ dropout_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long long n, fl
 __global__ void __launch_bounds__(256)
 lrn_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, bf16* __restrict__ scale, long long P, int C,
                    int size, float alpha, float beta, float k) {
+  geeps_pdl_enter();
   const long long total = P * C;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const int half = size / 2;
@@ -752,6 +771,7 @@ __global__ void __launch_bounds__(256)
 lrn_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ y, const bf16* __restrict__ scale,
                     const bf16* __restrict__ dy, bf16* __restrict__ dx, long long P, int C, int size, float alpha,
                     float beta, int relu_mask) {
+  geeps_pdl_enter();
   const long long total = P * C;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const int half = size / 2;
@@ -774,6 +794,7 @@ template <int HALF>
 __global__ void __launch_bounds__(256)
 lrn_forward_v8_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, bf16* __restrict__ scale, long long P, int C,
                       int size, float alpha, float beta, float k) {
+  geeps_pdl_enter();
   const int cv = C >> 3;
   const long long total = P * cv;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -817,6 +838,7 @@ __global__ void __launch_bounds__(256)
 lrn_backward_v8_kernel(const bf16* __restrict__ x, const bf16* __restrict__ y, const bf16* __restrict__ scale,
                        const bf16* __restrict__ dy, bf16* __restrict__ dx, long long P, int C, int size, float alpha,
                        float beta, int relu_mask, float* __restrict__ colsum) {
+  geeps_pdl_enter();
   // colsum (optional): per-channel sums of dx over all pixels - the bias gradient of the convolution whose
   // ReLU is folded in here.  The host sizes the grid so that gridDim * blockDim is a multiple of C/8: every
   // thread then keeps one channel group for all its pixels and sums in registers.
@@ -878,6 +900,7 @@ lrn_backward_v8_kernel(const bf16* __restrict__ x, const bf16* __restrict__ y, c
 template <typename T>
 __global__ void __launch_bounds__(256)
 nchw_to_nhwc_pix_kernel(const T* __restrict__ x, bf16* __restrict__ y, int B, int C, int HW, int Cpad) {
+  geeps_pdl_enter();
   const long long total = (long long)B * HW;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -900,6 +923,7 @@ nchw_to_nhwc_pix_kernel(const T* __restrict__ x, bf16* __restrict__ y, int B, in
 template <int S, int C, typename T>
 __global__ void __launch_bounds__(256)
 nchw_to_s2d_kernel(const T* __restrict__ x, bf16* __restrict__ y, int B, int H, int W, int Hs, int Ws, int Cpad) {
+  geeps_pdl_enter();
   constexpr int N = S * S * C;
   const long long total = (long long)B * Hs * Ws;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -942,6 +966,7 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 nchw_to_s2d43_tile_kernel(const T* __restrict__ x, bf16* __restrict__ y, int B, int H, int W, int Hs, int Ws, int Cpad,
                           int segs) {
+  geeps_pdl_enter();
   constexpr int S = 4, C = 3, PIX = 32, PITCH = 72;      // tile row pitch in elements: 144 bytes staggers the banks
   __shared__ __align__(16) bf16 tile[PIX * PITCH];
   const int lane = threadIdx.x & 31, dy = threadIdx.x >> 5;
@@ -982,6 +1007,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 nchw_to_s2d_generic_kernel(const T* __restrict__ x, bf16* __restrict__ y, int B, int C, int H, int W, int S,
                            int Hs, int Ws, int Cpad) {
+  geeps_pdl_enter();
   const long long total = (long long)B * Hs * Ws * Cpad;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -1089,6 +1115,7 @@ struct Bf16Quads {
 template <typename Src>
 __global__ void __launch_bounds__(256)
 s2d43_quad_kernel(Src src, bf16* __restrict__ y, unsigned npix, int Hs, int Ws, int Cpad) {
+  geeps_pdl_enter();
   __shared__ uint4 tile[8][16 * 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane & 1, px = lane >> 1;
   const unsigned base = (blockIdx.x * (blockDim.x >> 5) + warp) * 16u;
@@ -1170,13 +1197,14 @@ void launch_s2d43_quads(const Src& src, void* y, long long npix, int Hs, int Ws,
   const long long warps = (npix + 15) / 16;
   long long per_block = warps / (2 * geeps_sm_count());
   per_block = per_block < 1 ? 1 : (per_block > 8 ? 8 : per_block);
-  s2d43_quad_kernel<<<(unsigned)((warps + per_block - 1) / per_block), (unsigned)(32 * per_block), 0, st>>>(
+  geeps_launch(s2d43_quad_kernel<Src>, (unsigned)((warps + per_block - 1) / per_block), (unsigned)(32 * per_block), 0, st,
       src, (bf16*)y, (unsigned)npix, Hs, Ws, Cpad);
 }
 
 // any S >= 1 (S = 1: plain NHWC) and C <= 4: one thread per output element
 __global__ void __launch_bounds__(256)
 u8_xform_generic_kernel(XformDev t, bf16* __restrict__ y, int B, int C, int S, int Hs, int Ws, int Cpad) {
+  geeps_pdl_enter();
   const long long total = (long long)B * Hs * Ws * Cpad;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -1203,6 +1231,7 @@ u8_xform_generic_kernel(XformDev t, bf16* __restrict__ y, int B, int C, int S, i
 // g[r][c] = 0 where mask[c] == 0
 __global__ void __launch_bounds__(256)
 col_mask_kernel(float* __restrict__ g, const uint8_t* __restrict__ mask, long long rows, int cols, long long ld) {
+  geeps_pdl_enter();
   const long long total = rows * cols;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -1240,6 +1269,7 @@ __device__ __forceinline__ uint4 pool_bwd_pack(const __nv_bfloat162 (&acc)[4]) {
 __global__ void __launch_bounds__(256)
 maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, uint8_t* __restrict__ argmax,
                        const GeepsPoolGeom g) {
+  geeps_pdl_enter();
   const int cv = g.C >> 3;
   const int oh = blockIdx.x % g.OH, b = blockIdx.x / g.OH;
   const int ih0 = oh * g.stride - g.pad;
@@ -1286,6 +1316,7 @@ maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, uint8_t
 __global__ void __launch_bounds__(256)
 maxpool_backward_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ argmax, bf16* __restrict__ dx,
                         const GeepsPoolGeom g, int accumulate) {
+  geeps_pdl_enter();
   const int cv = g.C >> 3;
   const int ih = blockIdx.x % g.H, b = blockIdx.x / g.H;
   const int th = ih + g.pad;
@@ -1330,6 +1361,7 @@ maxpool_backward_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__
 __global__ void __launch_bounds__(256)
 maxpool_backward_smem_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ argmax, bf16* __restrict__ dx,
                              const GeepsPoolGeom g, int accumulate, int rows_per_block, int max_oh) {
+  geeps_pdl_enter();
   extern __shared__ __align__(16) uint8_t pool_smem[];
   const int cv = g.C >> 3;
   const int row_blocks = (g.H + rows_per_block - 1) / rows_per_block;
@@ -1407,6 +1439,7 @@ __device__ __forceinline__ unsigned pool_row() { return ROWS ? blockIdx.x * bloc
 template <bool ROWS>
 __global__ void __launch_bounds__(256)
 avgpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const GeepsPoolGeom g) {
+  geeps_pdl_enter();
   const int cv = g.C >> 3;
   const unsigned row = pool_row<ROWS>();
   if (ROWS && row >= (unsigned)g.B * (unsigned)g.OH) return;
@@ -1453,6 +1486,7 @@ avgpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const G
 template <bool ROWS>
 __global__ void __launch_bounds__(256)
 avgpool_backward_kernel(const bf16* __restrict__ dy, bf16* __restrict__ dx, const GeepsPoolGeom g, int accumulate) {
+  geeps_pdl_enter();
   const int cv = g.C >> 3;
   const unsigned row = pool_row<ROWS>();
   if (ROWS && row >= (unsigned)g.B * (unsigned)g.H) return;
@@ -1537,6 +1571,7 @@ __global__ void __launch_bounds__(256)
 softmax_ce_small_kernel(const float* __restrict__ logits, const long long* __restrict__ labels, float* loss_sum,
                   float* __restrict__ per_sample, bf16* __restrict__ dlogits, int C, long long ldl, long long ldd,
                   float loss_scale, float grad_scale, int* status) {
+  geeps_pdl_enter();
   __shared__ float sh[32];
   const int b = blockIdx.x;
   const float* row = logits + (long long)b * ldl;
@@ -1574,6 +1609,7 @@ __global__ void __launch_bounds__(1024)
 softmax_ce_kernel(const float* __restrict__ logits, const long long* __restrict__ labels, float* loss_sum,
                   float* __restrict__ per_sample, bf16* __restrict__ dlogits, int C, long long ldl, long long ldd,
                   float loss_scale, float grad_scale, int* status) {
+  geeps_pdl_enter();
   __shared__ float sh[32];
   constexpr int R = 3;
   const int b = blockIdx.x, T = blockDim.x, tid = threadIdx.x;
@@ -1657,9 +1693,9 @@ template <typename T>
 static int nchw_to_nhwc_launch(const T* x, void* y, int B, int C, int H, int W, int Cpad, cudaStream_t st) {
   const long long n = (long long)B * H * W * Cpad;
   if (Cpad % 4 == 0)
-    nchw_to_nhwc_pix_kernel<T><<<grid_1d((long long)B * H * W), 256, 0, st>>>(x, (bf16*)y, B, C, H * W, Cpad);
+    geeps_launch(nchw_to_nhwc_pix_kernel<T>, grid_1d((long long)B * H * W), 256, 0, st, x, (bf16*)y, B, C, H * W, Cpad);
   else
-    nchw_f32_to_nhwc_bf16_kernel<T><<<grid_1d(n), 256, 0, st>>>(x, (bf16*)y, B, C, H, W, Cpad);
+    geeps_launch(nchw_f32_to_nhwc_bf16_kernel<T>, grid_1d(n), 256, 0, st, x, (bf16*)y, B, C, H, W, Cpad);
   return CK();
 }
 
@@ -1675,12 +1711,12 @@ static int nchw_to_s2d_launch(const T* x, void* y, int B, int C, int H, int W, i
   }
   if (S == 4 && C == 3 && Cpad % 8 == 0 && Cpad >= 48 && Cpad <= 64 && (((uintptr_t)y) & 15) == 0) {
     const int segs = (Ws + 31) / 32;
-    nchw_to_s2d43_tile_kernel<T><<<(unsigned)((long long)B * Hs * segs), 128, 0, st>>>(x, (bf16*)y, B, H, W, Hs, Ws, Cpad,
+    geeps_launch(nchw_to_s2d43_tile_kernel<T>, (unsigned)((long long)B * Hs * segs), 128, 0, st, x, (bf16*)y, B, H, W, Hs, Ws, Cpad,
                                                                                       segs);
   } else if (S == 4 && C == 3)
-    nchw_to_s2d_kernel<4, 3, T><<<grid_1d((long long)B * Hs * Ws), 256, 0, st>>>(x, (bf16*)y, B, H, W, Hs, Ws, Cpad);
+    geeps_launch(nchw_to_s2d_kernel<4, 3, T>, grid_1d((long long)B * Hs * Ws), 256, 0, st, x, (bf16*)y, B, H, W, Hs, Ws, Cpad);
   else
-    nchw_to_s2d_generic_kernel<T><<<grid_1d((long long)B * Hs * Ws * Cpad), 256, 0, st>>>(x, (bf16*)y, B, C, H, W, S,
+    geeps_launch(nchw_to_s2d_generic_kernel<T>, grid_1d((long long)B * Hs * Ws * Cpad), 256, 0, st, x, (bf16*)y, B, C, H, W, S,
                                                                                          Hs, Ws, Cpad);
   return CK();
 }
@@ -1726,14 +1762,14 @@ int geeps_u8_transform_bf16(const GeepsU8Transform* p, void* stream) {
     q.end = p->x + (long long)p->B * 3 * p->Hin * p->Win;
     launch_s2d43_quads(q, p->y, npix, p->Hs, p->Ws, p->Cpad, st);
   } else {
-    u8_xform_generic_kernel<<<grid_1d((long long)p->B * p->Hs * p->Ws * p->Cpad), 256, 0, st>>>(t, (bf16*)p->y, p->B, p->C,
+    geeps_launch(u8_xform_generic_kernel, grid_1d((long long)p->B * p->Hs * p->Ws * p->Cpad), 256, 0, st, t, (bf16*)p->y, p->B, p->C,
                                                                                               S, p->Hs, p->Ws, p->Cpad);
   }
   return CK();
 }
 
 int geeps_col_mask_f32(float* g, const unsigned char* mask, long long rows, int cols, long long ld, void* stream) {
-  col_mask_kernel<<<grid_1d(rows * cols), 256, 0, (cudaStream_t)stream>>>(g, mask, rows, cols, ld);
+  geeps_launch(col_mask_kernel, grid_1d(rows * cols), 256, 0, (cudaStream_t)stream, g, mask, rows, cols, ld);
   return CK();
 }
 
@@ -1742,13 +1778,13 @@ int geeps_im2col(const void* x, void* col, const GeepsConvGeom* g, void* stream)
   const long long rows = (long long)g->B * g->OH * g->OW;
   const int kd = g->KH * g->KW * g->Cg;
   if (g->ldcol > kd)
-    zero_col_pad_kernel<<<grid_1d(rows * (g->ldcol - kd)), 256, 0, st>>>((bf16*)col, rows, kd, g->ldcol);
+    geeps_launch(zero_col_pad_kernel, grid_1d(rows * (g->ldcol - kd)), 256, 0, st, (bf16*)col, rows, kd, g->ldcol);
   const bool a8 = (g->Cg % 8 == 0) && (g->C % 8 == 0) && (g->c0 % 8 == 0) && (g->ldcol % 8 == 0);
   const bool a4 = (g->Cg % 4 == 0) && (g->C % 4 == 0) && (g->c0 % 4 == 0) && (g->ldcol % 4 == 0);
   const int wgrid = grid_1d(rows * 32);   // one warp per patch-matrix row
-  if (a8) im2col_kernel<8><<<wgrid, 256, 0, st>>>((const bf16*)x, (bf16*)col, *g);
-  else if (a4) im2col_kernel<4><<<wgrid, 256, 0, st>>>((const bf16*)x, (bf16*)col, *g);
-  else im2col_kernel<1><<<wgrid, 256, 0, st>>>((const bf16*)x, (bf16*)col, *g);
+  if (a8) geeps_launch(im2col_kernel<8>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
+  else if (a4) geeps_launch(im2col_kernel<4>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
+  else geeps_launch(im2col_kernel<1>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
   return CK();
 }
 
@@ -1756,8 +1792,8 @@ int geeps_col2im(const void* dcol, void* dx, const GeepsConvGeom* g, int accumul
   cudaStream_t st = (cudaStream_t)stream;
   const long long pix = (long long)g->B * g->H * g->W;
   const bool a8 = (g->Cg % 8 == 0) && (g->C % 8 == 0) && (g->c0 % 8 == 0) && (g->ldcol % 8 == 0);
-  if (a8) col2im_kernel<8><<<grid_1d(pix * (g->Cg / 8)), 256, 0, st>>>((const bf16*)dcol, (bf16*)dx, *g, accumulate);
-  else col2im_kernel<1><<<grid_1d(pix * g->Cg), 256, 0, st>>>((const bf16*)dcol, (bf16*)dx, *g, accumulate);
+  if (a8) geeps_launch(col2im_kernel<8>, grid_1d(pix * (g->Cg / 8)), 256, 0, st, (const bf16*)dcol, (bf16*)dx, *g, accumulate);
+  else geeps_launch(col2im_kernel<1>, grid_1d(pix * g->Cg), 256, 0, st, (const bf16*)dcol, (bf16*)dx, *g, accumulate);
   return CK();
 }
 
@@ -1777,11 +1813,11 @@ int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* be
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
-  channel_reduce_kernel<0><<<rg.grid, rg.threads, rg.smem, st>>>(
+  geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
-  bn_finalize_kernel<<<(C + 127) / 128, 128, 0, st>>>(sums, mean_rstd, running_mean, running_var, C,
+  geeps_launch(bn_finalize_kernel, (C + 127) / 128, 128, 0, st, sums, mean_rstd, running_mean, running_var, C,
                                                       1.f / (float)P, eps, momentum);
-  bn_apply_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
+  geeps_launch(bn_apply_kernel, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
                                                         ldy, relu);
   return CK();
 }
@@ -1793,9 +1829,9 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
-  channel_reduce_kernel<1><<<rg.grid, rg.threads, rg.smem, st>>>(
+  geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  bn_backward_kernel<false><<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
+  geeps_launch(bn_backward_kernel<false>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)y,
                                                            (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
                                                            ldx, lddy, lddx, relu, grad_scale, nullptr);
   return CK();
@@ -1836,9 +1872,9 @@ int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, cons
     return e == cudaSuccess ? CK() : (int)e;
   }
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
-  channel_reduce_kernel<0><<<rg.grid, rg.threads, rg.smem, st>>>(
+  geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
-  bn_apply_fused_kernel<<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
+  geeps_launch(bn_apply_fused_kernel, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
                                                               running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                                                               1.f / (float)P, eps, momentum, bits);
   return CK();
@@ -1862,16 +1898,16 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
   }
   const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
   if (bits != nullptr && relu) {
-    channel_reduce_kernel<3><<<rg.grid, rg.threads, rg.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)bits,
+    geeps_launch(channel_reduce_kernel<3>, rg.grid, rg.threads, rg.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits,
                                                                    mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-    bn_backward_kernel<true><<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
+    geeps_launch(bn_backward_kernel<true>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
                                                              mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx,
                                                              relu, grad_scale, zero_after);
     return CK();
   }
-  channel_reduce_kernel<1><<<rg.grid, rg.threads, rg.smem, st>>>(
+  geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  bn_backward_kernel<false><<<ag.grid, ag.threads, ag.smem, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y,
+  geeps_launch(bn_backward_kernel<false>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)y,
                                                            (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
                                                            ldx, lddy, lddx, relu, grad_scale, zero_after);
   return CK();
@@ -1881,12 +1917,12 @@ int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, f
                  void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if ((C % 8) || (ldx % 8) || C > 4096) {
-    colsum_simple_kernel<<<(C + 127) / 128, 128, 0, st>>>((const bf16*)x, out, P, C, ldx, scale, !zero_first);
+    geeps_launch(colsum_simple_kernel, (C + 127) / 128, 128, 0, st, (const bf16*)x, out, P, C, ldx, scale, !zero_first);
     return CK();
   }
   if (zero_first) cudaMemsetAsync(out, 0, sizeof(float) * C, st);
   const SlotGrid rg = reduce_grid(P, C, 1);
-  channel_reduce_kernel<2><<<rg.grid, rg.threads, rg.smem, st>>>(
+  geeps_launch(channel_reduce_kernel<2>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, out, P, C, ldx, 0, 0, scale);
   return CK();
 }
@@ -1897,14 +1933,14 @@ int geeps_copy_f32(float* dst, const float* src, long long n, void* stream) {
 
 int geeps_relu_backward(const void* dy, const void* y, void* dx, long long n, void* stream) {
   if (n % 8) return (int)cudaErrorInvalidValue;
-  relu_backward_kernel<<<grid_1d(n / 8), 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const bf16*)y, (bf16*)dx, n / 8);
+  geeps_launch(relu_backward_kernel, grid_1d(n / 8), 256, 0, (cudaStream_t)stream, (const bf16*)dy, (const bf16*)y, (bf16*)dx, n / 8);
   return CK();
 }
 
 int geeps_relu_backward_2d(const void* dy, const void* y, void* dx, long long P, int C, long long lddy, long long ldy,
                            long long lddx, void* stream) {
   if (C % 8 || lddy % 8 || ldy % 8 || lddx % 8) return (int)cudaErrorInvalidValue;
-  relu_backward_2d_kernel<<<grid_1d(P * (C / 8)), 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const bf16*)y,
+  geeps_launch(relu_backward_2d_kernel, grid_1d(P * (C / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)dy, (const bf16*)y,
                                                                                  (bf16*)dx, P, C, lddy, ldy, lddx);
   return CK();
 }
@@ -1914,14 +1950,14 @@ int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* c
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(colsum, 0, sizeof(float) * C, st);
   const SlotGrid rg = slot_grid(P, C, 4, 8, 1);
-  relu_backward_colsum_kernel<<<rg.grid, rg.threads, rg.smem, st>>>(
+  geeps_launch(relu_backward_colsum_kernel, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)dy, (const bf16*)y, (bf16*)dx, colsum, P, C, lddy, ldy, lddx);
   return CK();
 }
 int geeps_f32_to_bf16_2d(const float* src, void* dst, long long P, int C, long long lds, long long ldd, int relu,
                          void* stream) {
   if (C % 8 || lds % 4 || ldd % 8 || ((uintptr_t)src & 15) || ((uintptr_t)dst & 15)) return (int)cudaErrorInvalidValue;
-  f32_to_bf16_2d_kernel<<<grid_1d(P * (C / 8)), 256, 0, (cudaStream_t)stream>>>(src, (bf16*)dst, P, C, lds, ldd, relu);
+  geeps_launch(f32_to_bf16_2d_kernel, grid_1d(P * (C / 8)), 256, 0, (cudaStream_t)stream, src, (bf16*)dst, P, C, lds, ldd, relu);
   return CK();
 }
 int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s2, long long P, int C, long long ldd,
@@ -1934,7 +1970,7 @@ int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s
   const bool dense = ldd == C && ld0 == C && (n < 2 || ld1 == C) && (n < 3 || ld2 == C);
   const int grid = grid_1d(total);
   cudaStream_t st = (cudaStream_t)stream;
-#define ADD_2D(N, DENSE) add_2d_kernel<N, DENSE><<<grid, 256, 0, st>>>((bf16*)dst, src, total, C / 8, ldd)
+#define ADD_2D(N, DENSE) geeps_launch(add_2d_kernel<N, DENSE>, grid, 256, 0, st, (bf16*)dst, src, total, C / 8, ldd)
   if (dense) { if (n == 3) ADD_2D(3, true); else if (n == 2) ADD_2D(2, true); else ADD_2D(1, true); }
   else { if (n == 3) ADD_2D(3, false); else if (n == 2) ADD_2D(2, false); else ADD_2D(1, false); }
 #undef ADD_2D
@@ -1942,12 +1978,12 @@ int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s
 }
 
 int geeps_dropout(const void* x, void* y, long long n, float p, unsigned long long seed, void* stream) {
-  dropout_kernel<<<grid_1d(n), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, n, p, seed, nullptr);
+  geeps_launch(dropout_kernel, grid_1d(n), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, n, p, seed, nullptr);
   return CK();
 }
 int geeps_dropout_ref(const void* x, void* y, long long n, float p, unsigned long long seed, const int* step_ref,
                       void* stream) {
-  dropout_kernel<<<grid_1d(n), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, n, p, seed, step_ref);
+  geeps_launch(dropout_kernel, grid_1d(n), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, n, p, seed, step_ref);
   return CK();
 }
 
@@ -1956,13 +1992,13 @@ int geeps_lrn_forward(const void* x, void* y, void* rscale, long long P, int C, 
   const int g8 = grid_1d(P * (C / 8));
   cudaStream_t st8 = (cudaStream_t)stream;
   if (C % 8 == 0 && size == 5)
-    lrn_forward_v8_kernel<2><<<g8, 256, 0, st8>>>((const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
+    geeps_launch(lrn_forward_v8_kernel<2>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
   else if (C % 8 == 0 && size == 3)
-    lrn_forward_v8_kernel<1><<<g8, 256, 0, st8>>>((const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
+    geeps_launch(lrn_forward_v8_kernel<1>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
   else if (C % 8 == 0 && size == 7)
-    lrn_forward_v8_kernel<3><<<g8, 256, 0, st8>>>((const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
+    geeps_launch(lrn_forward_v8_kernel<3>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
   else
-    lrn_forward_kernel<<<grid_1d(P * C), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size,
+    geeps_launch(lrn_forward_kernel, grid_1d(P * C), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size,
                                                                         alpha, beta, k);
   return CK();
 }
@@ -1982,13 +2018,13 @@ int geeps_lrn_backward(const void* x, const void* y, const void* rscale, const v
     cudaMemsetAsync(colsum, 0, sizeof(float) * C, st8);
   }
   if (C % 8 == 0 && size == 5)
-    lrn_backward_v8_kernel<2><<<g8, 256, cs_smem, st8>>>((const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
+    geeps_launch(lrn_backward_v8_kernel<2>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
   else if (C % 8 == 0 && size == 3)
-    lrn_backward_v8_kernel<1><<<g8, 256, cs_smem, st8>>>((const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
+    geeps_launch(lrn_backward_v8_kernel<1>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
   else if (C % 8 == 0 && size == 7)
-    lrn_backward_v8_kernel<3><<<g8, 256, cs_smem, st8>>>((const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
+    geeps_launch(lrn_backward_v8_kernel<3>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
   else
-    lrn_backward_kernel<<<grid_1d(P * C), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (const bf16*)y, (const bf16*)rscale,
+    geeps_launch(lrn_backward_kernel, grid_1d(P * C), 256, 0, (cudaStream_t)stream, (const bf16*)x, (const bf16*)y, (const bf16*)rscale,
                                                                          (const bf16*)dy, (bf16*)dx, P, C, size, alpha,
                                                                          beta, relu_mask);
   return CK();
@@ -1996,7 +2032,7 @@ int geeps_lrn_backward(const void* x, const void* y, const void* rscale, const v
 
 int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream) {
   if (g->C % 8 || g->ldx % 8 || g->ldy % 8 || g->K * g->K > 255) return (int)cudaErrorInvalidValue;
-  maxpool_forward_kernel<<<g->B * g->OH, pool_block(g->C / 8), 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y,
+  geeps_launch(maxpool_forward_kernel, g->B * g->OH, pool_block(g->C / 8), 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y,
                                                                                         (uint8_t*)argmax, *g);
   return CK();
 }
@@ -2014,11 +2050,11 @@ int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const G
       attr_set = true;
     }
     const int row_blocks = (g->H + rows_per_block - 1) / rows_per_block;
-    maxpool_backward_smem_kernel<<<g->B * row_blocks, pool_block(g->C / 8), smem, (cudaStream_t)stream>>>(
+    geeps_launch(maxpool_backward_smem_kernel, g->B * row_blocks, pool_block(g->C / 8), smem, (cudaStream_t)stream,
         (const bf16*)dy, (const uint8_t*)argmax, (bf16*)dx, *g, accumulate, rows_per_block, max_oh);
     return CK();
   }
-  maxpool_backward_kernel<<<g->B * g->H, pool_block(g->C / 8), 0, (cudaStream_t)stream>>>(
+  geeps_launch(maxpool_backward_kernel, g->B * g->H, pool_block(g->C / 8), 0, (cudaStream_t)stream,
       (const bf16*)dy, (const uint8_t*)argmax, (bf16*)dx, *g, accumulate);
   return CK();
 }
@@ -2038,8 +2074,8 @@ int geeps_avgpool_forward(const void* x, void* y, const GeepsPoolGeom* g, void* 
   const PoolGrid pg = avgpool_grid(g->C / 8, g->OW, (long long)g->B * g->OH, g->K <= 3);
   cudaStream_t st = (cudaStream_t)stream;
   if (pg.grid.x == 0) return 0;
-  if (pg.block.z == 1) avgpool_forward_kernel<false><<<pg.grid, pg.block, 0, st>>>((const bf16*)x, (bf16*)y, *g);
-  else avgpool_forward_kernel<true><<<pg.grid, pg.block, 0, st>>>((const bf16*)x, (bf16*)y, *g);
+  if (pg.block.z == 1) geeps_launch(avgpool_forward_kernel<false>, pg.grid, pg.block, 0, st, (const bf16*)x, (bf16*)y, *g);
+  else geeps_launch(avgpool_forward_kernel<true>, pg.grid, pg.block, 0, st, (const bf16*)x, (bf16*)y, *g);
   return CK();
 }
 int geeps_avgpool_backward(const void* dy, void* dx, const GeepsPoolGeom* g, int accumulate, void* stream) {
@@ -2048,9 +2084,9 @@ int geeps_avgpool_backward(const void* dy, void* dx, const GeepsPoolGeom* g, int
   cudaStream_t st = (cudaStream_t)stream;
   if (pg.grid.x == 0) return 0;
   if (pg.block.z == 1)
-    avgpool_backward_kernel<false><<<pg.grid, pg.block, 0, st>>>((const bf16*)dy, (bf16*)dx, *g, accumulate);
+    geeps_launch(avgpool_backward_kernel<false>, pg.grid, pg.block, 0, st, (const bf16*)dy, (bf16*)dx, *g, accumulate);
   else
-    avgpool_backward_kernel<true><<<pg.grid, pg.block, 0, st>>>((const bf16*)dy, (bf16*)dx, *g, accumulate);
+    geeps_launch(avgpool_backward_kernel<true>, pg.grid, pg.block, 0, st, (const bf16*)dy, (bf16*)dx, *g, accumulate);
   return CK();
 }
 
@@ -2063,7 +2099,7 @@ int geeps_softmax_ce(const float* logits, const long long* labels, float* loss_s
   // 1000 classes and less from there (32 x 2000 8.5 -> 6.5 us, 32 x 4000 10.5 -> 7.0, 256 x 4000 10.6 -> 8.7; rows off a
   // 16-byte boundary 8.5, 8.5 and 10.6), 32 x 6000 12.6 -> 8.5, 32 x 21841 54 -> 8.
   if (C < 4096) {
-    softmax_ce_small_kernel<<<B, 256, 0, st>>>(logits, labels, loss_sum, per_sample, (bf16*)dlogits, C, ldl, ldd, loss_scale,
+    geeps_launch(softmax_ce_small_kernel, B, 256, 0, st, logits, labels, loss_sum, per_sample, (bf16*)dlogits, C, ldl, ldd, loss_scale,
                                                grad_scale, status);
     return CK();
   }
@@ -2072,10 +2108,10 @@ int geeps_softmax_ce(const float* logits, const long long* labels, float* loss_s
   const bool vec = ldl % 4 == 0 && ((uintptr_t)logits & 15) == 0 &&
                    (dlogits == nullptr || (ldd % 8 == 0 && ((uintptr_t)dlogits & 15) == 0));
   if (vec)
-    softmax_ce_kernel<true><<<B, threads, 0, st>>>(logits, labels, loss_sum, per_sample, (bf16*)dlogits, C, ldl, ldd,
+    geeps_launch(softmax_ce_kernel<true>, B, threads, 0, st, logits, labels, loss_sum, per_sample, (bf16*)dlogits, C, ldl, ldd,
                                                    loss_scale, grad_scale, status);
   else
-    softmax_ce_kernel<false><<<B, threads, 0, st>>>(logits, labels, loss_sum, per_sample, (bf16*)dlogits, C, ldl, ldd,
+    geeps_launch(softmax_ce_kernel<false>, B, threads, 0, st, logits, labels, loss_sum, per_sample, (bf16*)dlogits, C, ldl, ldd,
                                                     loss_scale, grad_scale, status);
   return CK();
 }
