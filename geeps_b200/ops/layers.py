@@ -201,6 +201,7 @@ class Conv2d(Layer):
         self.s2d, self.orig_k = s2d, k
         self.dy_is_masked = False       # set by Net when the consumer of the output applies this layer's ReLU mask
         self.bias_grad_src = None       # set by Net: the consumer's backward already summed dy per channel into this
+        self.wgrad_side = None          # set by Concat: (stream, event) its weight gradient runs on during a backward pass
         if s2d:
             assert stride == s2d and pad == 0 and groups == 1
             k, stride = -(-k // s2d), 1
@@ -320,39 +321,49 @@ class Conv2d(Layer):
                 bias_done = True
             else:
                 dy = self._relu_mask(dy)
-        gw = self.g32["weight"]
         if self.has_bias and not bias_done:
             if self.bias_grad_src is not None:
                 F.copy_f32(self.g32["bias"], self.bias_grad_src)
             else:
                 F.colsum(dy, self.g32["bias"])
-        w16 = self.p16["weight"]
+        if self.wgrad_side is not None and self.need_dx:
+            # nothing of this pass waits for the weight gradient: it runs beside what follows the data gradient
+            side, event = self.wgrad_side
+            F.stream_order(torch.cuda.current_stream(self.device), side, event)
+            self._data_gradient(dy)
+            with torch.cuda.stream(side):
+                self._weight_gradient(dy)
+            return self.dx
         for g in range(self.groups):
+            self._weight_gradient(dy, g)
+            if self.need_dx:
+                self._data_gradient(dy, g)
+        return self.dx
+
+    def _weight_gradient(self, dy, group=None):
+        gw = self.g32["weight"]
+        for g in range(self.groups) if group is None else (group,):
+            rows = slice(g * self.og, (g + 1) * self.og)
             if self.implicit:
-                xg, dy4 = self._x4(self.x, g), self._y4(dy, g)
-                F.conv_tc(F.CONV_WGRAD, xg, dy4, gw[g * self.og:(g + 1) * self.og], self.k, self.pad,
-                          stride=self.stride)
-                if self.need_dx and self.implicit_dgrad:
-                    F.conv_tc(F.CONV_DGRAD, self._x4(self.dx, g), dy4, w16[g * self.og:(g + 1) * self.og],
-                              self.k, self.pad, stride=self.stride)
-                elif self.need_dx:
-                    F.gemm(dy[:, g * self.og:(g + 1) * self.og], w16[g * self.og:(g + 1) * self.og], self.dcol, b_mn=True)
-                    F.col2im(self.dcol, self.dx, self.geoms[g])
+                F.conv_tc(F.CONV_WGRAD, self._x4(self.x, g), self._y4(dy, g), gw[rows], self.k, self.pad, stride=self.stride)
                 continue
-            dyg = dy[:, g * self.og:(g + 1) * self.og]
             a = self.x.view(self.M, -1) if self.pointwise else self.cols[g]
             # dW_g[og, ld] = dy_g^T @ col_g      (both operands stored K-outermost)
-            F.gemm(dyg, a, gw[g * self.og:(g + 1) * self.og], a_mn=True, b_mn=True, split_k=0)
-            if self.need_dx:
-                wg = w16[g * self.og:(g + 1) * self.og]
-                if self.pointwise:
-                    F.gemm(dyg, wg, self.dx.view(self.M, -1), b_mn=True)
-                else:
-                    F.gemm(dyg, wg, self.dcol, b_mn=True)
-                    F.col2im(self.dcol, self.dx, self.geoms[g])
-        if self.col_mask_dev is not None:
+            F.gemm(dy[:, rows], a, gw[rows], a_mn=True, b_mn=True, split_k=0)
+        if self.col_mask_dev is not None and group in (None, self.groups - 1):
             F.col_mask(gw, self.col_mask_dev)
-        return self.dx
+
+    def _data_gradient(self, dy, group=None):
+        w16 = self.p16["weight"]
+        for g in range(self.groups) if group is None else (group,):
+            rows = slice(g * self.og, (g + 1) * self.og)
+            if self.implicit and self.implicit_dgrad:
+                F.conv_tc(F.CONV_DGRAD, self._x4(self.dx, g), self._y4(dy, g), w16[rows], self.k, self.pad, stride=self.stride)
+            elif self.pointwise:
+                F.gemm(dy[:, rows], w16[rows], self.dx.view(self.M, -1), b_mn=True)
+            else:
+                F.gemm(dy[:, rows], w16[rows], self.dcol, b_mn=True)
+                F.col2im(self.dcol, self.dx, self.geoms[g])
 
     def _relu_mask(self, dy, colsum=None):
         if not hasattr(self, "_dy_masked"):

@@ -389,3 +389,35 @@ def test_bf16_only_weight_publish_trains_identically():
             assert mod.ps.last_error() == 0
             mod.close()
     assert losses[True] == pytest.approx(losses[False], rel=1e-3), losses
+
+
+def test_concurrent_module_backward_matches_the_serial_one():
+    """Branches and weight gradients on side streams against one stream: gradients complete when backward returns.  The
+    slices of a weight gradient meet in fp32 atomics, in any order; everything else is the same arithmetic."""
+    from geeps_b200.models.net import Concat
+    dev = torch.device("cuda:0")
+    conv = lambda n, c, k: [Conv2d(n, c, k, pad=k // 2, bias=False, std=0.0), BatchNorm(n + "_bn", relu=True)]   # noqa: E731
+    results = []
+    for concurrent in (True, False):
+        gen = torch.Generator(device=dev).manual_seed(3)
+        m = Concat("m", [conv("a", 32, 1), conv("b", 32, 1) + conv("c", 48, 3), conv("d", 16, 3) + conv("e", 16, 3) + conv("f", 24, 3),
+                         [Pool("avg", 3, 1, pad=1, ceil_mode=False)] + conv("g", 32, 1)], concurrent=concurrent)
+        m.setup((4, 14, 14, 64), dev)
+        for l in m.sublayers():
+            for sp in l.param_specs():
+                w = torch.randn(sp.shape, device=dev, generator=gen) * 0.1 + (1.0 if sp.name == "gamma" else 0.0)
+                l.p32[sp.name], l.p16[sp.name], l.g32[sp.name] = w, w.to(torch.bfloat16), torch.full_like(w, 9.0)
+        x = torch.randn(4, 14, 14, 64, device=dev, generator=gen).to(torch.bfloat16)
+        dy = torch.randn(4 * 14 * 14, 136, device=dev, generator=gen).to(torch.bfloat16)
+        torch.cuda.synchronize()
+        for _ in range(3):
+            y = m.forward(x)
+            dx = m.backward(dy)
+            grads = [l.g32[sp.name].clone() for l in m.sublayers() for sp in l.param_specs()]    # on the caller's stream
+        assert all(l.wgrad_side is None for l in m.sublayers() if isinstance(l, Conv2d))
+        results.append([y.clone(), dx.clone()] + grads)
+    torch.cuda.synchronize()
+    for a, b in zip(*results):
+        # sums of BatchNorm statistics and of gradient slices in another order: some 2^-24 per addition, roundings to bf16
+        # between the layers of a branch where such a difference meets a tie
+        assert (a.float() - b.float()).norm() <= 2e-3 * b.float().norm()
