@@ -37,6 +37,8 @@ constexpr int PANEL_BYTES = 64 * BK * 2;     // one MN-major panel: 64 k-rows x 
 constexpr int MAX_STAGES = 8;
 constexpr uint64_t WAIT_BUDGET_NS = 2000000000ull;
 constexpr int C_SLAB_BYTES = BM * 128;
+constexpr int kGroups = 2;                   // epilogue groups of four warps, which take alternate column slabs
+constexpr int kThreads = 64 + 128 * kGroups;
 
 enum { MODE_FWD = 0, MODE_DGRAD = 1, MODE_WGRAD = 2 };
 
@@ -57,6 +59,7 @@ struct ConvDev {
   int rows;                       // bw * bh * bnb
   int bn, n_valid;                // tile width; valid output columns (fwd: Og, dgrad: Cg, wgrad: panels * 64)
   int m_tiles, n_tiles, kt_total, split_k, stages, tmem_cols;
+  int slabs;                      // staging slabs: two per epilogue group that has one to fill
   int relu, zero_fill_c;          // wgrad: a channel coordinate outside X, for panels past the last one
   int ch_valid;                   // wgrad: channels per tap (cg)
   int narrow;                     // fwd / dgrad: result leaves in 32-channel (64-byte) slabs, see the host code
@@ -96,7 +99,7 @@ __device__ __forceinline__ Box decode_box(const ConvDev& d, int i, int wt, int h
 // tmA: activations of the M side (fwd: X, dgrad: dY, wgrad: dY); tmB: fwd/dgrad: W as (ci, tap, co),
 // wgrad: X; tmC: fwd: Y, dgrad: dX (4-D bf16), wgrad: dW as (ci, tap, co) fp32.
 template <int MODE>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ OutMaps tmC, const ConvDev d) {
   constexpr bool A_MN = MODE == MODE_WGRAD;
@@ -107,7 +110,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* cslab = tiles + (size_t)d.stages * STAGE_BYTES;
-  SmemCtl* ctl = (SmemCtl*)(cslab + 2 * C_SLAB_BYTES);
+  SmemCtl* ctl = (SmemCtl*)(cslab + d.slabs * C_SLAB_BYTES);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = d.stages;
@@ -125,7 +128,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) { tc05::mbar_init(&ctl->full[s], 1); tc05::mbar_init(&ctl->empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { tc05::mbar_init(&ctl->tmem_full[a], 1); tc05::mbar_init(&ctl->tmem_empty[a], 4); }
+    for (int a = 0; a < 2; ++a) { tc05::mbar_init(&ctl->tmem_full[a], 1); tc05::mbar_init(&ctl->tmem_empty[a], 4 * kGroups); }
     ctl->abort_flag = 0;
     tc05::mbar_fence_init();
   }
@@ -258,10 +261,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else {
     // ---------------- epilogue: TMEM -> registers -> swizzled slab -> TMA store ----------------
-    const int q = warp & 3;
+    const int q = warp & 3, grp = (warp - 2) >> 2;
     uint32_t tile_i = 0, slab_i = 0;
     const int cols_per_slab = (MODE == MODE_WGRAD || d.narrow) ? 32 : 64;
-    const bool issuer = threadIdx.x == 64;
+    const bool issuer = threadIdx.x == 64 + 128 * grp;
     const int rloc = q * 32 + lane;
     // wide slab: 128-byte rows, 128-byte swizzle (16-byte chunk ^ row % 8); narrow slab: 64-byte rows, 64-byte
     // swizzle (chunk ^ (row / 2) % 4)
@@ -284,11 +287,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (MODE == MODE_FWD) mb = decode_box(d, mi, d.wt, d.ht);
       if (MODE == MODE_DGRAD) mb = decode_box(d, mi, cq.wt, cq.ht);
 #pragma unroll 1
-      for (int c = 0; c < BN; c += cols_per_slab) {
+      for (int c = grp * cols_per_slab; c < BN; c += kGroups * cols_per_slab) {
         if (n0 + c >= d.n_valid) break;
-        uint8_t* slab = cslab + (size_t)(slab_i & 1u) * C_SLAB_BYTES;
+        uint8_t* slab = cslab + (size_t)(2 * grp + (slab_i & 1u)) * C_SLAB_BYTES;
         if (issuer) tc05::bulk_wait_read<1>();
-        tc05::named_bar_sync(1, 128);
+        tc05::named_bar_sync(1 + grp, 128);
         for (int h = 0; h < cols_per_slab; h += 32) {
           if (n0 + c + h >= d.n_valid) break;      // columns past the tensor's extent are clipped by the store anyway
           uint32_t r[32];
@@ -325,7 +328,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         tc05::fence_proxy_async_smem();
-        tc05::named_bar_sync(1, 128);
+        tc05::named_bar_sync(1 + grp, 128);
         if (issuer) {
           if (MODE == MODE_WGRAD) {
             const int panel = (n0 + c) >> 6;
@@ -348,7 +351,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   }
 
-  if (threadIdx.x == 64) tc05::bulk_wait<0>();
+  if (threadIdx.x == 64 || threadIdx.x == 192) tc05::bulk_wait<0>();
   tc05::fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0 && ctl->abort_flag)
@@ -448,14 +451,14 @@ template <int MODE>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tc, const ConvDev& d, int grid,
            cudaStream_t st) {
   const int stage_bytes = A_STAGE_BYTES + d.bn * BK * 2;
-  const size_t smem = (size_t)d.stages * stage_bytes + 2 * C_SLAB_BYTES + sizeof(SmemCtl) + 1024;
+  const size_t smem = (size_t)d.stages * stage_bytes + d.slabs * C_SLAB_BYTES + sizeof(SmemCtl) + 1024;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(conv_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  geeps_launch(conv_tc_kernel<MODE>, grid, 192, smem, st, ta, tb, tc, d);
+  geeps_launch(conv_tc_kernel<MODE>, grid, kThreads, smem, st, ta, tb, tc, d);
   return (int)cudaGetLastError();
 }
 
@@ -682,7 +685,8 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
   while (tmem_cols < 2 * d.bn) tmem_cols <<= 1;
   d.tmem_cols = tmem_cols;
   const int stage_bytes = A_STAGE_BYTES + d.bn * BK * 2;
-  d.stages = (200 * 1024 - 2 * C_SLAB_BYTES) / stage_bytes;
+  d.slabs = d.bn > (p->mode == MODE_WGRAD || d.narrow ? 32 : 64) ? 4 : 2;
+  d.stages = (224 * 1024 - d.slabs * C_SLAB_BYTES) / stage_bytes;
   if (d.stages > MAX_STAGES) d.stages = MAX_STAGES;
   if (d.stages < 2) d.stages = 2;
   const long long num_tiles = (long long)d.m_tiles * d.n_tiles * d.split_k;

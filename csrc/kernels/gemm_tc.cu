@@ -7,8 +7,9 @@
 // forward (X W^T), data-gradient (dY W) and weight-gradient (dY^T X) products of FC and
 // im2col-conv layers all run here without materialising a transpose.
 //
-// Persistent CTAs (one per SM) of 6 warps: warp 0 TMA producer, warp 1 MMA issuer + TMEM owner,
-// warps 2-5 epilogue (one TMEM lane quarter each).  Two accumulators live in TMEM, so the epilogue
+// Persistent CTAs (one per SM) of 10 warps: warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, two groups of four
+// epilogue warps (one TMEM lane quarter each), which take alternate column slabs: a product with a short K is bound by its
+// epilogue (fp32 gradients: 21841 x 1024, K = 32: 22.5 us with one group, 18.2 with two; 4096 x 4096, K = 256: 20.0, 18.4).  Two accumulators live in TMEM, so the epilogue
 // of a tile overlaps the main loop of the next one.  Tile 128 x BN x 64 with BN any multiple of 32
 // up to 256 (chosen per problem so that narrow outputs do not pad the MMA); partial tiles are
 // handled by TMA zero fill on loads and bounds checks on stores, so any M, N, K work as
@@ -37,7 +38,9 @@ constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2;   // 16 KB
 constexpr int MAX_STAGES = 8;
 constexpr uint64_t WAIT_BUDGET_NS = 2000000000ull;  // 2 s
-constexpr int C_SLAB_BYTES = BM * 128;       // epilogue staging slab: 128 rows x 128 bytes, two of them
+constexpr int C_SLAB_BYTES = BM * 128;       // epilogue staging slab: 128 rows x 128 bytes, two per epilogue group
+constexpr int epi_groups(bool cl) { return cl ? 1 : 2; }
+constexpr int gemm_threads(bool cl) { return 64 + 128 * epi_groups(cl); }
 
 struct GemmDev {
   void* C; const float* bias; int* status;
@@ -48,6 +51,7 @@ struct GemmDev {
   int tmem_cols;    // power of two >= 2 * bn: two accumulators, so the epilogue of a tile overlaps the next main loop
   int m_tiles, n_tiles;
   int cluster;      // > 1: K slices of one tile per cluster of this many CTAs (split_k is then the same number)
+  int slabs;        // staging slabs: two per epilogue group that has one to fill
   int tma_store;    // 1: epilogue stages 128-byte-wide slabs in swizzled smem and stores them with TMA
 };
 
@@ -87,7 +91,7 @@ __device__ __forceinline__ uint32_t part_off(int r, int q, int bn) { return (uin
 // Consecutive CTAs take consecutive M tiles of the same N tile, so the B tile they share stays in L2.
 // CL: a cluster of d.cluster CTAs per tile, one K slice each.
 template <bool A_MN, bool B_MN, bool CL>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(gemm_threads(CL), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const GemmDev d) {
   extern __shared__ uint8_t smem_raw[];
@@ -95,8 +99,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int B_STAGE_BYTES = BN * BK * 2;
   const int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* cslab = tiles + (size_t)d.stages * STAGE_BYTES;          // 2 x C_SLAB_BYTES, 1024-byte aligned
-  SmemCtl* ctl = (SmemCtl*)(cslab + (CL ? 0 : 2 * C_SLAB_BYTES));   // a cluster stages its tile in the operand ring
+  uint8_t* cslab = tiles + (size_t)d.stages * STAGE_BYTES;          // the slabs, 1024-byte aligned
+  SmemCtl* ctl = (SmemCtl*)(cslab + (CL ? 0 : d.slabs * C_SLAB_BYTES));   // a cluster stages its tile in the operand ring
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = d.stages;
@@ -110,7 +114,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) { tc05::mbar_init(&ctl->full[s], 1); tc05::mbar_init(&ctl->empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { tc05::mbar_init(&ctl->tmem_full[a], 1); tc05::mbar_init(&ctl->tmem_empty[a], 4); }
+    for (int a = 0; a < 2; ++a) { tc05::mbar_init(&ctl->tmem_full[a], 1); tc05::mbar_init(&ctl->tmem_empty[a], 4 * epi_groups(CL)); }
     ctl->abort_flag = 0;
     tc05::mbar_fence_init();
   }
@@ -207,6 +211,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else {
     // ---------------- epilogue: TMEM -> registers -> global ----------------
     const int q = warp & 3;  // TMEM lane quarter this warp may access
+    constexpr int G = epi_groups(CL);
+    const int grp = (warp - 2) >> 2;
     uint32_t tile_i = 0, slab_i = 0;
     for (int t = t_first; t < num_tiles; t += t_step, ++tile_i) {
       const int mn = t % tiles_mn, z = t / tiles_mn;
@@ -237,7 +243,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // 128-byte-wide slabs (64 bf16 or 32 fp32 columns) go through swizzled smem and leave with one
         // TMA store (or reduce-add for split-K) each: coalesced, asynchronous, clipped at the matrix edge
         const int cols_per_slab = d.out_fp32 ? 32 : 64;
-        const bool issuer = threadIdx.x == 64;
+        const bool issuer = threadIdx.x == 64 + 128 * grp;
         const int rloc = q * 32 + lane;          // row inside the tile = TMEM lane
         const uint32_t row_off = (uint32_t)rloc * 128u, rsw = (uint32_t)(rloc & 7);
         // everything that does not depend on the column is hoisted out of the slab loop
@@ -247,11 +253,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const bool relu = d.relu != 0;
         const int n_lim = (int)d.N;
 #pragma unroll 1
-        for (int c = 0; c < BN; c += cols_per_slab) {
+        for (int c = grp * cols_per_slab; c < BN; c += G * cols_per_slab) {
           if ((long long)n0 + c >= d.N) break;
-          uint8_t* slab = cslab + (size_t)(slab_i & 1u) * C_SLAB_BYTES;
-          if (issuer) tc05::bulk_wait_read<1>();   // the slab stored two slabs ago has been read out
-          tc05::named_bar_sync(1, 128);
+          uint8_t* slab = cslab + (size_t)(2 * grp + (slab_i & 1u)) * C_SLAB_BYTES;
+          if (issuer) tc05::bulk_wait_read<1>();   // the slab this group stored two slabs ago has been read out
+          tc05::named_bar_sync(1 + grp, 128);
           for (int h = 0; h < cols_per_slab; h += 32) {
             uint32_t r[32];
             tc05::tmem_ld_32x32(tacc + (uint32_t)(c + h), r);
@@ -293,7 +299,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
           }
           tc05::fence_proxy_async_smem();
-          tc05::named_bar_sync(1, 128);
+          tc05::named_bar_sync(1 + grp, 128);
           if (issuer) {
             if (d.split_k > 1) tc05::tma_reduce_add_2d(&tmC, slab, n0 + c, m0);
             else tc05::tma_store_2d(&tmC, slab, n0 + c, m0);
@@ -303,7 +309,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
       } else {
   #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = grp * 32; c < BN; c += G * 32) {
           uint32_t r[32];
           tc05::tmem_ld_32x32(tacc + (uint32_t)c, r);
           tc05::tmem_ld_wait();
@@ -444,7 +450,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncwarp();
     cluster_sync_all();      // nobody leaves while a peer still reads its partial tile
   }
-  if (!CL && d.tma_store && threadIdx.x == 64) tc05::bulk_wait<0>();   // all TMA stores of this CTA have landed
+  if (!CL && d.tma_store && (threadIdx.x == 64 || threadIdx.x == 192)) tc05::bulk_wait<0>();   // all TMA stores of this CTA have landed
   tc05::fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0 && ctl->abort_flag)
@@ -492,21 +498,21 @@ template <bool A_MN, bool B_MN, bool CL>
 int launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmDev& d, int grid,
                   cudaStream_t st) {
   const int stage_bytes = A_STAGE_BYTES + d.bn * BK * 2;
-  const size_t smem = (size_t)d.stages * stage_bytes + (CL ? 0 : 2 * C_SLAB_BYTES) + sizeof(SmemCtl) + 1024;
+  const size_t smem = (size_t)d.stages * stage_bytes + (CL ? 0 : d.slabs * C_SLAB_BYTES) + sizeof(SmemCtl) + 1024;
   static bool attr_set = false;  // per instantiation
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<A_MN, B_MN, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         220 * 1024);
+                                         227 * 1024);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
   if (!CL) {
-    geeps_launch(gemm_tc_kernel<A_MN, B_MN, CL>, grid, 192, smem, st, ta, tb, tc, d);
+    geeps_launch(gemm_tc_kernel<A_MN, B_MN, CL>, grid, gemm_threads(CL), smem, st, ta, tb, tc, d);
     return (int)cudaGetLastError();
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(192);
+  cfg.blockDim = dim3(gemm_threads(CL));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[2];
@@ -698,7 +704,8 @@ int geeps_gemm_bf16(const GeepsGemmParams* p, void* stream) {
   }
   if (!d.tma_store) tc = ta;   // unused by the kernel
   const int stage_bytes = A_STAGE_BYTES + bn * BK * 2;
-  d.stages = (200 * 1024 - (cluster > 1 ? 0 : 2 * C_SLAB_BYTES)) / stage_bytes;
+  d.slabs = bn > (p->out_fp32 ? 32 : 64) ? 4 : 2;
+  d.stages = (cluster > 1 ? 200 * 1024 : 224 * 1024 - d.slabs * C_SLAB_BYTES) / stage_bytes;
   if (d.stages > MAX_STAGES) d.stages = MAX_STAGES;
   if (d.stages < 2) d.stages = 2;
   const long long num_tiles = (long long)m_tiles * n_tiles * d.split_k;
