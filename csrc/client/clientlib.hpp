@@ -143,6 +143,10 @@ struct Fabric {
   std::vector<PushTiming> push_timing;
   size_t push_timing_next = 0;
   std::vector<void*> table_events;
+  // one worker: what a table's freshness wait needs is its latest push on the comm stream, an event
+  struct Applied { void* event = nullptr; int clock = -1; };
+  std::vector<Applied> applied;           // by table; clock: of the push that the event follows
+  void* joined_stream = nullptr;          // device-clock mode: the stream that the comm lanes last joined
   void* join_event = nullptr;             // device-clock mode: comm lanes -> application stream at the end of a clock
   int* host_status = nullptr;             // pinned mirror of the device status block
 };
@@ -203,7 +207,7 @@ class ClientLib {
   RouterHandler* client_router() { return router_.get(); }
   ServerThreadEntry* server() { return server_.get(); }
   void inject_skip_heartbeats(bool on) { skip_heartbeats_ = on; }
-  void inject_withhold_push_signal(bool on) { withhold_push_signal_ = on; }
+  void inject_withhold_push_signal(bool on) { withhold_push_signal_ = on; if (on) flags_only_ = true; }
 
   // ---- decoder callbacks (router handler thread) ----
   void recv_row_batch_cbk(uint server_id, uint table_id, iter_t data_age, iter_t self_clock, const RowKey* keys,
@@ -263,6 +267,7 @@ class ClientLib {
   bool fabric_setup(std::string* err);
   void fabric_teardown();
   void fabric_wait_data_age(CachedTable& ct, uint table_id, iter_t needed_age, void* stream);
+  bool fabric_by_events(const CachedTable& ct) const;
   void fabric_push(iter_t clock, uint table_id, bool is_init, void* stream);
   bool fabric_check_status(bool sync = false);
   void fabric_end_iteration_device_clock();
@@ -339,7 +344,7 @@ class ClientLib {
   // failure detection
   std::thread heartbeat_thread_;
   std::atomic<bool> stop_heartbeat_{false};
-  std::atomic<bool> skip_heartbeats_{false}, withhold_push_signal_{false};
+  std::atomic<bool> skip_heartbeats_{false}, withhold_push_signal_{false}, flags_only_{false};
   std::mutex peers_mu_;
   std::vector<double> last_heartbeat_;
   std::vector<iter_t> peer_clock_;

@@ -124,3 +124,36 @@ def test_second_stream_gets_its_own_wait():
         assert torch.all(x == 4.0)
         assert g.last_error() == 0
         g.close()
+
+
+@pytest.mark.parametrize("slack", [0, 1])
+def test_one_worker_reads_see_the_last_push_on_any_stream(slack):
+    """One worker orders its reads after its pushes by events (slack 0) or by the flags (an older push is enough): read and
+    update on streams that change from clock to clock, nothing synchronised, a table large enough for a push of some us."""
+    dev = torch.device("cuda:0")
+    cfg = GeePsConfig(device=DEVICE_CUDA, cuda_device=0, transport=TRANSPORT_NVLINK, tcp_base_port=28451 + 20 * slack)
+    streams = [torch.cuda.Stream(device=dev) for _ in range(3)]
+    with torch.cuda.stream(streams[0]):
+        g = GeePs(0, cfg)
+        rows = list(range(20000))
+        r = g.virtual_read(0, rows, slack); u = g.virtual_pre_update(0, rows)
+        pr = g.virtual_post_read(r); up = g.virtual_update(u); g.virtual_clock()
+        g.finish_virtual_iteration()
+        g.pre_update(u).fill_(1.0); g.update(up); g.clock(); g.start_iterations()
+        seen = []
+        for c in range(8):
+            s = streams[c % 3]
+            with torch.cuda.stream(s):
+                x = g.read(r, stream=s)
+                seen.append(torch.stack([x.min(), x.max()]))
+                b = g.pre_update(u, stream=s)
+                g.post_read(pr, stream=s)
+                b.fill_(1.0)
+                g.update(up, stream=s); g.clock()
+            streams[(c + 1) % 3].wait_stream(s)
+        torch.cuda.synchronize()
+        assert g.last_error() == 0
+        for c, mm in enumerate(seen):
+            lo, hi = mm.tolist()
+            assert c + 1 - slack <= lo and hi <= c + 1 and (slack or lo == hi), (c, lo, hi)
+        g.close()
