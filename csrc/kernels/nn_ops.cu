@@ -358,8 +358,13 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
   }
   slot_sums<MODE == 2 ? 1 : 2>(m, a0, a1, out, C, MODE == 2 ? scale : 1.f, sacc);
 }
+// Blocks per SM that the registers of a kernel allow (its launch bounds) and its grid asks for: a second round of blocks
+// would fetch the constants and meet in atomics once more.  32 x 56 x 56 x 192, forward and backward: 69.3 us with grids of
+// 4 (sums) and 8 (normalisation) blocks per SM, 63.7 with these; the backward sums spill at three blocks or four.
+constexpr int reduce_blocks(int mode) { return mode == 1 || mode == 3 ? 2 : 4; }
+constexpr int kApplyBlocks = 4, kBackwardBlocks = 3;
 template <int MODE>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, reduce_blocks(MODE))
 channel_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                       const float* __restrict__ mean_rstd, float* __restrict__ out, long long P, int C,
                       long long ldx, long long lddy, int relu, float scale) {
@@ -482,7 +487,7 @@ __device__ __forceinline__ void bn_apply_fused_body(const bf16* __restrict__ x, 
   if (!s.on) return;
   bn_apply_pixels(s, x, y, mkb, P, ldx, ldy, relu, bits, C >> 3);
 }
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kApplyBlocks)
 bn_apply_fused_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ sums,
                       float* __restrict__ mean_rstd, float* running_mean, float* running_var,
                       const float* __restrict__ gamma, const float* __restrict__ beta, float* zero_after, long long P,
@@ -527,7 +532,7 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
     }
     return o;
   };
-  constexpr int U = BITS ? 4 : 2;
+  constexpr int U = 2;
   long long p = s.p0;
   for (; p + (U - 1) * s.step < P; p += U * s.step) {
     Bf8 xv[U], dv[U], yv[U];
@@ -549,7 +554,7 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
   }
 }
 template <bool BITS>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, kBackwardBlocks)
 bn_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                    bf16* __restrict__ dx, const float* __restrict__ mean_rstd, const float* __restrict__ gamma,
                    const float* __restrict__ sums, float* dgamma, float* dbeta, long long P, int C,
@@ -1797,11 +1802,11 @@ int geeps_col2im(const void* dcol, void* dx, const GeepsConvGeom* g, int accumul
   return CK();
 }
 
-// reductions: one batch of four pixels per thread where that leaves SMs idle, at most four blocks per SM beyond
-static SlotGrid reduce_grid(long long P, int C, int nq = 2) { return slot_grid(P, C, 4, 4, nq); }
-// element-wise passes with per-channel constants: up to eight blocks per SM
-static SlotGrid apply_grid(long long P, int C) {
-  SlotGrid g = slot_grid(P, C, 4, 8, 0);
+// reductions: one batch of four pixels per thread where that leaves SMs idle
+static SlotGrid reduce_grid(int mode, long long P, int C) { return slot_grid(P, C, 4, reduce_blocks(mode), mode == 2 ? 1 : 2); }
+// element-wise passes with per-channel constants
+static SlotGrid apply_grid(long long P, int C, int per_sm = kApplyBlocks) {
+  SlotGrid g = slot_grid(P, C, 4, per_sm, 0);
   g.smem = ((size_t)(C / 8) + g.grid.x - 1) / g.grid.x * 8 * 4 * sizeof(float);      // four constants per channel
   return g;
 }
@@ -1812,7 +1817,7 @@ int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* be
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
-  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  const SlotGrid rg = reduce_grid(0, P, C), ag = apply_grid(P, C);
   geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   geeps_launch(bn_finalize_kernel, (C + 127) / 128, 128, 0, st, sums, mean_rstd, running_mean, running_var, C,
@@ -1828,7 +1833,7 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
-  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  const SlotGrid rg = reduce_grid(1, P, C), ag = apply_grid(P, C, kBackwardBlocks);
   geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
   geeps_launch(bn_backward_kernel<false>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)y,
@@ -1871,7 +1876,7 @@ int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, cons
     cudaError_t e = cudaLaunchCooperativeKernel((void*)bn_forward_coop_kernel, cg.grid, dim3(cg.threads), args, cg.smem, st);
     return e == cudaSuccess ? CK() : (int)e;
   }
-  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  const SlotGrid rg = reduce_grid(0, P, C), ag = apply_grid(P, C);
   geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   geeps_launch(bn_apply_fused_kernel, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
@@ -1896,7 +1901,7 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
     cudaError_t e = cudaLaunchCooperativeKernel(kernel, cg.grid, dim3(cg.threads), args, cg.smem, st);
     return e == cudaSuccess ? CK() : (int)e;
   }
-  const SlotGrid rg = reduce_grid(P, C), ag = apply_grid(P, C);
+  const SlotGrid rg = reduce_grid(3, P, C), ag = apply_grid(P, C, kBackwardBlocks);
   if (bits != nullptr && relu) {
     geeps_launch(channel_reduce_kernel<3>, rg.grid, rg.threads, rg.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits,
                                                                    mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
@@ -1921,7 +1926,7 @@ int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, f
     return CK();
   }
   if (zero_first) cudaMemsetAsync(out, 0, sizeof(float) * C, st);
-  const SlotGrid rg = reduce_grid(P, C, 1);
+  const SlotGrid rg = reduce_grid(2, P, C);
   geeps_launch(channel_reduce_kernel<2>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, out, P, C, ldx, 0, 0, scale);
   return CK();
