@@ -345,6 +345,24 @@ int geeps_conv_dgrad_rows_applicable(const GeepsConvTcParams* p) {
   return plan_rows(p).ok ? 1 : 0;
 }
 
+int geeps_conv_dgrad_rows_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {
+  memset(out, 0, sizeof(*out));
+  if (!geeps_conv_tc_supported(p)) return 0;
+  const RowsPlan rp = plan_rows(p);
+  if (!rp.ok) return 0;
+  const RowsDev& d = rp.d;
+  out->ok = 1;
+  out->routed = geeps_conv_dgrad_rows_applicable(p);
+  out->PW = d.PW; out->R = d.R; out->row_tiles = d.pairs + d.single; out->m_tiles = 1;
+  out->positions = BM; out->ncols2 = out->ncols1 = d.n_cols;
+  out->n_blocks = 2 * d.pairs + d.single;
+  out->stages_x = d.stages_x; out->stages_w = d.stages_w; out->x_stage_bytes = d.x_stage_bytes;
+  out->tmem_cols = 2 * ACC_COLS;
+  out->smem_bytes = (long long)rp.smem;
+  out->util = rp.util;
+  return 1;
+}
+
 int geeps_conv_dgrad_rows(const GeepsConvTcParams* p, void* stream) {
   if (!geeps_conv_tc_supported(p)) return (int)cudaErrorInvalidValue;
   RowsPlan rp = plan_rows(p);

@@ -178,7 +178,7 @@ int geeps_conv_wgrad_halo(const GeepsConvTcParams* p, void* stream);
 // Data gradient with the taps of a filter row side by side in an MMA's columns (conv_dgrad_rows.cu); same routing.
 int geeps_conv_dgrad_rows_applicable(const GeepsConvTcParams* p);
 int geeps_conv_dgrad_rows(const GeepsConvTcParams* p, void* stream);
-// The geometry the two halo kernels would use for a call (host arithmetic only; for tests and tuning).  `ok` = 0 when
+// The geometry these kernels would use for a call (host arithmetic only; for tests and tuning).  `ok` = 0 when
 // the kernel does not accept the call.
 typedef struct GeepsHaloPlanInfo {
   int ok, routed;                       // accepted; geeps_conv_tc() would route the call to this kernel
@@ -191,6 +191,7 @@ typedef struct GeepsHaloPlanInfo {
 } GeepsHaloPlanInfo;
 int geeps_conv_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
 int geeps_conv_wgrad_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
+int geeps_conv_dgrad_rows_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
 
 // ---------------- parameter pull fused with the consuming GEMM ----------------
 // Y[M,N] = X[M,K] * W[N,K]^T + bias (+ReLU), M <= 256, K a multiple of 64.  W's rows live on the server
