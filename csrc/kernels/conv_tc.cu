@@ -494,7 +494,6 @@ extern "C" {
 
 int geeps_conv_tc(const GeepsConvTcParams* p, void* stream) {
   if (!geeps_conv_tc_supported(p)) return (int)cudaErrorInvalidValue;
-  if (p->mode == MODE_DGRAD && p->split_k >= 0 && geeps_conv_dgrad_rows_applicable(p)) return geeps_conv_dgrad_rows(p, stream);
   if (p->mode != MODE_WGRAD && p->split_k >= 0 && geeps_conv_halo_applicable(p)) return geeps_conv_halo(p, stream);
   if (p->mode == MODE_WGRAD && p->split_k >= 0 && geeps_conv_wgrad_halo_applicable(p))
     return geeps_conv_wgrad_halo(p, stream);

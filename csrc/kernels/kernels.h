@@ -175,9 +175,6 @@ int geeps_conv_halo(const GeepsConvTcParams* p, void* stream);
 // Weight gradient with the taps of a filter row served by one activation tile (conv_wgrad_halo.cu); same routing.
 int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p);
 int geeps_conv_wgrad_halo(const GeepsConvTcParams* p, void* stream);
-// Data gradient with the taps of a filter row side by side in an MMA's columns (conv_dgrad_rows.cu); same routing.
-int geeps_conv_dgrad_rows_applicable(const GeepsConvTcParams* p);
-int geeps_conv_dgrad_rows(const GeepsConvTcParams* p, void* stream);
 // The geometry these kernels would use for a call (host arithmetic only; for tests and tuning).  `ok` = 0 when
 // the kernel does not accept the call.
 typedef struct GeepsHaloPlanInfo {
@@ -191,7 +188,6 @@ typedef struct GeepsHaloPlanInfo {
 } GeepsHaloPlanInfo;
 int geeps_conv_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
 int geeps_conv_wgrad_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
-int geeps_conv_dgrad_rows_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
 
 // ---------------- parameter pull fused with the consuming GEMM ----------------
 // Y[M,N] = X[M,K] * W[N,K]^T + bias (+ReLU), M <= 256, K a multiple of 64.  W's rows live on the server

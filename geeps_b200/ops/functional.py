@@ -120,14 +120,6 @@ def conv_halo(mode: int, x, y, w, k: int, pad: int, **kw) -> None:
     launch(lib().geeps_conv_halo, "conv_halo", C.byref(p), stream_ptr())
 
 
-def conv_dgrad_rows(dx, dy, w, k: int, pad: int, **kw) -> None:
-    """The filter-row data-gradient kernel called directly (16 to 64 input channels, images up to 33 - k wide)."""
-    L.require_cuda()
-    assert dx.dtype == bf16 and dy.dtype == bf16 and w.dtype == bf16
-    p = conv_tc_params(CONV_DGRAD, dx, dy, w, k, pad, **kw)
-    launch(lib().geeps_conv_dgrad_rows, "conv_dgrad_rows", C.byref(p), stream_ptr())
-
-
 def conv_wgrad_halo(x, dy, dw, k: int, pad: int, **kw) -> None:
     """The filter-row weight-gradient kernel called directly (dw fp32 [og, ldw], overwritten)."""
     L.require_cuda()

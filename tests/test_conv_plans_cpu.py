@@ -95,26 +95,3 @@ def test_weight_gradient_plans_respect_the_hardware_limits():
         assert rows_read * 128 <= info.x_stage_bytes
         assert info.stages_x >= 2 and info.smem_bytes <= SMEM_LIMIT
     assert seen > 100 and routed > 0
-
-
-def test_filter_row_data_gradient_plans_respect_the_hardware_limits():
-    lib = L.lib()
-    seen = 0
-    for B, H, cg, og, k, pad in SHAPES + [(3, H, cg, 72, k, k // 2) for H in range(1, 34) for cg in (16, 24, 48, 64) for k in (2, 4, 6, 7)]:
-        p, _, _ = _params(1, B, H, H, cg, og, k, pad)
-        info = L.HaloPlanInfo()
-        fits = 16 <= cg <= 64 and cg % 16 == 0 and k * cg <= 256 and H + k - 1 <= 32 and k - 1 - pad >= 0 and p.OH > 0
-        if not lib.geeps_conv_dgrad_rows_plan(C.byref(p), C.byref(info)):
-            assert not fits, (B, H, cg, og, k, pad)
-            continue
-        seen += 1
-        assert fits and info.routed
-        assert info.PW in (16, 32) and H + k - 1 <= info.PW                  # no window crosses a warp's 32 lanes
-        assert info.R * info.PW == info.positions == 128
-        assert info.R * info.n_blocks >= H > info.R * (info.n_blocks - 1)    # every block has a row of the image
-        assert k * cg <= info.ncols2 <= 256 and info.ncols2 % 64 == 0
-        assert (2 * info.R + k - 1) * info.PW * 128 == info.x_stage_bytes    # what the last tap of the second block reads
-        assert info.x_stage_bytes % 1024 == 0 and info.stages_x == 2 and info.stages_w >= 2
-        assert info.smem_bytes <= SMEM_LIMIT and info.tmem_cols == 512
-        assert 0.0 < info.util <= 1.0
-    assert seen > 100

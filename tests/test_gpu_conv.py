@@ -125,42 +125,6 @@ def test_strided_conv_forward_and_gradients_match_torch(case):
     assert status.tolist()[0] == 0
 
 
-DGRAD_ROWS = [
-    # B, H, W, C_total, c_off, cg, O_total, o_off, og, k, pad
-    (3, 27, 27, 96, 48, 48, 256, 128, 128, 5, 2),       # AlexNet conv2: three tiles of two blocks and one of one
-    (2, 9, 28, 16, 0, 16, 72, 0, 72, 5, 2),             # pitch 32 without a spare column, second chunk of 8 channels
-    (5, 14, 14, 64, 0, 64, 96, 0, 96, 3, 1),            # pitch 16: two image rows per warp, 192 columns
-    (2, 3, 10, 64, 16, 48, 24, 0, 24, 3, 0),            # one block, 24 of 64 gradient channels, no padding
-    (160, 7, 7, 32, 0, 32, 40, 0, 40, 7, 3),            # 7 taps, more tiles than SMs
-    (2, 17, 12, 48, 0, 48, 64, 0, 64, 5, 1),            # padding 1 of 2: halo 3
-]
-
-
-@pytest.mark.parametrize("case", DGRAD_ROWS)
-def test_filter_row_data_gradient_matches_torch(case):
-    """256 columns of (tap of a filter row, channel) per MMA, summed over the taps by lane shifts in the epilogue."""
-    from geeps_b200.ops import functional as F
-    B, H, W, Ct, c_off, cg, Ot, o_off, og, k, pad = case
-    dev = torch.device("cuda:0")
-    gen = torch.Generator(device=dev).manual_seed(11)
-    OH, OW, kd = H + 2 * pad - k + 1, W + 2 * pad - k + 1, k * k * cg
-    ld = (kd + 7) // 8 * 8
-    w = torch.zeros(og, ld, device=dev, dtype=BF)
-    w[:, :kd] = (torch.randn(og, kd, device=dev, generator=gen) / kd ** 0.5).to(BF)
-    dy = torch.randn(B, OH, OW, Ot, device=dev, generator=gen).to(BF)[..., o_off:o_off + og]
-    wr = w[:, :kd].double().view(og, k, k, cg).permute(0, 3, 1, 2)
-    ref = torch.nn.functional.conv_transpose2d(dy.double().permute(0, 3, 1, 2), wr, padding=pad).permute(0, 2, 3, 1)
-    dx_full = torch.full((B, H, W, Ct), 3.0, device=dev, dtype=BF)
-    dx = dx_full[..., c_off:c_off + cg]
-    status = torch.zeros(4, dtype=torch.int32, device=dev)
-    F.conv_dgrad_rows(dx, dy, w, k, pad, status=status)
-    torch.cuda.synchronize()
-    # fp32 sums rounded once to bf16: uniform relative rounding errors of up to 2^-9, 2^-9 / sqrt(3) = 1.1e-3 in the 2-norm
-    assert _rel(dx, ref) < 2.5e-3
-    assert bool((dx_full[..., :c_off] == 3.0).all()) and bool((dx_full[..., c_off + cg:] == 3.0).all())
-    assert status.tolist()[0] == 0
-
-
 HALO_CASES = CASES + [
     (3, 57, 57, 48, 0, 48, 96, 0, 96, 3, 0),            # AlexNet conv1 after space-to-depth: 96 channels leave in 32-wide slabs
     (3, 28, 28, 192, 0, 192, 96, 0, 96, 3, 1),          # three chunks, rows split 4 + 4 per tile, last tile short
