@@ -142,6 +142,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const uint32_t tmem = ctl->tmem_base;
   geeps_pdl_wait();          // everything above touches this CTA's own memory only
   volatile int* abort_flag = &ctl->abort_flag;
+  const uint32_t tiles_u = tc05::smem_u32(tiles), empty_u = tc05::smem_u32(ctl->empty);
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -242,18 +243,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int kt = kt_begin; kt < kt_end; ++kt) {
           if (!tc05::mbar_wait_warp(&ctl->full[s], ph, abort_flag, WAIT_BUDGET_NS)) { ok = false; break; }
           tc05::fence_after_sync();
-          const uint32_t sa = tc05::smem_u32(tiles + (size_t)s * STAGE_BYTES);
-          const uint32_t sb = sa + A_STAGE_BYTES;
-          if (leader) {
-          // descriptors as 32-bit halves: per MMA this one thread spends an add per operand, not a rebuild
+          const uint32_t sa = tiles_u + (uint32_t)(s * STAGE_BYTES), sb = sa + A_STAGE_BYTES;
           const uint32_t a_lo = tc05::desc_lo(sa, A_MN ? PANEL_BYTES : 16), b_lo = tc05::desc_lo(sb, B_MN ? PANEL_BYTES : 16);
-          constexpr uint32_t d_hi = tc05::desc_hi(1024);
-#pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            tc05::mma_bf16_ss_lohi(tacc, a_lo + (A_MN ? 128 : 2) * k, d_hi, b_lo + (B_MN ? 128 : 2) * k, d_hi, idesc,
-                                   (kt > kt_begin || k > 0) ? 1u : 0u);
-          tc05::mma_commit(&ctl->empty[s]);
-          }
+          tc05::mma_ktile_warp<A_MN ? 128 : 2, B_MN ? 128 : 2>(tacc, a_lo, b_lo, tc05::desc_hi(1024), idesc,
+                                                               kt > kt_begin ? 1u : 0u, empty_u + 8u * (uint32_t)s);
           if (++s == S) { s = 0; ph ^= 1u; }
         }
         if (ok && leader) tc05::mma_commit(&ctl->tmem_full[acc]);
