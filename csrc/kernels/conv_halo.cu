@@ -55,19 +55,33 @@ constexpr int UMMA_K = 16;
 constexpr int PANEL_BYTES = 64 * BK * 2;
 constexpr int W_STAGE_BYTES = BM * BK * 2;    // 128 channels x 64 k (forward) or two [64 k][64 channels] panels (dgrad)
 constexpr int MAX_X_STAGES = 2;
-constexpr int MAX_W_STAGES = 8;
+constexpr int MAX_W_STAGES = 16;
 constexpr uint64_t WAIT_BUDGET_NS = 2000000000ull;
 constexpr int C_SLAB_BYTES = 128 * 128;       // 128 positions x 64 channels bf16
 constexpr int ACC_COLS = 256;
+constexpr int SMEM_BUDGET = 224 * 1024;       // tiles, weights and slabs
 constexpr int kEpilogueWarps = 8;             // two per TMEM lane quarter: they take alternate column groups
 constexpr int kThreads = 64 + 32 * kEpilogueWarps;
 
-enum { MODE_FWD = 0, MODE_DGRAD = 1 };
+// MODE_DGRAD2: a data gradient with at most 64 channels, whose 128 accumulator rows hold them twice: once for the even and
+// once for the odd column of a pair, a position being a pair.  Both read the same activations one column apart, so a filter
+// row of KW taps takes KW + 1 steps - the even column has no tap in the last, the odd one none in the first - of half
+// the positions: (KW + 1) / 2 KW of the products that MODE_DGRAD spends with half its rows empty.  The activations are
+// loaded by column parity (two maps with twice the pixel pitch) and step s reads parity s % 2 from column s / 2 on; the two
+// halves leave through the maps of dX's even and odd columns.  Step s multiplies taps s (even column) and s - 1 (odd): a tap
+// is loaded once for both, as two steps read it from neighbouring panels - with a load for each the weights' rows (96 bytes
+// of every 2400 for 48 channels and 5 x 5) were the bound, 109 us below.  A half without a tap is left out of the step's
+// products (disabled lanes), so every output adds the same products in the same order as in MODE_DGRAD and nothing else.
+// 256 x 27 x 27, 128 -> 48, 5 x 5: 114 us in MODE_DGRAD, 85.5 here.
+enum { MODE_FWD = 0, MODE_DGRAD = 1, MODE_DGRAD2 = 2 };
 
 struct HaloDev {
   const float* bias; int* status;
   int KH, KW, taps, cchunks, k_last;   // k_last: MMA k-substeps (of 16) in the last chunk (zero channels are skipped)
   int PW, Rb, px, py;                  // padded pitch, image rows per store block (two blocks per tile), halo left / top
+  int KWs;                             // steps per filter row: KW, or KW + 1 (MODE_DGRAD2)
+  int w_bytes, slab_bytes;             // all weight stages; one store slab
+  int x0, x1, x_tile_bytes;            // MODE_DGRAD2: first column of the two parity maps; bytes of a parity's halo tile
   int split, ncols2, ncols1;           // positions per block (Rb * PW); MMA N for a tile of two blocks / one block
   int GH;                              // output rows of the image
   int row_tiles, m_tiles, n_images;    // tiles = m_tiles * n_images * row_tiles
@@ -102,13 +116,16 @@ __device__ __forceinline__ Tile decode_tile(const HaloDev& d, int t) {
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
-                 const __grid_constant__ CUtensorMap tmC, const HaloDev d) {
-  constexpr bool W_MN = MODE == MODE_DGRAD;
+                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX1,
+                 const __grid_constant__ CUtensorMap tmC1, const HaloDev d) {
+  constexpr bool W_MN = MODE != MODE_FWD;
+  constexpr bool PAIR = MODE == MODE_DGRAD2;
+  constexpr int CH = PAIR ? 64 : BM;            // channels per tile
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles_x = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles_w = tiles_x + (size_t)d.stages_x * d.x_stage_bytes;
-  uint8_t* cslab = tiles_w + (size_t)d.stages_w * W_STAGE_BYTES;
-  SmemCtl* ctl = (SmemCtl*)(cslab + 2 * C_SLAB_BYTES);          // one slab per 64 channels
+  uint8_t* cslab = tiles_w + d.w_bytes;
+  SmemCtl* ctl = (SmemCtl*)(cslab + 2 * d.slab_bytes);          // one slab per 64 channels
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = d.m_tiles * d.n_images * d.row_tiles;
 
@@ -138,13 +155,13 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   geeps_pdl_wait();          // everything above touches this CTA's own memory only
   volatile int* abort_flag = &ctl->abort_flag;
   const int NR = 2 * d.Rb + d.KH - 1;
-  const uint32_t x_tx = (uint32_t)(NR * d.PW * 128);
+  const uint32_t x_tx = (uint32_t)(NR * d.PW * 128) * (PAIR ? 2u : 1u);
 
   if (warp == 0) {
     // ---------------- TMA producer: one halo tile per chunk, one weight tile per (tap, chunk) ----------------
     const bool leader = tc05::elect_one();
     if (leader) { tc05::tma_prefetch_desc(&tmX); tc05::tma_prefetch_desc(&tmW); }
-    int sx = 0, sw = 0;
+    int sx = 0, sw = 0, wrow = 0;
     uint32_t phx = 0, phw = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
@@ -153,24 +170,34 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (!tc05::mbar_wait_warp(&ctl->empty_x[sx], phx ^ 1u, abort_flag, WAIT_BUDGET_NS)) { ok = false; break; }
         if (leader) {
           tc05::mbar_expect_tx(&ctl->full_x[sx], x_tx);
-          tc05::tma_load_4d(tiles_x + (size_t)sx * d.x_stage_bytes, &tmX, &ctl->full_x[sx], cc * 64, -d.px, q.y0 - d.py, q.b);
+          uint8_t* xt = tiles_x + (size_t)sx * d.x_stage_bytes;
+          tc05::tma_load_4d(xt, &tmX, &ctl->full_x[sx], cc * 64, PAIR ? d.x0 : -d.px, q.y0 - d.py, q.b);
+          if (PAIR) tc05::tma_load_4d(xt + d.x_tile_bytes, &tmX1, &ctl->full_x[sx], cc * 64, d.x1, q.y0 - d.py, q.b);
         }
         if (++sx == d.stages_x) { sx = 0; phx ^= 1u; }
-        for (int tap = 0; tap < d.taps; ++tap) {
+        const int loads = d.KH * d.KW;
+        int panel = d.KW - 1;                        // MODE_DGRAD2: where in its row's panels (from wrow on) the tap goes
+        for (int tap = 0; tap < loads; ++tap) {
           if (!tc05::mbar_wait_warp(&ctl->empty_w[sw], phw ^ 1u, abort_flag, WAIT_BUDGET_NS)) { ok = false; break; }
           if (leader) {
-            uint8_t* dst = tiles_w + (size_t)sw * W_STAGE_BYTES;
-            tc05::mbar_expect_tx(&ctl->full_w[sw], W_STAGE_BYTES);
+            uint8_t* dst = tiles_w + (PAIR ? (size_t)(wrow + panel) * PANEL_BYTES : (size_t)sw * W_STAGE_BYTES);
+            tc05::mbar_expect_tx(&ctl->full_w[sw], PAIR ? PANEL_BYTES : W_STAGE_BYTES);
             if (MODE == MODE_FWD) {
               tc05::tma_load_3d(dst, &tmW, &ctl->full_w[sw], cc * 64, tap, q.mi * BM);
+            } else if (PAIR) {
+              tc05::tma_load_3d(dst, &tmW, &ctl->full_w[sw], q.mi * CH, loads - 1 - tap, cc * 64);
             } else {
               // data gradient: the filter is applied mirrored; rows of the product are input channels
-              const int wtap = d.taps - 1 - tap;
+              const int wtap = loads - 1 - tap;
               tc05::tma_load_3d(dst, &tmW, &ctl->full_w[sw], q.mi * BM, wtap, cc * 64);
               tc05::tma_load_3d(dst + PANEL_BYTES, &tmW, &ctl->full_w[sw], q.mi * BM + 64, wtap, cc * 64);
             }
           }
           if (++sw == d.stages_w) { sw = 0; phw ^= 1u; }
+          if (PAIR && --panel < 0) {
+            panel = d.KW - 1;
+            wrow = sw;
+          }
         }
       }
     }
@@ -183,8 +210,11 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     constexpr uint32_t d_hi = tc05::desc_hi(1024);
     constexpr uint32_t w_kstep = W_MN ? 128u : 2u;      // 16 k: two 8-row groups of 1024 bytes, or 32 bytes in the row
     const uint32_t row_wrap8 = (uint32_t)(d.PW - d.KW + 1) * 8u;
+    // MODE_DGRAD2: from a step to the next alternately to the other parity's tile, and back and one column on
+    const uint32_t other = (uint32_t)d.x_tile_bytes >> 4;
+    const uint32_t pair_wrap = (uint32_t)d.PW * 8u - (uint32_t)(d.KW >> 1) * 8u - ((d.KW & 1) ? other : 0u);
     uint32_t tile_i = 0;
-    int sx = 0, sw = 0;
+    int sx = 0, sw = 0, wrow = 0;
     uint32_t phx = 0, phw = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_i) {
@@ -202,11 +232,26 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const bool full_k = cc + 1 < d.cchunks || d.k_last == BK / UMMA_K;
         int tx = 0;
         for (int tap = 0; tap < d.taps; ++tap) {
-          if (!tc05::mbar_wait_warp(&ctl->full_w[sw], phw, abort_flag, WAIT_BUDGET_NS)) { ok = false; break; }
+          // MODE_DGRAD2: the last step of a row has no tap of its own
+          if ((!PAIR || tx < d.KW) && !tc05::mbar_wait_warp(&ctl->full_w[sw], phw, abort_flag, WAIT_BUDGET_NS)) { ok = false; break; }
           tc05::fence_after_sync();
           if (leader) {
-            const uint32_t w_lo = tc05::desc_lo(tc05::smem_u32(tiles_w + (size_t)sw * W_STAGE_BYTES), W_MN ? PANEL_BYTES : 16);
-            if (full_k) {
+            const uint8_t* wt = tiles_w + (PAIR ? (ptrdiff_t)(wrow + d.KW - 1 - tx) * PANEL_BYTES : (ptrdiff_t)sw * W_STAGE_BYTES);
+            const uint32_t w_lo = tc05::desc_lo(tc05::smem_u32(wt), W_MN ? PANEL_BYTES : 16);
+            if (PAIR) {
+              // no product in the half whose column has no tap in this step; the odd column's first overwrites
+              const uint32_t no_even = tx == d.KW ? ~0u : 0u, no_odd = tx == 0 ? ~0u : 0u;
+              const int ks = full_k ? BK / UMMA_K : d.k_last;
+              if (cc == 0 && tap == 1) {
+                tc05::mma_bf16_ss_halves(tacc, w_lo, d_hi, x_lo, d_hi, idesc, 1u, no_even, ~0u);
+                tc05::mma_bf16_ss_halves(tacc, w_lo, d_hi, x_lo, d_hi, idesc, 0u, ~0u, 0u);
+              } else {
+                tc05::mma_bf16_ss_halves(tacc, w_lo, d_hi, x_lo, d_hi, idesc, accumulate, no_even, no_odd);
+              }
+#pragma unroll
+              for (int j = 1; j < BK / UMMA_K; ++j)
+                if (j < ks) tc05::mma_bf16_ss_halves(tacc, w_lo + j * w_kstep, d_hi, x_lo + 2 * j, d_hi, idesc, 1u, no_even, no_odd);
+            } else if (full_k) {
               tc05::mma_bf16_ss_lohi(tacc, w_lo, d_hi, x_lo, d_hi, idesc, accumulate);
               tc05::mma_bf16_ss_lohi(tacc, w_lo + w_kstep, d_hi, x_lo + 2, d_hi, idesc, 1u);
               tc05::mma_bf16_ss_lohi(tacc, w_lo + 2 * w_kstep, d_hi, x_lo + 4, d_hi, idesc, 1u);
@@ -216,11 +261,19 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
               if (d.k_last > 1) tc05::mma_bf16_ss_lohi(tacc, w_lo + w_kstep, d_hi, x_lo + 2, d_hi, idesc, 1u);
               if (d.k_last > 2) tc05::mma_bf16_ss_lohi(tacc, w_lo + 2 * w_kstep, d_hi, x_lo + 4, d_hi, idesc, 1u);
             }
-            tc05::mma_commit(&ctl->empty_w[sw]);
+            // MODE_DGRAD2: the tap of the step before is used up; it is the one in front of sw, or of 0 behind a turn
+            if (!PAIR) tc05::mma_commit(&ctl->empty_w[sw]);
+            else if (tx > 0) tc05::mma_commit(&ctl->empty_w[sw == 0 ? d.stages_w - 1 : sw - 1]);
           }
           accumulate = 1u;
-          if (++sw == d.stages_w) { sw = 0; phw ^= 1u; }
-          if (++tx == d.KW) { tx = 0; x_lo += row_wrap8; } else { x_lo += 8u; }
+          if (!PAIR || tx < d.KW) {
+            if (++sw == d.stages_w) { sw = 0; phw ^= 1u; }
+          }
+          if (PAIR) {
+            // step tx read parity tx % 2 at column tx / 2
+            if (tx == d.KW) { tx = 0; x_lo += pair_wrap; wrow = sw; }
+            else { x_lo += (tx & 1) ? 8u - other : other; ++tx; }
+          } else if (++tx == d.KW) { tx = 0; x_lo += row_wrap8; } else { x_lo += 8u; }
         }
         if (ok && leader) tc05::mma_commit(&ctl->empty_x[sx]);
         if (++sx == d.stages_x) { sx = 0; phx ^= 1u; }
@@ -240,7 +293,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     uint32_t cb[8];
 #pragma unroll
     for (int jj = 0; jj < 8; ++jj) cb[jj] = ((chunk ^ (uint32_t)jj) << 4) + within;
-    const uint32_t slab_base = tc05::smem_u32(cslab) + (uint32_t)(half * C_SLAB_BYTES);
+    const uint32_t slab_base = tc05::smem_u32(cslab) + (uint32_t)(half * d.slab_bytes);
     const bool storer = lane == 0 && (q4 & 1) == 0 && sub == 0;          // one thread per slab issues its stores
     const float floor_v = d.relu ? 0.f : -INFINITY;
     uint32_t tile_i = 0;
@@ -253,7 +306,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         bias_v = (MODE == MODE_FWD && d.bias != nullptr && ch < d.n_valid) ? __ldg(d.bias + ch) : 0.f;
         bias_mi = q.mi;
       }
-      const bool slab_valid = q.mi * BM + half * 64 < d.n_valid;           // same for every thread of the slab
+      const bool slab_valid = PAIR || q.mi * BM + half * 64 < d.n_valid;   // same for every thread of the slab
       const uint32_t acc = tile_i & 1u, acc_ph = (tile_i >> 1) & 1u;
       if (!tc05::mbar_wait(&ctl->tmem_full[acc], acc_ph, abort_flag, WAIT_BUDGET_NS)) break;
       tc05::fence_after_sync();
@@ -294,7 +347,8 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (storer && slab_valid) {
           // box (64 channels, PW, Rb, 1): columns past the image width, rows past its height and channels past
           // the extent are clipped by TMA
-          tc05::tma_store_4d_addr(&tmC, slab_base, q.mi * BM + half * 64, 0, q.y0 + p * d.Rb, q.b);
+          tc05::tma_store_4d_addr(PAIR && half ? &tmC1 : &tmC, slab_base, PAIR ? q.mi * CH : q.mi * BM + half * 64, 0,
+                                  q.y0 + p * d.Rb, q.b);
           tc05::bulk_commit();
         }
       }
@@ -348,35 +402,55 @@ bool make_act_map(CUtensorMap* map, const void* base, int ch, int W, int H, int 
   const int box[4] = {64, bw, bh, 1};
   return make_map(map, base, 4, dims, st, box);
 }
+// the columns of parity b of an NHWC tensor
+bool make_parity_map(CUtensorMap* map, const void* base, int ch, int W, int H, int B, long long pitch, int b, int bw, int bh) {
+  const long long dims[4] = {ch, (W - b + 1) / 2, H, B};
+  const long long st[3] = {pitch * 4, pitch * 2 * W, pitch * 2 * W * H};
+  const int box[4] = {64, bw, bh, 1};
+  return make_map(map, (const char*)base + pitch * 2 * b, 4, dims, st, box);
+}
 int round_up(long long v, int m) { return (int)((v + m - 1) / m * m); }
 
 template <int MODE>
-int launch(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tc, const HaloDev& d, int grid, size_t smem,
-           cudaStream_t st) {
+int launch(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tc, const CUtensorMap& tx1,
+           const CUtensorMap& tc1, const HaloDev& d, int grid, size_t smem, cudaStream_t st) {
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(conv_halo_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  geeps_launch(conv_halo_kernel<MODE>, grid, kThreads, smem, st, tx, tw, tc, d);
+  geeps_launch(conv_halo_kernel<MODE>, grid, kThreads, smem, st, tx, tw, tc, tx1, tc1, d);
   return (int)cudaGetLastError();
 }
 
 // geometry shared by the applicability check and the launch
-struct HaloPlan { HaloDev d; size_t smem; double util; bool ok; };
+struct HaloPlan { HaloDev d; size_t smem; double util, cost; bool ok; };      // cost: clocks of the steps on the busiest SM
 
-HaloPlan plan_halo(const GeepsConvTcParams* p) {
+// MODE_DGRAD2's weights: whole filter rows of KW panels of 64 channels, the taps of a row in descending order, so the 128
+// rows of a step's weights are two neighbouring panels and each tap is loaded once for both columns.  (The panel in front of
+// a row's last tap and the one behind its first belong to disabled lanes; at the ends they are a halo tile and a store slab.)
+// At least five panels: a tap is loaded again some KW steps after its last use.
+int pair_rows(int KW) { return (5 + KW - 1) / KW; }
+int pair_slab(int positions) { return round_up(positions > 64 ? positions * 128LL : PANEL_BYTES, 1024); }
+
+// a step of four 128 x n x 16 products takes 2 n clocks, but the tap's rows out of L2 and its issue some 520
+int step_clocks(int n) { return 2 * n > 520 ? 2 * n : 520; }
+
+// pair: MODE_DGRAD2
+HaloPlan plan_halo(const GeepsConvTcParams* p, bool pair = false) {
   HaloPlan hp;
   hp.ok = false;
   hp.smem = 0;
-  hp.util = 0;
+  hp.util = hp.cost = 0;
   HaloDev& d = hp.d;
   memset(&d, 0, sizeof(d));
   if ((p->mode != MODE_FWD && p->mode != MODE_DGRAD) || p->stride > 1) return hp;
   const bool fwd = p->mode == MODE_FWD;
-  const int GW = fwd ? p->OW : p->W, GH = fwd ? p->OH : p->H;
-  d.KH = p->KH; d.KW = p->KW; d.taps = p->KH * p->KW;
+  if (pair && (fwd || p->cg > 64 || p->W < 2 || p->OW < 2)) return hp;
+  const int GW = fwd ? p->OW : (pair ? (p->W + 1) / 2 : p->W), GH = fwd ? p->OH : p->H;
+  d.KH = p->KH; d.KW = p->KW; d.KWs = pair ? p->KW + 1 : p->KW; d.taps = p->KH * d.KWs;
+  const int span = pair ? p->KW / 2 : p->KW - 1;       // columns that a window reaches past its first
   d.px = fwd ? p->pad : p->KW - 1 - p->pad;
   d.py = fwd ? p->pad : p->KH - 1 - p->pad;
   if (d.px < 0 || d.py < 0 || d.taps < 2) return hp;
@@ -384,15 +458,28 @@ HaloPlan plan_halo(const GeepsConvTcParams* p) {
   // Two store blocks of Rb image rows per tile, at most 128 positions each; the rows are spread evenly over the
   // tiles so that the last tile is not mostly padding.  The pitch is the smallest one >= out_width + KW - 1 that
   // makes a block a multiple of 8 positions (the epilogue's constant swizzle offsets rely on it).
+  // MODE_DGRAD2 holds two halo tiles per stage, so its rows are also limited by shared memory, and of the pitches and rows
+  // that fit the cheapest is taken.
   bool found = false;
-  for (int pw = GW + p->KW - 1; pw <= GW + p->KW + 6 && pw <= 128; ++pw) {
-    const int rb_max = 128 / pw;
-    const int row_tiles = (GH + 2 * rb_max - 1) / (2 * rb_max);
-    const int rb = (GH + 2 * row_tiles - 1) / (2 * row_tiles);
-    if ((rb * pw) % 8) continue;
-    d.PW = pw; d.row_tiles = row_tiles; d.Rb = rb;
-    found = true;
-    break;
+  const int sms = geeps_sm_count();
+  for (int pw = GW + span; pw <= GW + span + 7 && pw <= 128 && (pair || !found); ++pw) {
+    for (int rb_max = 128 / pw; rb_max >= 1; --rb_max) {
+      const int row_tiles = (GH + 2 * rb_max - 1) / (2 * rb_max);
+      const int rb = (GH + 2 * row_tiles - 1) / (2 * row_tiles);
+      if ((rb * pw) % 8 == 0) {
+        const int ncols = round_up(2 * rb * pw, 16);
+        const long long x_bytes = round_up(((2LL * rb + p->KH - 1) * pw + ncols - 2 * rb * pw + p->KW) * 128, 1024);
+        const double cost = (double)(((long long)p->B * row_tiles + sms - 1) / sms) * step_clocks(ncols);
+        const bool fits = !pair || 4 * x_bytes + (long long)pair_rows(p->KW) * p->KW * PANEL_BYTES +
+                                       2 * pair_slab(rb * pw) <= SMEM_BUDGET;
+        if (fits && (!found || cost < hp.cost)) {
+          d.PW = pw; d.row_tiles = row_tiles; d.Rb = rb;
+          hp.cost = cost;
+          found = true;
+        }
+      }
+      if (!pair) break;
+    }
   }
   if (!found) return hp;
   d.split = d.Rb * d.PW;
@@ -403,23 +490,45 @@ HaloPlan plan_halo(const GeepsConvTcParams* p) {
   const int tail = kch - (d.cchunks - 1) * 64;
   d.k_last = (tail + UMMA_K - 1) / UMMA_K;
   d.n_valid = nch;
-  d.m_tiles = (nch + BM - 1) / BM;
+  d.m_tiles = pair ? 1 : (nch + BM - 1) / BM;
   d.n_images = p->B;
   const int NR = 2 * d.Rb + p->KH - 1;
   const int over = d.ncols2 - 2 * d.split + p->KW;     // rows an MMA may read past the halo tile
-  d.x_stage_bytes = round_up((long long)(NR * d.PW + over) * 128, 1024);
+  d.x_tile_bytes = round_up((long long)(NR * d.PW + over) * 128, 1024);
+  d.x_stage_bytes = (pair ? 2 : 1) * d.x_tile_bytes;
   d.stages_x = 2;
-  const long long budget = 224 * 1024 - 2 * C_SLAB_BYTES - (long long)d.stages_x * d.x_stage_bytes;
-  d.stages_w = (int)(budget / W_STAGE_BYTES);
-  if (d.stages_w > MAX_W_STAGES) d.stages_w = MAX_W_STAGES;
-  if (d.stages_w < 3) return hp;
-  hp.smem = (size_t)d.stages_x * d.x_stage_bytes + (size_t)d.stages_w * W_STAGE_BYTES + 2 * C_SLAB_BYTES + sizeof(SmemCtl) + 1024;
+  d.slab_bytes = pair ? pair_slab(d.split) : C_SLAB_BYTES;
+  const long long budget = SMEM_BUDGET - 2 * d.slab_bytes - (long long)d.stages_x * d.x_stage_bytes;
+  if (pair) {
+    int rows = pair_rows(p->KW);
+    while ((rows + 1) * p->KW <= MAX_W_STAGES && (long long)(rows + 1) * p->KW * PANEL_BYTES <= budget) ++rows;
+    d.stages_w = rows * p->KW;
+    d.w_bytes = d.stages_w * PANEL_BYTES;
+    if (d.stages_w > MAX_W_STAGES || d.w_bytes > budget) return hp;
+  } else {
+    d.stages_w = (int)(budget / W_STAGE_BYTES);
+    if (d.stages_w > 8) d.stages_w = 8;
+    if (d.stages_w < 3) return hp;
+    d.w_bytes = d.stages_w * W_STAGE_BYTES;
+  }
+  hp.smem = (size_t)d.stages_x * d.x_stage_bytes + d.w_bytes + 2 * d.slab_bytes + sizeof(SmemCtl) + 1024;
+  hp.cost *= (double)d.m_tiles * d.taps * d.cchunks;
   // share of the issued MMA work that lands in real outputs: positions x channels
   const double pos = (double)GH * GW / ((double)d.row_tiles * d.ncols2);
-  const double chn = (double)nch / ((double)d.m_tiles * BM);
+  const double chn = (double)nch / ((double)d.m_tiles * (pair ? 64 : BM)) * d.KW / d.KWs;
   hp.util = pos * chn;
   hp.ok = true;
   return hp;
+}
+
+// A data gradient with few channels goes by column pairs where the steps of its busiest SM then take fewer clocks.  Measured
+// (us, MODE_DGRAD and pairs): 64 x 28 x 28, 96 -> 64, 3 x 3: 18.4, 15.4; 300 x 14 x 14, 64 -> 32, 5 x 5: 52.2, 35.8; 128 x 20
+// x 20, 96 -> 48, 5 x 5: 32.8, 26.6; 64 x 27 x 27, 40 -> 48, 5 x 5: 24.6, 17.4; 256 x 28 x 28, 384 -> 64, 3 x 3: 120, 102.
+// Tiles of few rows look cheap by columns alone and are not: a step's weights take some 520 clocks (conv2 in tiles of two
+// image rows: 470 us).
+bool takes_pairs(const GeepsConvTcParams* p, const HaloPlan& plain) {
+  const HaloPlan pp = plan_halo(p, true);
+  return pp.ok && plain.ok && pp.cost < plain.cost;
 }
 
 int halo_mode() {
@@ -456,14 +565,11 @@ int geeps_conv_halo_applicable(const GeepsConvTcParams* p) {
   return d.taps >= 25 || (d.n_valid >= 64 && (d.n_valid <= 128 || chn >= 0.85)) ? 1 : 0;
 }
 
-int geeps_conv_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {
-  memset(out, 0, sizeof(*out));
-  if (!geeps_conv_tc_supported(p)) return 0;
-  const HaloPlan hp = plan_halo(p);
+static int fill_plan(const HaloPlan& hp, int routed, GeepsHaloPlanInfo* out) {
   if (!hp.ok) return 0;
   const HaloDev& d = hp.d;
   out->ok = 1;
-  out->routed = geeps_conv_halo_applicable(p);
+  out->routed = routed;
   out->PW = d.PW; out->R = d.Rb; out->row_tiles = d.row_tiles; out->m_tiles = d.m_tiles;
   out->positions = d.split; out->ncols2 = d.ncols2; out->ncols1 = d.ncols1;
   out->stages_x = d.stages_x; out->stages_w = d.stages_w; out->x_stage_bytes = d.x_stage_bytes;
@@ -472,20 +578,32 @@ int geeps_conv_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {
   out->util = hp.util;
   return 1;
 }
+int geeps_conv_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {
+  memset(out, 0, sizeof(*out));
+  if (!geeps_conv_tc_supported(p)) return 0;
+  return fill_plan(plan_halo(p), geeps_conv_halo_applicable(p), out);
+}
+int geeps_conv_halo_pair_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {
+  memset(out, 0, sizeof(*out));
+  if (!geeps_conv_tc_supported(p)) return 0;
+  return fill_plan(plan_halo(p, true), takes_pairs(p, plan_halo(p)), out);
+}
 
 int geeps_conv_halo(const GeepsConvTcParams* p, void* stream) {
   if (!geeps_conv_tc_supported(p)) return (int)cudaErrorInvalidValue;
   HaloPlan hp = plan_halo(p);
   if (!hp.ok) return (int)cudaErrorInvalidValue;
+  const bool pair = takes_pairs(p, hp);
+  if (pair) hp = plan_halo(p, true);
   HaloDev& d = hp.d;
   const bool fwd = p->mode == MODE_FWD;
   d.bias = fwd ? p->bias : nullptr;
   d.status = p->status;
   d.relu = fwd ? p->relu : 0;
   const int NR = 2 * d.Rb + p->KH - 1;
-  CUtensorMap tx, tw, tc;
+  CUtensorMap tx, tw, tc, tx1, tc1;
   bool ok;
-  const long long wdims[3] = {p->cg, d.taps, p->og};
+  const long long wdims[3] = {p->cg, d.KH * d.KW, p->og};
   const long long wst[2] = {(long long)p->cg * 2, p->ldw * 2};
   if (fwd) {
     ok = make_act_map(&tx, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, d.PW, NR);
@@ -493,17 +611,30 @@ int geeps_conv_halo(const GeepsConvTcParams* p, void* stream) {
     ok = ok && make_map(&tw, p->w, 3, wdims, wst, wbox);
     ok = ok && make_act_map(&tc, p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, d.PW, d.Rb);
   } else {
-    ok = make_act_map(&tx, p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, d.PW, NR);
     const int wbox[3] = {64, 1, 64};
-    ok = ok && make_map(&tw, p->w, 3, wdims, wst, wbox);
-    ok = ok && make_act_map(&tc, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, d.PW, d.Rb);
+    ok = make_map(&tw, p->w, 3, wdims, wst, wbox);
+    if (pair) {
+      // padded column 2 c + h is image column 2 c + h - px: column x0 (x1) + c of the image's columns of parity b
+      const int b0 = d.px & 1, b1 = (d.px + 1) & 1;
+      d.x0 = (-d.px - b0) / 2;
+      d.x1 = (1 - d.px - b1) / 2;
+      ok = ok && make_parity_map(&tx, p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, b0, d.PW, NR) &&
+           make_parity_map(&tx1, p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, b1, d.PW, NR) &&
+           make_parity_map(&tc, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, 0, d.PW, d.Rb) &&
+           make_parity_map(&tc1, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, 1, d.PW, d.Rb);
+    } else {
+      ok = ok && make_act_map(&tx, p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, d.PW, NR) &&
+           make_act_map(&tc, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, d.PW, d.Rb);
+    }
   }
+  if (!pair) { tx1 = tx; tc1 = tc; }      // unused by the kernel
   if (!ok) return (int)cudaErrorInvalidValue;
   const long long num_tiles = (long long)d.m_tiles * d.n_images * d.row_tiles;
   const int sms = geeps_sm_count();
   const int grid = (int)(num_tiles < sms ? num_tiles : sms);
-  if (fwd) return launch<MODE_FWD>(tx, tw, tc, d, grid, hp.smem, (cudaStream_t)stream);
-  return launch<MODE_DGRAD>(tx, tw, tc, d, grid, hp.smem, (cudaStream_t)stream);
+  if (fwd) return launch<MODE_FWD>(tx, tw, tc, tx1, tc1, d, grid, hp.smem, (cudaStream_t)stream);
+  if (pair) return launch<MODE_DGRAD2>(tx, tw, tc, tx1, tc1, d, grid, hp.smem, (cudaStream_t)stream);
+  return launch<MODE_DGRAD>(tx, tw, tc, tx1, tc1, d, grid, hp.smem, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -187,6 +187,8 @@ typedef struct GeepsHaloPlanInfo {
   double util;
 } GeepsHaloPlanInfo;
 int geeps_conv_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
+// ... and of a data gradient by column pairs; routed: geeps_conv_halo takes it that way
+int geeps_conv_halo_pair_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
 int geeps_conv_wgrad_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
 
 // ---------------- parameter pull fused with the consuming GEMM ----------------

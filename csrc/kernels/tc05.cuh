@@ -237,6 +237,19 @@ __device__ __forceinline__ void mma_bf16_ss_lohi(uint32_t tmem_d, uint32_t a_lo,
       : "memory");
 }
 
+// ... which leaves accumulator rows 0 to 63 (no_low = ~0) or 64 to 127 (no_high = ~0) as they are
+__device__ __forceinline__ void mma_bf16_ss_halves(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                                   uint32_t idesc, uint32_t accumulate, uint32_t no_low, uint32_t no_high) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %2};\n\t"
+      "mov.b64 db, {%3, %4};\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%7, %7, %8, %8}, p;\n\t}"
+      ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(no_low), "r"(no_high)
+      : "memory");
+}
+
 // ---------------- a k-tile's products issued by a converged warp ----------------
 // The lane is elected (always the same one) inside, so there is no divergent branch around the products: addresses and
 // descriptors stay in the warp's uniform registers, where the instructions want them.  Behind an `if (leader)` every one

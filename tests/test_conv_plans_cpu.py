@@ -95,3 +95,30 @@ def test_weight_gradient_plans_respect_the_hardware_limits():
         assert rows_read * 128 <= info.x_stage_bytes
         assert info.stages_x >= 2 and info.smem_bytes <= SMEM_LIMIT
     assert seen > 100 and routed > 0
+
+
+def test_column_pair_data_gradient_plans_respect_the_hardware_limits():
+    lib = L.lib()
+    seen = routed = 0
+    for B, H, cg, og, k, pad in SHAPES + [(256, H, cg, 96, k, k // 2) for H in (2, 3, 27, 31, 40, 55) for cg in (8, 48, 56, 64)
+                                          for k in (2, 3, 4, 5, 6, 7)]:
+        p, OH, OW = _params(1, B, H, H, cg, og, k, pad)
+        info = L.HaloPlanInfo()
+        if not lib.geeps_conv_halo_pair_plan(C.byref(p), C.byref(info)):
+            continue
+        seen += 1
+        routed += info.routed
+        assert cg <= 64 and H >= 2 and OW >= 2 and info.m_tiles == 1
+        assert info.PW >= (H + 1) // 2 + k // 2 and info.PW <= 128          # no window leaves its row
+        assert info.positions == info.R * info.PW and info.positions % 8 == 0 and 0 < info.positions <= 128
+        assert info.ncols2 % 16 == 0 and 2 * info.positions <= info.ncols2 <= 256
+        assert 2 * info.R * info.row_tiles >= H > 2 * info.R * (info.row_tiles - 1)
+        # the last step of a row reads k // 2 columns on, in either parity's tile
+        assert ((k - 1) * info.PW + k // 2 + info.ncols2) * 128 <= info.x_stage_bytes // 2
+        assert info.x_stage_bytes % 2048 == 0
+        # whole filter rows of panels (8192 bytes); a panel in front of them and one behind are read for disabled lanes
+        slab = max(8192, (info.positions * 128 + 1023) // 1024 * 1024)
+        assert info.stages_w % k == 0 and 5 <= info.stages_w <= 16 and info.stages_x * info.x_stage_bytes >= 8192
+        assert info.stages_x * info.x_stage_bytes + info.stages_w * 8192 + 2 * slab < info.smem_bytes <= SMEM_LIMIT
+        assert 0.0 < info.util <= 1.0
+    assert seen > 100 and routed > 0

@@ -125,6 +125,55 @@ def test_strided_conv_forward_and_gradients_match_torch(case):
     assert status.tolist()[0] == 0
 
 
+COLUMN_PAIRS = [
+    # B, H, W, C_total, c_off, cg, O_total, o_off, og, k, pad
+    (160, 27, 27, 96, 48, 48, 256, 128, 128, 5, 2),     # AlexNet conv2, channel slices on both sides
+    (2, 9, 28, 64, 0, 64, 72, 0, 72, 3, 1),             # even width, second chunk of 8 gradient channels
+    (4, 6, 2, 16, 0, 16, 24, 0, 24, 3, 1),              # one pair of columns
+    (2, 11, 13, 56, 0, 56, 40, 0, 40, 4, 1),            # even filter: halo of 2, the last step reads the even parity
+    (2, 17, 40, 8, 0, 8, 64, 0, 64, 7, 0),              # 7 taps, no padding
+    (400, 8, 7, 32, 0, 32, 40, 0, 40, 5, 2),            # more tiles than SMs
+    (3, 6, 9, 24, 0, 24, 16, 0, 16, 2, 0),              # two taps a row, few k
+]
+
+
+@pytest.mark.parametrize("case", COLUMN_PAIRS)
+def test_column_pair_data_gradient_matches_torch(case):
+    """The even and the odd column of a pair in the two halves of an accumulator, KW + 1 steps per filter row."""
+    import ctypes
+    from geeps_b200.ops import _lib as L
+    from geeps_b200.ops import functional as F
+    B, H, W, Ct, c_off, cg, Ot, o_off, og, k, pad = case
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(11)
+    OH, OW, kd = H + 2 * pad - k + 1, W + 2 * pad - k + 1, k * k * cg
+    ld = (kd + 7) // 8 * 8
+    w = torch.zeros(og, ld, device=dev, dtype=BF)
+    w[:, :kd] = (torch.randn(og, kd, device=dev, generator=gen) / kd ** 0.5).to(BF)
+    dy = torch.randn(B, OH, OW, Ot, device=dev, generator=gen).to(BF)[..., o_off:o_off + og]
+    dy[0, OH // 2, OW // 2, 0] = float("inf")           # spoils its own window only
+    wr = w[:, :kd].double().view(og, k, k, cg).permute(0, 3, 1, 2)
+    ref = torch.nn.functional.conv_transpose2d(dy.double().permute(0, 3, 1, 2), wr, padding=pad).permute(0, 2, 3, 1)
+    dx_full = torch.full((B, H, W, Ct), 3.0, device=dev, dtype=BF)
+    dx = dx_full[..., c_off:c_off + cg]
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    p, pairs = F.conv_tc_params(F.CONV_DGRAD, dx, dy, w, k, pad), L.HaloPlanInfo()
+    assert L.lib().geeps_conv_halo_pair_plan(ctypes.byref(p), ctypes.byref(pairs))
+    if not pairs.routed:
+        pytest.skip("the kernel takes this shape without pairs on this GPU")
+    F.conv_halo(F.CONV_DGRAD, dx, dy, w, k, pad, status=status)
+    torch.cuda.synchronize()
+    spoilt = torch.zeros(H, W, dtype=torch.bool, device=dev)
+    y0, x0 = OH // 2 - pad, OW // 2 - pad
+    spoilt[max(y0, 0):y0 + k, max(x0, 0):x0 + k] = True
+    fine = torch.isfinite(dx).all(-1)
+    assert bool(fine[1:].all()) and bool((fine[0] == ~spoilt).all())
+    # fp32 sums rounded once to bf16: uniform relative rounding errors of up to 2^-9, 2^-9 / sqrt(3) = 1.1e-3 in the 2-norm
+    assert _rel(dx[fine], ref[fine]) < 2.5e-3
+    assert bool((dx_full[..., :c_off] == 3.0).all()) and bool((dx_full[..., c_off + cg:] == 3.0).all())
+    assert status.tolist()[0] == 0
+
+
 HALO_CASES = CASES + [
     (3, 57, 57, 48, 0, 48, 96, 0, 96, 3, 0),            # AlexNet conv1 after space-to-depth: 96 channels leave in 32-wide slabs
     (3, 28, 28, 192, 0, 192, 96, 0, 96, 3, 1),          # three chunks, rows split 4 + 4 per tile, last tile short
