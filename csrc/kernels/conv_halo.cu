@@ -55,7 +55,7 @@ constexpr int UMMA_K = 16;
 constexpr int PANEL_BYTES = 64 * BK * 2;
 constexpr int W_STAGE_BYTES = BM * BK * 2;    // 128 channels x 64 k (forward) or two [64 k][64 channels] panels (dgrad)
 constexpr int MAX_X_STAGES = 2;
-constexpr int MAX_W_STAGES = 16;
+constexpr int MAX_W_STAGES = 16;             // of one panel; 8 of two
 constexpr uint64_t WAIT_BUDGET_NS = 2000000000ull;
 constexpr int C_SLAB_BYTES = 128 * 128;       // 128 positions x 64 channels bf16
 constexpr int ACC_COLS = 256;
@@ -112,7 +112,7 @@ __device__ __forceinline__ Tile decode_tile(const HaloDev& d, int t) {
 
 // tmX: the source activations (fwd: X, dgrad: dY) as (c, w, h, b) with box (64, PW, 2 Rb + KH - 1, 1);
 // tmW: weights (ci, tap, co): fwd box (64 ci, 1, 128 co) K-major, dgrad box (64 ci, 1, 64 co) = one MN-major panel;
-// tmC: the result (fwd: Y, dgrad: dX) with box (64, PW, Rb, 1).
+// tmC: the result (fwd: Y, dgrad: dX) with box (64, PW, Rb, 1); tmX1, tmC1: MODE_DGRAD2's second parity.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
@@ -233,7 +233,10 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         int tx = 0;
         for (int tap = 0; tap < d.taps; ++tap) {
           // MODE_DGRAD2: the last step of a row has no tap of its own
-          if ((!PAIR || tx < d.KW) && !tc05::mbar_wait_warp(&ctl->full_w[sw], phw, abort_flag, WAIT_BUDGET_NS)) { ok = false; break; }
+          if ((!PAIR || tx < d.KW) && !tc05::mbar_wait_warp(&ctl->full_w[sw], phw, abort_flag, WAIT_BUDGET_NS)) {
+            ok = false;
+            break;
+          }
           tc05::fence_after_sync();
           if (leader) {
             const uint8_t* wt = tiles_w + (PAIR ? (ptrdiff_t)(wrow + d.KW - 1 - tx) * PANEL_BYTES : (ptrdiff_t)sw * W_STAGE_BYTES);
@@ -507,7 +510,7 @@ HaloPlan plan_halo(const GeepsConvTcParams* p, bool pair = false) {
     if (d.stages_w > MAX_W_STAGES || d.w_bytes > budget) return hp;
   } else {
     d.stages_w = (int)(budget / W_STAGE_BYTES);
-    if (d.stages_w > 8) d.stages_w = 8;
+    if (d.stages_w > MAX_W_STAGES / 2) d.stages_w = MAX_W_STAGES / 2;
     if (d.stages_w < 3) return hp;
     d.w_bytes = d.stages_w * W_STAGE_BYTES;
   }
@@ -526,9 +529,8 @@ HaloPlan plan_halo(const GeepsConvTcParams* p, bool pair = false) {
 // x 20, 96 -> 48, 5 x 5: 32.8, 26.6; 64 x 27 x 27, 40 -> 48, 5 x 5: 24.6, 17.4; 256 x 28 x 28, 384 -> 64, 3 x 3: 120, 102.
 // Tiles of few rows look cheap by columns alone and are not: a step's weights take some 520 clocks (conv2 in tiles of two
 // image rows: 470 us).
-bool takes_pairs(const GeepsConvTcParams* p, const HaloPlan& plain) {
-  const HaloPlan pp = plan_halo(p, true);
-  return pp.ok && plain.ok && pp.cost < plain.cost;
+bool takes_pairs(const HaloPlan& plain, const HaloPlan& pairs) {
+  return plain.ok && pairs.ok && pairs.cost < plain.cost;
 }
 
 int halo_mode() {
@@ -586,15 +588,17 @@ int geeps_conv_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {
 int geeps_conv_halo_pair_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {
   memset(out, 0, sizeof(*out));
   if (!geeps_conv_tc_supported(p)) return 0;
-  return fill_plan(plan_halo(p, true), takes_pairs(p, plan_halo(p)), out);
+  const HaloPlan pairs = plan_halo(p, true);
+  return fill_plan(pairs, takes_pairs(plan_halo(p), pairs), out);
 }
 
 int geeps_conv_halo(const GeepsConvTcParams* p, void* stream) {
   if (!geeps_conv_tc_supported(p)) return (int)cudaErrorInvalidValue;
   HaloPlan hp = plan_halo(p);
   if (!hp.ok) return (int)cudaErrorInvalidValue;
-  const bool pair = takes_pairs(p, hp);
-  if (pair) hp = plan_halo(p, true);
+  const HaloPlan pairs = plan_halo(p, true);
+  const bool pair = takes_pairs(hp, pairs);
+  if (pair) hp = pairs;
   HaloDev& d = hp.d;
   const bool fwd = p->mode == MODE_FWD;
   d.bias = fwd ? p->bias : nullptr;
