@@ -266,6 +266,12 @@ void ClientLib::fabric_teardown() {
   fabric_.active = false;
 }
 
+static bool stream_capturing(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing((cudaStream_t)stream, &status) != cudaSuccess) cudaGetLastError();
+  return status != cudaStreamCaptureStatusNone;
+}
+
 // With one worker there is nobody to signal and nobody to wait for but the comm stream of this process, which an event
 // orders: no announcement kernel on the application's stream, no wait kernel on the comm stream, none in front of a read
 // (each 2 to 6 us of the stream; the announcement flushes its writes to system scope).  AlexNet's step 2218 -> 2176 us, a
@@ -288,7 +294,8 @@ void ClientLib::fabric_wait_data_age(CachedTable& ct, uint table_id, iter_t need
     // the latest push is the one that is asked for (slack 0), or the end of the last clock is behind it on this stream
     const Fabric::Applied& ap = fabric_.applied[table_id];
     const bool joined = device_clock_ != nullptr && stream == fabric_.joined_stream && needed_age < clock_;
-    if (joined || (device_clock_ == nullptr && ap.event != nullptr && ap.clock == needed_age)) {
+    // (a captured access takes the flags: a stream in capture cannot wait for an event recorded outside)
+    if (joined || (device_clock_ == nullptr && ap.event != nullptr && ap.clock == needed_age && !stream_capturing(stream))) {
       if (!joined) cudaStreamWaitEvent((cudaStream_t)stream, (cudaEvent_t)ap.event, 0);
       if (mine) mine->second = stamp; else ct.waited_by_stream.emplace_back(stream, stamp);
       stats_.device_waits_enqueued++;
@@ -365,9 +372,8 @@ void ClientLib::fabric_push(iter_t clock, uint table_id, bool is_init, void* str
   }
   // device time of the push kernel itself (the wait for the other workers is not part of it)
   Fabric::PushTiming* pt = nullptr;
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing((cudaStream_t)cs, &capturing);
-  if (!is_init && capturing == cudaStreamCaptureStatusNone) {   // an event recorded under capture cannot be queried
+  const bool capturing = stream_capturing(cs);
+  if (!is_init && !capturing) {   // an event recorded under capture cannot be queried
     if (fabric_.push_timing.empty()) fabric_.push_timing.resize(kPushTimingRing);
     pt = &fabric_.push_timing[fabric_.push_timing_next++ % kPushTimingRing];
     if (!pt->begin) {
@@ -435,7 +441,7 @@ void ClientLib::fabric_push(iter_t clock, uint table_id, bool is_init, void* str
   if (fabric_.applied.size() <= table_id) fabric_.applied.resize(table_id + 1);
   Fabric::Applied& ap = fabric_.applied[table_id];
   ap.clock = -1;
-  if (by_events && capturing == cudaStreamCaptureStatusNone) {
+  if (by_events && !capturing) {
     if (!ap.event) {
       cudaEvent_t e;
       cudaEventCreateWithFlags(&e, cudaEventDisableTiming);

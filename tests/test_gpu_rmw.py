@@ -157,3 +157,48 @@ def test_one_worker_reads_see_the_last_push_on_any_stream(slack):
             lo, hi = mm.tolist()
             assert c + 1 - slack <= lo and hi <= c + 1 and (slack or lo == hi), (c, lo, hi)
         g.close()
+
+
+def test_one_worker_read_and_pre_update_inside_a_callers_capture():
+    """A Read or PreUpdate that the application captures (no device clock): the freshness wait is a node of its graph."""
+    dev = torch.device("cuda:0")
+    cfg = GeePsConfig(device=DEVICE_CUDA, cuda_device=0, transport=TRANSPORT_NVLINK, tcp_base_port=28531)
+    sa, sb = torch.cuda.Stream(device=dev), torch.cuda.Stream(device=dev)
+    got = torch.zeros(40, 128, device=dev)
+    torch.cuda.synchronize()
+
+    def captured(stream, fn):
+        graph, nodes = C.c_void_p(), C.c_longlong(0)
+        assert lib().geeps_graph_begin(C.c_void_p(stream.cuda_stream)) == 0
+        with torch.cuda.stream(stream):
+            fn()
+        assert lib().geeps_graph_end(C.c_void_p(stream.cuda_stream), C.byref(graph), C.byref(nodes)) == 0
+        assert nodes.value == 2                        # the wait and the caller's own kernel
+        assert lib().geeps_graph_launch(graph, C.c_void_p(stream.cuda_stream)) == 0
+        return graph
+
+    with torch.cuda.stream(sa):
+        g = GeePs(0, cfg)
+        rows = list(range(40))
+        r = g.virtual_read(0, rows, 0); u = g.virtual_pre_update(0, rows)
+        pr = g.virtual_post_read(r); up = g.virtual_update(u); g.virtual_clock()
+        g.finish_virtual_iteration()
+        g.pre_update(u).fill_(1.0); g.update(up); g.clock(); g.start_iterations()
+        graphs = []
+        for c in range(4):
+            if c % 2 == 0:                             # clocks with and without captures follow one another
+                graphs.append(captured(sa, lambda: got.copy_(g.read(r, stream=sa))))
+                graphs.append(captured(sb, lambda: g.pre_update(u, stream=sb).fill_(1.0)))
+            else:
+                got.copy_(g.read(r, stream=sa))
+                with torch.cuda.stream(sb):
+                    g.pre_update(u, stream=sb).fill_(1.0)
+            g.post_read(pr, stream=sa)
+            sb.wait_stream(sa)
+            g.update(up, stream=sb); g.clock()
+            torch.cuda.synchronize()
+            assert torch.all(got == c + 1.0), c
+        assert g.last_error() == 0
+        for graph in graphs:
+            lib().geeps_graph_destroy(graph)
+        g.close()
