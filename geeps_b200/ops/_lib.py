@@ -166,6 +166,7 @@ class Tape:
 
     def __init__(self):
         self.ops = []          # (cfunc, args tuple, label)
+        self.held = []         # tensors that the arguments point into and that nothing else may keep
 
     def signature(self):
         sig = []
@@ -203,6 +204,7 @@ class StepGraph:
         self.stream = stream
         self.kernel_launches = tape.kernel_launches
         self.nodes = 0
+        self._held = tape.held
         self._exec = C.c_void_p()
         l = lib()
         err = l.geeps_graph_begin(C.c_void_p(stream.cuda_stream))
@@ -259,6 +261,13 @@ def launch(fn, label: str, *args) -> None:
     if _tape is not None:
         _tape.ops.append((fn, args, label))
     check(fn(*args), label)
+
+
+def hold(t):
+    """A tensor made during a step: a recorded step names its address and keeps it."""
+    if _tape is not None:
+        _tape.held.append(t)
+    return t
 
 
 def record_call(fn, label: str, *args):

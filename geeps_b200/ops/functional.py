@@ -133,7 +133,7 @@ def nchw_to_nhwc_bf16(x: torch.Tensor, cpad: int | None = None) -> torch.Tensor:
     B, Cc, H, W = x.shape
     cpad = cpad or Cc
     assert x.dtype in (torch.float32, bf16) and x.is_contiguous()
-    y = torch.empty((B, H, W, cpad), dtype=bf16, device=x.device)
+    y = L.hold(torch.empty((B, H, W, cpad), dtype=bf16, device=x.device))
     launch(lib().geeps_nchw_to_nhwc_bf16, "nchw_to_nhwc", ptr(x), int(x.dtype == bf16), ptr(y), B, Cc, H, W, cpad,
            stream_ptr())
     return y

@@ -17,6 +17,7 @@ from dataclasses import dataclass
 
 import torch
 
+from . import _lib as L
 from . import functional as F
 
 BF = torch.bfloat16
@@ -181,7 +182,7 @@ class Input(Layer):
                 self._src_hw = src_hw
                 self._centre_crop()
             self._src_hw = src_hw
-            y = self.y if self.s2d else torch.empty(self.out_shape, dtype=BF, device=x.device)
+            y = self.y if self.s2d else L.hold(torch.empty(self.out_shape, dtype=BF, device=x.device))
             return F.u8_transform(x, y, (H, W), self.s2d, self.aug, self.mean, self.scale)
         if self.s2d:
             return F.nchw_to_s2d_bf16(x, self.y, self.s2d)

@@ -589,3 +589,25 @@ def test_batchnorm_in_one_launch_keeps_and_reads_the_mask_bits():
     r = subprocess.run([sys.executable, "-c", _COOP], capture_output=True, text=True, timeout=300,
                        env=dict(os.environ, GEEPS_BN_COOP="1"), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.uint8])
+def test_recorded_step_keeps_the_input_layers_output(dtype):
+    """A plain NHWC input layer makes its output anew; the address that a recording names must not be given away."""
+    from geeps_b200.ops.layers import Input
+    inp = Input(cpad=8)
+    inp.setup((4, 3, 24, 24), DEV)
+    x = torch.zeros(4, 3, 24, 24, device=DEV).to(dtype)
+    stream = torch.cuda.Stream(device=DEV)
+    with torch.cuda.stream(stream):
+        inp.forward(x)
+        L.start_recording()
+        address = inp.forward(x).data_ptr()           # dropped at once
+        tape = L.stop_recording()
+        graph = L.StepGraph(tape, stream)
+        del tape
+        others = [torch.empty(4, 24, 24, 8, device=DEV, dtype=BF) for _ in range(8)]
+        assert address not in [t.data_ptr() for t in others]
+        graph.launch()
+    torch.cuda.synchronize()
+    graph.close()
