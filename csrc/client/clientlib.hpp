@@ -146,7 +146,8 @@ struct Fabric {
   // one worker: what a table's freshness wait needs is its latest push on the comm stream, an event
   struct Applied { void* event = nullptr; int clock = -1; };
   std::vector<Applied> applied;           // by table; clock: of the push that the event follows
-  void* joined_stream = nullptr;          // device-clock mode: the stream that the comm lanes last joined
+  void* joined_stream = nullptr;          // device-clock mode: the stream that the comm lanes last joined ...
+  bool joined = false;                    // ... in a host-run iteration that no replay has followed
   void* join_event = nullptr;             // device-clock mode: comm lanes -> application stream at the end of a clock
   int* host_status = nullptr;             // pinned mirror of the device status block
 };

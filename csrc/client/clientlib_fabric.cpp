@@ -291,11 +291,15 @@ void ClientLib::fabric_wait_data_age(CachedTable& ct, uint table_id, iter_t need
   for (auto& w : ct.waited_by_stream) if (w.first == stream) mine = &w;
   if (mine && stamp <= mine->second) return;
   if (fabric_by_events(ct) && table_id < fabric_.applied.size()) {
-    // the latest push is the one that is asked for (slack 0), or the end of the last clock is behind it on this stream
+    // The latest push is the one that is asked for (slack 0), or the end of the last clock is behind it on this stream.  With
+    // the device clock a captured access needs no wait of its own either: the clock word is advanced behind the end of all
+    // pushes, and a replay, whose stamps are relative to that word, follows the iteration before it on the device.  Without
+    // it a captured access takes the flags: a stream in capture cannot wait for an event recorded outside.
     const Fabric::Applied& ap = fabric_.applied[table_id];
-    const bool joined = device_clock_ != nullptr && stream == fabric_.joined_stream && needed_age < clock_;
-    // (a captured access takes the flags: a stream in capture cannot wait for an event recorded outside)
-    if (joined || (device_clock_ == nullptr && ap.event != nullptr && ap.clock == needed_age && !stream_capturing(stream))) {
+    const bool capturing = stream_capturing(stream);
+    const bool joined = device_clock_ != nullptr && needed_age < clock_ &&
+                        (capturing || (fabric_.joined && stream == fabric_.joined_stream));
+    if (joined || (device_clock_ == nullptr && ap.event != nullptr && ap.clock == needed_age && !capturing)) {
       if (!joined) cudaStreamWaitEvent((cudaStream_t)stream, (cudaEvent_t)ap.event, 0);
       if (mine) mine->second = stamp; else ct.waited_by_stream.emplace_back(stream, stamp);
       stats_.device_waits_enqueued++;
@@ -539,6 +543,7 @@ void ClientLib::fabric_end_iteration_device_clock() {
     cudaStreamWaitEvent(app, (cudaEvent_t)fabric_.join_event, 0);
   }
   fabric_.joined_stream = app;
+  fabric_.joined = true;
   geeps_clock_advance(device_clock_, app);
 }
 
@@ -560,6 +565,7 @@ void ClientLib::advance_replayed_iteration() {
     else if (op.type == OP_PRE_UPDATE) stats_.nr_preupdate++;
     else if (op.type == OP_UPDATE) { stats_.nr_update++; stats_.rows_updated += plan_.ops[op.prestep].rows.size(); }
   }
+  fabric_.joined = false;       // the replay joined the comm lanes into the stream that it ran on, not the last host-run one
   clock_++;
   last_handle_ = -1;
   stats_.nr_clock++;

@@ -149,7 +149,7 @@ class PSModule:
         self.use_tape = (use_tape or self.use_graph) and not manage_activations
         self._graphs, self._graph_failed = {}, False
         self._period = (slack + 1) if (slack + 1) % 2 == 0 else 2 * (slack + 1)
-        self._tapes, self._tape_sigs, self._tape_tries = {}, {}, {}     # keyed by (input ptr, label ptr, clock phase)
+        self._tapes, self._tape_sigs, self._tape_tries = {}, {}, {}     # keyed by _step_key()
         self.tape_mismatch = None
         # diagnostics: set to [] to collect CUDA events (step start, forward end, backward end, clock end) per step
         self.phase_events = None
@@ -255,13 +255,17 @@ class PSModule:
             for name, v in t.layer.p32.items():
                 self.captured[f"{t.layer.name}.{name}"] = v.clone()
 
+    def _step_key(self, x, labels):
+        """What a recorded step depends on.  The update ring has slack + 1 slots and staged buffers alternate between two
+        copies, so the pointers a step uses repeat with the least common multiple of the two; its launches name the stream."""
+        stream = torch.cuda.current_stream(self.device).cuda_stream if x.is_cuda else None
+        return (x.data_ptr(), labels.data_ptr(), self.steps % self._period, stream)
+
     def step(self, x: torch.Tensor, labels: torch.Tensor, capture: bool = False) -> torch.Tensor:
         """One clock: forward, backward, push.  Returns the mean loss as a 1-element device tensor.
         capture=True keeps clones of the parameters this clock read in `self.captured`."""
         net, tr = self.net, self.trace
-        # the update ring has slack + 1 slots and staged buffers alternate between two copies, so the pointers a
-        # step uses repeat with the least common multiple of the two
-        key = (x.data_ptr(), labels.data_ptr(), self.steps % self._period)
+        key = self._step_key(x, labels)
         graph = self._graphs.get(key) if self.use_graph and not capture else None
         if graph is not None:
             graph.launch()
@@ -367,7 +371,7 @@ class PSModule:
     def is_steady(self, x: torch.Tensor, labels: torch.Tensor) -> bool:
         """True when the next step with these buffers replays a captured graph (or, without graphs, a recorded
         tape): the Python layer code and the capture work are behind us."""
-        key = (x.data_ptr(), labels.data_ptr(), self.steps % self._period)
+        key = self._step_key(x, labels)
         if self.use_graph and not self._graph_failed:
             return key in self._graphs
         return (not self.use_tape) or key in self._tapes

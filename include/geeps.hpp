@@ -151,7 +151,8 @@ class GeePs {
    * changes from clock to clock and can be captured in a CUDA graph (one graph per phase of the update ring, i.e.
    * per clock modulo slack + 1).  From then on Clock() joins the runtime's streams into the stream of the latest
    * access call and advances the device word there.  After replaying a captured iteration, call
-   * AdvanceReplayedClock() instead of repeating the access calls.  DeviceClockPtr() is the device word (an int that
+   * AdvanceReplayedClock() instead of repeating the access calls.  Iterations follow one another on the device: an
+   * application that goes on in another stream orders it behind the last one.  DeviceClockPtr() is the device word (an int that
    * kernels of the application may read, e.g. to derive per-step random seeds). */
   bool EnableDeviceClock();
   void AdvanceReplayedClock();

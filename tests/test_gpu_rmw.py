@@ -202,3 +202,55 @@ def test_one_worker_read_and_pre_update_inside_a_callers_capture():
         for graph in graphs:
             lib().geeps_graph_destroy(graph)
         g.close()
+
+
+def test_device_clock_iterations_on_alternating_streams():
+    """Host-run, captured and replayed iterations on two streams, each ordered behind the iteration before it."""
+    dev = torch.device("cuda:0")
+    cfg = GeePsConfig(device=DEVICE_CUDA, cuda_device=0, transport=TRANSPORT_NVLINK, tcp_base_port=28551)
+    s0, s1 = torch.cuda.Stream(device=dev), torch.cuda.Stream(device=dev)
+    got = torch.zeros(20000, 128, device=dev)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s0):
+        g = GeePs(0, cfg)
+        rows = list(range(20000))
+        r = g.virtual_read(0, rows, 0); u = g.virtual_pre_update(0, rows)
+        pr = g.virtual_post_read(r); up = g.virtual_update(u); g.virtual_clock()
+        g.finish_virtual_iteration()
+        g.pre_update(u).fill_(1.0); g.update(up); g.clock(); g.start_iterations()
+        assert all(op["direct"] for op in g.plan()["ops"] if op["type"] in ("read", "pre_update"))
+        g.enable_device_clock()
+
+    def iteration(stream):
+        got.copy_(g.read(r, stream=stream))
+        b = g.pre_update(u, stream=stream)
+        g.post_read(pr, stream=stream)
+        b.fill_(1.0)
+        g.update(up, stream=stream); g.clock()
+
+    graphs, seen, last = {}, [], s0
+    plan = [(s0, 0), (s0, 0), (s1, 1), (s1, 1), (s0, 0), (s1, 1), (s0, 1), (s0, 1), (s1, 1), (s1, 0), (s0, 1), (s1, 0), (s0, 0)]
+    for stream, as_graph in plan:
+        stream.wait_stream(last)
+        last = stream
+        with torch.cuda.stream(stream):
+            if as_graph and stream in graphs:
+                assert lib().geeps_graph_launch(graphs[stream], C.c_void_p(stream.cuda_stream)) == 0
+                g.advance_replayed_clock()
+            elif as_graph:
+                graphs[stream] = C.c_void_p()
+                nodes = C.c_longlong(0)
+                assert lib().geeps_graph_begin(C.c_void_p(stream.cuda_stream)) == 0
+                iteration(stream)
+                assert lib().geeps_graph_end(C.c_void_p(stream.cuda_stream), C.byref(graphs[stream]), C.byref(nodes)) == 0
+                assert lib().geeps_graph_launch(graphs[stream], C.c_void_p(stream.cuda_stream)) == 0
+            else:
+                iteration(stream)
+            seen.append(torch.stack([got.min(), got.max()]))
+    torch.cuda.synchronize()
+    g.check()
+    for c, mm in enumerate(seen):
+        assert mm.tolist() == [c + 1.0, c + 1.0], (c, mm.tolist())
+    for graph in graphs.values():
+        lib().geeps_graph_destroy(graph)
+    g.close()

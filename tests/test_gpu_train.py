@@ -421,3 +421,37 @@ def test_concurrent_module_backward_matches_the_serial_one():
         # sums of BatchNorm statistics and of gradient slices in another order: some 2^-24 per addition, roundings to bf16
         # between the layers of a branch where such a difference meets a tie
         assert (a.float() - b.float()).norm() <= 2e-3 * b.float().norm()
+
+
+def test_graph_steps_follow_the_callers_stream():
+    """Steps on streams that change: each is ordered behind the last, its batch is written late on the stream that it is
+    called on, and recorded steps run there too - losses equal those of a module that stays on one stream."""
+    dev = torch.device("cuda:0")
+    B, steps = 16, 28
+    gen = torch.Generator(device=dev).manual_seed(11)
+    batches = [torch.randn(B, 3, 16, 16, device=dev, generator=gen) for _ in range(steps)]
+    y = torch.randint(0, 10, (B,), device=dev, generator=gen)
+    torch.cuda.synchronize()
+    losses = []
+    for changing in (False, True):
+        streams = [torch.cuda.Stream(device=dev) for _ in range(2)]
+        last = streams[0]
+        with torch.cuda.stream(last):
+            mod = PSModule(tiny_net(), (B, 3, 16, 16), cfg(TRANSPORT_NVLINK, learning_rate=0.05), device=dev, seed=3, use_graph=True)
+            x = torch.empty_like(batches[0])
+        out = []
+        for i in range(steps):
+            s = streams[(i // 7) % 2 if changing else 0]
+            s.wait_stream(last)
+            last = s
+            with torch.cuda.stream(s):
+                torch.cuda._sleep(200_000)
+                x.copy_(batches[i])
+                out.append(mod.step(x, y).clone())
+        torch.cuda.synchronize()
+        assert mod.ps.get_stats()["client"]["nr_replayed_clocks"] > 0
+        assert len({key[3] for key in mod._graphs}) == (2 if changing else 1)
+        losses.append(torch.cat(out))
+        mod.close()
+    # gradient slices meet in fp32 atomics in any order
+    assert torch.allclose(losses[0], losses[1], rtol=1e-3), losses
