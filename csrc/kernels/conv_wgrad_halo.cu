@@ -310,12 +310,19 @@ WgPlan plan_wgrad(const GeepsConvTcParams* p) {
   int tc = 32;
   while (tc < d.TY * d.KW * 64) tc <<= 1;
   d.tmem_cols = tc;
-  // slices of the positions: one item per SM, so that accumulators are drained once (nothing covers that: they take most
-  // of TMEM) and every part of dW is added to half as often: conv2 per group 74.2 us, with two items 77.8.  Items of
-  // several filter rows have more to drain and do better with two, the first drained while other SMs multiply (conv1: 105
-  // us, with one 109)
+  // Slices of the positions.  The busiest SM walks `waves` items, and each costs about five position blocks beside its own:
+  // its accumulators are drained (nothing covers that: they take most of TMEM) and its part of dW is added once more.  One
+  // wave of long items against two (us): conv2 per group, 5 items a slice: 72, 77; 200 x 20 x 20, 5 x 5, 128 -> 128 (10):
+  // 76, 80; 256 -> 128 (20): 140, 143.  Where a wave leaves SMs idle two win: 192 -> 128 (15): 112, 110; 256 -> 256 (40):
+  // 311, 270; 296 -> 344 (75): 896, 615.  Items of several filter rows (conv1, 105 us, with one wave 109) have unequal
+  // shares, which the second wave evens out.
+  const int sms = geeps_sm_count();
   const long long base_items = (long long)d.m_tiles * d.cchunks * d.passes;
-  long long split = ((d.TY > 1 ? 2LL : 1LL) * geeps_sm_count()) / base_items;
+  const long long most = 2LL * sms / base_items;
+  long long split = d.TY > 1 ? most : 1;
+  auto cost = [&](long long n) { return (base_items * n + sms - 1) / sms * ((d.n_blocks + n - 1) / n + 5); };
+  for (long long n = 2; d.TY == 1 && n <= most; ++n)
+    if (cost(n) < cost(split)) split = n;
   if (split > d.n_blocks) split = d.n_blocks;
   if (split < 1) split = 1;
   const int per = (int)((d.n_blocks + split - 1) / split);

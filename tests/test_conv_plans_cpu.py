@@ -122,3 +122,24 @@ def test_column_pair_data_gradient_plans_respect_the_hardware_limits():
         assert info.stages_x * info.x_stage_bytes + info.stages_w * 8192 + 2 * slab < info.smem_bytes <= SMEM_LIMIT
         assert 0.0 < info.util <= 1.0
     assert seen > 100 and routed > 0
+
+
+def test_weight_gradient_slices_do_not_leave_the_busiest_sm_longer_than_two_slices_per_sm():
+    """Position blocks on the busiest of 148 SMs, for layers of 5 to 150 (output block, channel chunk, filter row) items."""
+    lib, sms = L.lib(), 148
+    seen = set()
+    for B, H, cg, og, k in itertools.product((100, 200, 256), (14, 20, 28), range(64, 449, 64), range(128, 641, 128), (5, 7)):
+        p, OH, OW = _params(2, B, H, H, cg, og, k, k // 2)
+        info = L.HaloPlanInfo()
+        if not lib.geeps_conv_wgrad_halo_plan(C.byref(p), C.byref(info)):
+            continue
+        base = info.m_tiles * (-(-cg // 64)) * info.passes
+        assert info.TY == 1 and base == -(-og // 128) * -(-cg // 64) * k
+
+        def path(n):      # blocks walked, and five more for every item that is drained
+            waves, per = -(-base * n // sms), -(-info.n_blocks // n)
+            return waves * (per + 5)
+        # (a slice count that leaves the last slice empty is lowered until none is)
+        assert path(info.split) <= min(path(1), path(max(1, sms // base)), path(max(1, 2 * sms // base))), (B, H, cg, og, k)
+        seen.add(base)
+    assert min(seen) == 5 and len([b for b in seen if 50 <= b <= 148]) > 10
