@@ -362,7 +362,10 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
 // would fetch the constants and meet in atomics once more.  32 x 56 x 56 x 192, forward and backward: 69.3 us with grids of
 // 4 (sums) and 8 (normalisation) blocks per SM, 63.7 with these; the backward sums spill at three blocks or four.
 constexpr int reduce_blocks(int mode) { return mode == 1 || mode == 3 ? 2 : 4; }
-constexpr int kApplyBlocks = 4, kBackwardBlocks = 3;
+constexpr int kApplyBlocks = 4;
+enum { MASK_NONE = 0, MASK_Y = 1, MASK_BITS = 2 };      // what the backward pass reads a ReLU mask from
+// A third tensor's loads in flight spill at three blocks: backward of 100352 x 192 by the output 68.3 us at three, 56.0 at two.
+constexpr int backward_blocks(int mask) { return mask == MASK_Y ? 2 : 3; }
 template <int MODE>
 __global__ void __launch_bounds__(256, reduce_blocks(MODE))
 channel_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
@@ -498,7 +501,7 @@ bn_apply_fused_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const fl
 }
 
 // dx = gamma * rstd * (dy' - sum_dy/P - xhat * sum_dy_xhat/P); also emits dgamma, dbeta (scaled).
-template <bool BITS>
+template <int MASK>
 __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, const bf16* __restrict__ dy,
                                                  const bf16* __restrict__ y, bf16* __restrict__ dx,
                                                  const float* mean_rstd, const float* __restrict__ gamma,
@@ -527,7 +530,7 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       float d = bf(dv.v[e]);
-      if (BITS ? !(on >> e & 1u) : relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
+      if (MASK == MASK_BITS ? !(on >> e & 1u) : MASK == MASK_Y && relu && !(bf(yv.v[e]) > 0.f)) d = 0.f;
       o.v[e] = __float2bfloat16(q[1][e] * (d - q[2][e] - (bf(xv.v[e]) - q[0][e]) * q[3][e]));
     }
     return o;
@@ -541,27 +544,27 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
     for (int u = 0; u < U; ++u) {
       xv[u] = ld8(x + (p + u * s.step) * ldx + s.c);
       dv[u] = ld8(dy + (p + u * s.step) * lddy + s.c);
-      on[u] = BITS ? bits[(p + u * s.step) * cv + (s.c >> 3)] : 0u;
-      if (!BITS && relu) yv[u] = ld8(y + (p + u * s.step) * lddy + s.c);
+      on[u] = MASK == MASK_BITS ? bits[(p + u * s.step) * cv + (s.c >> 3)] : 0u;
+      if (MASK == MASK_Y && relu) yv[u] = ld8(y + (p + u * s.step) * lddy + s.c);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) st8(dx + (p + u * s.step) * lddx + s.c, one(xv[u], dv[u], yv[u], on[u]));
   }
   for (; p < P; p += s.step) {
     Bf8 xv = ld8(x + p * ldx + s.c), dv = ld8(dy + p * lddy + s.c), yv;
-    if (!BITS && relu) yv = ld8(y + p * lddy + s.c);
-    st8(dx + p * lddx + s.c, one(xv, dv, yv, BITS ? bits[p * cv + (s.c >> 3)] : 0u));
+    if (MASK == MASK_Y && relu) yv = ld8(y + p * lddy + s.c);
+    st8(dx + p * lddx + s.c, one(xv, dv, yv, MASK == MASK_BITS ? bits[p * cv + (s.c >> 3)] : 0u));
   }
 }
-template <bool BITS>
-__global__ void __launch_bounds__(256, kBackwardBlocks)
+template <int MASK>
+__global__ void __launch_bounds__(256, backward_blocks(MASK))
 bn_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                    bf16* __restrict__ dx, const float* __restrict__ mean_rstd, const float* __restrict__ gamma,
                    const float* __restrict__ sums, float* dgamma, float* dbeta, long long P, int C,
                    long long ldx, long long lddy, long long lddx, int relu, float grad_scale, float* zero_after) {
   geeps_pdl_enter();
-  bn_backward_body<BITS>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
-                   zero_after);
+  bn_backward_body<MASK>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
+                         zero_after);
 }
 
 // ---- one launch per direction: reduction, grid barrier, normalisation (cooperative launch: all blocks resident) ----
@@ -609,8 +612,8 @@ bn_backward_coop_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy,
   geeps_pdl_enter();
   channel_reduce_body<BITS ? 3 : 1>(x, dy, y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
   if (bn_grid_barrier(bar, (int)(gridDim.x * gridDim.y)))
-    bn_backward_body<BITS>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
-                           zero_after);
+    bn_backward_body<BITS ? MASK_BITS : MASK_Y>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx,
+                                                relu, grad_scale, zero_after);
   else if (threadIdx.x == 0) { bar[2] = 1; mean_rstd[0] = __int_as_float(0x7fc00000); }
   bn_grid_done(bar, (int)(gridDim.x * gridDim.y));
 }
@@ -1827,19 +1830,27 @@ int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* be
   return CK();
 }
 
+// the ReLU mask, where there is one, read from the output
+static int bn_backward_by_output(const void* x, const void* dy, const void* y, void* dx, const float* mean_rstd,
+                                 const float* gamma, float* sums, float* dgamma, float* dbeta, float* zero_after, long long P,
+                                 int C, long long ldx, long long lddy, long long lddx, int relu, float grad_scale,
+                                 cudaStream_t st) {
+  const SlotGrid rg = reduce_grid(1, P, C), ag = apply_grid(P, C, backward_blocks(relu ? MASK_Y : MASK_NONE));
+  geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
+      (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
+  geeps_launch(relu ? bn_backward_kernel<MASK_Y> : bn_backward_kernel<MASK_NONE>, ag.grid, ag.threads, ag.smem, st,
+               (const bf16*)x, (const bf16*)dy, (const bf16*)y, (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx,
+               lddy, lddx, relu, grad_scale, zero_after);
+  return CK();
+}
 int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, const float* mean_rstd,
                       const float* gamma, float* sums, float* dgamma, float* dbeta, long long P, int C,
                       long long ldx, long long lddy, long long lddx, int relu, float grad_scale, void* stream) {
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
-  const SlotGrid rg = reduce_grid(1, P, C), ag = apply_grid(P, C, kBackwardBlocks);
-  geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
-      (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  geeps_launch(bn_backward_kernel<false>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)y,
-                                                           (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
-                                                           ldx, lddy, lddx, relu, grad_scale, nullptr);
-  return CK();
+  return bn_backward_by_output(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, nullptr, P, C, ldx, lddy, lddx, relu,
+                               grad_scale, st);
 }
 
 // The training-loop forms: `sums` must be zero on entry (2 C floats) and `zero_after` (or NULL) is zeroed for the
@@ -1901,21 +1912,17 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
     cudaError_t e = cudaLaunchCooperativeKernel(kernel, cg.grid, dim3(cg.threads), args, cg.smem, st);
     return e == cudaSuccess ? CK() : (int)e;
   }
-  const SlotGrid rg = reduce_grid(3, P, C), ag = apply_grid(P, C, kBackwardBlocks);
   if (bits != nullptr && relu) {
+    const SlotGrid rg = reduce_grid(3, P, C), ag = apply_grid(P, C, backward_blocks(MASK_BITS));
     geeps_launch(channel_reduce_kernel<3>, rg.grid, rg.threads, rg.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits,
                                                                    mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-    geeps_launch(bn_backward_kernel<true>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
+    geeps_launch(bn_backward_kernel<MASK_BITS>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
                                                              mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx,
                                                              relu, grad_scale, zero_after);
     return CK();
   }
-  geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
-      (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  geeps_launch(bn_backward_kernel<false>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)y,
-                                                           (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C,
-                                                           ldx, lddy, lddx, relu, grad_scale, zero_after);
-  return CK();
+  return bn_backward_by_output(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, zero_after, P, C, ldx, lddy, lddx, relu,
+                               grad_scale, st);
 }
 
 int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, float scale, int zero_first,

@@ -1,7 +1,11 @@
 """Launch shapes of the element-wise and pooling kernels (host arithmetic only, no GPU)."""
 import ctypes as C
 import itertools
+import re
 
+import pytest
+
+from geeps_b200 import _native
 from geeps_b200.ops import _lib as L
 
 
@@ -55,3 +59,13 @@ def test_lrn_backward_lanes_fit_the_channels():
         assert (lp, nv) in ((1, 1), (2, 1), (2, 3), (4, 1), (4, 2), (4, 3), (8, 2), (8, 3), (16, 2), (16, 3), (32, 2))
         assert lp * nv >= cv
         assert pixels < 40000 or 3 * cv >= 2 * lp * nv, (cv, lp, nv)
+
+
+def test_channel_kernels_keep_to_registers_at_their_launch_bounds():
+    """What the compiler printed for the kernels whose blocks per SM are set by launch bounds: no spills."""
+    found = re.findall(r"entry function '\w*?(channel_reduce_kernel|bn_backward_kernel|bn_apply_fused_kernel)(\w*)'.*?(\d+) bytes spill stores",
+                       _native.ptxas_report(), re.S)
+    if not found:
+        pytest.skip("no compiler output here: the library was built elsewhere")
+    assert len(found) >= 6
+    assert [f for f in found if f[2] != "0"] == []
