@@ -30,9 +30,10 @@
 // rows past the image and the channels past the layer's extent.  A tile is two store blocks of Rb image rows; the
 // pitch PW is padded until a block has a multiple of 8 positions, which makes the swizzled chunk offsets of a
 // thread's channel constants; eight epilogue warps (two per TMEM lane quarter, alternate column groups) share the
-// conversion.  Both blocks leave through one pair of slabs, one after the other: the epilogue has time to wait for a slab
-// to be read, the main loop none to wait for its weights (16 KB per tap and chunk out of L2), and the 32 KB of a second
-// pair are two more weight stages: conv2 forward per group with 3 stages 66.6 us, with 5 60.4; conv1 with 4 99, with 6 96.
+// conversion.  Blocks leave through one pair of slabs, one after the other, where the main loop is long: the epilogue has
+// the time to wait for a slab to be read, the main loop none to wait for its weights (16 KB per tap and chunk out of L2), and
+// the 32 KB of a second pair are two more weight stages: conv2 forward per group with 3 stages 66.6 us, with 5 60.4; conv1
+// with 4 99, with 6 96.  Two pairs in turn where it is short (two_slab_pairs).
 //
 // conv_tc() routes a forward / data-gradient call here when the geometry wastes little (see
 // geeps_conv_halo_applicable); GEEPS_HALO_CONV=0 keeps every call on the box kernel.  Bounded waits and TMEM
@@ -80,7 +81,7 @@ struct HaloDev {
   int KH, KW, taps, cchunks, k_last;   // k_last: MMA k-substeps (of 16) in the last chunk (zero channels are skipped)
   int PW, Rb, px, py;                  // padded pitch, image rows per store block (two blocks per tile), halo left / top
   int KWs;                             // steps per filter row: KW, or KW + 1 (MODE_DGRAD2)
-  int w_bytes, slab_bytes;             // all weight stages; one store slab
+  int w_bytes, slab_bytes, slab_pairs; // all weight stages; one store slab; slabs per 64 channels
   int x0, x1, x_tile_bytes;            // MODE_DGRAD2: first column of the two parity maps; bytes of a parity's halo tile
   int split, ncols2, ncols1;           // positions per block (Rb * PW); MMA N for a tile of two blocks / one block
   int GH;                              // output rows of the image
@@ -125,7 +126,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   uint8_t* tiles_x = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles_w = tiles_x + (size_t)d.stages_x * d.x_stage_bytes;
   uint8_t* cslab = tiles_w + d.w_bytes;
-  SmemCtl* ctl = (SmemCtl*)(cslab + 2 * d.slab_bytes);          // one slab per 64 channels
+  SmemCtl* ctl = (SmemCtl*)(cslab + 2 * d.slab_pairs * d.slab_bytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_tiles = d.m_tiles * d.n_images * d.row_tiles;
 
@@ -297,6 +298,8 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 #pragma unroll
     for (int jj = 0; jj < 8; ++jj) cb[jj] = ((chunk ^ (uint32_t)jj) << 4) + within;
     const uint32_t slab_base = tc05::smem_u32(cslab) + (uint32_t)(half * d.slab_bytes);
+    const uint32_t next_pair = d.slab_pairs == 2 ? (uint32_t)(2 * d.slab_bytes) : 0u;
+    uint32_t slab_off = 0;                         // 0 and next_pair in turn: the slab of the next block stored
     const bool storer = lane == 0 && (q4 & 1) == 0 && sub == 0;          // one thread per slab issues its stores
     const float floor_v = d.relu ? 0.f : -INFINITY;
     uint32_t tile_i = 0;
@@ -315,8 +318,8 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       tc05::fence_after_sync();
       const uint32_t tacc = tmem + acc * (uint32_t)ACC_COLS + ((uint32_t)(q4 * 32) << 16);
       for (int p = 0; p < q.nb; ++p) {
-        // the previous block was stored out of this slab: that store must have read it
-        if (storer) tc05::bulk_wait_read<0>();
+        // the store out of this slab, the latest or (two pairs) the one before it, must have read it
+        if (storer) { if (next_pair) tc05::bulk_wait_read<1>(); else tc05::bulk_wait_read<0>(); }
         tc05::named_bar_sync(1, 32 * kEpilogueWarps);
         if (slab_valid) {
           const int c_begin = p * d.split, c_end = c_begin + d.split;
@@ -326,7 +329,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             tc05::tmem_ld_32x32(tacc + (uint32_t)g, r);
             tc05::tmem_ld_wait();
             const int row0 = g - c_begin;              // slab row of element 0: a multiple of 8, negative for a first
-            const uint32_t rbase = slab_base + (uint32_t)(row0 * 128);     // group that starts in the previous block
+            const uint32_t rbase = slab_base + slab_off + (uint32_t)(row0 * 128);     // group that starts in the previous block
             if (row0 >= 0 && row0 + 32 <= d.split) {
 #pragma unroll
               for (int e = 0; e < 32; ++e) {
@@ -350,10 +353,11 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (storer && slab_valid) {
           // box (64 channels, PW, Rb, 1): columns past the image width, rows past its height and channels past
           // the extent are clipped by TMA
-          tc05::tma_store_4d_addr(PAIR && half ? &tmC1 : &tmC, slab_base, PAIR ? q.mi * CH : q.mi * BM + half * 64, 0,
+          tc05::tma_store_4d_addr(PAIR && half ? &tmC1 : &tmC, slab_base + slab_off, PAIR ? q.mi * CH : q.mi * BM + half * 64, 0,
                                   q.y0 + p * d.Rb, q.b);
           tc05::bulk_commit();
         }
+        if (slab_valid) slab_off ^= next_pair;
       }
       tc05::fence_before_sync();
       __syncwarp();
@@ -440,6 +444,15 @@ int pair_slab(int positions) { return round_up(positions > 64 ? positions * 128L
 // a step of four 128 x n x 16 products takes 2 n clocks, but the tap's rows out of L2 and its issue some 520
 int step_clocks(int n) { return 2 * n > 520 ? 2 * n : 520; }
 
+// A second pair of store slabs instead of two weight stages: where a tile has few products its epilogue is the bound.  3 x 3
+// forward, us with one pair and with two: 256 x 28 x 28, 8 -> 96 77.3, 74.9; 32 -> 128 29.2, 27.5; 256 x 27 x 27, 48 -> 128
+// 41.8, 39.8.  One pair from a whole chunk or 5 x 5 taps on: 96 x 57 x 57, 64 -> 96 39.6, 41.3; 96 x 56 x 56, 96 -> 128 66.6,
+// 69.3; 256 x 27 x 27, 48 -> 128, 5 x 5 59.2, 65.7; and in the data gradient, whose taps are loaded in two panels: 96 x 56 x
+// 56, 16 channels of dY 62.6, 70.1.
+bool two_slab_pairs(const GeepsConvTcParams* p, const HaloDev& d) {
+  return p->mode == MODE_FWD && d.cchunks == 1 && d.k_last <= 3 && d.taps <= 9;
+}
+
 // pair: MODE_DGRAD2
 HaloPlan plan_halo(const GeepsConvTcParams* p, bool pair = false) {
   HaloPlan hp;
@@ -501,7 +514,8 @@ HaloPlan plan_halo(const GeepsConvTcParams* p, bool pair = false) {
   d.x_stage_bytes = (pair ? 2 : 1) * d.x_tile_bytes;
   d.stages_x = 2;
   d.slab_bytes = pair ? pair_slab(d.split) : C_SLAB_BYTES;
-  const long long budget = SMEM_BUDGET - 2 * d.slab_bytes - (long long)d.stages_x * d.x_stage_bytes;
+  d.slab_pairs = 1;
+  long long budget = SMEM_BUDGET - 2 * d.slab_bytes - (long long)d.stages_x * d.x_stage_bytes;
   if (pair) {
     int rows = pair_rows(p->KW);
     while ((rows + 1) * p->KW <= MAX_W_STAGES && (long long)(rows + 1) * p->KW * PANEL_BYTES <= budget) ++rows;
@@ -509,12 +523,16 @@ HaloPlan plan_halo(const GeepsConvTcParams* p, bool pair = false) {
     d.w_bytes = d.stages_w * PANEL_BYTES;
     if (d.stages_w > MAX_W_STAGES || d.w_bytes > budget) return hp;
   } else {
+    if (two_slab_pairs(p, d) && budget >= 2 * d.slab_bytes + 3LL * W_STAGE_BYTES) {
+      d.slab_pairs = 2;
+      budget -= 2 * d.slab_bytes;
+    }
     d.stages_w = (int)(budget / W_STAGE_BYTES);
     if (d.stages_w > MAX_W_STAGES / 2) d.stages_w = MAX_W_STAGES / 2;
     if (d.stages_w < 3) return hp;
     d.w_bytes = d.stages_w * W_STAGE_BYTES;
   }
-  hp.smem = (size_t)d.stages_x * d.x_stage_bytes + d.w_bytes + 2 * d.slab_bytes + sizeof(SmemCtl) + 1024;
+  hp.smem = (size_t)d.stages_x * d.x_stage_bytes + d.w_bytes + 2 * d.slab_pairs * d.slab_bytes + sizeof(SmemCtl) + 1024;
   hp.cost *= (double)d.m_tiles * d.taps * d.cchunks;
   // share of the issued MMA work that lands in real outputs: positions x channels
   const double pos = (double)GH * GW / ((double)d.row_tiles * d.ncols2);

@@ -143,3 +143,23 @@ def test_weight_gradient_slices_do_not_leave_the_busiest_sm_longer_than_two_slic
         assert path(info.split) <= min(path(1), path(max(1, sms // base)), path(max(1, 2 * sms // base))), (B, H, cg, og, k)
         seen.add(base)
     assert min(seen) == 5 and len([b for b in seen if 50 <= b <= 148]) > 10
+
+
+def test_short_forward_tiles_keep_two_pairs_of_store_slabs():
+    """3 x 3 layers of at most 48 input channels, wherever three weight stages remain; one pair and more stages elsewhere."""
+    lib = L.lib()
+    two = one = 0
+    for mode, (B, H, cg, og, k, pad) in itertools.product((0, 1), SHAPES):
+        p, OH, OW = _params(mode, B, H, H, cg, og, k, pad)
+        info = L.HaloPlanInfo()
+        if not lib.geeps_conv_halo_plan(C.byref(p), C.byref(info)):
+            continue
+        rest = info.smem_bytes - info.stages_x * info.x_stage_bytes - info.stages_w * 16384     # slabs and barriers
+        pairs = rest // 32768
+        assert pairs in (1, 2) and rest - pairs * 32768 < 2048 and info.smem_bytes <= SMEM_LIMIT
+        short = mode == 0 and k <= 3 and cg <= 48
+        room = 224 * 1024 - info.stages_x * info.x_stage_bytes >= 65536 + 3 * 16384
+        assert pairs == (2 if short and room else 1), (mode, B, H, cg, og, k)
+        two += pairs == 2
+        one += pairs == 1
+    assert two > 50 and one > 50

@@ -180,7 +180,15 @@ HALO_CASES = CASES + [
 ]
 
 
-@pytest.mark.parametrize("case", HALO_CASES)
+# several tiles per SM through two pairs of store slabs: a last tile of one block, a channel block with one slab to store
+SHORT_TILES = [
+    (60, 28, 28, 48, 0, 48, 160, 0, 160, 3, 1),
+    (160, 9, 27, 24, 8, 16, 104, 0, 104, 3, 1),
+    (90, 28, 28, 8, 0, 8, 96, 0, 96, 2, 0),
+]
+
+
+@pytest.mark.parametrize("case", HALO_CASES + SHORT_TILES)
 def test_conv_halo_forward_dgrad_match_torch(case):
     """The halo-tile kernel called directly on every shape it accepts (conv_tc() picks it only where it pays)."""
     from geeps_b200.ops import functional as F
