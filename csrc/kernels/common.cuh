@@ -52,14 +52,12 @@ __device__ __forceinline__ void geeps_pdl_wait() { asm volatile("griddepcontrol.
 // The blocks of the next kernel may start, as far as there is room for them, once every block has called this (or left).
 // Called before the wait of its own kernel has returned it would let a third kernel in; all kernels call it after.
 // Where it stands: in the tensor-core kernels behind the last load of a block, whose shared memory leaves no room for
-// another block before; in the others at the start.  us a pass, ordinary launches / dependent launches / with triggers:
-// an Inception module (some 50 kernels on four streams) 223 / 212 / 203; its 1024 x 21841 classifier 88 / 88 / 86;
-// AlexNet's training step 2275 / 2261 / 2218.
+// another block before (the pair GEMM has none: its successor comes up when it ends); in the others at the start.
 __device__ __forceinline__ void geeps_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void geeps_pdl_enter() { geeps_pdl_wait(); geeps_pdl_trigger(); }
 
 template <typename... P, typename... A>
-inline void geeps_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline void geeps_launch_as(int dependent, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -69,8 +67,29 @@ inline void geeps_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);      // an error is also what cudaGetLastError() returns
+}
+// Which launch a kernel gets (us in a captured chain of 16, ordinary / dependent, unless said otherwise).
+// geeps_launch, dependent: tensor-core kernels, channel sums, BatchNorm, softmax.  They have at most as many blocks as fit at
+// once (softmax: one a row), and in a network's chains the way from one kernel to the next is what is gained: 32 x 14 x 14, 128 ->
+// 160, 3 x 3 7.9 / 7.0; GEMM 6272 x 160, K = 576 5.6 / 4.8; BatchNorm of 100 x 16 x 16 x 144 forward and backward 22.6 / 21.2;
+// softmax of 256 x 1000 7.6 / 6.6; an Inception module with BatchNorm's launches ordinary 199, dependent 193, its classifier
+// 82.3, 80.9.  Forward and backward of 60 convolution layers take 4 % less.  Not every kernel gains: CTAs of a part of a wave
+// come up where the predecessor leaves room, and the other way round 35 x 8 x 8, 72 -> 312 takes 9.7 / 11.5 after itself.
+// geeps_launch_plain: kernels of many short blocks.  Early blocks wait on the SMs that have room first, as many as fit, and the
+// other SMs run dry: max pooling of 32 x 14 x 14 x 576 12.1 / 15.1, its backward at 608 channels 19.2 / 23.5; average pooling
+// of 8 x 14 x 14 x 576 4.1 / 4.4, backward 5.5 / 6.1; LRN + pooling backward of 2 x 43 x 43 x 88 8.8 / 10.2; layouts: fp32 to
+// space-to-depth at 16 x 227 x 227 3.9 / 4.2 (72 channels, 32 x 224 x 224 8.3 / 9.3), to NHWC at 100 x 32 x 32 2.3 / 2.5, from
+// 8 bits 9.1 / 9.6; the sum of three gradients of 16 Mi values 13.6 / 14.6, the ReLU mask 11.3 / 11.9.  Where a size does not
+// suffer it gains 0.1 to 0.3.  In a network: Inception module 192.0 / 192.8, AlexNet's training step 2212 / 2218.
+template <typename... P, typename... A>
+inline void geeps_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  geeps_launch_as(1, kernel, grid, block, smem, st, static_cast<A&&>(args)...);
+}
+template <typename... P, typename... A>
+inline void geeps_launch_plain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  geeps_launch_as(0, kernel, grid, block, smem, st, static_cast<A&&>(args)...);
 }
 
 __device__ __forceinline__ void geeps_report(int* status, int code, int kid, int detail, int seen) {

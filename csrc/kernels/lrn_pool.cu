@@ -677,7 +677,7 @@ int geeps_lrn_maxpool_forward(const void* x, void* p, void* argmax, const GeepsP
       if (e != cudaSuccess) return (int)e;                                                                         \
       attr_set = true;                                                                                             \
     }                                                                                                              \
-    geeps_launch(lrn_maxpool_forward_kernel<HALF, K3S2>, grid, block, smem, st, (const bf16*)x, (bf16*)p, (uint8_t*)argmax,   \
+    geeps_launch_plain(lrn_maxpool_forward_kernel<HALF, K3S2>, grid, block, smem, st, (const bf16*)x, (bf16*)p, (uint8_t*)argmax,   \
                                                                        *g, cf, RO);                                \
   } while (0)
   const bool k3s2 = g->K == 3 && g->stride == 2;
@@ -716,7 +716,7 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
     const long long cap = (long long)geeps_sm_count() * 2;
     if (blocks > cap) blocks = cap;
 #define LP_LANES(LP, NV)                                                                                           \
-  geeps_launch(lrn_maxpool_backward_lanes_kernel<LP, NV>, (int)blocks, 256, sizeof(float) * g->C, st,                          \
+  geeps_launch_plain(lrn_maxpool_backward_lanes_kernel<LP, NV>, (int)blocks, 256, sizeof(float) * g->C, st,                          \
       (const bf16*)x, (const bf16*)dp, (const uint8_t*)argmax, (bf16*)dx, *g, cf, coef, relu_mask, colsum)
     if (lp == 1) LP_LANES(1, 1);
     else if (lp == 2) { if (nv == 1) LP_LANES(2, 1); else LP_LANES(2, 3); }
@@ -736,7 +736,7 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
       if (e != cudaSuccess) return (int)e;                                                                         \
       attr_set = true;                                                                                             \
     }                                                                                                              \
-    geeps_launch(lrn_maxpool_backward_kernel<HALF, K3S2>, grid, block, smem, st, (const bf16*)x, (const bf16*)dp,             \
+    geeps_launch_plain(lrn_maxpool_backward_kernel<HALF, K3S2>, grid, block, smem, st, (const bf16*)x, (const bf16*)dp,             \
                                                                  (const uint8_t*)argmax, (bf16*)dx, *g, R, max_oh,  \
                                                                  cf, coef, relu_mask, colsum);                     \
   } while (0)

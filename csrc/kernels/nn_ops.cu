@@ -1697,13 +1697,23 @@ softmax_ce_kernel(const float* __restrict__ logits, const long long* __restrict_
 
 #define CK() ((int)cudaGetLastError())
 
+// A dependent launch, unless the blocks are more than one a SM and less than two: those that come up early pair up on the SMs
+// with room.  Forward and backward, us, ordinary / dependent: 8 x 56 x 56 x 64, 196 blocks 13.8 / 14.7; 64 x 14 x 14 x 160, 261
+// blocks 16.9 / 18.1; near one a SM either way (149 blocks 13.9 / 13.8, 171 13.4 / 14.0); beyond 100 x 14 x 14 x 128, 306
+// blocks 18.2 / 16.4.
+template <typename... P, typename... A>
+static void launch_channels(void (*kernel)(P...), const SlotGrid& g, cudaStream_t st, A&&... args) {
+  const long long blocks = (long long)g.grid.x * g.grid.y, sms = geeps_sm_count();
+  geeps_launch_as(blocks <= sms || blocks >= 2 * sms, kernel, g.grid, g.threads, g.smem, st, static_cast<A&&>(args)...);
+}
+
 template <typename T>
 static int nchw_to_nhwc_launch(const T* x, void* y, int B, int C, int H, int W, int Cpad, cudaStream_t st) {
   const long long n = (long long)B * H * W * Cpad;
   if (Cpad % 4 == 0)
-    geeps_launch(nchw_to_nhwc_pix_kernel<T>, grid_1d((long long)B * H * W), 256, 0, st, x, (bf16*)y, B, C, H * W, Cpad);
+    geeps_launch_plain(nchw_to_nhwc_pix_kernel<T>, grid_1d((long long)B * H * W), 256, 0, st, x, (bf16*)y, B, C, H * W, Cpad);
   else
-    geeps_launch(nchw_f32_to_nhwc_bf16_kernel<T>, grid_1d(n), 256, 0, st, x, (bf16*)y, B, C, H, W, Cpad);
+    geeps_launch_plain(nchw_f32_to_nhwc_bf16_kernel<T>, grid_1d(n), 256, 0, st, x, (bf16*)y, B, C, H, W, Cpad);
   return CK();
 }
 
@@ -1719,12 +1729,12 @@ static int nchw_to_s2d_launch(const T* x, void* y, int B, int C, int H, int W, i
   }
   if (S == 4 && C == 3 && Cpad % 8 == 0 && Cpad >= 48 && Cpad <= 64 && (((uintptr_t)y) & 15) == 0) {
     const int segs = (Ws + 31) / 32;
-    geeps_launch(nchw_to_s2d43_tile_kernel<T>, (unsigned)((long long)B * Hs * segs), 128, 0, st, x, (bf16*)y, B, H, W, Hs, Ws, Cpad,
+    geeps_launch_plain(nchw_to_s2d43_tile_kernel<T>, (unsigned)((long long)B * Hs * segs), 128, 0, st, x, (bf16*)y, B, H, W, Hs, Ws, Cpad,
                                                                                       segs);
   } else if (S == 4 && C == 3)
-    geeps_launch(nchw_to_s2d_kernel<4, 3, T>, grid_1d((long long)B * Hs * Ws), 256, 0, st, x, (bf16*)y, B, H, W, Hs, Ws, Cpad);
+    geeps_launch_plain(nchw_to_s2d_kernel<4, 3, T>, grid_1d((long long)B * Hs * Ws), 256, 0, st, x, (bf16*)y, B, H, W, Hs, Ws, Cpad);
   else
-    geeps_launch(nchw_to_s2d_generic_kernel<T>, grid_1d((long long)B * Hs * Ws * Cpad), 256, 0, st, x, (bf16*)y, B, C, H, W, S,
+    geeps_launch_plain(nchw_to_s2d_generic_kernel<T>, grid_1d((long long)B * Hs * Ws * Cpad), 256, 0, st, x, (bf16*)y, B, C, H, W, S,
                                                                                          Hs, Ws, Cpad);
   return CK();
 }
@@ -1770,14 +1780,14 @@ int geeps_u8_transform_bf16(const GeepsU8Transform* p, void* stream) {
     q.end = p->x + (long long)p->B * 3 * p->Hin * p->Win;
     launch_s2d43_quads(q, p->y, npix, p->Hs, p->Ws, p->Cpad, st);
   } else {
-    geeps_launch(u8_xform_generic_kernel, grid_1d((long long)p->B * p->Hs * p->Ws * p->Cpad), 256, 0, st, t, (bf16*)p->y, p->B, p->C,
+    geeps_launch_plain(u8_xform_generic_kernel, grid_1d((long long)p->B * p->Hs * p->Ws * p->Cpad), 256, 0, st, t, (bf16*)p->y, p->B, p->C,
                                                                                               S, p->Hs, p->Ws, p->Cpad);
   }
   return CK();
 }
 
 int geeps_col_mask_f32(float* g, const unsigned char* mask, long long rows, int cols, long long ld, void* stream) {
-  geeps_launch(col_mask_kernel, grid_1d(rows * cols), 256, 0, (cudaStream_t)stream, g, mask, rows, cols, ld);
+  geeps_launch_plain(col_mask_kernel, grid_1d(rows * cols), 256, 0, (cudaStream_t)stream, g, mask, rows, cols, ld);
   return CK();
 }
 
@@ -1786,13 +1796,13 @@ int geeps_im2col(const void* x, void* col, const GeepsConvGeom* g, void* stream)
   const long long rows = (long long)g->B * g->OH * g->OW;
   const int kd = g->KH * g->KW * g->Cg;
   if (g->ldcol > kd)
-    geeps_launch(zero_col_pad_kernel, grid_1d(rows * (g->ldcol - kd)), 256, 0, st, (bf16*)col, rows, kd, g->ldcol);
+    geeps_launch_plain(zero_col_pad_kernel, grid_1d(rows * (g->ldcol - kd)), 256, 0, st, (bf16*)col, rows, kd, g->ldcol);
   const bool a8 = (g->Cg % 8 == 0) && (g->C % 8 == 0) && (g->c0 % 8 == 0) && (g->ldcol % 8 == 0);
   const bool a4 = (g->Cg % 4 == 0) && (g->C % 4 == 0) && (g->c0 % 4 == 0) && (g->ldcol % 4 == 0);
   const int wgrid = grid_1d(rows * 32);   // one warp per patch-matrix row
-  if (a8) geeps_launch(im2col_kernel<8>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
-  else if (a4) geeps_launch(im2col_kernel<4>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
-  else geeps_launch(im2col_kernel<1>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
+  if (a8) geeps_launch_plain(im2col_kernel<8>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
+  else if (a4) geeps_launch_plain(im2col_kernel<4>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
+  else geeps_launch_plain(im2col_kernel<1>, wgrid, 256, 0, st, (const bf16*)x, (bf16*)col, *g);
   return CK();
 }
 
@@ -1800,8 +1810,8 @@ int geeps_col2im(const void* dcol, void* dx, const GeepsConvGeom* g, int accumul
   cudaStream_t st = (cudaStream_t)stream;
   const long long pix = (long long)g->B * g->H * g->W;
   const bool a8 = (g->Cg % 8 == 0) && (g->C % 8 == 0) && (g->c0 % 8 == 0) && (g->ldcol % 8 == 0);
-  if (a8) geeps_launch(col2im_kernel<8>, grid_1d(pix * (g->Cg / 8)), 256, 0, st, (const bf16*)dcol, (bf16*)dx, *g, accumulate);
-  else geeps_launch(col2im_kernel<1>, grid_1d(pix * g->Cg), 256, 0, st, (const bf16*)dcol, (bf16*)dx, *g, accumulate);
+  if (a8) geeps_launch_plain(col2im_kernel<8>, grid_1d(pix * (g->Cg / 8)), 256, 0, st, (const bf16*)dcol, (bf16*)dx, *g, accumulate);
+  else geeps_launch_plain(col2im_kernel<1>, grid_1d(pix * g->Cg), 256, 0, st, (const bf16*)dcol, (bf16*)dx, *g, accumulate);
   return CK();
 }
 
@@ -1821,11 +1831,11 @@ int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* be
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
   const SlotGrid rg = reduce_grid(0, P, C), ag = apply_grid(P, C);
-  geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
+  launch_channels(channel_reduce_kernel<0>, rg, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   geeps_launch(bn_finalize_kernel, (C + 127) / 128, 128, 0, st, sums, mean_rstd, running_mean, running_var, C,
                                                       1.f / (float)P, eps, momentum);
-  geeps_launch(bn_apply_kernel, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
+  launch_channels(bn_apply_kernel, ag, st, (const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
                                                         ldy, relu);
   return CK();
 }
@@ -1836,9 +1846,9 @@ static int bn_backward_by_output(const void* x, const void* dy, const void* y, v
                                  int C, long long ldx, long long lddy, long long lddx, int relu, float grad_scale,
                                  cudaStream_t st) {
   const SlotGrid rg = reduce_grid(1, P, C), ag = apply_grid(P, C, backward_blocks(relu ? MASK_Y : MASK_NONE));
-  geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
+  launch_channels(channel_reduce_kernel<1>, rg, st,
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  geeps_launch(relu ? bn_backward_kernel<MASK_Y> : bn_backward_kernel<MASK_NONE>, ag.grid, ag.threads, ag.smem, st,
+  launch_channels(relu ? bn_backward_kernel<MASK_Y> : bn_backward_kernel<MASK_NONE>, ag, st,
                (const bf16*)x, (const bf16*)dy, (const bf16*)y, (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx,
                lddy, lddx, relu, grad_scale, zero_after);
   return CK();
@@ -1888,9 +1898,9 @@ int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, cons
     return e == cudaSuccess ? CK() : (int)e;
   }
   const SlotGrid rg = reduce_grid(0, P, C), ag = apply_grid(P, C);
-  geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
+  launch_channels(channel_reduce_kernel<0>, rg, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
-  geeps_launch(bn_apply_fused_kernel, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
+  launch_channels(bn_apply_fused_kernel, ag, st, (const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
                                                               running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                                                               1.f / (float)P, eps, momentum, bits);
   return CK();
@@ -1914,9 +1924,9 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
   }
   if (bits != nullptr && relu) {
     const SlotGrid rg = reduce_grid(3, P, C), ag = apply_grid(P, C, backward_blocks(MASK_BITS));
-    geeps_launch(channel_reduce_kernel<3>, rg.grid, rg.threads, rg.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits,
+    launch_channels(channel_reduce_kernel<3>, rg, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits,
                                                                    mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-    geeps_launch(bn_backward_kernel<MASK_BITS>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
+    launch_channels(bn_backward_kernel<MASK_BITS>, ag, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
                                                              mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx,
                                                              relu, grad_scale, zero_after);
     return CK();
@@ -1934,7 +1944,7 @@ int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, f
   }
   if (zero_first) cudaMemsetAsync(out, 0, sizeof(float) * C, st);
   const SlotGrid rg = reduce_grid(2, P, C);
-  geeps_launch(channel_reduce_kernel<2>, rg.grid, rg.threads, rg.smem, st,
+  launch_channels(channel_reduce_kernel<2>, rg, st,
       (const bf16*)x, nullptr, nullptr, nullptr, out, P, C, ldx, 0, 0, scale);
   return CK();
 }
@@ -1945,14 +1955,14 @@ int geeps_copy_f32(float* dst, const float* src, long long n, void* stream) {
 
 int geeps_relu_backward(const void* dy, const void* y, void* dx, long long n, void* stream) {
   if (n % 8) return (int)cudaErrorInvalidValue;
-  geeps_launch(relu_backward_kernel, grid_1d(n / 8), 256, 0, (cudaStream_t)stream, (const bf16*)dy, (const bf16*)y, (bf16*)dx, n / 8);
+  geeps_launch_plain(relu_backward_kernel, grid_1d(n / 8), 256, 0, (cudaStream_t)stream, (const bf16*)dy, (const bf16*)y, (bf16*)dx, n / 8);
   return CK();
 }
 
 int geeps_relu_backward_2d(const void* dy, const void* y, void* dx, long long P, int C, long long lddy, long long ldy,
                            long long lddx, void* stream) {
   if (C % 8 || lddy % 8 || ldy % 8 || lddx % 8) return (int)cudaErrorInvalidValue;
-  geeps_launch(relu_backward_2d_kernel, grid_1d(P * (C / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)dy, (const bf16*)y,
+  geeps_launch_plain(relu_backward_2d_kernel, grid_1d(P * (C / 8)), 256, 0, (cudaStream_t)stream, (const bf16*)dy, (const bf16*)y,
                                                                                  (bf16*)dx, P, C, lddy, ldy, lddx);
   return CK();
 }
@@ -1962,14 +1972,14 @@ int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* c
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(colsum, 0, sizeof(float) * C, st);
   const SlotGrid rg = slot_grid(P, C, 4, 8, 1);
-  geeps_launch(relu_backward_colsum_kernel, rg.grid, rg.threads, rg.smem, st,
+  geeps_launch_plain(relu_backward_colsum_kernel, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)dy, (const bf16*)y, (bf16*)dx, colsum, P, C, lddy, ldy, lddx);
   return CK();
 }
 int geeps_f32_to_bf16_2d(const float* src, void* dst, long long P, int C, long long lds, long long ldd, int relu,
                          void* stream) {
   if (C % 8 || lds % 4 || ldd % 8 || ((uintptr_t)src & 15) || ((uintptr_t)dst & 15)) return (int)cudaErrorInvalidValue;
-  geeps_launch(f32_to_bf16_2d_kernel, grid_1d(P * (C / 8)), 256, 0, (cudaStream_t)stream, src, (bf16*)dst, P, C, lds, ldd, relu);
+  geeps_launch_plain(f32_to_bf16_2d_kernel, grid_1d(P * (C / 8)), 256, 0, (cudaStream_t)stream, src, (bf16*)dst, P, C, lds, ldd, relu);
   return CK();
 }
 int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s2, long long P, int C, long long ldd,
@@ -1982,7 +1992,7 @@ int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s
   const bool dense = ldd == C && ld0 == C && (n < 2 || ld1 == C) && (n < 3 || ld2 == C);
   const int grid = grid_1d(total);
   cudaStream_t st = (cudaStream_t)stream;
-#define ADD_2D(N, DENSE) geeps_launch(add_2d_kernel<N, DENSE>, grid, 256, 0, st, (bf16*)dst, src, total, C / 8, ldd)
+#define ADD_2D(N, DENSE) geeps_launch_plain(add_2d_kernel<N, DENSE>, grid, 256, 0, st, (bf16*)dst, src, total, C / 8, ldd)
   if (dense) { if (n == 3) ADD_2D(3, true); else if (n == 2) ADD_2D(2, true); else ADD_2D(1, true); }
   else { if (n == 3) ADD_2D(3, false); else if (n == 2) ADD_2D(2, false); else ADD_2D(1, false); }
 #undef ADD_2D
@@ -1990,12 +2000,12 @@ int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s
 }
 
 int geeps_dropout(const void* x, void* y, long long n, float p, unsigned long long seed, void* stream) {
-  geeps_launch(dropout_kernel, grid_1d(n), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, n, p, seed, nullptr);
+  geeps_launch_plain(dropout_kernel, grid_1d(n), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, n, p, seed, nullptr);
   return CK();
 }
 int geeps_dropout_ref(const void* x, void* y, long long n, float p, unsigned long long seed, const int* step_ref,
                       void* stream) {
-  geeps_launch(dropout_kernel, grid_1d(n), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, n, p, seed, step_ref);
+  geeps_launch_plain(dropout_kernel, grid_1d(n), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, n, p, seed, step_ref);
   return CK();
 }
 
@@ -2004,13 +2014,13 @@ int geeps_lrn_forward(const void* x, void* y, void* rscale, long long P, int C, 
   const int g8 = grid_1d(P * (C / 8));
   cudaStream_t st8 = (cudaStream_t)stream;
   if (C % 8 == 0 && size == 5)
-    geeps_launch(lrn_forward_v8_kernel<2>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
+    geeps_launch_plain(lrn_forward_v8_kernel<2>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
   else if (C % 8 == 0 && size == 3)
-    geeps_launch(lrn_forward_v8_kernel<1>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
+    geeps_launch_plain(lrn_forward_v8_kernel<1>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
   else if (C % 8 == 0 && size == 7)
-    geeps_launch(lrn_forward_v8_kernel<3>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
+    geeps_launch_plain(lrn_forward_v8_kernel<3>, g8, 256, 0, st8, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size, alpha, beta, k);
   else
-    geeps_launch(lrn_forward_kernel, grid_1d(P * C), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size,
+    geeps_launch_plain(lrn_forward_kernel, grid_1d(P * C), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, (bf16*)rscale, P, C, size,
                                                                         alpha, beta, k);
   return CK();
 }
@@ -2030,13 +2040,13 @@ int geeps_lrn_backward(const void* x, const void* y, const void* rscale, const v
     cudaMemsetAsync(colsum, 0, sizeof(float) * C, st8);
   }
   if (C % 8 == 0 && size == 5)
-    geeps_launch(lrn_backward_v8_kernel<2>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
+    geeps_launch_plain(lrn_backward_v8_kernel<2>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
   else if (C % 8 == 0 && size == 3)
-    geeps_launch(lrn_backward_v8_kernel<1>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
+    geeps_launch_plain(lrn_backward_v8_kernel<1>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
   else if (C % 8 == 0 && size == 7)
-    geeps_launch(lrn_backward_v8_kernel<3>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
+    geeps_launch_plain(lrn_backward_v8_kernel<3>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
   else
-    geeps_launch(lrn_backward_kernel, grid_1d(P * C), 256, 0, (cudaStream_t)stream, (const bf16*)x, (const bf16*)y, (const bf16*)rscale,
+    geeps_launch_plain(lrn_backward_kernel, grid_1d(P * C), 256, 0, (cudaStream_t)stream, (const bf16*)x, (const bf16*)y, (const bf16*)rscale,
                                                                          (const bf16*)dy, (bf16*)dx, P, C, size, alpha,
                                                                          beta, relu_mask);
   return CK();
@@ -2044,7 +2054,7 @@ int geeps_lrn_backward(const void* x, const void* y, const void* rscale, const v
 
 int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream) {
   if (g->C % 8 || g->ldx % 8 || g->ldy % 8 || g->K * g->K > 255) return (int)cudaErrorInvalidValue;
-  geeps_launch(maxpool_forward_kernel, g->B * g->OH, pool_block(g->C / 8), 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y,
+  geeps_launch_plain(maxpool_forward_kernel, g->B * g->OH, pool_block(g->C / 8), 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y,
                                                                                         (uint8_t*)argmax, *g);
   return CK();
 }
@@ -2062,11 +2072,11 @@ int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const G
       attr_set = true;
     }
     const int row_blocks = (g->H + rows_per_block - 1) / rows_per_block;
-    geeps_launch(maxpool_backward_smem_kernel, g->B * row_blocks, pool_block(g->C / 8), smem, (cudaStream_t)stream,
+    geeps_launch_plain(maxpool_backward_smem_kernel, g->B * row_blocks, pool_block(g->C / 8), smem, (cudaStream_t)stream,
         (const bf16*)dy, (const uint8_t*)argmax, (bf16*)dx, *g, accumulate, rows_per_block, max_oh);
     return CK();
   }
-  geeps_launch(maxpool_backward_kernel, g->B * g->H, pool_block(g->C / 8), 0, (cudaStream_t)stream,
+  geeps_launch_plain(maxpool_backward_kernel, g->B * g->H, pool_block(g->C / 8), 0, (cudaStream_t)stream,
       (const bf16*)dy, (const uint8_t*)argmax, (bf16*)dx, *g, accumulate);
   return CK();
 }
@@ -2086,8 +2096,8 @@ int geeps_avgpool_forward(const void* x, void* y, const GeepsPoolGeom* g, void* 
   const PoolGrid pg = avgpool_grid(g->C / 8, g->OW, (long long)g->B * g->OH, g->K <= 3);
   cudaStream_t st = (cudaStream_t)stream;
   if (pg.grid.x == 0) return 0;
-  if (pg.block.z == 1) geeps_launch(avgpool_forward_kernel<false>, pg.grid, pg.block, 0, st, (const bf16*)x, (bf16*)y, *g);
-  else geeps_launch(avgpool_forward_kernel<true>, pg.grid, pg.block, 0, st, (const bf16*)x, (bf16*)y, *g);
+  if (pg.block.z == 1) geeps_launch_plain(avgpool_forward_kernel<false>, pg.grid, pg.block, 0, st, (const bf16*)x, (bf16*)y, *g);
+  else geeps_launch_plain(avgpool_forward_kernel<true>, pg.grid, pg.block, 0, st, (const bf16*)x, (bf16*)y, *g);
   return CK();
 }
 int geeps_avgpool_backward(const void* dy, void* dx, const GeepsPoolGeom* g, int accumulate, void* stream) {
@@ -2096,9 +2106,9 @@ int geeps_avgpool_backward(const void* dy, void* dx, const GeepsPoolGeom* g, int
   cudaStream_t st = (cudaStream_t)stream;
   if (pg.grid.x == 0) return 0;
   if (pg.block.z == 1)
-    geeps_launch(avgpool_backward_kernel<false>, pg.grid, pg.block, 0, st, (const bf16*)dy, (bf16*)dx, *g, accumulate);
+    geeps_launch_plain(avgpool_backward_kernel<false>, pg.grid, pg.block, 0, st, (const bf16*)dy, (bf16*)dx, *g, accumulate);
   else
-    geeps_launch(avgpool_backward_kernel<true>, pg.grid, pg.block, 0, st, (const bf16*)dy, (bf16*)dx, *g, accumulate);
+    geeps_launch_plain(avgpool_backward_kernel<true>, pg.grid, pg.block, 0, st, (const bf16*)dy, (bf16*)dx, *g, accumulate);
   return CK();
 }
 

@@ -160,3 +160,59 @@ def test_gemm_cluster_split_k(M, N, K, b_mn, fp32, cluster):
     again = torch.empty_like(wide)[:, 8:8 + N]
     F.gemm(a, b, again, b_mn=b_mn, bias=bias, relu=True, alpha=0.5, impl="tc")
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_dependent_launches_keep_reads_and_writes_in_order(captured):
+    """A product may come up while its predecessor runs.  Each here overwrites what the one before reads, or reads what it
+    writes, in one stream, across an event and around a copy; results are those of one call at a time, bitwise."""
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(5)
+    n, deep = 256, 4096
+    rnd = lambda *s: (torch.randn(*s, device=dev, generator=gen) * 0.05).to(torch.bfloat16)      # noqa: E731
+    first, w, u, v, other = rnd(n, deep), rnd(n, deep), rnd(n, n), rnd(deep, n), rnd(n, deep)
+    main, side = torch.cuda.Stream(device=dev), torch.cuda.Stream(device=dev)
+    torch.cuda.synchronize()
+
+    def run(a, outs, pause):
+        event = iter(events)
+        with torch.cuda.stream(main):
+            a.copy_(first); pause()
+            F.gemm(a, w, outs[0]); pause()             # long K: the successor's blocks are there before it ends
+            F.gemm(u, v, a); pause()                   # overwrites the operand of the one before
+            F.gemm(a, w, outs[1]); pause()             # reads what was just written
+            a.copy_(other); pause()                    # a copy behind a product and in front of one
+            F.gemm(a, w, outs[2]); pause()
+            F.stream_order(main, side, next(event))
+        with torch.cuda.stream(side):
+            F.gemm(a, w, outs[3]); pause()             # beside the main stream
+            F.colsum(a, outs[5]); pause()
+        F.stream_order(side, main, next(event))
+        with torch.cuda.stream(main):
+            F.gemm(u, v, a); pause()                   # overwrites what the other stream reads
+            F.gemm(a, w, outs[4]); pause()
+
+    def buffers():
+        return rnd(n, deep), [torch.zeros(n, n, device=dev, dtype=torch.bfloat16) for _ in range(5)] + [torch.zeros(deep, device=dev)]
+
+    events = [F.new_event() for _ in range(2)]
+    a, ref = buffers()
+    run(a, ref, torch.cuda.synchronize)
+    a, got = buffers()
+    torch.cuda.synchronize()
+    if captured:
+        graph, nodes = ctypes.c_void_p(), ctypes.c_longlong(0)
+        assert L.lib().geeps_graph_begin(ctypes.c_void_p(main.cuda_stream)) == 0
+        run(a, got, lambda: None)
+        assert L.lib().geeps_graph_end(ctypes.c_void_p(main.cuda_stream), ctypes.byref(graph), ctypes.byref(nodes)) == 0
+        for _ in range(20):
+            assert L.lib().geeps_graph_launch(graph, ctypes.c_void_p(main.cuda_stream)) == 0
+        torch.cuda.synchronize()
+        L.lib().geeps_graph_destroy(graph)
+    else:
+        for _ in range(20):
+            run(a, got, lambda: None)
+        torch.cuda.synchronize()
+    for r, g in zip(ref[:5], got[:5]):
+        assert torch.equal(r, g)
+    assert torch.allclose(ref[5], got[5], atol=1e-4)   # block sums meet in atomics
