@@ -35,8 +35,7 @@ class Concat(Layer):
         self.branches = branches       # list of lists of layers
         import os
         self.concurrent = (os.environ.get("GEEPS_CONCAT_STREAMS", "1") != "0") if concurrent is None else concurrent
-        self._events = None
-        self._wgrad_events = None
+        self._event = None             # one serves all forks and joins: a wait is for the record before it
 
     def sublayers(self):
         for br in self.branches:
@@ -89,6 +88,11 @@ class Concat(Layer):
         for br in self.branches:
             br[0].set_input(x)
 
+    def _fork_event(self) -> int:
+        if self._event is None:
+            self._event = F.Event()
+        return self._event.handle
+
     def _run_branches(self, fn):
         """fn(i, branch) for every branch; branches 1.. on side streams between a fork and a join when concurrent."""
         n = len(self.branches)
@@ -98,15 +102,14 @@ class Concat(Layer):
             return
         main = torch.cuda.current_stream(self.y.device)
         sides = side_streams(self.y.device, n - 1)
-        if self._events is None:
-            self._events = [F.new_event() for _ in range(2 * (n - 1))]
+        event = self._fork_event()
         for i in range(1, n):
-            F.stream_order(main, sides[i - 1], self._events[i - 1])                 # fork
+            F.stream_order(main, sides[i - 1], event)                   # fork
         fn(0, self.branches[0])
         for i in range(1, n):
             with torch.cuda.stream(sides[i - 1]):
                 fn(i, self.branches[i])
-            F.stream_order(sides[i - 1], main, self._events[n - 1 + i - 1])         # join
+            F.stream_order(sides[i - 1], main, event)                   # join
 
     def forward(self, x):
         x4 = x if x.dim() == 4 else x.view(self.in_shape)
@@ -142,8 +145,8 @@ class Concat(Layer):
         total = grads[0]
         for i in range(1, len(grads), 3):
             F.add_2d_n(total, grads[i:i + 3])
-        for stream, event in wgrad:
-            F.stream_order(stream, torch.cuda.current_stream(self.y.device), event)
+        for stream in wgrad:
+            F.stream_order(stream, torch.cuda.current_stream(self.y.device), self._fork_event())
         return total
 
     def _fork_weight_gradients(self) -> list:
@@ -154,14 +157,12 @@ class Concat(Layer):
             return []
         convs = [[l for l in br if isinstance(l, Conv2d) and l.need_dx] for br in self.branches]
         streams = side_streams(self.y.device, len(self.branches), "wgrad")
-        if self._wgrad_events is None:
-            self._wgrad_events = [[F.new_event() for _ in range(len(ls) + 1)] for ls in convs]
         out = []
-        for ls, stream, events in zip(convs, streams, self._wgrad_events):
-            for l, e in zip(ls, events):
-                l.wgrad_side = (stream, e)
+        for ls, stream in zip(convs, streams):
+            for l in ls:
+                l.wgrad_side = (stream, self._fork_event())
             if ls:
-                out.append((stream, events[-1]))
+                out.append(stream)
         return out
 
 

@@ -278,6 +278,22 @@ def new_event() -> int:
     return int(lib().geeps_event_new())
 
 
+class Event:
+    """An event for stream_order() that lives as long as its owner."""
+
+    def __init__(self):
+        self.handle = new_event()
+
+    def __deepcopy__(self, memo):
+        return Event()
+
+    def __del__(self):
+        try:
+            lib().geeps_event_delete(C.c_void_p(self.handle))
+        except Exception:           # the interpreter is going down
+            pass
+
+
 def add_2d(dst2d, src2d) -> None:
     add_2d_n(dst2d, [src2d])
 

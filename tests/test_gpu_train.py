@@ -392,8 +392,10 @@ def test_bf16_only_weight_publish_trains_identically():
 
 
 def test_concurrent_module_backward_matches_the_serial_one():
-    """Branches and weight gradients on side streams against one stream: gradients complete when backward returns.  The
-    slices of a weight gradient meet in fp32 atomics, in any order; everything else is the same arithmetic."""
+    """Branches and weight gradients on side streams against one stream, on another batch in every pass: gradients are
+    complete when backward returns, and a pass does not touch what the one before still reads.  One weight gradient takes
+    longer than all that its branch has left to do.  The slices of a weight gradient meet in fp32 atomics, in any order;
+    everything else is the same arithmetic."""
     from geeps_b200.models.net import Concat
     dev = torch.device("cuda:0")
     conv = lambda n, c, k: [Conv2d(n, c, k, pad=k // 2, bias=False, std=0.0), BatchNorm(n + "_bn", relu=True)]   # noqa: E731
@@ -401,26 +403,73 @@ def test_concurrent_module_backward_matches_the_serial_one():
     for concurrent in (True, False):
         gen = torch.Generator(device=dev).manual_seed(3)
         m = Concat("m", [conv("a", 32, 1), conv("b", 32, 1) + conv("c", 48, 3), conv("d", 16, 3) + conv("e", 16, 3) + conv("f", 24, 3),
-                         [Pool("avg", 3, 1, pad=1, ceil_mode=False)] + conv("g", 32, 1)], concurrent=concurrent)
-        m.setup((4, 14, 14, 64), dev)
+                         [Pool("avg", 3, 1, pad=1, ceil_mode=False)] + conv("g", 512, 5)], concurrent=concurrent)
+        m.setup((8, 28, 28, 64), dev)
+        params = []
         for l in m.sublayers():
             for sp in l.param_specs():
                 w = torch.randn(sp.shape, device=dev, generator=gen) * 0.1 + (1.0 if sp.name == "gamma" else 0.0)
-                l.p32[sp.name], l.p16[sp.name], l.g32[sp.name] = w, w.to(torch.bfloat16), torch.full_like(w, 9.0)
-        x = torch.randn(4, 14, 14, 64, device=dev, generator=gen).to(torch.bfloat16)
-        dy = torch.randn(4 * 14 * 14, 136, device=dev, generator=gen).to(torch.bfloat16)
+                l.p32[sp.name], l.p16[sp.name], l.g32[sp.name] = w, w.to(torch.bfloat16), torch.empty_like(w)
+                params.append((l, sp.name))
+        x = torch.empty(8, 28, 28, 64, device=dev, dtype=torch.bfloat16)
+        dy = torch.empty(8 * 28 * 28, 616, device=dev, dtype=torch.bfloat16)
+        batches = [(torch.randn(x.shape, device=dev, generator=gen).to(torch.bfloat16),
+                    torch.randn(dy.shape, device=dev, generator=gen).to(torch.bfloat16)) for _ in range(4)]
         torch.cuda.synchronize()
-        for _ in range(3):
+        passes = []
+        for bx, bdy in batches:                                     # all on the caller's stream, nothing waited for
+            x.copy_(bx)
+            dy.copy_(bdy)
+            for l, name in params:
+                l.g32[name].fill_(float("nan"))                     # a gradient that is not there yet
             y = m.forward(x)
             dx = m.backward(dy)
-            grads = [l.g32[sp.name].clone() for l in m.sublayers() for sp in l.param_specs()]    # on the caller's stream
+            passes.append([y.clone(), dx.clone()] + [l.g32[name].clone() for l, name in params])
         assert all(l.wgrad_side is None for l in m.sublayers() if isinstance(l, Conv2d))
-        results.append([y.clone(), dx.clone()] + grads)
+        results.append(passes)
     torch.cuda.synchronize()
-    for a, b in zip(*results):
-        # sums of BatchNorm statistics and of gradient slices in another order: some 2^-24 per addition, roundings to bf16
-        # between the layers of a branch where such a difference meets a tie
-        assert (a.float() - b.float()).norm() <= 2e-3 * b.float().norm()
+    for concurrent, serial in zip(*results):
+        for a, b in zip(concurrent, serial):
+            # Sums of BatchNorm statistics and of gradient slices meet in another order, and a value that this brings over a
+            # rounding or over the zero of a ReLU changes what follows: one mask bit of the narrowest layer (6272 x 16, half
+            # of them on) is 1 / sqrt(50176) = 4.5e-3 of its gradient in the 2-norm, and sixteen of them 1.8e-2.  A gradient
+            # of another batch, or one that is not there, is off by more than 1.
+            assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm()
+
+
+def test_modules_give_their_event_back(monkeypatch):
+    """A module makes one event for its forks and joins, and destroys it when it goes."""
+    import gc
+    from geeps_b200.models.net import Concat
+    from geeps_b200.ops import functional as F
+    dev = torch.device("cuda:0")
+    made, deleted = [], []
+    new, lib = F.new_event, F.lib()
+    monkeypatch.setattr(F, "new_event", lambda: made.append(new()) or made[-1])
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def geeps_event_delete(self, handle):
+            deleted.append(handle.value)
+            lib.geeps_event_delete(handle)
+    monkeypatch.setattr(F, "lib", lambda: Lib())
+    m = Concat("m", [[Conv2d("a", 16, 1, bias=False)], [Conv2d("b", 16, 3, pad=1, bias=False)], [Conv2d("c", 16, 1, bias=False)]])
+    m.setup((2, 8, 8, 16), dev)
+    for l in m.sublayers():
+        for sp in l.param_specs():
+            w = torch.zeros(sp.shape, device=dev)
+            l.p32[sp.name], l.p16[sp.name], l.g32[sp.name] = w, w.to(torch.bfloat16), w.clone()
+    torch.cuda.synchronize()
+    for _ in range(2):
+        m.forward(torch.zeros(2, 8, 8, 16, device=dev, dtype=torch.bfloat16))
+        m.backward(torch.zeros(2 * 64, 48, device=dev, dtype=torch.bfloat16))
+    torch.cuda.synchronize()
+    assert len(made) == 1 and not deleted
+    del m, l
+    gc.collect()
+    assert deleted == made
 
 
 def test_graph_steps_follow_the_callers_stream():
