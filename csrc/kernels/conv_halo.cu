@@ -546,7 +546,8 @@ HaloPlan plan_halo(const GeepsConvTcParams* p, bool pair = false) {
 // (us, MODE_DGRAD and pairs): 64 x 28 x 28, 96 -> 64, 3 x 3: 18.4, 15.4; 300 x 14 x 14, 64 -> 32, 5 x 5: 52.2, 35.8; 128 x 20
 // x 20, 96 -> 48, 5 x 5: 32.8, 26.6; 64 x 27 x 27, 40 -> 48, 5 x 5: 24.6, 17.4; 256 x 28 x 28, 384 -> 64, 3 x 3: 120, 102.
 // Tiles of few rows look cheap by columns alone and are not: a step's weights take some 520 clocks (conv2 in tiles of two
-// image rows: 470 us).
+// image rows: 470 us).  Through conv_tc() only 64 channels or 5 x 5 taps and more come here; the rule for those is older than
+// the pairs, and fewer channels at 3 x 3 or 4 x 4 are on the box kernel.
 bool takes_pairs(const HaloPlan& plain, const HaloPlan& pairs) {
   return plain.ok && pairs.ok && pairs.cost < plain.cost;
 }
@@ -607,7 +608,7 @@ int geeps_conv_halo_pair_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out
   memset(out, 0, sizeof(*out));
   if (!geeps_conv_tc_supported(p)) return 0;
   const HaloPlan pairs = plan_halo(p, true);
-  return fill_plan(pairs, takes_pairs(plan_halo(p), pairs), out);
+  return fill_plan(pairs, geeps_conv_halo_applicable(p) && takes_pairs(plan_halo(p), pairs), out);
 }
 
 int geeps_conv_halo(const GeepsConvTcParams* p, void* stream) {
@@ -615,7 +616,8 @@ int geeps_conv_halo(const GeepsConvTcParams* p, void* stream) {
   HaloPlan hp = plan_halo(p);
   if (!hp.ok) return (int)cudaErrorInvalidValue;
   const HaloPlan pairs = plan_halo(p, true);
-  const bool pair = takes_pairs(hp, pairs);
+  const bool pair = p->columns == 0 ? takes_pairs(hp, pairs) : p->columns == 2;
+  if (pair && !pairs.ok) return (int)cudaErrorInvalidValue;
   if (pair) hp = pairs;
   HaloDev& d = hp.d;
   const bool fwd = p->mode == MODE_FWD;

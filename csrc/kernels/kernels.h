@@ -162,8 +162,10 @@ typedef struct GeepsConvTcParams {
   void* x; void* y; void* w; const float* bias; int* status;
   long long x_pitch, y_pitch, ldw;
   int B, H, W, cg, OH, OW, og, KH, KW, pad, relu, mode, split_k;
-  int stride;   // 0 or 1: stride 1; 2 .. 8: forward and weight gradient only (the activation boxes are loaded with
-                // that TMA element stride), the data gradient of a strided layer is not an implicit GEMM here
+  int stride;   // 0 or 1: stride 1; 2 .. 8: the activation boxes of forward and weight gradient are loaded with that TMA
+                // element stride, the data gradient is stride * stride problems of stride 1, one per parity class of dX
+  int columns;  // data gradient of the halo kernel: 0 by cost, 1 one image column per position, 2 column pairs (an error
+                // where they do not fit)
 } GeepsConvTcParams;
 int geeps_conv_tc(const GeepsConvTcParams* p, void* stream);
 int geeps_conv_tc_supported(const GeepsConvTcParams* p);
@@ -187,7 +189,7 @@ typedef struct GeepsHaloPlanInfo {
   double util;
 } GeepsHaloPlanInfo;
 int geeps_conv_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
-// ... and of a data gradient by column pairs; routed: geeps_conv_halo takes it that way
+// ... and of a data gradient by column pairs; routed: geeps_conv_tc() would run the call that way
 int geeps_conv_halo_pair_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
 int geeps_conv_wgrad_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out);
 

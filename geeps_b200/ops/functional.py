@@ -70,11 +70,12 @@ CONV_FWD, CONV_DGRAD, CONV_WGRAD = 0, 1, 2
 
 def conv_tc_params(mode: int, x: torch.Tensor, y: torch.Tensor, w: torch.Tensor, k: int, pad: int, *,
                    bias: torch.Tensor | None = None, relu: bool = False, split_k: int = 0,
-                   status: torch.Tensor | None = None, stride: int = 1) -> ConvTcParams:
+                   status: torch.Tensor | None = None, stride: int = 1, columns: int = 0) -> ConvTcParams:
     """Arguments of the implicit-GEMM convolution (stride 1 .. 8; the data gradient of a strided layer needs a
     filter at least as wide as the stride).  x: [B, H, W, cg] and y: [B, OH, OW, og] are NHWC
     bf16 tensors or channel slices of wider ones (last-dim stride 1, dense pixels); w: [og, ldw] with column
-    (kh * k + kw) * cg + ci, bf16 for forward / data gradient, fp32 (the gradient) for the weight gradient."""
+    (kh * k + kw) * cg + ci, bf16 for forward / data gradient, fp32 (the gradient) for the weight gradient.  columns: a
+    data gradient on the halo kernel by single columns (1) or column pairs (2), 0 = whichever costs less."""
     B, H, W, cg = x.shape
     _, OH, OW, og = y.shape
     assert x.stride(3) == 1 and y.stride(3) == 1 and w.stride(1) == 1
@@ -88,7 +89,7 @@ def conv_tc_params(mode: int, x: torch.Tensor, y: torch.Tensor, w: torch.Tensor,
     p.x_pitch, p.y_pitch, p.ldw = xp, yp, w.stride(0)
     p.B, p.H, p.W, p.cg, p.OH, p.OW, p.og = B, H, W, cg, OH, OW, og
     p.KH, p.KW, p.pad, p.relu, p.mode, p.split_k = k, k, pad, int(relu), mode, split_k
-    p.stride = stride
+    p.stride, p.columns = stride, columns
     return p
 
 

@@ -133,14 +133,16 @@ COLUMN_PAIRS = [
     (40, 17, 40, 8, 0, 8, 64, 0, 64, 7, 0),             # 7 taps, no padding
     (100, 20, 20, 24, 0, 24, 64, 0, 64, 7, 3),
     (75, 13, 28, 16, 0, 16, 24, 0, 24, 2, 0),           # two taps a row, few k
+    (1, 5, 2, 8, 0, 8, 8, 0, 8, 3, 1),                  # one pair of columns
+    (2, 7, 9, 64, 0, 64, 136, 0, 136, 5, 2),            # three chunks, the last of 8
+    (3, 11, 13, 24, 8, 16, 48, 0, 48, 6, 3),
 ]
 
 
 @pytest.mark.parametrize("case", COLUMN_PAIRS)
 def test_column_pair_data_gradient_matches_torch(case):
-    """The even and the odd column of a pair in the two halves of an accumulator, KW + 1 steps per filter row."""
-    import ctypes
-    from geeps_b200.ops import _lib as L
+    """The even and the odd column of a pair in the two halves of an accumulator, KW + 1 steps per filter row: against 64
+    bits, and bitwise against one column per position, which adds the same products in the same order."""
     from geeps_b200.ops import functional as F
     B, H, W, Ct, c_off, cg, Ot, o_off, og, k, pad = case
     dev = torch.device("cuda:0")
@@ -156,10 +158,9 @@ def test_column_pair_data_gradient_matches_torch(case):
     dx_full = torch.full((B, H, W, Ct), 3.0, device=dev, dtype=BF)
     dx = dx_full[..., c_off:c_off + cg]
     status = torch.zeros(4, dtype=torch.int32, device=dev)
-    p, pairs = F.conv_tc_params(F.CONV_DGRAD, dx, dy, w, k, pad), L.HaloPlanInfo()
-    assert L.lib().geeps_conv_halo_pair_plan(ctypes.byref(p), ctypes.byref(pairs))
-    assert pairs.routed
-    F.conv_halo(F.CONV_DGRAD, dx, dy, w, k, pad, status=status)
+    single = torch.full((B, H, W, Ct), 3.0, device=dev, dtype=BF)
+    F.conv_halo(F.CONV_DGRAD, single[..., c_off:c_off + cg], dy, w, k, pad, columns=1, status=status)
+    F.conv_halo(F.CONV_DGRAD, dx, dy, w, k, pad, columns=2, status=status)
     torch.cuda.synchronize()
     spoilt = torch.zeros(H, W, dtype=torch.bool, device=dev)
     y0, x0 = OH // 2 - pad, OW // 2 - pad
@@ -168,8 +169,32 @@ def test_column_pair_data_gradient_matches_torch(case):
     assert bool(fine[1:].all()) and bool((fine[0] == ~spoilt).all())
     # fp32 sums rounded once to bf16: uniform relative rounding errors of up to 2^-9, 2^-9 / sqrt(3) = 1.1e-3 in the 2-norm
     assert _rel(dx[fine], ref[fine]) < 2.5e-3
+    finite = torch.isfinite(dx_full)                    # what infinity and NaN are made of may differ
+    assert torch.equal(finite, torch.isfinite(single)) and torch.equal(dx_full[finite], single[finite])
     assert bool((dx_full[..., :c_off] == 3.0).all()) and bool((dx_full[..., c_off + cg:] == 3.0).all())
     assert status.tolist()[0] == 0
+
+
+@pytest.mark.parametrize("case", [(160, 27, 48, 128, 5, 2), (200, 28, 64, 96, 3, 1)])
+def test_conv_tc_runs_a_data_gradient_by_column_pairs(case):
+    """Layers that conv_tc() sends to the pairs: the result is that of the kernel asked for them."""
+    import ctypes
+    from geeps_b200.ops import _lib as L
+    from geeps_b200.ops import functional as F
+    B, H, cg, og, k, pad = case
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(12)
+    w = (torch.randn(og, k * k * cg, device=dev, generator=gen) / (k * k * cg) ** 0.5).to(BF)
+    dy = torch.randn(B, H, H, og, device=dev, generator=gen).to(BF)
+    out = [torch.zeros(B, H, H, cg, device=dev, dtype=BF) for _ in range(2)]
+    p, pairs = F.conv_tc_params(F.CONV_DGRAD, out[0], dy, w, k, pad), L.HaloPlanInfo()
+    assert L.lib().geeps_conv_halo_pair_plan(ctypes.byref(p), ctypes.byref(pairs)) and pairs.routed
+    F.conv_tc(F.CONV_DGRAD, out[0], dy, w, k, pad)
+    F.conv_halo(F.CONV_DGRAD, out[1], dy, w, k, pad, columns=2)
+    torch.cuda.synchronize()
+    assert torch.equal(*out)
+    p.mode, p.columns = F.CONV_FWD, 2                   # no such thing
+    assert L.lib().geeps_conv_halo(ctypes.byref(p), L.stream_ptr()) != 0
 
 
 HALO_CASES = CASES + [
