@@ -274,8 +274,8 @@ static bool stream_capturing(void* stream) {
 
 // With one worker there is nobody to signal and nobody to wait for but the comm stream of this process, which an event
 // orders: no announcement kernel on the application's stream, no wait kernel on the comm stream, none in front of a read
-// (each 2 to 6 us of the stream; the announcement flushes its writes to system scope).  AlexNet's step 2218 -> 2176 us, a
-// clock of 1 MiB 67 -> 53 us.  Not where a test withholds the announcements, and not where readers merge their own pending
+// (each 2 to 6 us of the stream; the announcement flushes its writes to system scope).  By flags and by events: AlexNet's step
+// 2265 and 2210 us, a clock of 1 MiB 48.4 and 40.9 us (medians of 9 x 1500 clocks, three processes each).  Not where a test withholds the announcements, and not where readers merge their own pending
 // updates at slack > 0 (they read the flags).
 bool ClientLib::fabric_by_events(const CachedTable& ct) const {
   return num_processes_ == 1 && !flags_only_ && !(config_.read_my_writes && ct.plan->slack > 0);

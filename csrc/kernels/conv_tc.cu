@@ -462,7 +462,7 @@ extern "C" {
 int geeps_conv_tc_supported(const GeepsConvTcParams* p) {
   if (p->B <= 0 || p->H <= 0 || p->W <= 0 || p->cg <= 0 || p->og <= 0 || p->KH <= 0 || p->KW <= 0) return 0;
   const int s = p->stride > 1 ? p->stride : 1;
-  // a strided data gradient runs per parity class of dX; a class without taps (filter narrower than the stride)
+  // a strided data gradient is a problem for each parity class of dX; a class without taps (filter narrower than the stride)
   // would have to be zeroed instead and is left to the caller
   if (s > 8 || (s > 1 && p->mode == MODE_DGRAD && (p->KH < s || p->KW < s))) return 0;
   if (p->OH != (p->H + 2 * p->pad - p->KH) / s + 1 || p->OW != (p->W + 2 * p->pad - p->KW) / s + 1) return 0;

@@ -344,8 +344,8 @@ int halo_mode() {
 extern "C" {
 
 // 1 when conv_tc() should route this weight-gradient call here.  Fitted to timings of both kernels at batch 128 .. 256
-// (python -m geeps_b200.utils.microbench conv): filter rows of 5 taps or more always win (AlexNet conv2 0.103 ->
-// 0.087 ms per group, Inception 5 x 5 0.054 -> 0.050 ms); 3-tap rows only when the layer is one item wide (one block
+// (python -m geeps_b200.utils.microbench conv): filter rows of 5 taps or more always win (AlexNet conv2 0.103 ms per group,
+// 0.087 here when the line was drawn and 0.074 now; Inception 5 x 5 0.054 -> 0.050 ms); 3-tap rows only when the layer is one item wide (one block
 // of output channels, one chunk of input channels: AlexNet conv1 0.120 -> 0.112 ms) - wider 3 x 3 layers are faster
 // on the box kernel, which covers four (tap, chunk) panels per MMA whatever the filter's shape.
 int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p) {

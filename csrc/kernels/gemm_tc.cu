@@ -528,12 +528,14 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, 
 
 int round_up(long long v, int m) { return (int)((v + m - 1) / m * m); }
 
-// Tile width and K slices (cluster size) for an output that 256-wide tiles would not spread over every SM.  Such a
-// product is bound by the operand bytes its CTAs pull through L2 (75 to 90 bytes per ns and SM: 256 x 4096, K = 9216 takes
-// 43, 51 and 80 us on widths 64, 128 and 256), so the choice is the one with the least traffic on the busiest SM: rounds x
-// k tiles per CTA x (A rows + B rows) x 128 bytes, plus kTileOver (2 us of that traffic) per round (fill, drain) and, for a
-// cluster, the exchange of its partial tile.  Narrow tiles spread an
-// output but re-read A once per tile; a cluster keeps the tile wide and cuts K instead.
+// Tile width and K slices (cluster size) for an output that 256-wide tiles would not spread over every SM: the choice with
+// the least operand traffic on the busiest SM, rounds x k tiles per CTA x (A rows + B rows) x 128 bytes, plus kTileOver per
+// round (fill, drain) and, for a cluster, the exchange of its partial tile.  Narrow tiles spread an output but re-read A
+// once per tile; a cluster keeps the tile wide and cuts K instead.  The traffic is not the bound (the issue of the MMAs
+// alone took 256 x 4096, K = 9216 from 38.9 to 32.8 us, L2 flushed), but it ranks the widths as they are now (64, 128, 192, 256; us
+// in a captured chain): 256 x 4096, K = 9216 27.0, 35.2, 48.9, 64.4; 256 x 9216, K = 4096 29.5, 20.1, 25.4, 30.0; 256 x 4096,
+// K = 4096 13.9, 13.7, 17.5, 22.6; 256 x 1000, K = 4096 13.3, 13.5, 17.5, 22.5; 100 x 512, K = 2048 7.9, 8.4, 10.6, 13.0.
+// The sizes of clusters it ranks less well (see plan_gemm).
 struct TileChoice { int bn, cluster; };
 TileChoice choose_tiles(const GeepsGemmParams* p, int unit, int kt, int sms, bool cluster_ok) {
   constexpr double kTileOver = 150e3, kClusterOver = 150e3;
@@ -591,11 +593,12 @@ GemmPlan plan_gemm(const GeepsGemmParams* p, int sms) {
       // a bf16 slab is 64 columns wide (see below): several tiles have widths that are multiples of it
       const int step = tma_c && !p->out_fp32 ? 64 : unit;
       // Clusters only for K above 8128 over at most sms / 8 narrow tiles: the data gradient of a wide classifier, 32 x 1024,
-      // K = 21841, 16 tiles: 80 us without a cluster, 37 on 64 x 8 (31 on 64 x 4).  The line is drawn by the order of the
+      // K = 21841, 16 tiles (tile width x cluster, us in a captured chain): 70 without a cluster, 26.6 on 64 x 8, which the
+      // cost picks (22.1 on 64 x 4, 16.4 on 128 x 8).  The line is drawn by the order of the
       // sums, not by speed: a cluster adds its K slices in another order than one running sum, and in a deep network with
       // near-ties in its pooling windows that changes which element a later step's maximum picks, so ordinary layers
-      // keep one sum.  What that leaves (tile width x cluster, L2 flushed): 256 x 4096, K = 9216: 45 us on 64 x 1, 53 on
-      // 128 x 1, 41 on 128 x 2; 32 rows: 43 on 64 x 1, 31 on 128 x 4; 256 x 1000, K = 4096: 24.5 on 64 x 1, 16.5 on 64 x 4.
+      // keep one sum.  What that leaves: 256 x 4096, K = 9216: 27.0 on 64 x 1, 25.1 on 128 x 2; 32 rows: 25.6 on 64 x 1, 13.9
+      // on 128 x 4; 256 x 1000, K = 4096: 13.3 on 64 x 1, 9.4 on 64 x 4.
       const bool cluster_ok = p->split_k <= 1 && p->beta == 0.f && kt >= 128 &&
                               m_tiles * ((p->N + 63) / 64) <= sms / 8;
       const TileChoice c = choose_tiles(p, step, kt, sms, cluster_ok);

@@ -243,8 +243,8 @@ class Conv2d(Layer):
             # 49 mostly-zero k-steps lose to 7 dense ones over a patch matrix (6.8 against 5.8 ms per step)
             self.implicit = False
         # a strided layer's forward and weight gradient load the activation boxes with a TMA element stride; its data
-        # gradient runs one parity class of dX at a time (stride^2 stride-1 problems with sub-filters), unless the
-        # filter is narrower than the stride (then some classes have no taps): GEMM + col2im for those
+        # gradient is a stride-1 problem with a sub-filter for each parity class of dX (stride^2 of them, four a launch),
+        # unless the filter is narrower than the stride (then some classes have no taps): GEMM + col2im for those
         self.implicit_dgrad = self.implicit and (self.stride == 1 or self.k >= self.stride)
         self.cols = self.dcol = None
         if not self.pointwise and not self.implicit:
