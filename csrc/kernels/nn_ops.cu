@@ -235,6 +235,13 @@ inline SlotGrid slot_grid(long long P, int C, int per_thread, int per_sm, int nq
   if (want * 8 < fill) want = one_each < fill ? one_each : fill;
   const long long cap = (long long)geeps_sm_count() * per_sm / chunks;
   if (want > cap) want = cap;
+  // More than one block a SM and less than two: one.  Blocks that come up before their predecessor has left (geeps_launch)
+  // pair up on the SMs with room, and the step waits for those.  BatchNorm forward and backward, us, ordinary launches /
+  // dependent / dependent with this: 8 x 56 x 56 x 64, 196 blocks 13.0 / 14.6 / 12.7; 64 x 14 x 14 x 160, 261 blocks 16.6 /
+  // 18.1 / 15.2; 32 x 28 x 28 x 48, 149 blocks 14.3 / 13.7 / 11.9.  In an Inception module of 31 x 28 x 28 x 352 ordinary
+  // launches of these layers cost 10 us (313), dependent ones 302, with this 298.
+  const long long one = geeps_sm_count() / chunks;
+  if (want > one && want < 2 * one) want = one;
   if (want < 1) want = 1;
   g.grid = dim3((unsigned)chunks, (unsigned)want, 1);
   g.smem = (size_t)rows_used * cvb * 8 * nq * sizeof(float);
@@ -1697,16 +1704,6 @@ softmax_ce_kernel(const float* __restrict__ logits, const long long* __restrict_
 
 #define CK() ((int)cudaGetLastError())
 
-// A dependent launch, unless the blocks are more than one a SM and less than two: those that come up early pair up on the SMs
-// with room.  Forward and backward, us, ordinary / dependent: 8 x 56 x 56 x 64, 196 blocks 13.8 / 14.7; 64 x 14 x 14 x 160, 261
-// blocks 16.9 / 18.1; near one a SM either way (149 blocks 13.9 / 13.8, 171 13.4 / 14.0); beyond 100 x 14 x 14 x 128, 306
-// blocks 18.2 / 16.4.
-template <typename... P, typename... A>
-static void launch_channels(void (*kernel)(P...), const SlotGrid& g, cudaStream_t st, A&&... args) {
-  const long long blocks = (long long)g.grid.x * g.grid.y, sms = geeps_sm_count();
-  geeps_launch_as(blocks <= sms || blocks >= 2 * sms, kernel, g.grid, g.threads, g.smem, st, static_cast<A&&>(args)...);
-}
-
 template <typename T>
 static int nchw_to_nhwc_launch(const T* x, void* y, int B, int C, int H, int W, int Cpad, cudaStream_t st) {
   const long long n = (long long)B * H * W * Cpad;
@@ -1831,11 +1828,11 @@ int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* be
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
   const SlotGrid rg = reduce_grid(0, P, C), ag = apply_grid(P, C);
-  launch_channels(channel_reduce_kernel<0>, rg, st,
+  geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
   geeps_launch(bn_finalize_kernel, (C + 127) / 128, 128, 0, st, sums, mean_rstd, running_mean, running_var, C,
                                                       1.f / (float)P, eps, momentum);
-  launch_channels(bn_apply_kernel, ag, st, (const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
+  geeps_launch(bn_apply_kernel, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (bf16*)y, mean_rstd, gamma, beta, P, C, ldx,
                                                         ldy, relu);
   return CK();
 }
@@ -1846,9 +1843,9 @@ static int bn_backward_by_output(const void* x, const void* dy, const void* y, v
                                  int C, long long ldx, long long lddy, long long lddx, int relu, float grad_scale,
                                  cudaStream_t st) {
   const SlotGrid rg = reduce_grid(1, P, C), ag = apply_grid(P, C, backward_blocks(relu ? MASK_Y : MASK_NONE));
-  launch_channels(channel_reduce_kernel<1>, rg, st,
+  geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-  launch_channels(relu ? bn_backward_kernel<MASK_Y> : bn_backward_kernel<MASK_NONE>, ag, st,
+  geeps_launch(relu ? bn_backward_kernel<MASK_Y> : bn_backward_kernel<MASK_NONE>, ag.grid, ag.threads, ag.smem, st,
                (const bf16*)x, (const bf16*)dy, (const bf16*)y, (bf16*)dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx,
                lddy, lddx, relu, grad_scale, zero_after);
   return CK();
@@ -1898,9 +1895,9 @@ int geeps_bn_forward_fused_bits(const void* x, void* y, const float* gamma, cons
     return e == cudaSuccess ? CK() : (int)e;
   }
   const SlotGrid rg = reduce_grid(0, P, C), ag = apply_grid(P, C);
-  launch_channels(channel_reduce_kernel<0>, rg, st,
+  geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
-  launch_channels(bn_apply_fused_kernel, ag, st, (const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
+  geeps_launch(bn_apply_fused_kernel, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (bf16*)y, sums, mean_rstd, running_mean,
                                                               running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                                                               1.f / (float)P, eps, momentum, bits);
   return CK();
@@ -1924,9 +1921,9 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
   }
   if (bits != nullptr && relu) {
     const SlotGrid rg = reduce_grid(3, P, C), ag = apply_grid(P, C, backward_blocks(MASK_BITS));
-    launch_channels(channel_reduce_kernel<3>, rg, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits,
+    geeps_launch(channel_reduce_kernel<3>, rg.grid, rg.threads, rg.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits,
                                                                    mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
-    launch_channels(bn_backward_kernel<MASK_BITS>, ag, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
+    geeps_launch(bn_backward_kernel<MASK_BITS>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
                                                              mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx,
                                                              relu, grad_scale, zero_after);
     return CK();
@@ -1944,7 +1941,7 @@ int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, f
   }
   if (zero_first) cudaMemsetAsync(out, 0, sizeof(float) * C, st);
   const SlotGrid rg = reduce_grid(2, P, C);
-  launch_channels(channel_reduce_kernel<2>, rg, st,
+  geeps_launch(channel_reduce_kernel<2>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, out, P, C, ldx, 0, 0, scale);
   return CK();
 }
