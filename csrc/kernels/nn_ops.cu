@@ -235,13 +235,6 @@ inline SlotGrid slot_grid(long long P, int C, int per_thread, int per_sm, int nq
   if (want * 8 < fill) want = one_each < fill ? one_each : fill;
   const long long cap = (long long)geeps_sm_count() * per_sm / chunks;
   if (want > cap) want = cap;
-  // More than one block a SM and less than two: one.  Blocks that come up before their predecessor has left (geeps_launch)
-  // pair up on the SMs with room, and the step waits for those.  BatchNorm forward and backward, us, ordinary launches /
-  // dependent / dependent with this: 8 x 56 x 56 x 64, 196 blocks 13.0 / 14.6 / 12.7; 64 x 14 x 14 x 160, 261 blocks 16.6 /
-  // 18.1 / 15.2; 32 x 28 x 28 x 48, 149 blocks 14.3 / 13.7 / 11.9.  In an Inception module of 31 x 28 x 28 x 352 ordinary
-  // launches of these layers cost 10 us (313), dependent ones 302, with this 298.
-  const long long one = geeps_sm_count() / chunks;
-  if (want > one && want < 2 * one) want = one;
   if (want < 1) want = 1;
   g.grid = dim3((unsigned)chunks, (unsigned)want, 1);
   g.smem = (size_t)rows_used * cvb * 8 * nq * sizeof(float);
@@ -1812,11 +1805,23 @@ int geeps_col2im(const void* dcol, void* dx, const GeepsConvGeom* g, int accumul
   return CK();
 }
 
+// More than one block a SM and less than two: one.  Blocks that come up before their predecessor has left (geeps_launch)
+// pair up on the SMs with room, and the step waits for those.  BatchNorm forward and backward, us, ordinary launches /
+// dependent / dependent with this: 8 x 56 x 56 x 64, 196 blocks 13.0 / 14.6 / 12.7; 64 x 14 x 14 x 160, 261 blocks 16.6 /
+// 18.1 / 15.2; 32 x 28 x 28 x 48, 149 blocks 14.3 / 13.7 / 11.9.  In an Inception module of 31 x 28 x 28 x 352 ordinary
+// launches of these layers cost 10 us (313), dependent ones 302, with this 298.
+static SlotGrid balanced(SlotGrid g) {
+  const unsigned one = (unsigned)geeps_sm_count() / g.grid.x;
+  if (g.grid.y > one && g.grid.y < 2 * one) g.grid.y = one;
+  return g;
+}
 // reductions: one batch of four pixels per thread where that leaves SMs idle
-static SlotGrid reduce_grid(int mode, long long P, int C) { return slot_grid(P, C, 4, reduce_blocks(mode), mode == 2 ? 1 : 2); }
+static SlotGrid reduce_grid(int mode, long long P, int C) {
+  return balanced(slot_grid(P, C, 4, reduce_blocks(mode), mode == 2 ? 1 : 2));
+}
 // element-wise passes with per-channel constants
 static SlotGrid apply_grid(long long P, int C, int per_sm = kApplyBlocks) {
-  SlotGrid g = slot_grid(P, C, 4, per_sm, 0);
+  SlotGrid g = balanced(slot_grid(P, C, 4, per_sm, 0));
   g.smem = ((size_t)(C / 8) + g.grid.x - 1) / g.grid.x * 8 * 4 * sizeof(float);      // four constants per channel
   return g;
 }
