@@ -59,6 +59,7 @@ struct ConvDev {
   int rows;                       // bw * bh * bnb
   int bn, n_valid;                // tile width; valid output columns (fwd: Og, dgrad: Cg, wgrad: panels * 64)
   int m_tiles, n_tiles, kt_total, split_k, stages, tmem_cols;
+  int groups;                     // epilogue groups that have columns to take
   int slabs;                      // staging slabs: two per epilogue group that has one to fill
   int relu, zero_fill_c;          // wgrad: a channel coordinate outside X, for panels past the last one
   int ch_valid;                   // wgrad: channels per tap (cg)
@@ -280,7 +281,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (MODE == MODE_FWD) mb = decode_box(d, mi, d.wt, d.ht);
       if (MODE == MODE_DGRAD) mb = decode_box(d, mi, cq.wt, cq.ht);
 #pragma unroll 1
-      for (int c = grp * cols_per_slab; c < BN; c += kGroups * cols_per_slab) {
+      for (int c = grp < d.groups ? grp * cols_per_slab : BN; c < BN; c += d.groups * cols_per_slab) {
         if (n0 + c >= d.n_valid) break;
         uint8_t* slab = cslab + (size_t)(2 * grp + (slab_i & 1u)) * C_SLAB_BYTES;
         if (issuer) tc05::bulk_wait_read<1>();
@@ -677,11 +678,17 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
   while (tmem_cols < 2 * d.bn) tmem_cols <<= 1;
   d.tmem_cols = tmem_cols;
   const int stage_bytes = A_STAGE_BYTES + d.bn * BK * 2;
-  d.slabs = d.bn > (p->mode == MODE_WGRAD || d.narrow ? 32 : 64) ? 4 : 2;
+  const long long num_tiles = (long long)d.m_tiles * d.n_tiles * d.split_k;
+  // Two groups share a tile of three slabs unevenly, and where many tiles follow one another the epilogue is covered anyway:
+  // one group takes them.  3 x 3 forward, us before there were two groups / with two / so: 47 x 52 x 52, 64 -> 312 48.9 / 50.8 /
+  // 49.1; 128 x 28 x 28, 64 -> 320 37.7 / 39.1 / 37.0; 32 x 56 x 56, 64 -> 192 (5.3 tiles an SM) 22.0 / 22.2 / 21.3.  Few
+  // tiles are faster with two: 64 x 28 x 28, 64 -> 160 (2.6) 12.7 / 11.9 / 12.1; 128 -> 192 at batch 32 14.8 / 13.7 / 13.9.
+  const int slab_cols = p->mode == MODE_WGRAD || d.narrow ? 32 : 64;
+  d.groups = p->mode == MODE_FWD && !d.narrow && (d.bn + 63) / 64 == 3 && num_tiles >= 4LL * kSMs ? 1 : kGroups;
+  d.slabs = d.groups == 2 && d.bn > slab_cols ? 4 : 2;
   d.stages = (224 * 1024 - d.slabs * C_SLAB_BYTES) / stage_bytes;
   if (d.stages > MAX_STAGES) d.stages = MAX_STAGES;
   if (d.stages < 2) d.stages = 2;
-  const long long num_tiles = (long long)d.m_tiles * d.n_tiles * d.split_k;
   const int grid = (int)(num_tiles < kSMs ? num_tiles : kSMs);
   if (p->mode == MODE_FWD) return launch<MODE_FWD>(ta, tb, tc, d, grid, st);
   if (p->mode == MODE_DGRAD) return launch<MODE_DGRAD>(ta, tb, tc, d, grid, st);

@@ -22,7 +22,14 @@ CASES = [
 ]
 
 
-@pytest.mark.parametrize("case", CASES)
+# three column slabs a tile and four tiles or more per SM: one epilogue group; the last tile of 312 channels has two slabs
+LONG_ROWS = [
+    (25, 56, 56, 16, 0, 16, 160, 0, 160, 3, 1),
+    (47, 30, 30, 24, 8, 16, 320, 0, 312, 3, 1),
+]
+
+
+@pytest.mark.parametrize("case", CASES + LONG_ROWS)
 def test_conv_tc_forward_dgrad_wgrad_match_torch(case):
     from geeps_b200.ops import functional as F
     B, H, W, Ct, c_off, cg, Ot, o_off, og, k, pad = case
