@@ -147,6 +147,7 @@ int geeps_gemm_pair_supported(const GeepsGemmParams* p);
 // Returns 0 if the tcgen05 path does not accept p.
 typedef struct GeepsGemmPlan { int pair, block_n, split_k, cluster; long long tiles; } GeepsGemmPlan;
 int geeps_gemm_plan(const GeepsGemmParams* p, GeepsGemmPlan* out);
+int geeps_clear_f32(float* c, long long n, void* stream);           // n zeros
 // C[m][n] = beta * C[m][n] (exactly 0 when beta == 0) over an M x N view with pitch ldc
 int geeps_scale_matrix_f32(float* c, long long M, long long N, long long ldc, float beta, void* stream);
 

@@ -19,6 +19,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "kernels.h"
 #include "nn_ops.h"
 
 namespace {
@@ -704,7 +705,7 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
   const int per_sm = smem <= kLpTwoPerSm ? 2 : 1;
   int grid = geeps_sm_count() * per_sm;
   if (grid > total) grid = (int)total;
-  if (colsum != nullptr) cudaMemsetAsync(colsum, 0, sizeof(float) * g->C, st);
+  if (colsum != nullptr) geeps_clear_f32(colsum, g->C, st);
   const bool k3s2 = g->K == 3 && g->stride == 2;
   // the register kernel covers the usual pair (5 channels, 3 x 3 stride 2) up to 512 channels; its item count is 32 bits
   const int cv = g->C / 8;

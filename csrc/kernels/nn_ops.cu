@@ -7,6 +7,7 @@
 // .gitmodules:1-4 of the reference); layer maths follows the usual Caffe definitions so that
 // the AlexNet / Inception-BN configurations behave as the originals did.
 #include "common.cuh"
+#include "kernels.h"
 #include "nn_ops.h"
 
 namespace {
@@ -1831,7 +1832,7 @@ int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* be
                      long long ldx, long long ldy, float eps, float momentum, int relu, void* stream) {
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
+  geeps_clear_f32(sums, 2LL * C, st);
   const SlotGrid rg = reduce_grid(0, P, C), ag = apply_grid(P, C);
   geeps_launch(channel_reduce_kernel<0>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, sums, P, C, ldx, 0, 0, 1.f);
@@ -1860,7 +1861,7 @@ int geeps_bn_backward(const void* x, const void* dy, const void* y, void* dx, co
                       long long ldx, long long lddy, long long lddx, int relu, float grad_scale, void* stream) {
   if (C % 8) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaMemsetAsync(sums, 0, sizeof(float) * 2 * C, st);
+  geeps_clear_f32(sums, 2LL * C, st);
   return bn_backward_by_output(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, nullptr, P, C, ldx, lddy, lddx, relu,
                                grad_scale, st);
 }
@@ -1944,7 +1945,7 @@ int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, f
     geeps_launch(colsum_simple_kernel, (C + 127) / 128, 128, 0, st, (const bf16*)x, out, P, C, ldx, scale, !zero_first);
     return CK();
   }
-  if (zero_first) cudaMemsetAsync(out, 0, sizeof(float) * C, st);
+  if (zero_first) geeps_clear_f32(out, C, st);
   const SlotGrid rg = reduce_grid(2, P, C);
   geeps_launch(channel_reduce_kernel<2>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, nullptr, nullptr, nullptr, out, P, C, ldx, 0, 0, scale);
@@ -1972,7 +1973,7 @@ int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* c
                                long long lddy, long long ldy, long long lddx, void* stream) {
   if (C % 8 || lddy % 8 || ldy % 8 || lddx % 8 || C > 8192) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaMemsetAsync(colsum, 0, sizeof(float) * C, st);
+  geeps_clear_f32(colsum, C, st);
   const SlotGrid rg = slot_grid(P, C, 4, 8, 1);
   geeps_launch_plain(relu_backward_colsum_kernel, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)dy, (const bf16*)y, (bf16*)dx, colsum, P, C, lddy, ldy, lddx);
@@ -2039,7 +2040,7 @@ int geeps_lrn_backward(const void* x, const void* y, const void* rscale, const v
     const int m = cv / a;
     g8 = g8 >= m ? g8 / m * m : m;
     cs_smem = sizeof(float) * C;
-    cudaMemsetAsync(colsum, 0, sizeof(float) * C, st8);
+    geeps_clear_f32(colsum, C, st8);
   }
   if (C % 8 == 0 && size == 5)
     geeps_launch_plain(lrn_backward_v8_kernel<2>, g8, 256, cs_smem, st8, (const bf16*)x, (const bf16*)y, (const bf16*)rscale, (const bf16*)dy, (bf16*)dx, P, C, size, alpha, beta, relu_mask, colsum);
@@ -2118,7 +2119,7 @@ int geeps_softmax_ce(const float* logits, const long long* labels, float* loss_s
                      void* dlogits, int B, int C, long long ldl, long long ldd, float loss_scale, float grad_scale,
                      int zero_loss, int* status, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  if (zero_loss && loss_sum) cudaMemsetAsync(loss_sum, 0, sizeof(float), st);
+  if (zero_loss && loss_sum) geeps_clear_f32(loss_sum, 1, st);
   // Narrow rows keep the order in which 256 threads have always summed them.  The register kernel takes the same time up to
   // 1000 classes and less from there (32 x 2000 8.5 -> 6.5 us, 32 x 4000 10.5 -> 7.0, 256 x 4000 10.6 -> 8.7; rows off a
   // 16-byte boundary 8.5, 8.5 and 10.6), 32 x 6000 12.6 -> 8.5, 32 x 21841 54 -> 8.

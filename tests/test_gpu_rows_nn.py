@@ -1,4 +1,6 @@
 """Row ops and training-op kernels vs plain PyTorch fp32 references."""
+import ctypes
+
 import pytest
 import torch
 import torch.nn.functional as TF
@@ -611,3 +613,13 @@ def test_recorded_step_keeps_the_input_layers_output(dtype):
         graph.launch()
     torch.cuda.synchronize()
     graph.close()
+
+
+@pytest.mark.parametrize("off", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 1023, 4099, 2_000_003])
+def test_clear_covers_exactly_its_range(off, n):
+    """Heads and tails around 16-byte boundaries; more vectors than threads at the largest."""
+    buf = torch.full((n + 16,), 2.0, device=DEV)
+    L.check(L.lib().geeps_clear_f32(ctypes.c_void_p(buf.data_ptr() + 4 * (4 + off)), ctypes.c_longlong(n), L.stream_ptr()), "clear")
+    assert (buf[4 + off:4 + off + n] == 0).all()
+    assert (buf[:4 + off] == 2).all() and (buf[4 + off + n:] == 2).all()
