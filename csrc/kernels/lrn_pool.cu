@@ -425,6 +425,232 @@ lrn_maxpool_backward_lanes_kernel(const bf16* __restrict__ x, const bf16* __rest
   }
 }
 
+// ---------------- backward, 3 x 3 windows with stride 2, window of 5 channels, many pixels ----------------
+// The 2 x 2 input pixels between two window rows and two window columns (a quad) lie under the same four windows, so a
+// lane takes the four pixels of a quad in one vector of 8 channels: four window loads instead of nine, all of a lane's
+// loads in flight at once, and which windows cover a pixel is known when the kernel is compiled.  Neighbouring lanes
+// hold neighbouring vectors of the flat (image, quad row, quad, vector) index; the first and the last lane of a warp repeat
+// a vector of their neighbours for the halo channels and store nothing, so 30 of 32 lanes work at every channel count.
+// The window codes are spread to 16-bit numbers between 0.5 and 2; one packed comparison then is a mask.  The polynomials
+// are evaluated without a branch around them (a pixel beyond their range is done again, exactly), so the arithmetic of
+// neighbouring pixels overlaps.  Sums over windows and channels are those of the lanes kernel above, in its order: the
+// results have the same bits.
+// Bound by instruction issue (64 % of the slots, half-rate integer pipe 62 %) at 16 warps per SM: 256 x 55 x 55 x 96
+// 170 us (lanes kernel) -> 138, 256 x 27 x 27 x 256 110 -> 95, 64 x 55 x 55 x 264 150 -> 98.  Three blocks per SM spill: 165 us;
+// two pixels at a time spill too: 147; fp32 without the register pairs: 151; without the last four of the savings named at
+// the lines below (codes expanded at use, packed sign test, merged halo words, match test only beyond the range): 153.
+
+// c + the two bf16 of w (a mixed-precision sum needs no conversion in front of it)
+__device__ __forceinline__ float2 add_bf16(float2 c, uint32_t w) {
+  asm("{.reg .b16 l, h; mov.b32 {l, h}, %2; add.f32.bf16 %0, l, %0; add.f32.bf16 %1, h, %1;}" : "+f"(c.x), "+f"(c.y) : "r"(w));
+  return c;
+}
+// o, 0 where x <= lim (never for a NaN)
+__device__ __forceinline__ float2 zero_where_le(float2 o, uint32_t x, uint32_t lim) {
+  asm("{.reg .pred p, q; setp.le.bf16x2 p|q, %2, %3; selp.f32 %0, 0f00000000, %0, p; selp.f32 %1, 0f00000000, %1, q;}"
+      : "+f"(o.x), "+f"(o.y) : "r"(x), "r"(lim));
+  return o;
+}
+// A walk over the mixed-radix index (image, quad row, quad) in steps of a constant.
+struct QuadWalk {
+  int b, h, w;
+  int db, dh, dw;
+  __device__ __forceinline__ QuadWalk(int first, int step, int QH, int QW) {
+    const int r = first / QW, t = step / QW;
+    w = first - r * QW;
+    b = r / QH;
+    h = r - b * QH;
+    dw = step - t * QW;
+    db = t / QH;
+    dh = t - db * QH;
+  }
+  __device__ __forceinline__ void next(int QH, int QW) {
+    w += dw;
+    h += dh;
+    b += db;
+    if (w >= QW) { w -= QW; ++h; }
+    if (h >= QH) { h -= QH; ++b; }
+  }
+};
+
+// total: vectors of all quads.  warps: those that work, each at vectors 30 warp, 30 (warp + warps), ...; 30 warps is a
+// multiple of cv unless every warp takes one step.
+__global__ void __launch_bounds__(256, 2)
+lrn_maxpool_backward_quad_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dp,
+                                 const uint8_t* __restrict__ argmax, bf16* __restrict__ dx, const GeepsPoolGeom g,
+                                 const LrnCoef cf, float coef, int relu_mask, float* __restrict__ colsum, int QH, int QW,
+                                 int total, int warps) {
+  geeps_pdl_enter();
+  __shared__ float cs_sh[8][30 * 8 + 1];        // by channel of the vector: the block's 8 x 30 working lanes
+  const int C = g.C, cv = C >> 3, W = g.W, OW = g.OW;
+  const int lane = threadIdx.x & 31;
+  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int step = warps * 30;
+  // the lane before vector 0 has no quad; the values that it hands on are not used
+  int f = warp * 30 + lane - 1;
+  const int f0 = f < 0 ? 0 : f;
+  const int vec = f0 % cv;
+  float2 cs[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) cs[k] = both(0.f);
+  QuadWalk q(f0 / cv, step / cv, QH, QW);
+  // the channels beside a vector: none at the ends of a pixel, loaded at the ends of a warp, else the neighbour's
+  const bool first_vec = vec == 0, last_vec = vec == cv - 1;
+  const uint32_t keep_b = lane == 0 || first_vec ? 0u : 0xffffffffu, keep_a = lane == 31 || last_vec ? 0u : 0xffffffffu;
+  const bool stores = lane != 0 && lane != 31;
+  const uint32_t lim = relu_mask ? 0u : 0x7fc07fc0u;
+  const int q0 = g.pad >> 1;                     // quad rows and columns begin on a window's first row and column
+  for (int it0 = warp * 30; warp < warps && it0 < total; it0 += step, f += step, q.next(QH, QW)) {
+    const bool on = f >= 0 && f < total;
+    const int h0 = 2 * (q.h + q0) - g.pad, w0 = 2 * (q.w + q0) - g.pad;
+    const long long px = (((long long)q.b * g.H + h0) * W + w0) * C + vec * 8;
+    uint4 xq[4];
+    uint32_t edge[4];
+    bool in[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      in[i] = on && (unsigned)(h0 + (i >> 1)) < (unsigned)g.H && (unsigned)(w0 + (i & 1)) < (unsigned)W;
+      const bf16* xp = x + px + ((i >> 1) * W + (i & 1)) * C;
+      xq[i] = in[i] ? *reinterpret_cast<const uint4*>(xp) : make_uint4(0u, 0u, 0u, 0u);
+      edge[i] = 0u;
+      if (in[i] && ((lane == 0 && !first_vec) || (lane == 31 && !last_vec)))
+        edge[i] = *reinterpret_cast<const uint32_t*>(xp + (lane == 0 ? -2 : 8));
+    }
+    // windows (row before, column before), (row before, column), (row, column before), (row, column)
+    uint32_t d[4][4];
+    uint2 raw[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int oh = q.h + q0 - 1 + (i >> 1), ow = q.w + q0 - 1 + (i & 1);
+      const bool there = on && (unsigned)oh < (unsigned)g.OH && (unsigned)ow < (unsigned)OW;
+      const long long opix = ((long long)q.b * g.OH + oh) * OW + ow;
+      raw[i] = there ? *reinterpret_cast<const uint2*>(argmax + opix * C + vec * 8) : make_uint2(0xffffffffu, 0xffffffffu);
+      const uint4 dv = there ? *reinterpret_cast<const uint4*>(dp + opix * g.ldy + vec * 8) : make_uint4(0u, 0u, 0u, 0u);
+      d[i][0] = dv.x; d[i][1] = dv.y; d[i][2] = dv.z; d[i][3] = dv.w;
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      if (!__any_sync(0xffffffffu, in[2 * r] || in[2 * r + 1])) continue;       // beyond the last row
+      uint32_t code[4][4];
+#pragma unroll
+      for (int j = 2 * r; j < 4; ++j) {
+        code[j][0] = __byte_perm(raw[j].x, 0x3f3f3f3fu, 0x4140); code[j][1] = __byte_perm(raw[j].x, 0x3f3f3f3fu, 0x4342);
+        code[j][2] = __byte_perm(raw[j].y, 0x3f3f3f3fu, 0x4140); code[j][3] = __byte_perm(raw[j].y, 0x3f3f3f3fu, 0x4342);
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int i = 2 * r + c;
+        // pooling gradient: window j covers the pixel unless it begins in the row (column) before and the pixel is in
+        // the quad's second row (column)
+        float2 dy[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) dy[k] = both(0.f);
+#pragma unroll
+        for (int j = 2 * r; j < 4; ++j) {
+          if ((j & 1) == 0 && c == 1) continue;
+          const int kh = j < 2 ? 2 : r, kw = (j & 1) == 0 ? 2 : c;
+          const uint32_t want = 0x3f003f00u | (uint32_t)((kh * 3 + kw) * 0x00010001u);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            dy[k] = add_bf16(dy[k], d[j][k] & __heq2_mask(reinterpret_cast<const __nv_bfloat162&>(code[j][k]),
+                                                          reinterpret_cast<const __nv_bfloat162&>(want)));
+        }
+        // a = dy * scale^-beta, rt = dy * x * scale^-(beta+1), both rounded to bf16
+        uint32_t before = __shfl_up_sync(0xffffffffu, xq[i].w, 1), after = __shfl_down_sync(0xffffffffu, xq[i].x, 1);
+        before = (before & keep_b) | (lane == 0 ? edge[i] : 0u);
+        after = (after & keep_a) | (lane == 31 ? edge[i] : 0u);
+        const float2 v[4] = {unpack2(xq[i].x), unpack2(xq[i].y), unpack2(xq[i].z), unpack2(xq[i].w)};
+        float2 t[6], ws[4], a[4], rt[4];
+        t[0] = unpack2(before); t[5] = unpack2(after);
+        t[0] = mul2(t[0], t[0]); t[5] = mul2(t[5], t[5]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) t[k + 1] = mul2(v[k], v[k]);
+        window5(t, ws);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[k] = mul2(dy[k], fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.p3), both(cf.p2)), both(cf.p1)), both(cf.p0)));
+          rt[k] = mul2(mul2(dy[k], v[k]),
+                       fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.q3), both(cf.q2)), both(cf.q1)), both(cf.q0)));
+        }
+        // the sum of all twelve squares bounds every window's
+        if (!((ws[0].x + ws[2].y) + (t[5].x + t[5].y) <= cf.w_max)) {
+          uint32_t hit = 0u;                      // a vector without a gradient has none here either (no 0 x inf)
+#pragma unroll
+          for (int j = 2 * r; j < 4; ++j) {
+            if ((j & 1) == 0 && c == 1) continue;
+            const uint32_t c4 = (uint32_t)((j < 2 ? 2 : r) * 3 + ((j & 1) == 0 ? 2 : c)) * 0x01010101u;
+            hit |= __vcmpeq4(raw[j].x, c4) | __vcmpeq4(raw[j].y, c4);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float s0 = cf.k * fmaf(cf.es, ws[k].x, 1.f), s1 = cf.k * fmaf(cf.es, ws[k].y, 1.f);
+            a[k] = make_float2(dy[k].x * __powf(s0, -cf.beta), dy[k].y * __powf(s1, -cf.beta));
+            rt[k] = make_float2(a[k].x * v[k].x * __frcp_rn(s0), a[k].y * v[k].y * __frcp_rn(s1));
+            if (hit == 0u) { a[k] = both(0.f); rt[k] = both(0.f); }
+          }
+        }
+        const uint32_t aw[4] = {pack_bf16x2(a[0].x, a[0].y), pack_bf16x2(a[1].x, a[1].y), pack_bf16x2(a[2].x, a[2].y),
+                                pack_bf16x2(a[3].x, a[3].y)};
+        const uint4 rv = make_uint4(pack_bf16x2(rt[0].x, rt[0].y), pack_bf16x2(rt[1].x, rt[1].y),
+                                    pack_bf16x2(rt[2].x, rt[2].y), pack_bf16x2(rt[3].x, rt[3].y));
+        // dx = a - coef * x * (window sum of rt), ReLU mask, per-channel sums
+        before = __shfl_up_sync(0xffffffffu, rv.w, 1);
+        after = __shfl_down_sync(0xffffffffu, rv.x, 1);
+        if (first_vec) before = 0u;
+        if (last_vec) after = 0u;
+        const float2 u[6] = {unpack2(before), unpack2(rv.x), unpack2(rv.y), unpack2(rv.z), unpack2(rv.w), unpack2(after)};
+        window5(u, ws);
+        const uint32_t xw[4] = {xq[i].x, xq[i].y, xq[i].z, xq[i].w};
+        float2 o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          o[k] = zero_where_le(fma2(mul2(both(-coef), v[k]), ws[k], unpack2(aw[k])), xw[k], lim);
+        if (in[i] && stores) {
+          *reinterpret_cast<uint4*>(dx + px + (r * W + c) * C) =
+              make_uint4(pack_bf16x2(o[0].x, o[0].y), pack_bf16x2(o[1].x, o[1].y), pack_bf16x2(o[2].x, o[2].y),
+                         pack_bf16x2(o[3].x, o[3].y));
+#pragma unroll
+          for (int k = 0; k < 4; ++k) cs[k] = add2(cs[k], o[k]);
+        }
+      }
+    }
+  }
+  if (colsum != nullptr) {
+    // the working lanes of a block hold consecutive vectors, each for all of its steps
+    if (stores) {
+      const int at = (threadIdx.x >> 5) * 30 + lane - 1;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) { cs_sh[2 * k][at] = cs[k].x; cs_sh[2 * k + 1][at] = cs[k].y; }
+    }
+    __syncthreads();
+    const int base = (int)(blockIdx.x * 240u % (unsigned)cv);
+    // several threads a channel where there are few channels, their sums met in the places of the first ones' vectors
+    const int parts = C < 256 ? 256 / C : 1;
+    for (int i = threadIdx.x; i < C * parts; i += blockDim.x) {
+      const int c = i % C, part = i / C;
+      int at = (c >> 3) - base;
+      if (at < 0) at += cv;
+      at += part * cv;
+      const int first = at;
+      float sum = 0.f;
+      for (; at < 240; at += parts * cv) sum += cs_sh[c & 7][at];
+      if (parts == 1) { if (first < 240) atomicAdd(colsum + c, sum); }
+      else if (first < 240) cs_sh[c & 7][first] = sum;
+    }
+    if (parts > 1) {
+      __syncthreads();
+      const int c = threadIdx.x;
+      if (c < C) {
+        int at = (c >> 3) - base;
+        if (at < 0) at += cv;
+        float sum = 0.f;
+        for (int part = 0; part < parts && at < 240; ++part, at += cv) sum += cs_sh[c & 7][at];
+        atomicAdd(colsum + c, sum);
+      }
+    }
+  }
+}
+
 // ---------------- backward, any window ----------------
 // Persistent: CTA i handles row blocks i, i + gridDim, ... (a row block = R input rows of one image).
 // Shared memory: as, rs [R][W][C] bf16, dps [max_oh][OW][C] bf16, args [max_oh][OW][C] u8, cs [C] float.
@@ -709,6 +935,25 @@ int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax
   const bool k3s2 = g->K == 3 && g->stride == 2;
   // the register kernel covers the usual pair (5 channels, 3 x 3 stride 2) up to 512 channels; its item count is 32 bits
   const int cv = g->C / 8;
+  const int q0 = g->pad >> 1, QH = ((g->H - 1 + g->pad) >> 1) - q0 + 1, QW = ((g->W - 1 + g->pad) >> 1) - q0 + 1;
+  const long long vectors = (long long)g->B * QH * QW * cv;
+  // Below some 100 vectors an SM the lanes kernel has more warps at work (captured chains of 16, lanes / quads, us: 13 x 13 x 32
+  // 2.5 / 3.6, 8 x 27 x 27 x 64 3.2 / 3.8, 3 x 33 x 33 x 88 3.7 / 3.8; above, 16 x 27 x 27 x 64 4.0 / 3.8, 64 x 13 x 13 x 40
+  // 4.2 / 3.8, 2 x 55 x 55 x 96 3.9 / 3.8, 64 x 27 x 27 x 104 16.2 / 10.5); the quad kernel counts vectors in 32 bits.
+  if (k3s2 && size == 5 && vectors >= 96LL * geeps_sm_count() && vectors < (1LL << 30)) {
+    // a warp of several steps keeps its channels: then the warps' vectors are a multiple of a pixel's
+    long long warps = (vectors + 29) / 30;
+    const long long cap = (long long)geeps_sm_count() * 16;
+    if (warps > cap) {
+      int a = cv, b = 30;
+      while (b) { const int t = a % b; a = b; b = t; }
+      const int m = cv / a;                                   // 30 m vectors are whole pixels
+      warps = m <= cap ? cap / m * m : m;
+    }
+    geeps_launch_plain(lrn_maxpool_backward_quad_kernel, (int)((warps + 7) / 8), 256, 0, st, (const bf16*)x, (const bf16*)dp,
+                       (const uint8_t*)argmax, (bf16*)dx, *g, cf, coef, relu_mask, colsum, QH, QW, (int)vectors, (int)warps);
+    return (int)cudaGetLastError();
+  }
   if (k3s2 && size == 5 && cv <= 64 && (long long)g->B * g->H * (g->W + 64) < 0x7fffffffLL) {
     const LrnLanes ln = lrn_lanes(cv, (long long)g->B * g->H * g->W);
     const int lp = ln.lp, nv = ln.nv;

@@ -623,3 +623,36 @@ def test_clear_covers_exactly_its_range(off, n):
     L.check(L.lib().geeps_clear_f32(ctypes.c_void_p(buf.data_ptr() + 4 * (4 + off)), ctypes.c_longlong(n), L.stream_ptr()), "clear")
     assert (buf[4 + off:4 + off + n] == 0).all()
     assert (buf[:4 + off] == 2).all() and (buf[4 + off + n:] == 2).all()
+
+
+@pytest.mark.parametrize("B,H,Cc,pad,ldy", [(64, 29, 8, 0, 8), (61, 31, 8, 1, 8), (40, 13, 120, 0, 136), (9, 61, 40, 1, 40),
+                                            (3, 27, 240, 0, 240), (2, 28, 312, 0, 312), (100, 14, 88, 1, 88),
+                                            (260, 27, 32, 0, 32), (24, 55, 296, 0, 296), (36, 15, 520, 0, 520)])
+@pytest.mark.parametrize("alpha", [1e-4, 0.5])
+def test_lrn_maxpool_backward_by_quads_matches_small_batches(B, H, Cc, pad, ldy, alpha):
+    """A batch large enough for the quad kernel (one step a warp and several, ends of rows and images inside a warp,
+    one vector a pixel, vector counts without a common factor with 30) against single images, which the other kernels take:
+    the same bits in the range of the polynomials, and each within two roundings of bf16 beyond it."""
+    torch.manual_seed(B * Cc)
+    size, beta, kk = 5, 0.75, 1.0
+    x = (torch.randn(B, H, H, Cc, device=DEV) * 3).clamp_min(-0.5).to(BF)        # some negative inputs: masked by sign
+    g = F.pool_geom(x.shape, 3, 2, pad, Cc, ldy)
+    assert B * ((H + pad + 1) // 2) ** 2 * Cc // 8 >= 96 * torch.cuda.get_device_properties(0).multi_processor_count
+    arg = torch.randint(0, 9, (B, g.OH, g.OW, Cc), device=DEV, dtype=torch.uint8)
+    dp = torch.randn(B, g.OH, g.OW, ldy, device=DEV).to(BF)
+    dx, cs = torch.empty_like(x), torch.empty(Cc, device=DEV)
+    F.lrn_maxpool_backward(x, dp, arg, dx, g, size, alpha, beta, kk, relu_mask=True, colsum=cs)
+    one = F.pool_geom(x[:1].shape, 3, 2, pad, Cc, ldy)
+    ref, part, total = torch.empty_like(x[:1]), torch.empty(Cc, device=DEV), torch.zeros(Cc, dtype=torch.float64, device=DEV)
+    for b in range(B):
+        F.lrn_maxpool_backward(x[b:b + 1], dp[b:b + 1], arg[b:b + 1], ref, one, size, alpha, beta, kk, relu_mask=True, colsum=part)
+        total += part
+        if alpha < 1e-2:
+            assert torch.equal(dx[b:b + 1], ref), b
+        else:
+            assert (dx[b:b + 1].double() - ref.double()).norm() <= 2.0 ** -8 * ref.double().norm(), b
+    # n additions, each rounded by at most 2^-24 of the sum of magnitudes, with random signs: four deviations; beyond the
+    # polynomials' range the two kernels may also take different paths, 4e-4 of every value apart
+    mag = dx.double().abs().sum((0, 1, 2))
+    bound = (4 * 2.0 ** -24 * (B * H * H) ** 0.5 + (4e-4 if alpha > 1e-2 else 0.0)) * mag
+    assert ((cs.double() - total).abs() <= bound).all()
