@@ -138,7 +138,7 @@ __device__ __forceinline__ void window5(const float2 (&t)[6], float2 (&w)[4]) {
 // a window of 3 or 7 channels), normalised once per element into shared memory ([n_in][W][C] bf16), and pooled from there.
 // K3S2: 3 x 3 windows with stride 2 (window size and stride are then constants of the pooling loops)
 template <int HALF, bool K3S2>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(512, 2)
 lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uint8_t* __restrict__ argmax,
                            const GeepsPoolGeom g, const LrnCoef cf, int RO) {
   geeps_pdl_enter();
@@ -158,36 +158,56 @@ lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uin
     const bf16* xbase = x + ((long long)b * g.H + ih_base + r_lo) * row_elems;
     bf16* ybase = ys + (size_t)r_lo * row_elems;
     const int nrows = r_hi - r_lo;
-    for (ItemWalk it(tid, nt, W, cv); it.r < nrows; it.next(W, cv)) {
-      const int c = it.cvi * 8;
-      const int pix = it.r * row_elems + it.w * C;          // offsets inside a block of a few rows: 32 bits
-      if constexpr (HALF == 2) {
-        // pairs of channels: half the fp32 instructions, and a halo of one word per side instead of two
-        const bf16* px = xbase + pix + c;
-        const uint32_t before = c > 0 ? *reinterpret_cast<const uint32_t*>(px - 2) : 0u;
-        const uint4 xv = *reinterpret_cast<const uint4*>(px);
-        const uint32_t after = c + 8 < C ? *reinterpret_cast<const uint32_t*>(px + 8) : 0u;
-        const float2 v[6] = {unpack2(before), unpack2(xv.x), unpack2(xv.y), unpack2(xv.z), unpack2(xv.w), unpack2(after)};
-        float2 t[6], ws[4], o[4];
+    if constexpr (HALF == 2) {
+      // Pairs of channels: half the fp32 instructions, and a halo of one word per side instead of two.  Three items are
+      // loaded before the first is computed: with one, half of the time went on waiting for it (256 x 55 x 55 x 96: 96 us;
+      // two 84, three 82, four spill).
+      constexpr int U = 3;
+      for (ItemWalk it(tid, nt, W, cv); it.r < nrows;) {
+        uint32_t before[U], after[U];
+        uint4 xv[U];
+        int at[U];                                            // offsets inside a block of a few rows: 32 bits
 #pragma unroll
-        for (int k = 0; k < 6; ++k) t[k] = mul2(v[k], v[k]);
-        window5(t, ws);
-        const float top = fmaxf(fmaxf(fmaxf(ws[0].x, ws[0].y), fmaxf(ws[1].x, ws[1].y)),
-                                fmaxf(fmaxf(ws[2].x, ws[2].y), fmaxf(ws[3].x, ws[3].y)));
-        if (top <= cf.w_max) {
+        for (int u = 0; u < U; ++u) {
+          at[u] = -1;
+          if (it.r < nrows) {
+            const int c = it.cvi * 8;
+            at[u] = it.r * row_elems + it.w * C + c;
+            const bf16* px = xbase + at[u];
+            before[u] = c > 0 ? *reinterpret_cast<const uint32_t*>(px - 2) : 0u;
+            xv[u] = *reinterpret_cast<const uint4*>(px);
+            after[u] = c + 8 < C ? *reinterpret_cast<const uint32_t*>(px + 8) : 0u;
+            it.next(W, cv);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (at[u] < 0) break;
+          const float2 v[6] = {unpack2(before[u]), unpack2(xv[u].x), unpack2(xv[u].y), unpack2(xv[u].z), unpack2(xv[u].w),
+                               unpack2(after[u])};
+          float2 t[6], ws[4], o[4];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) t[k] = mul2(v[k], v[k]);
+          window5(t, ws);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             o[k] = mul2(v[k + 1], fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.p3), both(cf.p2)), both(cf.p1)), both(cf.p0)));
-        } else {
+          // the sum of all twelve squares bounds every window's
+          if (!((ws[0].x + ws[2].y) + (t[5].x + t[5].y) <= cf.w_max)) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            o[k] = make_float2(v[k + 1].x * __powf(cf.k * fmaf(cf.es, ws[k].x, 1.f), -cf.beta),
-                               v[k + 1].y * __powf(cf.k * fmaf(cf.es, ws[k].y, 1.f), -cf.beta));
+            for (int k = 0; k < 4; ++k)
+              o[k] = make_float2(v[k + 1].x * __powf(cf.k * fmaf(cf.es, ws[k].x, 1.f), -cf.beta),
+                                 v[k + 1].y * __powf(cf.k * fmaf(cf.es, ws[k].y, 1.f), -cf.beta));
+          }
+          *reinterpret_cast<uint4*>(ybase + at[u]) =
+              make_uint4(pack_bf16x2(o[0].x, o[0].y), pack_bf16x2(o[1].x, o[1].y), pack_bf16x2(o[2].x, o[2].y),
+                         pack_bf16x2(o[3].x, o[3].y));
         }
-        *reinterpret_cast<uint4*>(ybase + pix + c) =
-            make_uint4(pack_bf16x2(o[0].x, o[0].y), pack_bf16x2(o[1].x, o[1].y), pack_bf16x2(o[2].x, o[2].y),
-                       pack_bf16x2(o[3].x, o[3].y));
-      } else {
+      }
+    } else {
+      for (ItemWalk it(tid, nt, W, cv); it.r < nrows; it.next(W, cv)) {
+        const int c = it.cvi * 8;
+        const int pix = it.r * row_elems + it.w * C;
         float v[16], t[16], ws[8], o[8];
         load16(xbase + pix, c, C, v);
 #pragma unroll
