@@ -656,3 +656,30 @@ def test_lrn_maxpool_backward_by_quads_matches_small_batches(B, H, Cc, pad, ldy,
     mag = dx.double().abs().sum((0, 1, 2))
     bound = (4 * 2.0 ** -24 * (B * H * H) ** 0.5 + (4e-4 if alpha > 1e-2 else 0.0)) * mag
     assert ((cs.double() - total).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("B,H,W,Cc,pad,ldx,ldy", [(33, 15, 14, 96, 1, 96, 112), (40, 8, 9, 256, 0, 272, 256), (65, 5, 7, 304, 2, 304, 304),
+                                                  (30, 3, 3, 2312, 1, 2312, 2320), (2, 1, 9, 8, 1, 8, 8), (3, 4, 5, 16, 2, 24, 32)])
+def test_average_pooling_3x3_stride_1(B, H, W, Cc, pad, ldx, ldy):
+    """Four rows a thread and one, rows that are no multiple of four, images of one row, pitched input and output, and the
+    backward pass added to what is there."""
+    torch.manual_seed(H * W + Cc)
+    x = torch.randn(B, H, W, ldx, device=DEV).to(BF)
+    g = F.pool_geom((B, H, W, Cc), 3, 1, pad, ldx, ldy, ceil_mode=False)
+    y = torch.full((B, g.OH, g.OW, ldy), 7.0, dtype=BF, device=DEV)
+    F.avgpool_forward(x, y, g)
+    dy = torch.randn_like(y)
+    xr = x[..., :Cc].double().permute(0, 3, 1, 2).contiguous().requires_grad_(True)
+    ref = TF.avg_pool2d(TF.pad(xr, (pad, pad, pad, pad)), 3, 1)
+    ref.backward(dy[..., :Cc].double().permute(0, 3, 1, 2).contiguous())
+    want, grad = ref.detach().permute(0, 2, 3, 1), xr.grad.permute(0, 2, 3, 1)
+    # one rounding to bf16 of fp32 sums of at most ten terms
+    assert torch.allclose(y[..., :Cc].double(), want, atol=1e-5, rtol=2.0 ** -8)
+    assert (y[..., Cc:] == 7).all()
+    dx = torch.randn(B, H, W, ldx, device=DEV).to(BF)
+    old = dx.clone()
+    for accumulate in (1, 0):
+        dx.copy_(old)
+        L.check(L.lib().geeps_avgpool_backward(L.ptr(dy), L.ptr(dx), ctypes.byref(g), accumulate, L.stream_ptr()), "avgpool_backward")
+        assert torch.allclose(dx[..., :Cc].double(), grad + (old[..., :Cc].double() if accumulate else 0.0), atol=1e-5, rtol=2.0 ** -8)
+        assert torch.equal(dx[..., Cc:], old[..., Cc:])
