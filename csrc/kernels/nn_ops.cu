@@ -741,7 +741,10 @@ __device__ __forceinline__ uint32_t mix32(uint64_t z) {
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return (uint32_t)((z ^ (z >> 31)) >> 32);
 }
-// y = x * keep(seed, idx) / (1 - p); the same call with dy as input gives dx.
+// y = x * keep(seed, idx) / (1 - p); the same call with dy as input gives dx.  VEC: eight values a thread and step (n a
+// multiple of 8, both pointers on 16 bytes): fewer, wider accesses and an eighth of the blocks, which also have to find room
+// beside a parameter push that holds half of every SM.  256 x 4096 5.4 -> 2.9 us, 6.5 M values 12.8 -> 9.5.
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 dropout_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long long n, float p, unsigned long long seed,
                const int* __restrict__ step_ref) {
@@ -749,9 +752,20 @@ dropout_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long long n, fl
   if (step_ref != nullptr) seed += (unsigned long long)(long long)*step_ref;
   const float inv = 1.f / (1.f - p);
   const uint32_t thresh = (uint32_t)(p * 4294967296.0);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    y[i] = mix32(seed * 0x100000001B3ull + (uint64_t)i) >= thresh ? __float2bfloat16(bf(x[i]) * inv) : __float2bfloat16(0.f);
+  auto one = [&](bf16 v, long long i) {
+    return mix32(seed * 0x100000001B3ull + (uint64_t)i) >= thresh ? __float2bfloat16(bf(v) * inv) : __float2bfloat16(0.f);
+  };
+  const long long stride = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (VEC) {
+    for (long long i = first * 8; i < n; i += stride * 8) {
+      Bf8 v = ld8(x + i);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v.v[e] = one(v.v[e], i + e);
+      st8(y + i, v);
+    }
+  } else {
+    for (long long i = first; i < n; i += stride) y[i] = one(x[i], i);
+  }
 }
 
 // ---------------- LRN across channels ----------------
@@ -2069,12 +2083,13 @@ int geeps_add_bf16_2d_n(void* dst, const void* s0, const void* s1, const void* s
 }
 
 int geeps_dropout(const void* x, void* y, long long n, float p, unsigned long long seed, void* stream) {
-  geeps_launch_plain(dropout_kernel, grid_1d(n), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, n, p, seed, nullptr);
-  return CK();
+  return geeps_dropout_ref(x, y, n, p, seed, nullptr, stream);
 }
 int geeps_dropout_ref(const void* x, void* y, long long n, float p, unsigned long long seed, const int* step_ref,
                       void* stream) {
-  geeps_launch_plain(dropout_kernel, grid_1d(n), 256, 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y, n, p, seed, step_ref);
+  const bool vec = n % 8 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
+  geeps_launch_plain(vec ? dropout_kernel<true> : dropout_kernel<false>, grid_1d(vec ? n / 8 : n), 256, 0, (cudaStream_t)stream,
+                     (const bf16*)x, (bf16*)y, n, p, seed, step_ref);
   return CK();
 }
 
