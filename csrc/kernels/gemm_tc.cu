@@ -535,7 +535,7 @@ int round_up(long long v, int m) { return (int)((v + m - 1) / m * m); }
 // alone took 256 x 4096, K = 9216 from 38.9 to 32.8 us, L2 flushed), but it ranks the widths as they are now (64, 128, 192, 256; us
 // in a captured chain): 256 x 4096, K = 9216 27.0, 35.2, 48.9, 64.4; 256 x 9216, K = 4096 29.5, 20.1, 25.4, 30.0; 256 x 4096,
 // K = 4096 13.9, 13.7, 17.5, 22.6; 256 x 1000, K = 4096 13.3, 13.5, 17.5, 22.5; 100 x 512, K = 2048 7.9, 8.4, 10.6, 13.0.
-// The sizes of clusters it ranks less well (see plan_gemm).
+// Clusters: see plan_gemm.
 struct TileChoice { int bn, cluster; };
 TileChoice choose_tiles(const GeepsGemmParams* p, int unit, int kt, int sms, bool cluster_ok) {
   constexpr double kTileOver = 150e3, kClusterOver = 150e3;
@@ -548,9 +548,11 @@ TileChoice choose_tiles(const GeepsGemmParams* p, int unit, int kt, int sms, boo
     for (int cs = 1; cs <= (cluster_ok ? 8 : 1); cs *= 2) {
       const int per = (kt + cs - 1) / cs;
       if (cs > 1 && (per < 4 || (long long)(cs - 1) * per >= kt)) continue;    // every slice needs k tiles
-      const long long slots = cs <= 2 ? sms : sms / 18 * 16;                   // whole clusters per GPC
+      // SMs that whole clusters find in GPCs of different sizes: 33 clusters of four and 15 of eight are resident on 148 SMs
+      const long long slots = cs <= 2 ? sms : cs == 4 ? sms * 8 / 9 : sms * 5 / 6 / 8 * 8;
       const long long rounds = (tiles * cs + slots - 1) / slots;
-      double cost = rounds * (per * (a_rows + bn) * 128.0 + kTileOver);
+      // a k step of a slice has its price even for a few rows (4 x 1024, K = 21841: 21.5 us on 64 x 4, 16 on 128 x 8)
+      double cost = rounds * (per * ((cs > 1 && a_rows < 32 ? 32.0 : a_rows) + bn) * 128.0 + kTileOver);
       if (cs > 1) cost += rounds * (kClusterOver + a_rows * bn * 8.0);
       if (cost < best_cost * 0.98) { best_cost = cost; best = {bn, cs}; }
     }
@@ -593,8 +595,9 @@ GemmPlan plan_gemm(const GeepsGemmParams* p, int sms) {
       // a bf16 slab is 64 columns wide (see below): several tiles have widths that are multiples of it
       const int step = tma_c && !p->out_fp32 ? 64 : unit;
       // Clusters only for K above 8128 over at most sms / 8 narrow tiles: the data gradient of a wide classifier, 32 x 1024,
-      // K = 21841, 16 tiles (tile width x cluster, us in a captured chain): 70 without a cluster, 26.6 on 64 x 8, which the
-      // cost picks (22.1 on 64 x 4, 16.4 on 128 x 8).  The line is drawn by the order of the
+      // K = 21841, 16 tiles (tile width x cluster, us in a captured chain): 70 without a cluster, 27.3 on 64 x 8 (16 clusters,
+      // of which 15 are resident at once: picked before the cost knew), 22.1 on 64 x 4, 17.0 on 128 x 8, which the cost picks;
+      // K = 12000 19.5 on 64 x 8, 12.5, K = 8200 16.7, 11.0.  The line is drawn by the order of the
       // sums, not by speed: a cluster adds its K slices in another order than one running sum, and in a deep network with
       // near-ties in its pooling windows that changes which element a later step's maximum picks, so ordinary layers
       // keep one sum.  What that leaves: 256 x 4096, K = 9216: 27.0 on 64 x 1, 25.1 on 128 x 2; 32 rows: 25.6 on 64 x 1, 13.9
