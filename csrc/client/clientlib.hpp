@@ -137,8 +137,8 @@ struct Fabric {
   void* timeline_origin = nullptr;
   std::vector<TimelineRec> timeline_recs;
   void* push_done_event = nullptr;
-  // Device time of the latest pushes: a ring of event pairs around the reduce + apply + publish kernel on the comm
-  // stream, summed by GetStats() over the pairs that have completed (device_push_ms / device_push_gb_per_s).
+  // Device time of the latest pushes of every eighth clock: a ring of event pairs around the reduce + apply + publish
+  // kernel on the comm stream, summed by GetStats() over the pairs that have completed (device_push_ms / device_push_gb_per_s).
   struct PushTiming { void* begin = nullptr; void* end = nullptr; size_t table_bytes = 0; bool armed = false; };
   std::vector<PushTiming> push_timing;
   size_t push_timing_next = 0;
@@ -149,7 +149,8 @@ struct Fabric {
   void* joined_stream = nullptr;          // device-clock mode: the stream that the comm lanes last joined ...
   bool joined = false;                    // ... in a host-run iteration that no replay has followed
   void* join_event = nullptr;             // device-clock mode: comm lanes -> application stream at the end of a clock
-  int* host_status = nullptr;             // pinned mirror of the device status block
+  int* host_status = nullptr;             // pinned mirror of the device status block ...
+  bool status_mirrored = false;           // ... which a push enqueued since the last look keeps up to date
 };
 
 struct LocalStore {

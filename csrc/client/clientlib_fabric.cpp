@@ -377,7 +377,8 @@ void ClientLib::fabric_push(iter_t clock, uint table_id, bool is_init, void* str
   // device time of the push kernel itself (the wait for the other workers is not part of it)
   Fabric::PushTiming* pt = nullptr;
   const bool capturing = stream_capturing(cs);
-  if (!is_init && !capturing) {   // an event recorded under capture cannot be queried
+  // every eighth clock; an event recorded under capture cannot be queried
+  if (!is_init && !capturing && clock % 8 == 0) {
     if (fabric_.push_timing.empty()) fabric_.push_timing.resize(kPushTimingRing);
     pt = &fabric_.push_timing[fabric_.push_timing_next++ % kPushTimingRing];
     if (!pt->begin) {
@@ -421,6 +422,7 @@ void ClientLib::fabric_push(iter_t clock, uint table_id, bool is_init, void* str
   p.global_clock = reinterpret_cast<int*>(fabric_.base + ta.flags_off + kGlobalClockOff);
   p.cta_counter = reinterpret_cast<int*>(fabric_.base + ta.flags_off + kCtaCounterOff);
   p.status = status;
+  p.status_mirror = fabric_.host_status;
   p.n_owned = (long long)own.count;
   p.row_start = (long long)own.start;
   p.row_stride = (long long)own.stride;
@@ -441,6 +443,7 @@ void ClientLib::fabric_push(iter_t clock, uint table_id, bool is_init, void* str
                         ? (long long)config_.table_fp32_from_row[table_id] : 0;
   if (timed) cudaEventRecord((cudaEvent_t)rec.arrived, (cudaStream_t)cs);
   geeps_ps_push_apply(&p, fabric_.push_ctas, cs);
+  fabric_.status_mirrored = true;
   if (pt) cudaEventRecord((cudaEvent_t)pt->end, (cudaStream_t)cs);
   if (fabric_.applied.size() <= table_id) fabric_.applied.resize(table_id + 1);
   Fabric::Applied& ap = fabric_.applied[table_id];
@@ -614,8 +617,8 @@ void ClientLib::fabric_pull_rows(uint table_id, RowData* dst, size_t row_from, v
 }
 
 // Errors recorded by kernels (expired waits, failed bounds checks) surface here.  The device block
-// is mirrored into pinned memory asynchronously, so a problem is seen at most one clock late
-// without ever synchronising the streams.
+// is mirrored into pinned memory asynchronously - by the clock's pushes, or by a copy where it had none -, so a
+// problem is seen at most one clock late without ever synchronising the streams.
 bool ClientLib::fabric_check_status(bool sync) {
   if (!fabric_.active) return true;
   bool ok = true;
@@ -630,8 +633,10 @@ bool ClientLib::fabric_check_status(bool sync) {
                   std::to_string(fabric_.host_status[1]) + ", detail " + std::to_string(fabric_.host_status[2]) +
                   ", seen " + std::to_string(fabric_.host_status[3]) + ")");
   }
-  cudaMemcpyAsync(fabric_.host_status, fabric_.base + fabric_.status_off, 4 * sizeof(int), cudaMemcpyDeviceToHost,
-                  (cudaStream_t)fabric_.comm_stream);
+  if (!fabric_.status_mirrored)
+    cudaMemcpyAsync(fabric_.host_status, fabric_.base + fabric_.status_off, 4 * sizeof(int), cudaMemcpyDeviceToHost,
+                    (cudaStream_t)fabric_.comm_stream);
+  fabric_.status_mirrored = false;
   return ok;
 }
 

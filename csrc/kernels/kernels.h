@@ -60,6 +60,7 @@ typedef struct GeepsPushApplyParams {
   const float* upd_mc;
   float* cache_mc;
   void* cache16_mc;
+  int* status_mirror;                  // NULL, or 4 ints of pinned host memory that receive a non-zero status block
 } GeepsPushApplyParams;
 int geeps_ps_push_apply(const GeepsPushApplyParams* p, int max_ctas, void* stream);
 

@@ -176,6 +176,17 @@ push_apply_kernel(const GeepsPushApplyParams p) {
         for (int q = 0; q < p.n_ranks; ++q)
           if (p.data_age[q] != nullptr) st_release_sys(p.data_age[q] + p.rank, clock_stamp);
     }
+    // what the host looks at without synchronising: written only when something went wrong (a copy of the block behind
+    // every clock is a driver call and a turn of the copy engine)
+    if (p.status_mirror != nullptr && p.status != nullptr) {
+      const int code = ld_relaxed_sys(p.status);
+      if (code != 0) {
+        volatile int* m = p.status_mirror;
+        for (int k = 1; k < 4; ++k) m[k] = ld_relaxed_sys(p.status + k);
+        __threadfence_system();
+        m[0] = code;
+      }
+    }
   }
 }
 

@@ -64,6 +64,7 @@ class PushApplyParams(C.Structure):
         ("lr", C.c_float), ("momentum_coef", C.c_float), ("weight_decay", C.c_float),
         ("grad_scale", C.c_float), ("fp32_from_row", C.c_longlong), ("clock_ref", C.c_void_p),
         ("master16", C.c_void_p), ("upd_mc", C.c_void_p), ("cache_mc", C.c_void_p), ("cache16_mc", C.c_void_p),
+        ("status_mirror", C.c_void_p),
     ]
 
 
@@ -142,9 +143,16 @@ def require_cuda() -> None:
         raise RuntimeError("geeps_b200 kernels need a CUDA device (sm_100a); none is visible")
 
 
+def current_stream_handle() -> int:
+    """The current device's current stream as a CUDA handle, without the stream object that torch.cuda.current_stream()
+    builds for every call."""
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def stream_ptr(stream=None) -> C.c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    return C.c_void_p(current_stream_handle() if stream is None else stream.cuda_stream)
 
 
 def ptr(t) -> C.c_void_p:

@@ -198,9 +198,8 @@ class GeePs:
     def _stream(self, stream):
         if not self._cuda:
             return C.c_void_p(0)
-        s = stream if stream is not None else torch.cuda.current_stream()
         # handle 0 means "the runtime's own stream" to the C API; CUDA's legacy default stream is 0x1
-        return C.c_void_p(s.cuda_stream or 1)
+        return C.c_void_p((_L.current_stream_handle() if stream is None else stream.cuda_stream) or 1)
 
     def _wrap(self, ptr: int, nrows: int, dtype=torch.float32) -> torch.Tensor:
         if not ptr:

@@ -254,3 +254,26 @@ def test_device_clock_iterations_on_alternating_streams():
     for graph in graphs.values():
         lib().geeps_graph_destroy(graph)
     g.close()
+
+
+@pytest.mark.parametrize("rows", [1, 5000])
+def test_push_mirrors_a_status_block_that_is_not_zero(rows):
+    """The pinned words that the host looks at without synchronising: untouched by a clean push, a copy of the block
+    behind one that finds it set (a failed bounds check of this push included)."""
+    dev = torch.device("cuda:0")
+    upd, master, cache = (torch.ones(rows, 128, device=dev) for _ in range(3))
+    words = torch.zeros(64, dtype=torch.int32, device=dev)
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    mirror = torch.full((4,), -1, dtype=torch.int32).pin_memory()
+    p = L.PushApplyParams()
+    p.upd[0], p.cache[0], p.master = upd.data_ptr(), cache.data_ptr(), master.data_ptr()
+    p.global_clock, p.cta_counter, p.status, p.status_mirror = words.data_ptr(), words.data_ptr() + 4, status.data_ptr(), mirror.data_ptr()
+    p.n_owned, p.row_start, p.row_stride, p.total_rows = rows, 0, 1, rows
+    p.wait_budget_ns, p.n_ranks, p.publish, p.clock_stamp = 10 ** 9, 1, 1, 1
+    L.check(lib().geeps_ps_push_apply(C.byref(p), 0, stream_ptr()), "push_apply")
+    torch.cuda.synchronize()
+    assert mirror.tolist() == [-1] * 4 and (master == 2).all()
+    p.row_start = 1                              # the last row lies behind the table: refused by the kernel's check
+    L.check(lib().geeps_ps_push_apply(C.byref(p), 0, stream_ptr()), "push_apply")
+    torch.cuda.synchronize()
+    assert mirror.tolist() == status.tolist() and mirror[0].item() == 2 and mirror[2].item() == rows - 1
