@@ -1077,25 +1077,24 @@ __device__ __forceinline__ void xform_image(const XformDev& t, long long b, int&
 // the one to three aligned 32-bit words that cover them, converts them in registers and builds three 16-byte pieces of
 // the pixel; a warp's 16 pixels meet in shared memory and leave as one contiguous run.  256 images of 8 bits, cropped to
 // 227 x 227: one element per load and 2-byte shared-memory stores, 32 pixels of one output row per block, 59 us; this
-// 34 us, of which the 106 MB written are 16.  Bound by instruction issue.
+// 30 us, of which the 106 MB written are 16.
 // An 8-bit source may start and end inside a word (a batch slice, odd image sizes): the lanes whose words could reach past
 // it fetch by elements, every other lane by words (by elements throughout: 423 us).
 struct U8Quads {
+  static constexpr bool kBytes = true;
   XformDev t;
   const uint8_t* end;       // one past the source
   int h_off, w_off, mirror;
   __device__ __forceinline__ void image(long long b) { xform_image(t, b, h_off, w_off, mirror); }
   __device__ __forceinline__ int height() const { return t.H; }
+  __device__ __forceinline__ int pitch() const { return t.Win; }
+  __device__ __forceinline__ long long plane() const { return (long long)t.Hin * t.Win; }
   __device__ __forceinline__ int width() const { return t.W; }
-  __device__ __forceinline__ float value(uint32_t byte, int c) const {
-    return (__uint_as_float(0x4b000000u | byte) - 8388608.f - t.mean[c]) * t.scale;      // 2^23 + byte: exact
-  }
-  __device__ __forceinline__ uint32_t bits(float v) const { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(v)); }
   __device__ __forceinline__ const uint8_t* row(long long b, int c, int h) const {
     return t.x + ((b * 3 + c) * t.Hin + (h + h_off)) * (long long)t.Win + w_off;
   }
-  __device__ __forceinline__ uint32_t one(long long b, int c, int h, int w) const {
-    return bits(value(__ldg(row(b, c, h) + (mirror ? t.W - 1 - w : w)), c));
+  __device__ __forceinline__ uint32_t byte(long long b, int c, int h, int w) const {
+    return __ldg(row(b, c, h) + (mirror ? t.W - 1 - w : w));
   }
   __device__ __forceinline__ const uint8_t* quad_at(long long b, int c, int h, int w) const {
     return row(b, c, h) + (mirror ? t.W - 4 - w : w);
@@ -1105,19 +1104,48 @@ struct U8Quads {
     const uint8_t* first = quad_at(b, 0, h, w);
     return first - ((uintptr_t)first & 3) >= t.x && end - quad_at(b, 2, h1, w) >= 8;
   }
-  // columns w .. w + 3 as two packed words (the second word is read only when it holds one of the columns)
-  __device__ __forceinline__ uint2 quad(long long b, int c, int h, int w) const {
-    const uint8_t* p = quad_at(b, c, h, w);
+  // columns w .. w + 3, a byte each (the second word is read only when it holds one of the columns)
+  __device__ __forceinline__ uint32_t quad(const uint8_t* p) const {
     const uint32_t sh = (uint32_t)((uintptr_t)p & 3) * 8;
     const uint32_t* q = reinterpret_cast<const uint32_t*>((uintptr_t)p & ~(uintptr_t)3);
     const uint32_t lo = __ldg(q), hi = sh ? __ldg(q + 1) : 0u;
-    uint32_t v = __funnelshift_r(lo, hi, sh);
-    if (mirror) v = __byte_perm(v, 0, 0x0123);
-    return make_uint2(pack_bf16x2(value(v & 255u, c), value((v >> 8) & 255u, c)),
-                      pack_bf16x2(value((v >> 16) & 255u, c), value(v >> 24, c)));
+    const uint32_t v = __funnelshift_r(lo, hi, sh);
+    return mirror ? __byte_perm(v, 0, 0x0123) : v;
+  }
+  // (byte - mean) * scale of byte i of u and byte j of v, packed; 2^23 + byte is exact; m: minus the two colours' means
+  __device__ __forceinline__ uint32_t two(uint32_t u, int i, uint32_t v, int j, float2 m) const {
+    const float2 f = make_float2(__uint_as_float(__byte_perm(u, 0x4b000000u, 0x7650u | (uint32_t)i)),
+                                 __uint_as_float(__byte_perm(v, 0x4b000000u, 0x7650u | (uint32_t)j)));
+    const float2 base = make_float2(-8388608.f, -8388608.f), k = make_float2(t.scale, t.scale);
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;\n\tadd.rn.f32x2 %0, %0, %3;\n\tmul.rn.f32x2 %0, %0, %4;"
+        : "=&l"(r)
+        : "l"(reinterpret_cast<const unsigned long long&>(f)), "l"(reinterpret_cast<const unsigned long long&>(base)),
+          "l"(reinterpret_cast<const unsigned long long&>(m)), "l"(reinterpret_cast<const unsigned long long&>(k)));
+    const float2 o = reinterpret_cast<float2&>(r);
+    return pack_bf16x2(o.x, o.y);
+  }
+  // the twelve values of a row, column-major, colour fastest; columns from n on are zero (n >= 4: none)
+  __device__ __forceinline__ void row12(const uint32_t (&v)[3], int n, uint32_t* o) const {
+    const float2 m01 = make_float2(-t.mean[0], -t.mean[1]), m20 = make_float2(-t.mean[2], -t.mean[0]),
+                 m12 = make_float2(-t.mean[1], -t.mean[2]);
+#pragma unroll
+    for (int k = 0; k < 4; k += 2) {
+      o[3 * (k / 2)] = two(v[0], k, v[1], k, m01);
+      o[3 * (k / 2) + 1] = two(v[2], k, v[0], k + 1, m20);
+      o[3 * (k / 2) + 2] = two(v[1], k + 1, v[2], k + 1, m12);
+    }
+    if (n < 4) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        const int first = 2 * i / 3, second = (2 * i + 1) / 3;       // columns of the word's halves
+        if (second >= n) o[i] &= first >= n ? 0u : 0xffffu;
+      }
+    }
   }
 };
 struct Bf16Quads {
+  static constexpr bool kBytes = false;
   const bf16* x;
   int H, W;
   __device__ __forceinline__ void image(long long) {}
@@ -1151,48 +1179,78 @@ s2d43_quad_kernel(Src src, bf16* __restrict__ y, unsigned npix, int Hs, int Ws, 
     const unsigned row = pix / (unsigned)Ws, b = row / (unsigned)Hs;
     const int w = (int)(pix - row * Ws) * 4, h0 = (int)(row - b * Hs) * 4 + half * 2;
     src.image(b);
-    unsigned long long q[2][3];          // four columns of 16 bits
     const int last = src.height() - 1, wq = min(w, src.width() - 4);
     // All fetches of a lane are in flight together, then masked.  (A branch per colour that fetched the one to three
     // columns of a ragged right edge waited for each: 256 images 45 us, 35 us without; one image 4.9 and 2.5 us.)
-    if (wq >= 0 && src.inside(b, min(h0, last), min(h0 + 1, last), wq)) {
-      const int shift = (w - wq) * 16;   // past the right edge: the last four columns, shifted
+    const bool words = wq >= 0 && src.inside(b, min(h0, last), min(h0 + 1, last), wq);
+    if constexpr (Src::kBytes) {
+      // bytes stay bytes until they are packed in the output's order (converted a colour at a time and interleaved as
+      // 16-bit values: 256 images 33.8 us, 29.8 now, of which the 157 MB in and out are 24)
+      const int shift = (w - wq) * 8;    // past the right edge: the last four columns, shifted
+      uint32_t v[2][3];
+      if (words) {
+        const uint8_t* at = src.quad_at(b, 0, min(h0, last), wq);
+        const long long plane = src.plane(), down = h0 < last ? src.pitch() : 0;
 #pragma unroll
-      for (int d = 0; d < 2; ++d)
+        for (int d = 0; d < 2; ++d)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const uint2 v = src.quad(b, c, min(h0 + d, last), wq);
-          q[d][c] = shift < 64 ? ((unsigned long long)v.y << 32 | v.x) >> shift : 0ull;
-        }
-    } else {
-      const int n = src.width() - w;
-      const unsigned long long keep = n >= 4 ? ~0ull : (n > 0 ? (1ull << (16 * n)) - 1 : 0ull);
+          for (int c = 0; c < 3; ++c) {
+            v[d][c] = src.quad(at + (c * plane + d * down));
+            v[d][c] = shift < 32 ? v[d][c] >> shift : 0u;
+          }
+      } else {
 #pragma unroll
-      for (int d = 0; d < 2; ++d)
+        for (int d = 0; d < 2; ++d)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          unsigned long long v = 0;
+          for (int c = 0; c < 3; ++c) {
+            v[d][c] = 0u;
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            v |= (unsigned long long)src.one(b, c, min(h0 + d, last), min(w + k, src.width() - 1)) << (16 * k);
-          q[d][c] = v & keep;
-        }
-    }
-    // interleave: column-major, colour fastest
-#pragma unroll
-    for (int d = 0; d < 2; ++d) {
-      uint32_t lo[3], hi[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        lo[c] = h0 + d <= last ? (uint32_t)q[d][c] : 0u;
-        hi[c] = h0 + d <= last ? (uint32_t)(q[d][c] >> 32) : 0u;
+            for (int k = 0; k < 4; ++k) v[d][c] |= src.byte(b, c, min(h0 + d, last), min(w + k, src.width() - 1)) << (8 * k);
+          }
       }
-      o[6 * d + 0] = __byte_perm(lo[0], lo[1], 0x5410);
-      o[6 * d + 1] = __byte_perm(lo[2], lo[0], 0x7610);
-      o[6 * d + 2] = __byte_perm(lo[1], lo[2], 0x7632);
-      o[6 * d + 3] = __byte_perm(hi[0], hi[1], 0x5410);
-      o[6 * d + 4] = __byte_perm(hi[2], hi[0], 0x7610);
-      o[6 * d + 5] = __byte_perm(hi[1], hi[2], 0x7632);
+#pragma unroll
+      for (int d = 0; d < 2; ++d) src.row12(v[d], h0 + d <= last ? src.width() - w : 0, o + 6 * d);
+    } else {
+      unsigned long long q[2][3];          // four columns of 16 bits
+      if (words) {
+        const int shift = (w - wq) * 16;
+#pragma unroll
+        for (int d = 0; d < 2; ++d)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const uint2 v = src.quad(b, c, min(h0 + d, last), wq);
+            q[d][c] = shift < 64 ? ((unsigned long long)v.y << 32 | v.x) >> shift : 0ull;
+          }
+      } else {
+        const int n = src.width() - w;
+        const unsigned long long keep = n >= 4 ? ~0ull : (n > 0 ? (1ull << (16 * n)) - 1 : 0ull);
+#pragma unroll
+        for (int d = 0; d < 2; ++d)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            unsigned long long v = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              v |= (unsigned long long)src.one(b, c, min(h0 + d, last), min(w + k, src.width() - 1)) << (16 * k);
+            q[d][c] = v & keep;
+          }
+      }
+      // interleave: column-major, colour fastest
+#pragma unroll
+      for (int d = 0; d < 2; ++d) {
+        uint32_t lo[3], hi[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          lo[c] = h0 + d <= last ? (uint32_t)q[d][c] : 0u;
+          hi[c] = h0 + d <= last ? (uint32_t)(q[d][c] >> 32) : 0u;
+        }
+        o[6 * d + 0] = __byte_perm(lo[0], lo[1], 0x5410);
+        o[6 * d + 1] = __byte_perm(lo[2], lo[0], 0x7610);
+        o[6 * d + 2] = __byte_perm(lo[1], lo[2], 0x7632);
+        o[6 * d + 3] = __byte_perm(hi[0], hi[1], 0x5410);
+        o[6 * d + 4] = __byte_perm(hi[2], hi[0], 0x7610);
+        o[6 * d + 5] = __byte_perm(hi[1], hi[2], 0x7632);
+      }
     }
   }
   // pieces of a pixel XOR-ed with the pixel number: the 16-byte stores spread over the banks
