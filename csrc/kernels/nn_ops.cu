@@ -267,6 +267,17 @@ __device__ __forceinline__ void slot_sums(const SlotMap& m, const float (&a0)[8]
   }
 }
 
+// The pixels p0, p0 + step, ... below P in batches whose loads are in flight together: U at a time, and what is left over in
+// batches of halves of it (a wait each, where single pixels would wait U - 1 times).  batch(count, first pixel)
+template <int N> struct Count { static constexpr int value = N; };
+template <int U, typename Fn>
+__device__ __forceinline__ void pixel_batches(long long p, long long step, long long P, Fn batch) {
+  for (; p + (U - 1) * step < P; p += U * step) batch(Count<U>(), p);
+  if constexpr (U > 4) if (p + 3 * step < P) { batch(Count<4>(), p); p += 4 * step; }
+  if constexpr (U > 2) if (p + step < P) { batch(Count<2>(), p); p += 2 * step; }
+  if (U > 1 && p < P) batch(Count<1>(), p);
+}
+
 // Per-channel constants of a block's slots meet in shared memory ([n][8 * slots]): computed or loaded once per block with
 // coalesced reads, then eight consecutive ones per thread.  Read from global memory by every thread (32 bytes apart per
 // lane) they were 39 of the 52 us of a 32 x 56 x 56 x 192 normalisation.
@@ -326,11 +337,10 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
         for (int e = 0; e < 8; ++e) { const float f = bf(xv.v[e]); a0[e] += f; if (MODE == 0) a1[e] += f * f; }
       }
     };
-    // pixels whose loads are in flight together; two where there are three tensors to load: four took 153 registers, one
-    // block per SM (BatchNorm backward of 100352 x 192 by its output 73 us, 56 now)
-    constexpr int U = MODE == 1 ? 2 : 4;
-    long long p = m.p0;
-    for (; p + (U - 1) * m.step < P; p += U * m.step) {
+    // two pixels where there are three tensors to load: four took 153 registers, one block per SM (BatchNorm backward of
+    // 100352 x 192 by its output 73 us, 56 with two)
+    pixel_batches<MODE == 1 ? 2 : MODE == 3 ? 4 : 8>(m.p0, m.step, P, [&](auto count, long long p) {
+      constexpr int U = decltype(count)::value;
       Bf8 xv[U], dv[U], yv[U];
       uint32_t on[U];
 #pragma unroll
@@ -345,13 +355,7 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) add(xv[u], dv[u], yv[u], on[u]);
-    }
-    for (; p < P; p += m.step) {
-      Bf8 xv = ld8(x + p * ldx + m.c), dv, yv;
-      if (BWD) dv = ld8(dy + p * lddy + m.c);
-      if (MODE == 1 && relu) yv = ld8(y + p * lddy + m.c);
-      add(xv, dv, yv, MODE == 3 ? bits[p * cv + (m.c >> 3)] : 0u);
-    }
+    });
     if (BWD) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) a1[e] *= mr[1][e];
@@ -359,16 +363,15 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
   }
   slot_sums<MODE == 2 ? 1 : 2>(m, a0, a1, out, C, MODE == 2 ? scale : 1.f, sacc);
 }
-// Blocks per SM that the registers of a kernel allow (its launch bounds) and its grid asks for: a second round of blocks
-// would fetch the constants and meet in atomics once more.  32 x 56 x 56 x 192, forward and backward: 69.3 us with grids of
-// 4 (sums) and 8 (normalisation) blocks per SM, 63.7 with these; the backward sums spill at three blocks or four.
-constexpr int reduce_blocks(int mode) { return mode == 1 || mode == 3 ? 2 : 4; }
-constexpr int kApplyBlocks = 4;
+// Blocks per SM of the channel kernels (launch bounds and grids).  Two with eight pixels of a thread in flight (four where
+// there are two tensors to load, two where there are three) instead of four with four: the same bytes in flight, half the
+// atomics and constants.  BatchNorm with ReLU bits, forward and backward, us: 100352 x 192 61.3 -> 57.4, 25088 x 192 24.5 ->
+// 22.0, 25088 x 320 32.2 -> 28.7, 25600 x 144 22.8 -> 20.0, 50000 x 48 18.1 -> 15.7, 6272 x 160 12.8 -> 11.8; one block per SM
+// with eight pixels of the sums 62.1, 20.9, 28.3, 18.4, 16.4, 12.8.
+constexpr int kChannelBlocks = 2;
 enum { MASK_NONE = 0, MASK_Y = 1, MASK_BITS = 2 };      // what the backward pass reads a ReLU mask from
-// A third tensor's loads in flight spill at three blocks: backward of 100352 x 192 by the output 68.3 us at three, 56.0 at two.
-constexpr int backward_blocks(int mask) { return mask == MASK_Y ? 2 : 3; }
 template <int MODE>
-__global__ void __launch_bounds__(256, reduce_blocks(MODE))
+__global__ void __launch_bounds__(256, kChannelBlocks)
 channel_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                       const float* __restrict__ mean_rstd, float* __restrict__ out, long long P, int C,
                       long long ldx, long long lddy, int relu, float scale) {
@@ -427,9 +430,8 @@ __device__ __forceinline__ void bn_apply_pixels(const SlotMap& s, const bf16* __
     }
     return o;
   };
-  constexpr int U = 4;
-  long long p = s.p0;
-  for (; p + (U - 1) * s.step < P; p += U * s.step) {
+  pixel_batches<8>(s.p0, s.step, P, [&](auto count, long long p) {
+    constexpr int U = decltype(count)::value;
     Bf8 v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) v[u] = ld8(x + (p + u * s.step) * ldx + s.c);
@@ -439,12 +441,7 @@ __device__ __forceinline__ void bn_apply_pixels(const SlotMap& s, const bf16* __
       st8(y + (p + u * s.step) * ldy + s.c, o);
       if (bits) mark(p + u * s.step, o);
     }
-  }
-  for (; p < P; p += s.step) {
-    const Bf8 o = one(ld8(x + p * ldx + s.c));
-    st8(y + p * ldy + s.c, o);
-    if (bits) mark(p, o);
-  }
+  });
 }
 
 __global__ void __launch_bounds__(256)
@@ -491,7 +488,7 @@ __device__ __forceinline__ void bn_apply_fused_body(const bf16* __restrict__ x, 
   if (!s.on) return;
   bn_apply_pixels(s, x, y, mkb, P, ldx, ldy, relu, bits, C >> 3);
 }
-__global__ void __launch_bounds__(256, kApplyBlocks)
+__global__ void __launch_bounds__(256, kChannelBlocks)
 bn_apply_fused_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const float* __restrict__ sums,
                       float* __restrict__ mean_rstd, float* running_mean, float* running_var,
                       const float* __restrict__ gamma, const float* __restrict__ beta, float* zero_after, long long P,
@@ -536,9 +533,8 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
     }
     return o;
   };
-  constexpr int U = 2;
-  long long p = s.p0;
-  for (; p + (U - 1) * s.step < P; p += U * s.step) {
+  pixel_batches<MASK == MASK_Y ? 2 : 4>(s.p0, s.step, P, [&](auto count, long long p) {
+    constexpr int U = decltype(count)::value;
     Bf8 xv[U], dv[U], yv[U];
     uint32_t on[U];
 #pragma unroll
@@ -550,15 +546,10 @@ __device__ __forceinline__ void bn_backward_body(const bf16* __restrict__ x, con
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) st8(dx + (p + u * s.step) * lddx + s.c, one(xv[u], dv[u], yv[u], on[u]));
-  }
-  for (; p < P; p += s.step) {
-    Bf8 xv = ld8(x + p * ldx + s.c), dv = ld8(dy + p * lddy + s.c), yv;
-    if (MASK == MASK_Y && relu) yv = ld8(y + p * lddy + s.c);
-    st8(dx + p * lddx + s.c, one(xv, dv, yv, MASK == MASK_BITS ? bits[p * cv + (s.c >> 3)] : 0u));
-  }
+  });
 }
 template <int MASK>
-__global__ void __launch_bounds__(256, backward_blocks(MASK))
+__global__ void __launch_bounds__(256, kChannelBlocks)
 bn_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                    bf16* __restrict__ dx, const float* __restrict__ mean_rstd, const float* __restrict__ gamma,
                    const float* __restrict__ sums, float* dgamma, float* dbeta, long long P, int C,
@@ -670,7 +661,8 @@ f32_to_bf16_2d_kernel(const float* __restrict__ src, bf16* __restrict__ dst, lon
   }
 }
 // ReLU backward fused with the per-channel sums of its result (the bias gradient of the layer whose output y is):
-// dx = y > 0 ? dy : 0, out[c] += sum over pixels of dx.
+// dx = y > 0 ? dy : 0, out[c] += sum over pixels of dx.  Four blocks per SM with eight pixels of a thread in flight; eight with
+// four: 43264 x 384 22.3 us, 18.0 now, 43264 x 256 16.4, 12.4, 186624 x 256 53.4, 50.9 (of which 44 are the bytes).
 __global__ void __launch_bounds__(256)
 relu_backward_colsum_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ y, bf16* __restrict__ dx,
                             float* __restrict__ out, long long P, int C, long long lddy, long long ldy, long long lddx) {
@@ -691,9 +683,8 @@ relu_backward_colsum_kernel(const bf16* __restrict__ dy, const bf16* __restrict_
       }
       return o;
     };
-    constexpr int U = 4;
-    long long p = m.p0;
-    for (; p + (U - 1) * m.step < P; p += U * m.step) {
+    pixel_batches<8>(m.p0, m.step, P, [&](auto count, long long p) {
+      constexpr int U = decltype(count)::value;
       Bf8 d[U], v[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -702,8 +693,7 @@ relu_backward_colsum_kernel(const bf16* __restrict__ dy, const bf16* __restrict_
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) st8(dx + (p + u * m.step) * lddx + m.c, one(d[u], v[u]));
-    }
-    for (; p < P; p += m.step) st8(dx + p * lddx + m.c, one(ld8(dy + p * lddy + m.c), ld8(y + p * ldy + m.c)));
+    });
   }
   slot_sums<1>(m, a, a, out, C, 1.f, sacc);
 }
@@ -1956,11 +1946,11 @@ static SlotGrid balanced(SlotGrid g) {
 }
 // reductions: one batch of four pixels per thread where that leaves SMs idle
 static SlotGrid reduce_grid(int mode, long long P, int C) {
-  return balanced(slot_grid(P, C, 4, reduce_blocks(mode), mode == 2 ? 1 : 2));
+  return balanced(slot_grid(P, C, 4, kChannelBlocks, mode == 2 ? 1 : 2));
 }
 // element-wise passes with per-channel constants
-static SlotGrid apply_grid(long long P, int C, int per_sm = kApplyBlocks) {
-  SlotGrid g = balanced(slot_grid(P, C, 4, per_sm, 0));
+static SlotGrid apply_grid(long long P, int C) {
+  SlotGrid g = balanced(slot_grid(P, C, 4, kChannelBlocks, 0));
   g.smem = ((size_t)(C / 8) + g.grid.x - 1) / g.grid.x * 8 * 4 * sizeof(float);      // four constants per channel
   return g;
 }
@@ -1986,7 +1976,7 @@ static int bn_backward_by_output(const void* x, const void* dy, const void* y, v
                                  const float* gamma, float* sums, float* dgamma, float* dbeta, float* zero_after, long long P,
                                  int C, long long ldx, long long lddy, long long lddx, int relu, float grad_scale,
                                  cudaStream_t st) {
-  const SlotGrid rg = reduce_grid(1, P, C), ag = apply_grid(P, C, backward_blocks(relu ? MASK_Y : MASK_NONE));
+  const SlotGrid rg = reduce_grid(1, P, C), ag = apply_grid(P, C);
   geeps_launch(channel_reduce_kernel<1>, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)x, (const bf16*)dy, (const bf16*)y, mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
   geeps_launch(relu ? bn_backward_kernel<MASK_Y> : bn_backward_kernel<MASK_NONE>, ag.grid, ag.threads, ag.smem, st,
@@ -2064,7 +2054,7 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
     return e == cudaSuccess ? CK() : (int)e;
   }
   if (bits != nullptr && relu) {
-    const SlotGrid rg = reduce_grid(3, P, C), ag = apply_grid(P, C, backward_blocks(MASK_BITS));
+    const SlotGrid rg = reduce_grid(3, P, C), ag = apply_grid(P, C);
     geeps_launch(channel_reduce_kernel<3>, rg.grid, rg.threads, rg.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits,
                                                                    mean_rstd, sums, P, C, ldx, lddy, relu, 1.f);
     geeps_launch(bn_backward_kernel<MASK_BITS>, ag.grid, ag.threads, ag.smem, st, (const bf16*)x, (const bf16*)dy, (const bf16*)bits, (bf16*)dx,
@@ -2112,7 +2102,7 @@ int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* c
   if (C % 8 || lddy % 8 || ldy % 8 || lddx % 8 || C > 8192) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   geeps_clear_f32(colsum, C, st);
-  const SlotGrid rg = slot_grid(P, C, 4, 8, 1);
+  const SlotGrid rg = slot_grid(P, C, 4, 4, 1);
   geeps_launch_plain(relu_backward_colsum_kernel, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)dy, (const bf16*)y, (bf16*)dx, colsum, P, C, lddy, ldy, lddx);
   return CK();
