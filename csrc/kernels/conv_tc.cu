@@ -47,6 +47,7 @@ enum { MODE_FWD = 0, MODE_DGRAD = 1, MODE_WGRAD = 2 };
 struct DgradDev {
   int t0;                         // first tile of the class
   int wt, ht, m_tiles;            // pixel boxes along W, along H, in all
+  int m_units;                    // boxes or, on CTA pairs, pairs of neighbouring boxes
   int KW, kt_total;               // taps per row of the sub-filter; its taps x channel chunks
   int pad_w, pad_h, tap0;         // dY offset of sub-filter tap (0, 0) and its place in the whole filter
 };
@@ -58,7 +59,7 @@ struct ConvDev {
   int bw, bh, bnb, wt, ht;        // pixel box and number of boxes along W and H (batch boxes follow)
   int rows;                       // bw * bh * bnb
   int bn, n_valid;                // tile width; valid output columns (fwd: Og, dgrad: Cg, wgrad: panels * 64)
-  int m_tiles, n_tiles, kt_total, split_k, stages, tmem_cols;
+  int m_tiles, m_units, n_tiles, kt_total, split_k, stages, tmem_cols;
   int groups;                     // epilogue groups that have columns to take
   int slabs;                      // staging slabs: two per epilogue group that has one to fill
   int relu, zero_fill_c;          // wgrad: a channel coordinate outside X, for panels past the last one
@@ -99,7 +100,12 @@ __device__ __forceinline__ Box decode_box(const ConvDev& d, int i, int wt, int h
 
 // tmA: activations of the M side (fwd: X, dgrad: dY, wgrad: dY); tmB: fwd/dgrad: W as (ci, tap, co),
 // wgrad: X; tmC: fwd: Y, dgrad: dX (4-D bf16), wgrad: dW as (ci, tap, co) fp32.
-template <int MODE>
+//
+// PAIR (forward and data gradient): the two CTAs of a cluster compute the tiles of two neighbouring pixel boxes with one
+// MMA of 256 rows (cta_group::2).  Each loads its own box and half of the weight tile, so an SM takes 28 KB instead of 40
+// from L2 for a k-tile of 192 columns, and that (some 64 bytes a clock) is what bounds the main loop.  The even CTA issues
+// the products for both; its barriers count the bytes of both.
+template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ OutMaps tmC, const ConvDev d) {
@@ -107,16 +113,19 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   constexpr bool B_MN = MODE != MODE_FWD;
   extern __shared__ uint8_t smem_raw[];
   const int BN = d.bn;
-  const int B_STAGE_BYTES = BN * BK * 2;
+  const int BNC = PAIR ? BN / 2 : BN;                   // columns of the weight tile that this CTA loads
+  const int B_STAGE_BYTES = BNC * BK * 2;
   const int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* cslab = tiles + (size_t)d.stages * STAGE_BYTES;
   SmemCtl* ctl = (SmemCtl*)(cslab + d.slabs * C_SLAB_BYTES);
+  const int rank = PAIR ? (int)tc05::cluster_ctarank() : 0;
+  const int unit0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, units = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = d.stages;
   const int kt_per = (d.kt_total + d.split_k - 1) / d.split_k;
-  const int tiles_mn = d.m_tiles * d.n_tiles;
+  const int tiles_mn = d.m_units * d.n_tiles;
   const int num_tiles = tiles_mn * d.split_k;
   const int acc_stride = d.tmem_cols >> 1;
 
@@ -129,16 +138,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) { tc05::mbar_init(&ctl->full[s], 1); tc05::mbar_init(&ctl->empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { tc05::mbar_init(&ctl->tmem_full[a], 1); tc05::mbar_init(&ctl->tmem_empty[a], 4 * kGroups); }
+    for (int a = 0; a < 2; ++a) { tc05::mbar_init(&ctl->tmem_full[a], 1); tc05::mbar_init(&ctl->tmem_empty[a], (PAIR ? 2 : 1) * 4 * kGroups); }
     ctl->abort_flag = 0;
     tc05::mbar_fence_init();
   }
   if (warp == 1) {
-    tc05::tmem_alloc(&ctl->tmem_base, (uint32_t)d.tmem_cols);
-    tc05::tmem_relinquish();
+    if (PAIR) { tc05::tmem_alloc_pair(&ctl->tmem_base, (uint32_t)d.tmem_cols); tc05::tmem_relinquish_pair(); }
+    else { tc05::tmem_alloc(&ctl->tmem_base, (uint32_t)d.tmem_cols); tc05::tmem_relinquish(); }
   }
   tc05::fence_before_sync();
   __syncthreads();
+  if (PAIR) tc05::cluster_sync();      // the peer's barriers are initialised before anything signals them
   tc05::fence_after_sync();
   const uint32_t tmem = ctl->tmem_base;
   geeps_pdl_wait();          // everything above touches this CTA's own memory only
@@ -157,13 +167,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       uint32_t ph = 0;
       bool ok = true;
       const uint32_t tx_bytes = MODE == MODE_WGRAD ? (uint32_t)((2 + BN / 64) * d.rows * 128)
-                                                   : (uint32_t)(d.rows * 128 + BN * 128);
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+                                                   : (uint32_t)((PAIR ? 2 : 1) * (d.rows * 128 + BNC * 128));
+      for (int t = unit0; t < num_tiles && ok; t += units) {
         const DgradDev& q = d.cls[MODE == MODE_DGRAD ? dgrad_class(d, t) : 0];
         const int tq = MODE == MODE_DGRAD ? t - q.t0 : t;
         const int mn = MODE == MODE_DGRAD ? tq : tq % tiles_mn, z = MODE == MODE_DGRAD ? 0 : tq / tiles_mn;
-        const int mts = MODE == MODE_DGRAD ? q.m_tiles : d.m_tiles;
-        const int mi = mn % mts, ni = mn / mts;
+        const int mts = MODE == MODE_DGRAD ? q.m_units : d.m_units;
+        const int ni = mn / mts, mi = PAIR ? (mn - ni * mts) * 2 + rank : mn - ni * mts;    // a second box past the last is all zeros
         const int kt_begin = z * kt_per, kt_end = MODE == MODE_DGRAD ? q.kt_total : min(d.kt_total, kt_begin + kt_per);
         const int KW = MODE == MODE_DGRAD ? q.KW : d.KW;
         Box mb = {0, 0, 0};
@@ -195,8 +205,19 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           uint8_t* sb = sa + A_STAGE_BYTES;
           uint64_t* bar = &ctl->full[s];
           if (leader) {
-          tc05::mbar_expect_tx(bar, tx_bytes);
-          if (MODE == MODE_FWD) {
+          if (!PAIR || rank == 0) tc05::mbar_expect_tx(bar, tx_bytes);
+          if (PAIR) {
+            const uint32_t both = tc05::map_to_cta(tc05::smem_u32(bar), 0);
+            const int n = ni * BN + rank * BNC;
+            if (MODE == MODE_FWD) {
+              tc05::tma_load_4d_pair(sa, &tmA, both, cc * 64, mb.w0 * d.stride + kw - d.pad, mb.h0 * d.stride + kh - d.pad, mb.b0);
+              tc05::tma_load_3d_pair(sb, &tmB, both, cc * 64, tap, n);
+            } else {
+              tc05::tma_load_4d_pair(sa, &tmA, both, cc * 64, mb.w0 - kw, mb.h0 - kh, mb.b0);
+              for (int h = 0; h < BNC / 64; ++h)
+                tc05::tma_load_3d_pair(sb + h * PANEL_BYTES, &tmB, both, n + 64 * h, wtap, cc * 64);
+            }
+          } else if (MODE == MODE_FWD) {
             tc05::tma_load_4d(sa, &tmA, bar, cc * 64, mb.w0 * d.stride + kw - d.pad, mb.h0 * d.stride + kh - d.pad, mb.b0);
             tc05::tma_load_3d(sb, &tmB, bar, cc * 64, tap, ni * BN);
           } else if (MODE == MODE_DGRAD) {
@@ -226,14 +247,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
     geeps_pdl_trigger();       // every operand is on its way: the rest of this CTA is its last products and stores
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    {
+    // ---------------- MMA issuer (of a pair: the even CTA's) ----------------
+    if (!PAIR || rank == 0) {
       const bool leader = tc05::elect_one();
-      const uint32_t idesc = tc05::make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const uint32_t idesc = tc05::make_idesc_bf16(PAIR ? 2 * BM : BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       uint32_t tile_i = 0, ph = 0;
       int s = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_i) {
+      for (int t = unit0; t < num_tiles && ok; t += units, ++tile_i) {
         const int z = MODE == MODE_DGRAD ? 0 : t / tiles_mn;
         const int kt_begin = z * kt_per;
         const int kt_end = MODE == MODE_DGRAD ? d.cls[dgrad_class(d, t)].kt_total : min(d.kt_total, kt_begin + kt_per);
@@ -246,11 +267,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tc05::fence_after_sync();
           const uint32_t sa = tiles_u + (uint32_t)(s * STAGE_BYTES), sb = sa + A_STAGE_BYTES;
           const uint32_t a_lo = tc05::desc_lo(sa, A_MN ? PANEL_BYTES : 16), b_lo = tc05::desc_lo(sb, B_MN ? PANEL_BYTES : 16);
-          tc05::mma_ktile_warp<A_MN ? 128 : 2, B_MN ? 128 : 2>(tacc, a_lo, b_lo, tc05::desc_hi(1024), idesc,
-                                                               kt > kt_begin ? 1u : 0u, empty_u + 8u * (uint32_t)s);
+          if (PAIR)
+            tc05::mma_ktile_warp_pair<A_MN ? 128 : 2, B_MN ? 128 : 2>(tacc, a_lo, b_lo, tc05::desc_hi(1024), idesc,
+                                                                      kt > kt_begin ? 1u : 0u, empty_u + 8u * (uint32_t)s);
+          else
+            tc05::mma_ktile_warp<A_MN ? 128 : 2, B_MN ? 128 : 2>(tacc, a_lo, b_lo, tc05::desc_hi(1024), idesc,
+                                                                 kt > kt_begin ? 1u : 0u, empty_u + 8u * (uint32_t)s);
           if (++s == S) { s = 0; ph ^= 1u; }
         }
-        if (ok && leader) tc05::mma_commit(&ctl->tmem_full[acc]);
+        if (ok && leader) {
+          if (PAIR) tc05::mma_commit_pair(&ctl->tmem_full[acc], 3);
+          else tc05::mma_commit(&ctl->tmem_full[acc]);
+        }
       }
     }
   } else {
@@ -266,12 +294,13 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t row_off = (uint32_t)rloc * (narrow ? 64u : 128u);
     const uint32_t rsw = narrow ? (uint32_t)((rloc >> 1) & 3) : (uint32_t)(rloc & 7);
     const bool relu = d.relu != 0;
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tile_i) {
+    for (int t = unit0; t < num_tiles; t += units, ++tile_i) {
       const int cl = MODE == MODE_DGRAD ? dgrad_class(d, t) : 0;
       const DgradDev& cq = d.cls[cl];
       const int mn = MODE == MODE_DGRAD ? t - cq.t0 : t % tiles_mn;
-      const int mts = MODE == MODE_DGRAD ? cq.m_tiles : d.m_tiles;
-      const int mi = mn % mts, ni = mn / mts;
+      const int mts = MODE == MODE_DGRAD ? cq.m_units : d.m_units;
+      const int ni = mn / mts, mi = PAIR ? (mn - ni * mts) * 2 + rank : mn - ni * mts;
+      const bool there = !PAIR || mi < (MODE == MODE_DGRAD ? cq.m_tiles : d.m_tiles);
       const int n0 = ni * BN;
       const uint32_t acc = tile_i & 1u, acc_ph = (tile_i >> 1) & 1u;
       if (!tc05::mbar_wait(&ctl->tmem_full[acc], acc_ph, abort_flag, WAIT_BUDGET_NS)) break;
@@ -281,7 +310,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (MODE == MODE_FWD) mb = decode_box(d, mi, d.wt, d.ht);
       if (MODE == MODE_DGRAD) mb = decode_box(d, mi, cq.wt, cq.ht);
 #pragma unroll 1
-      for (int c = grp < d.groups ? grp * cols_per_slab : BN; c < BN; c += d.groups * cols_per_slab) {
+      for (int c = grp < d.groups && there ? grp * cols_per_slab : BN; c < BN; c += d.groups * cols_per_slab) {
         if (n0 + c >= d.n_valid) break;
         uint8_t* slab = cslab + (size_t)(2 * grp + (slab_i & 1u)) * C_SLAB_BYTES;
         if (issuer) tc05::bulk_wait_read<1>();
@@ -341,7 +370,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       tc05::fence_before_sync();
       __syncwarp();
-      if (lane == 0) tc05::mbar_arrive(&ctl->tmem_empty[acc]);
+      if (lane == 0) {
+        if (PAIR) tc05::mbar_arrive_cluster(tc05::map_to_cta(tc05::smem_u32(&ctl->tmem_empty[acc]), 0));
+        else tc05::mbar_arrive(&ctl->tmem_empty[acc]);
+      }
     }
   }
 
@@ -350,9 +382,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __syncthreads();
   if (threadIdx.x == 0 && ctl->abort_flag)
     geeps_report(d.status, GEEPS_ERR_TIMEOUT, KID_CONV_TC, (int)blockIdx.x, 0);
+  // neither CTA of a pair may release TMEM or leave while the other can still signal its barriers or use the pair's TMEM
+  if (PAIR) tc05::cluster_sync();
   if (warp == 1) {
     tc05::fence_after_sync();
-    tc05::tmem_dealloc(tmem, (uint32_t)d.tmem_cols);
+    if (PAIR) tc05::tmem_dealloc_pair(tmem, (uint32_t)d.tmem_cols);
+    else tc05::tmem_dealloc(tmem, (uint32_t)d.tmem_cols);
   }
 }
 
@@ -416,8 +451,11 @@ bool make_act_view(CUtensorMap* map, const void* base, int ch, int W, int H, int
 }
 
 // Pick the pixel box (bw, bh, bnb) with at most `cap` pixels that covers the W x H x B grid with the fewest
-// boxes; ties go to the wider box (longer contiguous runs).
+// boxes; ties go to the wider box (longer contiguous runs).  A call asks twice (which kernel, how it is cut): the last answer is
+// kept for the thread.
 void pick_box(int W, int H, int B, int cap, int* bw, int* bh, int* bnb) {
+  thread_local int last[7] = {0, 0, 0, 0, 0, 0, 0};
+  if (last[0] == W && last[1] == H && last[2] == B && last[3] == cap) { *bw = last[4]; *bh = last[5]; *bnb = last[6]; return; }
   long long best = -1;
   *bw = 1; *bh = 1; *bnb = 1;
   for (int w = 1; w <= W && w <= cap; ++w) {
@@ -429,6 +467,8 @@ void pick_box(int W, int H, int B, int cap, int* bw, int* bh, int* bnb) {
       if (best < 0 || boxes < best || (boxes == best && w > *bw)) { best = boxes; *bw = w; *bh = h; *bnb = n; }
     }
   }
+  const int now[7] = {W, H, B, cap, *bw, *bh, *bnb};
+  memcpy(last, now, sizeof(last));
 }
 
 int round_up(long long v, int m) { return (int)((v + m - 1) / m * m); }
@@ -441,19 +481,89 @@ int narrow_store(int channels, long long pitch) {
   return (channels % 64 == 32 && (pitch * 2) % 128 != 0) ? 1 : 0;
 }
 
-template <int MODE>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tc, const ConvDev& d, int grid,
-           cudaStream_t st) {
-  const int stage_bytes = A_STAGE_BYTES + d.bn * BK * 2;
+// How a forward or data-gradient product is cut into tiles, and what its two kernels take.
+// (the parity classes of a strided data gradient share one box, which the largest class is cut into)
+struct BoxPlan {
+  int bw, bh, bnb;                // pixel box
+  long long m_tiles;              // boxes: of the whole problem, or of the largest class
+  int bn, n_tiles, kt;            // tile width, tiles along the channels, k-tiles (whole filter)
+  double one, pair;               // us on single CTAs and on pairs; pair < 0: no pairs
+};
+// Times (us, captured chain) of 364 forward and 364 data-gradient products with 7 x 7 to 56 x 56 pixels, 32 to 384 channels,
+// 3 x 3 and 5 x 5 taps, as launch + waves * (tile + k-tiles * (k-tile + width * per column)); half of the fits lie within
+// 13 % of the measurement.  Rows of activations or weights that do not begin on 128-byte lines cost a k-tile more, above all
+// where one CTA loads the whole weight tile: 24 x 24 x 296 -> 240 at batch 197 219 us on single CTAs, 151 on pairs.
+struct KernelCost { double launch, tile, tile_col, kt, kt_col, kt_mis, kt_mis_col; };
+constexpr KernelCost kFwdOne = {4.09, 1.52, 0.146, 0.143, 0.028, 0., 0.062}, kFwdPair = {4.98, 1.19, 0.326, 0.152, 0.021, 0.012, 0.028},
+                     kDgradOne = {3.47, 1.73, 0., 0.182, 0.033, 0., 0.044}, kDgradPair = {5.22, 0., 0.603, 0.208, 0.019, 0.023, 0.008};
+double tiles_us(const KernelCost& c, long long waves, int kt, int bn, bool mis) {
+  const double cols = bn / 64.0;
+  return c.launch + waves * (c.tile + cols * c.tile_col + kt * (c.kt + cols * c.kt_col + (mis ? c.kt_mis + cols * c.kt_mis_col : 0.)));
+}
+
+// s, n_cls: stride and classes of this launch of a strided data gradient
+BoxPlan plan_box(const GeepsConvTcParams* p, int s, int n_cls, int sms) {
+  const bool fwd = p->mode == MODE_FWD;
+  BoxPlan b;
+  // rows of the tile: pixels of the output (fwd) or of the input gradient (dgrad)
+  const int GW = fwd ? p->OW : (p->W + s - 1) / s, GH = fwd ? p->OH : (p->H + s - 1) / s;
+  pick_box(GW, GH, p->B, BM, &b.bw, &b.bh, &b.bnb);
+  b.m_tiles = (long long)((GW + b.bw - 1) / b.bw) * ((GH + b.bh - 1) / b.bh) * ((p->B + b.bnb - 1) / b.bnb);
+  const int kch = fwd ? p->cg : p->og, nch = fwd ? p->og : p->cg;          // reduced and produced channels
+  b.kt = p->KH * p->KW * ((kch + 63) / 64);
+  const int nt = (nch + 255) / 256;
+  b.bn = round_up((nch + nt - 1) / nt, (fwd && nt == 1) ? 32 : 64);
+  if (b.bn > 256) b.bn = 256;
+  // too few tiles for the machine: narrower ones, while the operand rows (the bound here) of the busiest SM go down:
+  // 32 x 14 x 14 pixels, 160 channels: 3 x 3 forward 14.7 -> 12.2 us (160 in), 11.5 -> 9.7 us (128 in)
+  const long long all = b.m_tiles * n_cls;
+  if (all * ((nch + b.bn - 1) / b.bn) < sms) {
+    auto cost = [&](int w) { return (all * ((nch + w - 1) / w) + sms - 1) / sms * (BM + w); };
+    for (int w = 64, top = b.bn; w < top; w += 64)
+      if (cost(w) < cost(b.bn)) b.bn = w;
+  }
+  b.n_tiles = (nch + b.bn - 1) / b.bn;
+  const void* act = fwd ? p->x : p->y;
+  const bool mis = ((fwd ? p->x_pitch : p->y_pitch) % 64) != 0 || p->cg % 64 != 0 || ((uintptr_t)act & 127) != 0;
+  b.one = tiles_us(fwd ? kFwdOne : kDgradOne, (b.m_tiles * b.n_tiles + sms - 1) / sms, b.kt, b.bn, mis);
+  // Not below the channels that the fits know.  Pairs need whole 64-column panels of a transposed weight tile in each half.  Where the lines are aligned and the
+  // k-tiles few the epilogue is the bound (32 x 56 x 56, 64 -> 192: 23.4 us on single CTAs, 26.8 on pairs).
+  b.pair = -1;
+  if (p->stride <= 1 && s == 1 && b.bn % (fwd ? 32 : 128) == 0 && (mis || b.kt >= 18) && kch >= 32 && nch >= 32)
+    b.pair = tiles_us(fwd ? kFwdPair : kDgradPair, ((b.m_tiles + 1) / 2 * b.n_tiles + sms / 2 - 1) / (sms / 2), b.kt, b.bn, mis);
+  return b;
+}
+bool takes_pairs(const BoxPlan& b) { return b.pair >= 0 && b.pair < 0.97 * b.one; }
+
+template <int MODE, bool PAIR>
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const OutMaps& tc, const ConvDev& d, int units, cudaStream_t st) {
+  const int stage_bytes = A_STAGE_BYTES + (PAIR ? d.bn / 2 : d.bn) * BK * 2;
   const size_t smem = (size_t)d.stages * stage_bytes + d.slabs * C_SLAB_BYTES + sizeof(SmemCtl) + 1024;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(conv_tc_kernel<MODE, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  geeps_launch(conv_tc_kernel<MODE>, grid, kThreads, smem, st, ta, tb, tc, d);
-  return (int)cudaGetLastError();
+  if (!PAIR) {
+    geeps_launch(conv_tc_kernel<MODE, PAIR>, units, kThreads, smem, st, ta, tb, tc, d);
+    return (int)cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * units));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, conv_tc_kernel<MODE, PAIR>, ta, tb, tc, d);
+  return e == cudaSuccess ? (int)cudaGetLastError() : (int)e;
 }
 
 }  // namespace
@@ -474,6 +584,19 @@ int geeps_conv_tc_supported(const GeepsConvTcParams* p) {
   if (p->ldw < (long long)p->KH * p->KW * p->cg) return 0;
   if (p->mode < 0 || p->mode > 2) return 0;
   return 1;
+}
+
+}  // extern "C"
+
+extern "C" {
+
+// us that the better of the box kernels is expected to take for a stride-1 forward or data-gradient product
+double geeps_conv_box_us(const GeepsConvTcParams* p) {
+  const BoxPlan b = plan_box(p, 1, 1, geeps_sm_count());
+  return takes_pairs(b) ? b.pair : b.one;
+}
+int geeps_conv_box_pairs(const GeepsConvTcParams* p) {
+  return p->mode != MODE_WGRAD && p->stride <= 1 && geeps_conv_tc_supported(p) && takes_pairs(plan_box(p, 1, 1, geeps_sm_count())) ? 1 : 0;
 }
 
 }  // extern "C"
@@ -545,15 +668,14 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
   CUtensorMap ta, tb;
   OutMaps tc;
   memset(&tc, 0, sizeof(tc));
-  bool ok = true;
+  bool ok = true, pair = false;
   const long long wdims[3] = {p->cg, d.taps, p->og};
   if (p->mode == MODE_FWD || p->mode == MODE_DGRAD) {
     const bool fwd = p->mode == MODE_FWD;
-    // rows of the tile: pixels of the output (fwd) or of the input gradient (dgrad)
-    // (the classes share one box, which the largest class is cut into)
     const int GW = fwd ? p->OW : (p->W + cls.s - 1) / cls.s, GH = fwd ? p->OH : (p->H + cls.s - 1) / cls.s;
     if (!fwd) d.stride = 1;
-    pick_box(GW, GH, p->B, BM, &d.bw, &d.bh, &d.bnb);
+    const BoxPlan plan = plan_box(p, cls.s, cls.n, kSMs);
+    d.bw = plan.bw; d.bh = plan.bh; d.bnb = plan.bnb;
     d.rows = d.bw * d.bh * d.bnb;
     d.wt = (GW + d.bw - 1) / d.bw; d.ht = (GH + d.bh - 1) / d.bh;
     const int bt = (p->B + d.bnb - 1) / d.bnb;
@@ -579,30 +701,23 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
     d.cchunks = (kch + 63) / 64;
     d.kt_total = d.taps * d.cchunks;
     d.n_valid = nch;
-    const int nt = (nch + 255) / 256;
-    int bn = round_up((nch + nt - 1) / nt, (fwd && nt == 1) ? 32 : 64);
-    if (bn > 256) bn = 256;
-    // too few tiles for the machine: narrower ones, while the operand rows (the bound here) of the busiest SM go down:
-    // 32 x 14 x 14 pixels, 160 channels: 3 x 3 forward 14.7 -> 12.2 us (160 in), 11.5 -> 9.7 us (128 in)
-    if ((long long)d.m_tiles * ((nch + bn - 1) / bn) < kSMs) {
-      auto cost = [&](int w) {
-        const long long t = (long long)d.m_tiles * ((nch + w - 1) / w);
-        return (t + kSMs - 1) / kSMs * (BM + w);
-      };
-      for (int w = 64, top = bn; w < top; w += 64)
-        if (cost(w) < cost(bn)) bn = w;
-    }
-    d.bn = bn;
-    d.n_tiles = (nch + bn - 1) / bn;
+    d.bn = plan.bn;
+    d.n_tiles = plan.n_tiles;
+    pair = p->split_k != -2 && takes_pairs(plan);
+    d.m_units = pair ? (d.m_tiles + 1) / 2 : d.m_tiles;
+    if (!fwd) d.m_units = 0;
     for (int i = 0, t0 = 0; !fwd && i < cls.n; ++i) {
-      d.cls[i].kt_total *= d.cchunks;
-      d.cls[i].t0 = t0;
-      t0 += d.cls[i].m_tiles * d.n_tiles;
+      DgradDev& q = d.cls[i];
+      q.kt_total *= d.cchunks;
+      q.m_units = pair ? (q.m_tiles + 1) / 2 : q.m_tiles;
+      d.m_units += q.m_units;
+      q.t0 = t0;
+      t0 += q.m_units * d.n_tiles;
     }
     const long long wst[2] = {(long long)p->cg * 2, p->ldw * 2};
     if (fwd) {
       ok = make_act_map(&ta, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, d.bw, d.bh, d.bnb, false, d.stride);
-      const int wbox[3] = {64, 1, bn};
+      const int wbox[3] = {64, 1, pair ? d.bn / 2 : d.bn};
       ok = ok && make_map(&tb, p->w, 3, wdims, wst, wbox, false);
       d.narrow = narrow_store(p->og, p->y_pitch);
       ok = ok && make_act_map(&tc.m[0], p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, d.bw, d.bh, d.bnb, d.narrow != 0);
@@ -621,7 +736,7 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
     d.rows = d.bw * d.bh * d.bnb;
     d.wt = (p->OW + d.bw - 1) / d.bw; d.ht = (p->OH + d.bh - 1) / d.bh;
     d.kt_total = d.wt * d.ht * ((p->B + d.bnb - 1) / d.bnb);
-    d.m_tiles = (p->og + BM - 1) / BM;
+    d.m_tiles = d.m_units = (p->og + BM - 1) / BM;
     d.cchunks = (p->cg + 63) / 64;
     const int panels = d.taps * d.cchunks;
     d.n_valid = panels * 64;
@@ -677,7 +792,7 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
   int tmem_cols = 32;
   while (tmem_cols < 2 * d.bn) tmem_cols <<= 1;
   d.tmem_cols = tmem_cols;
-  const int stage_bytes = A_STAGE_BYTES + d.bn * BK * 2;
+  const int stage_bytes = A_STAGE_BYTES + (pair ? d.bn / 2 : d.bn) * BK * 2;
   const long long num_tiles = (long long)d.m_tiles * d.n_tiles * d.split_k;
   // Two groups share a tile of three slabs unevenly, and where many tiles follow one another the epilogue is covered anyway:
   // one group takes them.  3 x 3 forward, us before there were two groups / with two / so: 47 x 52 x 52, 64 -> 312 48.9 / 50.8 /
@@ -689,10 +804,12 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
   d.stages = (224 * 1024 - d.slabs * C_SLAB_BYTES) / stage_bytes;
   if (d.stages > MAX_STAGES) d.stages = MAX_STAGES;
   if (d.stages < 2) d.stages = 2;
-  const int grid = (int)(num_tiles < kSMs ? num_tiles : kSMs);
-  if (p->mode == MODE_FWD) return launch<MODE_FWD>(ta, tb, tc, d, grid, st);
-  if (p->mode == MODE_DGRAD) return launch<MODE_DGRAD>(ta, tb, tc, d, grid, st);
-  return launch<MODE_WGRAD>(ta, tb, tc, d, grid, st);
+  const long long work = (long long)d.m_units * d.n_tiles * d.split_k, room = pair ? kSMs / 2 : kSMs;
+  const int units = (int)(work < room ? work : room);
+  if (p->mode == MODE_FWD) return pair ? launch<MODE_FWD, true>(ta, tb, tc, d, units, st) : launch<MODE_FWD, false>(ta, tb, tc, d, units, st);
+  if (p->mode == MODE_DGRAD)
+    return pair ? launch<MODE_DGRAD, true>(ta, tb, tc, d, units, st) : launch<MODE_DGRAD, false>(ta, tb, tc, d, units, st);
+  return launch<MODE_WGRAD, false>(ta, tb, tc, d, units, st);
 }
 
 }  // namespace

@@ -311,6 +311,20 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tma
       ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar_cluster_addr), "r"(x), "r"(y)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr, int x, int y,
+                                                 int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr, int x, int y,
+                                                 int z, int w) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_holder, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_holder)),
                "r"(ncols) : "memory");
@@ -334,6 +348,29 @@ __device__ __forceinline__ void mma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc_
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// mma_ktile_warp() for a pair, by the leader's warp; the commit arrives at `bar` in both CTAs
+template <uint32_t A_STEP, uint32_t B_STEP>
+__device__ __forceinline__ void mma_ktile_warp_pair(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                                    uint32_t accumulate, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a, b;\n\t.reg .b64 da, db;\n\t.reg .b16 both;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "mov.b16 both, 3;\n\t"
+      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t"
+      "add.u32 a, %1, %7;\n\tadd.u32 b, %2, %8;\n\tmov.b64 da, {a, %3};\n\tmov.b64 db, {b, %3};\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, t;\n\t"
+      "add.u32 a, a, %7;\n\tadd.u32 b, b, %8;\n\tmov.b64 da, {a, %3};\n\tmov.b64 db, {b, %3};\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, t;\n\t"
+      "add.u32 a, a, %7;\n\tadd.u32 b, b, %8;\n\tmov.b64 da, {a, %3};\n\tmov.b64 db, {b, %3};\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, t;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%6], both;\n\t}"
+      ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(bar), "n"(A_STEP), "n"(B_STEP)
       : "memory");
 }
 

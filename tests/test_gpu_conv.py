@@ -455,3 +455,46 @@ def test_8_bit_sources_on_any_byte_take_the_fast_kernel():
         return best
     aligned = ms(0)
     assert ms(1) < 2.5 * aligned and ms(2) < 2.5 * aligned
+
+
+@pytest.mark.parametrize("mode,B,H,W,cg,og,k,pad,wide", [
+    ("fwd", 3, 7, 6, 152, 80, 5, 2, 0),           # one box and an empty half of a pair
+    ("fwd", 4, 5, 5, 368, 40, 5, 2, 8),           # N = 64 in halves of 32, pitched activations
+    ("fwd", 37, 17, 5, 144, 280, 3, 1, 0),        # two tiles of 192 columns, the second one ragged
+    ("fwd", 39, 28, 17, 72, 80, 3, 1, 16),        # ragged boxes, columns past the last channel
+    ("fwd", 19, 18, 6, 328, 360, 2, 1, 0),
+    ("dgrad", 26, 30, 23, 80, 136, 2, 1, 0),      # more pairs than fit at once
+    ("dgrad", 26, 27, 26, 72, 72, 3, 0, 0), ("dgrad", 11, 29, 27, 72, 208, 3, 1, 16), ("dgrad", 17, 17, 30, 72, 72, 5, 0, 0),
+    ("dgrad", 24, 20, 21, 248, 136, 3, 1, 0)])    # 256 columns: two panels of the weights in each half
+def test_box_convolution_on_cta_pairs_gives_the_bits_of_single_ctas(mode, B, H, W, cg, og, k, pad, wide):
+    """Two neighbouring pixel boxes by one product of 256 rows: the same terms in the same order, so the same bits as one CTA per
+    box; nothing outside the result is written."""
+    import ctypes
+    from geeps_b200.ops import _lib as L
+    from geeps_b200.ops import functional as F
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(B * cg)
+    fwd, OH, OW, kd = mode == "fwd", H + 2 * pad - k + 1, W + 2 * pad - k + 1, k * k * cg
+    w = (torch.randn(og, (kd + 7) // 8 * 8, device=dev, generator=gen) / kd ** 0.5).to(BF)
+    full = [torch.randn(B, h, v, c + wide, device=dev, generator=gen).to(BF) for h, v, c in ((H, W, cg), (OH, OW, og))]
+    src, c_out = (full[0], og) if fwd else (full[1], cg)
+    bias = torch.randn(og, device=dev, generator=gen) if fwd else None
+    got = []
+    for split_k in (-1, -2):
+        dst = torch.full(full[1 if fwd else 0].shape, 3.0, device=dev, dtype=BF)
+        x, y = ((src, dst) if fwd else (dst, src))
+        status = torch.zeros(4, dtype=torch.int32, device=dev)
+        p = F.conv_tc_params(F.CONV_FWD if fwd else F.CONV_DGRAD, x[..., :cg], y[..., :og], w, k, pad, bias=bias, relu=fwd,
+                             split_k=split_k, status=status)
+        L.check(L.lib().geeps_conv_tc(ctypes.byref(p), L.stream_ptr()), "conv_tc")
+        assert status.tolist()[0] == 0 and (dst[..., c_out:] == 3.0).all()
+        got.append(dst)
+    assert L.lib().geeps_conv_box_pairs(ctypes.byref(p))
+    assert torch.equal(got[0], got[1])
+    x64 = full[0][..., :cg].double().permute(0, 3, 1, 2)
+    w64 = w[:, :kd].double().view(og, k, k, cg).permute(0, 3, 1, 2)
+    ref = (torch.relu(torch.nn.functional.conv2d(x64, w64, bias.double(), padding=pad)) if fwd else
+           torch.nn.functional.conv_transpose2d(full[1][..., :og].double().permute(0, 3, 1, 2), w64, padding=pad))
+    # fp32 sums rounded once to bf16: 2^-9 / sqrt(3) = 1.1e-3 in the 2-norm
+    assert _rel(got[0][..., :c_out], ref.permute(0, 2, 3, 1)) < 2.5e-3
+
