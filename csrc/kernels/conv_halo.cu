@@ -562,28 +562,42 @@ int halo_mode() {
 
 extern "C" {
 
-// 1 when conv_tc() should route this call here.  The rule is fitted to timings of both kernels on AlexNet and
-// Inception layers at batch 128 .. 256 (python -m geeps_b200.utils.microbench conv): the activations must be re-read
-// often enough by the box kernel (>= 9 taps), and the 128-channel row blocks must be mostly real channels - a 192- or
-// 384-channel layer on 13 x 13 .. 56 x 56 maps is still faster on the box kernel, whose tile is exactly as wide as the
-// layer.  A 5 x 5 data gradient always wins here (the box kernel runs it with N = 48 .. 64 MMAs).
+// 1 when conv_tc() should route this call here.  The activations must be re-read often enough by the box kernel (>= 9 taps).
+//
+// Activations whose rows are whole 128-byte lines (64 channels): the 128-channel row blocks must be mostly real channels, and
+// there must be two tiles an SM (a layer of one channel block still wins from 1.7: AlexNet conv5 per group, 256 tiles); a
+// 5 x 5 data gradient, which the box kernel runs with narrow products, always comes here.  Fitted to AlexNet and Inception layers.
+//
+// Other rows straddle lines, and the box kernel fetches them once per tap, this one once per chunk.  There the expected times
+// decide, each a fit to measured ones (geeps_conv_box_us says how; here half of the fits lie within 5 % of the measurement):
+// launch + waves * (tile + chunks * (its activations + taps * step)), and within a tenth of one another, or below the 32
+// channels that the fits know, the rule above.  us,
+// halo / box: data gradient 48 x 48, 288 -> 360 at batch 48 204 / 317; forward 27 x 27, 136 -> 80, 5 x 5 at batch 30 29.5 / 60, 51 x 51,
+// 104 -> 80 at batch 73 62.8 / 158, but 29 x 29, 56 -> 32 at batch 26 11.4 / 9.9 (a block of 32 real rows is better than its fit).
+// The rule for whole lines loses up to a fifth too (13 x 13, 256 -> 384 at batch 256, data gradient: 70 / 59) and stays: the kernels
+// add their terms in different orders (taps of a chunk, chunks of a tap), and in a deep network with near-ties in its pooling
+// windows another order changes which element a later step's maximum picks.
 int geeps_conv_halo_applicable(const GeepsConvTcParams* p) {
   if (!halo_mode()) return 0;
   if (!geeps_conv_tc_supported(p)) return 0;
   const HaloPlan hp = plan_halo(p);
   if (!hp.ok || hp.d.taps < 9) return 0;
   const HaloDev& d = hp.d;
-  const int GW = p->mode == MODE_FWD ? p->OW : p->W;
-  const double pos = (double)d.GH * GW / ((double)d.row_tiles * d.ncols2);
-  const double chn = (double)d.n_valid / ((double)d.m_tiles * BM);
+  const bool fwd = p->mode == MODE_FWD;
+  const double pos = (double)d.GH * (fwd ? p->OW : p->W) / ((double)d.row_tiles * d.ncols2);
   if (pos < 0.6) return 0;
-  // its tiles are large (up to 256 positions x 128 channels): with fewer than two per SM the box kernel's smaller
-  // tiles spread better (Inception at batch 32 .. 100: 5.60 against 5.79 ms per step of the 22K net); a layer of one
-  // channel block still wins from 1.7 tiles per SM on (AlexNet conv5 per group, 256 tiles: 0.030 against 0.038 ms)
+  const int sms = geeps_sm_count();
   const long long tiles = (long long)d.m_tiles * d.n_images * d.row_tiles;
-  if (tiles * 10 < (d.m_tiles == 1 ? 17LL : 20LL) * geeps_sm_count()) return 0;
-  if (p->mode == MODE_FWD) return (d.m_tiles == 1 && d.n_valid >= 96) || (chn >= 0.85 && pos >= 0.8) ? 1 : 0;
-  return d.taps >= 25 || (d.n_valid >= 64 && (d.n_valid <= 128 || chn >= 0.85)) ? 1 : 0;
+  const double chn = (double)d.n_valid / ((double)d.m_tiles * BM);
+  const bool shares = tiles * 10 >= (d.m_tiles == 1 ? 17LL : 20LL) * sms &&
+                      (fwd ? (d.m_tiles == 1 && d.n_valid >= 96) || (chn >= 0.85 && pos >= 0.8)
+                           : d.taps >= 25 || (d.n_valid >= 64 && (d.n_valid <= 128 || chn >= 0.85)));
+  const bool lines = (fwd ? p->x_pitch : p->y_pitch) % 64 == 0 && (fwd ? p->cg : p->og) % 64 == 0;
+  if (lines || p->cg < 32 || p->og < 32) return shares ? 1 : 0;
+  const double waves = (double)((tiles + sms - 1) / sms), cols = d.ncols2 / 100.0;
+  const double us = fwd ? 4.28 + waves * (1.44 + 0.364 * cols + d.cchunks * (0.035 * cols + d.taps * (0.214 + 0.023 * cols)))
+                        : 5.14 + waves * (0.65 + 0.107 * cols + d.cchunks * (0.142 * cols + d.taps * (0.214 + 0.025 * cols)));
+  return us < (shares ? 1.11 : d.n_valid > 32 ? 0.9 : 0.75) * geeps_conv_box_us(p) ? 1 : 0;
 }
 
 static int fill_plan(const HaloPlan& hp, int routed, GeepsHaloPlanInfo* out) {

@@ -498,3 +498,29 @@ def test_box_convolution_on_cta_pairs_gives_the_bits_of_single_ctas(mode, B, H, 
     # fp32 sums rounded once to bf16: 2^-9 / sqrt(3) = 1.1e-3 in the 2-norm
     assert _rel(got[0][..., :c_out], ref.permute(0, 2, 3, 1)) < 2.5e-3
 
+
+@pytest.mark.parametrize("B,H,cg,og,k", [(30, 27, 136, 80, 5), (22, 47, 168, 88, 3), (8, 52, 176, 128, 3), (13, 39, 80, 104, 5),
+                                         (33, 38, 184, 96, 3), (37, 30, 184, 88, 3), (10, 32, 264, 40, 5), (6, 43, 240, 376, 3)])
+def test_layers_off_128_byte_lines_agree_on_both_kernels(B, H, cg, og, k):
+    """Layers that the expected times send to the halo kernel, as conv_tc() runs them and kept on the box kernel: fp32 sums in two
+    orders, so a rounding to bf16 differs now and then."""
+    import ctypes
+    from geeps_b200.ops import _lib as L
+    from geeps_b200.ops import functional as F
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(H * cg)
+    kd = k * k * cg
+    x = torch.randn(B, H, H, cg, device=dev, generator=gen).to(BF)
+    dy = torch.randn(B, H, H, og, device=dev, generator=gen).to(BF)
+    w = (torch.randn(og, (kd + 7) // 8 * 8, device=dev, generator=gen) / kd ** 0.5).to(BF)
+    routed = 0
+    for mode in (F.CONV_FWD, F.CONV_DGRAD):
+        out = [torch.full_like(dy if mode == F.CONV_FWD else x, 3.0) for _ in range(2)]
+        for o, split_k in zip(out, (0, -2)):
+            a = (x, o) if mode == F.CONV_FWD else (o, dy)
+            p = F.conv_tc_params(mode, *a, w, k, k // 2, split_k=split_k)
+            routed += split_k == 0 and L.lib().geeps_conv_halo_applicable(ctypes.byref(p))
+            L.check(L.lib().geeps_conv_tc(ctypes.byref(p), L.stream_ptr()), "conv_tc")
+        # a term's rounding is 2^-24 of a partial sum of norm about sqrt(kd): few results cross a rounding boundary of bf16
+        assert _rel(out[0], out[1].double()) < 5e-4
+    assert routed
