@@ -568,15 +568,17 @@ extern "C" {
 // there must be two tiles an SM (a layer of one channel block still wins from 1.7: AlexNet conv5 per group, 256 tiles); a
 // 5 x 5 data gradient, which the box kernel runs with narrow products, always comes here.  Fitted to AlexNet and Inception layers.
 //
-// Other rows straddle lines, and the box kernel fetches them once per tap, this one once per chunk.  There the expected times
-// decide, each a fit to measured ones (geeps_conv_box_us says how; here half of the fits lie within 5 % of the measurement):
+// Other rows straddle lines, and the box kernel fetches them once per tap, this one once per chunk.  There, in the data gradient
+// and in a forward pass of one chunk, the expected times decide, each a fit to measured ones (geeps_conv_box_us says how; here half of the fits lie within 5 % of the measurement):
 // launch + waves * (tile + chunks * (its activations + taps * step)), and within a tenth of one another, or below the 32
-// channels that the fits know, the rule above.  us,
-// halo / box: data gradient 48 x 48, 288 -> 360 at batch 48 204 / 317; forward 27 x 27, 136 -> 80, 5 x 5 at batch 30 29.5 / 60, 51 x 51,
-// 104 -> 80 at batch 73 62.8 / 158, but 29 x 29, 56 -> 32 at batch 26 11.4 / 9.9 (a block of 32 real rows is better than its fit).
-// The rule for whole lines loses up to a fifth too (13 x 13, 256 -> 384 at batch 256, data gradient: 70 / 59) and stays: the kernels
-// add their terms in different orders (taps of a chunk, chunks of a tap), and in a deep network with near-ties in its pooling
-// windows another order changes which element a later step's maximum picks.
+// channels that the fits know, the rule above.  us, halo / box: data gradient 48 x 48, 288 -> 360 at batch 48 204 / 317, 40 x 40,
+// 280 -> 120 at batch 81 110 / 162; forward 48 x 48, 56 -> 272, 5 x 5 at batch 25 63 / 105, but 29 x 29, 56 -> 32 at batch 26
+// 11.4 / 9.9 (a block of 32 real rows is better than its fit).
+// The rule for whole lines loses up to a fifth too (13 x 13, 256 -> 384 at batch 256, data gradient: 70 / 59) and stays, as it does
+// for a forward pass of several chunks (27 x 27, 136 -> 80, 5 x 5 at batch 30 29.5 / 60): the kernels add their terms in different
+// orders (taps of a chunk, chunks of a tap; one chunk gives the same bits).  In a deep network with near-ties in its pooling
+// windows another order changes which element a later step's maximum picks, and behind a ReLU whether an output next to zero
+// is one, and with it the gradients under it.
 int geeps_conv_halo_applicable(const GeepsConvTcParams* p) {
   if (!halo_mode()) return 0;
   if (!geeps_conv_tc_supported(p)) return 0;
@@ -593,11 +595,12 @@ int geeps_conv_halo_applicable(const GeepsConvTcParams* p) {
                       (fwd ? (d.m_tiles == 1 && d.n_valid >= 96) || (chn >= 0.85 && pos >= 0.8)
                            : d.taps >= 25 || (d.n_valid >= 64 && (d.n_valid <= 128 || chn >= 0.85)));
   const bool lines = (fwd ? p->x_pitch : p->y_pitch) % 64 == 0 && (fwd ? p->cg : p->og) % 64 == 0;
-  if (lines || p->cg < 32 || p->og < 32) return shares ? 1 : 0;
+  if (lines || (fwd && d.cchunks > 1) || p->cg < 32 || p->og < 32) return shares ? 1 : 0;
   const double waves = (double)((tiles + sms - 1) / sms), cols = d.ncols2 / 100.0;
   const double us = fwd ? 4.28 + waves * (1.44 + 0.364 * cols + d.cchunks * (0.035 * cols + d.taps * (0.214 + 0.023 * cols)))
                         : 5.14 + waves * (0.65 + 0.107 * cols + d.cchunks * (0.142 * cols + d.taps * (0.214 + 0.025 * cols)));
-  return us < (shares ? 1.11 : d.n_valid > 32 ? 0.9 : 0.75) * geeps_conv_box_us(p) ? 1 : 0;
+  // (column pairs make a 5 x 5 data gradient of few channels better than its fit: 14 x 14, 40 -> 184 at batch 181 65 / 77)
+  return us < (shares ? (d.taps >= 25 ? 1.25 : 1.11) : d.n_valid > 32 ? 0.9 : 0.75) * geeps_conv_box_us(p) ? 1 : 0;
 }
 
 static int fill_plan(const HaloPlan& hp, int routed, GeepsHaloPlanInfo* out) {
