@@ -533,6 +533,50 @@ BoxPlan plan_box(const GeepsConvTcParams* p, int s, int n_cls, int sms) {
     b.pair = tiles_us(fwd ? kFwdPair : kDgradPair, ((b.m_tiles + 1) / 2 * b.n_tiles + sms / 2 - 1) / (sms / 2), b.kt, b.bn, mis);
   return b;
 }
+// How a weight gradient is cut.  us: as tiles_us, fitted to 391 products of both kernels (here half of them within 14 %).
+struct WgradPlan { int bw, bh, bnb, kt, m_tiles, per, n_tiles, split; double us; };      // per: panels (tap, chunk) per tile
+WgradPlan plan_wgrad_box(const GeepsConvTcParams* p, int sms) {
+  WgradPlan g;
+  // reduction over output pixels in boxes of up to 64
+  pick_box(p->OW, p->OH, p->B, 64, &g.bw, &g.bh, &g.bnb);
+  g.kt = ((p->OW + g.bw - 1) / g.bw) * ((p->OH + g.bh - 1) / g.bh) * ((p->B + g.bnb - 1) / g.bnb);
+  g.m_tiles = (p->og + BM - 1) / BM;
+  const int panels = p->KH * p->KW * ((p->cg + 63) / 64);
+  // panels per tile: fewest panel loads per pixel box over the whole product (2 dY panels + `per` patch panels
+  // for each of ceil(panels / per) tiles); ties go to the wider tile
+  g.per = 1;
+  long long best_cost = -1;
+  for (int c = 1; c <= 4 && c <= panels; ++c) {
+    const long long cost = (long long)((panels + c - 1) / c) * (2 + c);
+    if (best_cost < 0 || cost <= best_cost) { best_cost = cost; g.per = c; }
+  }
+  g.n_tiles = (panels + g.per - 1) / g.per;
+  int split = p->split_k;
+  const long long tiles = (long long)g.m_tiles * g.n_tiles;
+  if (split <= 0) {
+    split = 1;
+    if (tiles < sms && g.kt >= 8) {
+      // the busiest SM walks `waves` slices, and each costs about eight k-tiles of time beside its own: filling the
+      // pipeline, and a read-modify-write of its part of the gradient.  That prefers one wave of longer slices where
+      // it fills the machine.  One wave against two, us: 256 x 13 x 13, 256 -> 384: 64.0, 66.6; 192 -> 128: 24.6, 27.7;
+      // 32 x 14 x 14, 128 -> 160: 13.3, 17.9; 100 x 32 x 32 stride 2, 80 -> 80: 16.4, 18.4
+      auto cost = [&](long long n) { return (tiles * n + sms - 1) / sms * ((g.kt + n - 1) / n + 8); };
+      const long long most = (2 * sms) / tiles < g.kt / 4 ? (2 * sms) / tiles : g.kt / 4;
+      for (long long n = 2; n <= most; ++n)
+        if (cost(n) < cost(split)) split = (int)n;
+    }
+  }
+  if (split > g.kt) split = g.kt;
+  if (split > 1) {
+    const int per_k = (g.kt + split - 1) / split;
+    split = (g.kt + per_k - 1) / per_k;      // every k-slice non-empty
+  }
+  g.split = split;
+  const bool mis_x = p->x_pitch % 64 != 0 || p->cg % 64 != 0, mis_y = p->y_pitch % 64 != 0 || p->og % 64 != 0;
+  const double waves = (double)((tiles * split + sms - 1) / sms), kt = (g.kt + split - 1) / split;
+  g.us = 5.46 + waves * (0.841 * g.per + kt * (0.332 + (mis_y ? 0.092 : 0.) + (mis_x ? 0.042 * g.per : 0.)));
+  return g;
+}
 bool takes_pairs(const BoxPlan& b) { return b.pair >= 0 && b.pair < 0.97 * b.one; }
 
 template <int MODE, bool PAIR>
@@ -595,6 +639,7 @@ double geeps_conv_box_us(const GeepsConvTcParams* p) {
   const BoxPlan b = plan_box(p, 1, 1, geeps_sm_count());
   return takes_pairs(b) ? b.pair : b.one;
 }
+double geeps_conv_box_wgrad_us(const GeepsConvTcParams* p) { return plan_wgrad_box(p, geeps_sm_count()).us; }
 int geeps_conv_box_pairs(const GeepsConvTcParams* p) {
   return p->mode != MODE_WGRAD && p->stride <= 1 && geeps_conv_tc_supported(p) && takes_pairs(plan_box(p, 1, 1, geeps_sm_count())) ? 1 : 0;
 }
@@ -731,51 +776,23 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
                                  d.bw, d.bh, d.bnb, d.narrow != 0);
     }
   } else {
-    // reduction over output pixels in boxes of up to 64
-    pick_box(p->OW, p->OH, p->B, 64, &d.bw, &d.bh, &d.bnb);
+    const WgradPlan plan = plan_wgrad_box(p, kSMs);
+    d.bw = plan.bw; d.bh = plan.bh; d.bnb = plan.bnb;
     d.rows = d.bw * d.bh * d.bnb;
     d.wt = (p->OW + d.bw - 1) / d.bw; d.ht = (p->OH + d.bh - 1) / d.bh;
-    d.kt_total = d.wt * d.ht * ((p->B + d.bnb - 1) / d.bnb);
-    d.m_tiles = d.m_units = (p->og + BM - 1) / BM;
+    d.kt_total = plan.kt;
+    d.m_tiles = d.m_units = plan.m_tiles;
     d.cchunks = (p->cg + 63) / 64;
-    const int panels = d.taps * d.cchunks;
-    d.n_valid = panels * 64;
-    // panels per tile: fewest panel loads per pixel box over the whole product (2 dY panels + `per` patch panels
-    // for each of ceil(panels / per) tiles); ties go to the wider tile
-    int per = 1;
-    long long best_cost = -1;
-    for (int c = 1; c <= 4 && c <= panels; ++c) {
-      const long long cost = (long long)((panels + c - 1) / c) * (2 + c);
-      if (best_cost < 0 || cost <= best_cost) { best_cost = cost; per = c; }
-    }
-    d.bn = per * 64;
-    d.n_tiles = (panels + per - 1) / per;
+    d.n_valid = d.taps * d.cchunks * 64;
+    d.bn = plan.per * 64;
+    d.n_tiles = plan.n_tiles;
     d.zero_fill_c = d.cchunks * 64;
     ok = make_act_map(&ta, p->y, p->og, p->OW, p->OH, p->B, p->y_pitch, d.bw, d.bh, d.bnb);
     ok = ok && make_act_map(&tb, p->x, p->cg, p->W, p->H, p->B, p->x_pitch, d.bw, d.bh, d.bnb, false, d.stride);
     const long long wst[2] = {(long long)p->cg * 4, p->ldw * 4};
     const int wbox[3] = {32, 1, BM};
     ok = ok && make_map(&tc.m[0], p->w, 3, wdims, wst, wbox, true);
-    int split = p->split_k;
-    const long long tiles = (long long)d.m_tiles * d.n_tiles;
-    if (split <= 0) {
-      split = 1;
-      if (tiles < kSMs && d.kt_total >= 8) {
-        // the busiest SM walks `waves` slices, and each costs about eight k-tiles of time beside its own: filling the
-        // pipeline, and a read-modify-write of its part of the gradient.  That prefers one wave of longer slices where
-        // it fills the machine.  One wave against two, us: 256 x 13 x 13, 256 -> 384: 64.0, 66.6; 192 -> 128: 24.6, 27.7;
-        // 32 x 14 x 14, 128 -> 160: 13.3, 17.9; 100 x 32 x 32 stride 2, 80 -> 80: 16.4, 18.4
-        auto cost = [&](long long n) { return (tiles * n + kSMs - 1) / kSMs * ((d.kt_total + n - 1) / n + 8); };
-        const long long most = (2 * kSMs) / tiles < d.kt_total / 4 ? (2 * kSMs) / tiles : d.kt_total / 4;
-        for (long long n = 2; n <= most; ++n)
-          if (cost(n) < cost(split)) split = (int)n;
-      }
-    }
-    if (split > d.kt_total) split = d.kt_total;
-    if (split > 1) {
-      const int per_k = (d.kt_total + split - 1) / split;
-      split = (d.kt_total + per_k - 1) / per_k;      // every k-slice non-empty
-    }
+    const int split = plan.split;
     d.split_k = split;
     const long long kd = (long long)d.taps * p->cg;
     if (split > 1) {

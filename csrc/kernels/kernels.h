@@ -175,6 +175,7 @@ int geeps_conv_tc_supported(const GeepsConvTcParams* p);
 // chunk and the filter taps are shifted MMA-descriptor starts.  geeps_conv_tc() routes to it when applicable
 // (a negative split_k on a forward / data-gradient call keeps the call on the box kernel, -2 on its single CTAs).
 double geeps_conv_box_us(const GeepsConvTcParams* p);          // expected time of the box kernel, stride 1 (host arithmetic)
+double geeps_conv_box_wgrad_us(const GeepsConvTcParams* p);
 int geeps_conv_box_pairs(const GeepsConvTcParams* p);          // 1 if the box kernel runs p on CTA pairs
 int geeps_conv_halo_applicable(const GeepsConvTcParams* p);
 int geeps_conv_halo(const GeepsConvTcParams* p, void* stream);

@@ -528,3 +528,21 @@ def test_layers_off_128_byte_lines_agree_on_both_kernels(B, H, cg, og, k):
         assert _rel(out[0], out[1].double()) < 5e-4
     assert routed
 
+
+@pytest.mark.parametrize("B,H,cg,og,k", [(68, 53, 40, 208, 3), (41, 28, 136, 104, 5), (5, 26, 280, 200, 5), (37, 27, 168, 368, 3), (20, 47, 104, 112, 5),
+                                         (40, 28, 136, 72, 3), (95, 33, 64, 360, 5)])
+def test_weight_gradients_off_128_byte_lines_agree_on_both_kernels(B, H, cg, og, k):
+    """Layers that the expected times send to the filter-row kernel (and one that they keep off it), as conv_tc() runs them and on the
+    box kernel: the same products, summed in fp32 in other slices."""
+    from geeps_b200.ops import functional as F
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(H * cg)
+    ld = (k * k * cg + 7) // 8 * 8 + 8
+    x = torch.randn(B, H, H, cg, device=dev, generator=gen).to(BF)
+    dy = torch.randn(B, H, H, og, device=dev, generator=gen).to(BF)
+    out = [torch.full((og, ld), 3.0, device=dev) for _ in range(2)]
+    for o, split_k in zip(out, (0, -1)):
+        F.conv_tc(F.CONV_WGRAD, x, dy, o, k, k // 2, split_k=split_k)
+        assert (o[:, k * k * cg:] == 0).all()
+    # n additions of terms of norm one, each rounded by 2^-24 of a partial sum of norm at most sqrt(n): sqrt(n) 2^-24 of the result's
+    assert _rel(out[0], out[1].double()) < 2 * (B * H * H) ** 0.5 * 2.0 ** -24
