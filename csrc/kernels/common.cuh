@@ -150,6 +150,18 @@ __device__ __forceinline__ bool geeps_wait_ge(const int* flag, int expected, uin
 // 16-byte vector helpers
 __device__ __forceinline__ float4 ld_f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st_f4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+// Zeros to c[0, n) by the threads at, at + stride, ...: `head` single values up to a 16-byte boundary, vectors, the rest
+__device__ __forceinline__ void clear_range(float* c, long long n, int head, long long at, long long stride) {
+  if (at < head) c[at] = 0.f;
+  const long long n4 = (n - head) >> 2;
+  for (long long i = at; i < n4; i += stride) st_f4(c + head + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
+  const long long tail = head + 4 * n4;
+  if (at < n - tail) c[tail + at] = 0.f;
+}
+inline long long clear_head(const float* c, long long n) {
+  const long long head = ((16 - ((uintptr_t)c & 15)) & 15) / 4;
+  return head < n ? head : n;
+}
 __device__ __forceinline__ float4 ld_f4_nc_stream(const float* p) {
   float4 v;
   asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"

@@ -654,6 +654,10 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
 
 extern "C" {
 
+int geeps_conv_wgrad_adds(const GeepsConvTcParams* p) {
+  if (p->mode != MODE_WGRAD || !geeps_conv_tc_supported(p)) return 0;
+  return (p->split_k >= 0 && geeps_conv_wgrad_halo_applicable(p)) || plan_wgrad_box(p, geeps_sm_count()).split > 1;
+}
 int geeps_conv_tc(const GeepsConvTcParams* p, void* stream) {
   if (!geeps_conv_tc_supported(p)) return (int)cudaErrorInvalidValue;
   if (p->mode != MODE_WGRAD && p->split_k >= 0 && geeps_conv_halo_applicable(p)) return geeps_conv_halo(p, stream);
@@ -797,7 +801,7 @@ int conv_tc_run(const GeepsConvTcParams* p, const DgradClasses& cls, void* strea
     const long long kd = (long long)d.taps * p->cg;
     if (split > 1) {
       // partial sums are reduce-added: the whole [og][ldw] block starts at zero
-      int e = geeps_scale_matrix_f32((float*)p->w, p->og, p->ldw, p->ldw, 0.f, stream);
+      int e = p->cleared ? 0 : geeps_scale_matrix_f32((float*)p->w, p->og, p->ldw, p->ldw, 0.f, stream);
       if (e) return e;
     } else if (p->ldw > kd) {
       // the pad columns past the last tap are never stored: keep them at zero

@@ -402,7 +402,7 @@ int geeps_conv_wgrad_halo(const GeepsConvTcParams* p, void* stream) {
   ok = ok && make_map(&tw, p->w, true, 3, wdims, wst, wbox);
   if (!ok) return (int)cudaErrorInvalidValue;
   // every item reduce-adds: the whole [og][ldw] block starts at zero (pad columns past the last tap included)
-  int e = geeps_scale_matrix_f32((float*)p->w, p->og, p->ldw, p->ldw, 0.f, stream);
+  int e = p->cleared ? 0 : geeps_scale_matrix_f32((float*)p->w, p->og, p->ldw, p->ldw, 0.f, stream);
   if (e) return e;
   static bool attr_set = false;
   if (!attr_set) {

@@ -76,15 +76,10 @@ __global__ void scale_matrix_kernel(float* c, long long M, long long N, long lon
   }
 }
 
-// zeros, a matrix without gaps between its rows: `head` single values up to a 16-byte boundary, vectors, the rest
+// zeros, a matrix without gaps between its rows
 __global__ void __launch_bounds__(256) clear_kernel(float* c, long long n, int head) {
   geeps_pdl_enter();
-  const long long stride = (long long)gridDim.x * blockDim.x, at = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (at < head) c[at] = 0.f;
-  const long long n4 = (n - head) >> 2;
-  for (long long i = at; i < n4; i += stride) st_f4(c + head + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
-  const long long tail = head + 4 * n4;
-  if (at < n - tail) c[tail + at] = 0.f;
+  clear_range(c, n, head, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
 }  // namespace
@@ -105,8 +100,7 @@ int geeps_gemm_bf16_simt(const GeepsGemmParams* p, void* stream) {
 // for each value.
 int geeps_clear_f32(float* c, long long n, void* stream) {
   if (n <= 0) return 0;
-  long long head = ((16 - ((uintptr_t)c & 15)) & 15) / 4;
-  if (head > n) head = n;
+  const long long head = clear_head(c, n);
   long long blocks = ((n - head) / 4 + 255) / 256;
   if (blocks > geeps_sm_count() * 8) blocks = geeps_sm_count() * 8;
   if (blocks < 1) blocks = 1;

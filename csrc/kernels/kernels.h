@@ -168,6 +168,7 @@ typedef struct GeepsConvTcParams {
                 // element stride, the data gradient is stride * stride problems of stride 1, one per parity class of dX
   int columns;  // data gradient of the halo kernel: 0 by cost, 1 one image column per position, 2 column pairs (an error
                 // where they do not fit)
+  int cleared;  // weight gradient: 1, w holds zeros already (a gradient that is summed in slices clears it otherwise)
 } GeepsConvTcParams;
 int geeps_conv_tc(const GeepsConvTcParams* p, void* stream);
 int geeps_conv_tc_supported(const GeepsConvTcParams* p);
@@ -182,6 +183,7 @@ int geeps_conv_halo(const GeepsConvTcParams* p, void* stream);
 // Weight gradient with the taps of a filter row served by one activation tile (conv_wgrad_halo.cu); same routing.
 int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p);
 int geeps_conv_wgrad_halo(const GeepsConvTcParams* p, void* stream);
+int geeps_conv_wgrad_adds(const GeepsConvTcParams* p);         // 1 if geeps_conv_tc() adds p's weight gradient to zeros in w
 // The geometry these kernels would use for a call (host arithmetic only; for tests and tuning).  `ok` = 0 when
 // the kernel does not accept the call.
 typedef struct GeepsHaloPlanInfo {

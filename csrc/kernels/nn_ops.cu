@@ -663,11 +663,15 @@ f32_to_bf16_2d_kernel(const float* __restrict__ src, bf16* __restrict__ dst, lon
 // ReLU backward fused with the per-channel sums of its result (the bias gradient of the layer whose output y is):
 // dx = y > 0 ? dy : 0, out[c] += sum over pixels of dx.  Four blocks per SM with eight pixels of a thread in flight; eight with
 // four: 43264 x 384 22.3 us, 18.0 now, 43264 x 256 16.4, 12.4, 186624 x 256 53.4, 50.9 (of which 44 are the bytes).
+// `clear`: the weight gradient that the next kernels add to, zeroed on the way.
 __global__ void __launch_bounds__(256)
 relu_backward_colsum_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ y, bf16* __restrict__ dx,
-                            float* __restrict__ out, long long P, int C, long long lddy, long long ldy, long long lddx) {
+                            float* __restrict__ out, long long P, int C, long long lddy, long long ldy, long long lddx,
+                            float* __restrict__ clear, long long clear_n, int clear_head) {
   geeps_pdl_enter();
   extern __shared__ __align__(16) float sacc[];  // [rows][8 * slots]
+  clear_range(clear, clear_n, clear_head, ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x,
+              (long long)gridDim.y * gridDim.x * blockDim.x);
   const SlotMap m(C);
   float a[8];
 #pragma unroll
@@ -2097,14 +2101,24 @@ int geeps_relu_backward_2d(const void* dy, const void* y, void* dx, long long P,
                                                                                  (bf16*)dx, P, C, lddy, ldy, lddx);
   return CK();
 }
+// Zeros to the clear_n values at `clear` as well: on the way in a short pass, where a launch for them in front of each group's
+// weight gradient costs more than its bytes (backward passes of layers, us, a launch each / so: 1000 x 48 from 80 channels
+// 15.5 / 13.7, two groups 1922 x 96 from 128 31.2 / 27.2, 6100 x 232 from 88 32.0 / 29.8, 22275 x 176 from 40 49.9 / 46.8).
+// After a long pass they keep a launch, one for all groups: the blocks of a weight gradient that follows it directly come up
+// in the order in which its blocks leave, on other SMs than the tiles they share lie well on (44800 x 264 from 144, 5 x 5
+// 295.5 us, 306.3 without the launch; 93600 x 352 from 88 632, 650; though 43264 x 384 from 256 145.8, 143.2).
 int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* colsum, long long P, int C,
-                               long long lddy, long long ldy, long long lddx, void* stream) {
-  if (C % 8 || lddy % 8 || ldy % 8 || lddx % 8 || C > 8192) return (int)cudaErrorInvalidValue;
+                               long long lddy, long long ldy, long long lddx, float* clear, long long clear_n, void* stream) {
+  if (C % 8 || lddy % 8 || ldy % 8 || lddx % 8 || C > 8192 || clear_n < 0 || (clear_n > 0 && !clear)) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   geeps_clear_f32(colsum, C, st);
+  const bool apart = P * C > (1LL << 22);
+  float* const along = apart ? nullptr : clear;
+  const long long along_n = apart ? 0 : clear_n;
   const SlotGrid rg = slot_grid(P, C, 4, 4, 1);
   geeps_launch_plain(relu_backward_colsum_kernel, rg.grid, rg.threads, rg.smem, st,
-      (const bf16*)dy, (const bf16*)y, (bf16*)dx, colsum, P, C, lddy, ldy, lddx);
+      (const bf16*)dy, (const bf16*)y, (bf16*)dx, colsum, P, C, lddy, ldy, lddx, along, along_n, (int)clear_head(along, along_n));
+  if (apart && clear_n > 0) geeps_clear_f32(clear, clear_n, st);
   return CK();
 }
 int geeps_f32_to_bf16_2d(const float* src, void* dst, long long P, int C, long long lds, long long ldd, int relu,

@@ -67,7 +67,7 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
 // out[c] (+)= scale * sum_p x[p][c]
 // dx = y > 0 ? dy : 0 and colsum[c] = sum over the P pixels of dx (C % 8 == 0, C <= 8192), one pass
 int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* colsum, long long P, int C,
-                               long long lddy, long long ldy, long long lddx, void* stream);
+                               long long lddy, long long ldy, long long lddx, float* clear, long long clear_n, void* stream);
 int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, float scale, int zero_first,
                  void* stream);
 int geeps_relu_backward(const void* dy, const void* y, void* dx, long long n, void* stream);

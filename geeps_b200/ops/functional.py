@@ -70,12 +70,14 @@ CONV_FWD, CONV_DGRAD, CONV_WGRAD = 0, 1, 2
 
 def conv_tc_params(mode: int, x: torch.Tensor, y: torch.Tensor, w: torch.Tensor, k: int, pad: int, *,
                    bias: torch.Tensor | None = None, relu: bool = False, split_k: int = 0,
-                   status: torch.Tensor | None = None, stride: int = 1, columns: int = 0) -> ConvTcParams:
+                   status: torch.Tensor | None = None, stride: int = 1, columns: int = 0,
+                   cleared: bool = False) -> ConvTcParams:
     """Arguments of the implicit-GEMM convolution (stride 1 .. 8; the data gradient of a strided layer needs a
     filter at least as wide as the stride).  x: [B, H, W, cg] and y: [B, OH, OW, og] are NHWC
     bf16 tensors or channel slices of wider ones (last-dim stride 1, dense pixels); w: [og, ldw] with column
     (kh * k + kw) * cg + ci, bf16 for forward / data gradient, fp32 (the gradient) for the weight gradient.  columns: a
-    data gradient on the halo kernel by single columns (1) or column pairs (2), 0 = whichever costs less."""
+    data gradient on the halo kernel by single columns (1) or column pairs (2), 0 = whichever costs less.  cleared: w, the
+    weight gradient to write, holds zeros already."""
     B, H, W, cg = x.shape
     _, OH, OW, og = y.shape
     assert x.stride(3) == 1 and y.stride(3) == 1 and w.stride(1) == 1
@@ -89,7 +91,7 @@ def conv_tc_params(mode: int, x: torch.Tensor, y: torch.Tensor, w: torch.Tensor,
     p.x_pitch, p.y_pitch, p.ldw = xp, yp, w.stride(0)
     p.B, p.H, p.W, p.cg, p.OH, p.OW, p.og = B, H, W, cg, OH, OW, og
     p.KH, p.KW, p.pad, p.relu, p.mode, p.split_k = k, k, pad, int(relu), mode, split_k
-    p.stride, p.columns = stride, columns
+    p.stride, p.columns, p.cleared = stride, columns, int(cleared)
     return p
 
 
@@ -106,6 +108,11 @@ def conv_tc(mode: int, x, y, w, k: int, pad: int, **kw) -> None:
     assert w.dtype == (torch.float32 if mode == CONV_WGRAD else bf16)
     p = conv_tc_params(mode, x, y, w, k, pad, **kw)
     launch(lib().geeps_conv_tc, "conv_tc", C.byref(p), stream_ptr())
+
+
+def conv_wgrad_adds(x, dy, dw, k: int, pad: int, **kw) -> bool:
+    """Does conv_tc() add this weight gradient to zeros, which it puts there first unless told that dw is `cleared`?"""
+    return bool(lib().geeps_conv_wgrad_adds(C.byref(conv_tc_params(CONV_WGRAD, x, dy, dw, k, pad, **kw))))
 
 
 def conv_halo_applicable(p: ConvTcParams) -> bool:
@@ -259,12 +266,19 @@ def relu_backward_2d(dy2d, y2d, dx2d) -> None:
                                        C.c_longlong(_ld(y2d)), C.c_longlong(_ld(dx2d)), stream_ptr())
 
 
-def relu_backward_colsum(dy2d, y2d, dx2d, colsum_out) -> None:
-    """dx = dy where y > 0 else 0, and colsum_out[c] = sum of dx over the rows, in one pass."""
+def clear_f32(t) -> None:
+    assert t.dtype == torch.float32 and t.is_contiguous()
+    launch(lib().geeps_clear_f32, "clear_f32", ptr(t), C.c_longlong(t.numel()), stream_ptr())
+
+
+def relu_backward_colsum(dy2d, y2d, dx2d, colsum_out, clear: torch.Tensor | None = None) -> None:
+    """dx = dy where y > 0 else 0, and colsum_out[c] = sum of dx over the rows, in one pass, which also zeroes `clear`."""
     P, Cc = dy2d.shape
     assert colsum_out.dtype == torch.float32 and colsum_out.numel() == Cc and colsum_out.is_contiguous()
+    assert clear is None or clear.dtype == torch.float32 and clear.is_contiguous()
     launch(lib().geeps_relu_backward_colsum, "relu_backward_colsum", ptr(dy2d), ptr(y2d), ptr(dx2d), ptr(colsum_out),
-           C.c_longlong(P), Cc, C.c_longlong(_ld(dy2d)), C.c_longlong(_ld(y2d)), C.c_longlong(_ld(dx2d)), stream_ptr())
+           C.c_longlong(P), Cc, C.c_longlong(_ld(dy2d)), C.c_longlong(_ld(y2d)), C.c_longlong(_ld(dx2d)),
+           ptr(clear), C.c_longlong(0 if clear is None else clear.numel()), stream_ptr())
 
 
 def stream_order(src_stream, dst_stream, event) -> None:

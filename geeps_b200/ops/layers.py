@@ -315,10 +315,13 @@ class Conv2d(Layer):
         # dy: [M, cout] bf16 (possibly a slice view of a wider tensor)
         if dy.dim() != 2:
             dy = dy.view(self.M, self.cout)
-        bias_done = False
+        aside = self.wgrad_side is not None and self.need_dx
+        bias_done, clear = False, None
         if self.relu and not self.dy_is_masked:
             if self.has_bias and self.bias_grad_src is None and self.cout % 8 == 0 and self.cout <= 8192:
-                dy = self._relu_mask(dy, colsum=self.g32["bias"])     # mask and bias gradient in one pass
+                # mask and bias gradient in one pass, which also puts the zeros that the weight gradient is added to
+                clear = None if aside else self._gradient_to_clear(self._masked())
+                dy = self._relu_mask(dy, colsum=self.g32["bias"], clear=clear)
                 bias_done = True
             else:
                 dy = self._relu_mask(dy)
@@ -327,7 +330,7 @@ class Conv2d(Layer):
                 F.copy_f32(self.g32["bias"], self.bias_grad_src)
             else:
                 F.colsum(dy, self.g32["bias"])
-        if self.wgrad_side is not None and self.need_dx:
+        if aside:
             # nothing of this pass waits for the weight gradient: it runs beside what follows the data gradient
             side, event = self.wgrad_side
             F.stream_order(torch.cuda.current_stream(self.device), side, event)
@@ -335,18 +338,31 @@ class Conv2d(Layer):
             with torch.cuda.stream(side):
                 self._weight_gradient(dy)
             return self.dx
+        if clear is None and self.groups > 1:
+            clear = self._gradient_to_clear(dy)               # one launch for all groups
+            if clear is not None:
+                F.clear_f32(clear)
         for g in range(self.groups):
-            self._weight_gradient(dy, g)
+            self._weight_gradient(dy, g, cleared=clear is not None)
             if self.need_dx:
                 self._data_gradient(dy, g)
         return self.dx
 
-    def _weight_gradient(self, dy, group=None):
+    def _gradient_to_clear(self, dy):
+        """The weight gradient if its groups are added to zeros."""
+        gw = self.g32["weight"]
+        if not self.implicit or not gw.is_contiguous():
+            return None
+        rows = slice(0, self.og)
+        return gw if F.conv_wgrad_adds(self._x4(self.x, 0), self._y4(dy, 0), gw[rows], self.k, self.pad, stride=self.stride) else None
+
+    def _weight_gradient(self, dy, group=None, cleared=False):
         gw = self.g32["weight"]
         for g in range(self.groups) if group is None else (group,):
             rows = slice(g * self.og, (g + 1) * self.og)
             if self.implicit:
-                F.conv_tc(F.CONV_WGRAD, self._x4(self.x, g), self._y4(dy, g), gw[rows], self.k, self.pad, stride=self.stride)
+                F.conv_tc(F.CONV_WGRAD, self._x4(self.x, g), self._y4(dy, g), gw[rows], self.k, self.pad, stride=self.stride,
+                          cleared=cleared)
                 continue
             a = self.x.view(self.M, -1) if self.pointwise else self.cols[g]
             # dW_g[og, ld] = dy_g^T @ col_g      (both operands stored K-outermost)
@@ -366,14 +382,18 @@ class Conv2d(Layer):
                 F.gemm(dy[:, rows], w16[rows], self.dcol, b_mn=True)
                 F.col2im(self.dcol, self.dx, self.geoms[g])
 
-    def _relu_mask(self, dy, colsum=None):
+    def _masked(self):
         if not hasattr(self, "_dy_masked"):
             self._dy_masked = torch.empty(self.M, self.cout, dtype=BF, device=self.device)
-        if colsum is not None:
-            F.relu_backward_colsum(dy, self.y, self._dy_masked, colsum)
-        else:
-            F.relu_backward_2d(dy, self.y, self._dy_masked)
         return self._dy_masked
+
+    def _relu_mask(self, dy, colsum=None, clear=None):
+        masked = self._masked()
+        if colsum is not None:
+            F.relu_backward_colsum(dy, self.y, masked, colsum, clear=clear)
+        else:
+            F.relu_backward_2d(dy, self.y, masked)
+        return masked
 
 
 class Linear(Layer):

@@ -546,3 +546,36 @@ def test_weight_gradients_off_128_byte_lines_agree_on_both_kernels(B, H, cg, og,
         assert (o[:, k * k * cg:] == 0).all()
     # n additions of terms of norm one, each rounded by 2^-24 of a partial sum of norm at most sqrt(n): sqrt(n) 2^-24 of the result's
     assert _rel(out[0], out[1].double()) < 2 * (B * H * H) ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("B,H,cin,cout,k,groups,masked", [(64, 27, 96, 256, 5, 2, False), (64, 27, 96, 256, 5, 2, True), (50, 13, 128, 96, 3, 2, False),
+                                                          (20, 13, 64, 200, 3, 1, False), (1, 7, 32, 48, 3, 2, True), (2, 8, 16, 8, 1, 1, False)])
+def test_layer_gradient_is_cleared_once(B, H, cin, cout, k, groups, masked):
+    """Weight gradients whose zeros come with the ReLU mask or from one launch for all groups, and such that need none (summed
+    in one piece, 1 x 1): two backward passes over a gradient that held other values; whole numbers, so every sum is exact."""
+    from geeps_b200.ops import functional as F
+    from geeps_b200.ops.layers import Conv2d
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(B + cout)
+    rnd = lambda *s: torch.randint(-1, 2, s, device=dev, generator=gen).to(BF)      # noqa: E731
+    layer = Conv2d("c", cout, k, pad=k // 2, groups=groups, relu=True)
+    layer.setup((B, H, H, cin), dev)
+    shapes = {s.name.split(".")[-1]: s.shape for s in layer.param_specs()}
+    (wname, wshape), (bname, bshape) = shapes.items()
+    layer.p16["weight"], layer.p32["bias"] = rnd(*wshape), torch.zeros(bshape, device=dev)
+    layer.g32["weight"], layer.g32["bias"] = torch.full(wshape, 5.0, device=dev), torch.full(bshape, 5.0, device=dev)
+    x, dy = rnd(B, H, H, cin), rnd(B * H * H, cout)
+    y = layer.forward(x).view(B * H * H, cout)
+    dz = dy if masked else torch.where(y > 0, dy, torch.zeros_like(dy))
+    if masked:
+        layer.dy_is_masked, layer.bias_grad_src = True, dz.float().sum(0)
+    ref = torch.full(wshape, 3.0, device=dev)
+    cg, og = cin // groups, cout // groups
+    for g in range(groups):
+        if k == 1:
+            ref[:, :cin] = dz.float().t() @ x.float().view(-1, cin)
+        else:
+            F.conv_tc(F.CONV_WGRAD, x[..., g * cg:(g + 1) * cg], dz.view(B, H, H, cout)[..., g * og:(g + 1) * og], ref[g * og:(g + 1) * og], k, k // 2)
+    for _ in range(2):
+        layer.backward(dy)
+        assert torch.equal(layer.g32["weight"], ref) and torch.equal(layer.g32["bias"], dz.float().sum(0))

@@ -625,6 +625,21 @@ def test_clear_covers_exactly_its_range(off, n):
     assert (buf[:4 + off] == 2).all() and (buf[4 + off + n:] == 2).all()
 
 
+@pytest.mark.parametrize("off,n", [(0, 1), (1, 2), (3, 4), (2, 1023), (0, 614400), (1, 5_000_001)])
+@pytest.mark.parametrize("P,C", [(3, 8), (5000, 384), (11000, 384)])
+def test_relu_backward_clears_a_range_on_the_way(off, n, P, C):
+    """Fewer and more values than the launch has threads, off 16-byte boundaries, and a pass that leaves them to a launch of their
+    own: the range, nothing beside it, and the results of
+    a call without one."""
+    dy, y = torch.randn(P, C, device=DEV).to(BF), torch.randn(P, C, device=DEV).to(BF)
+    buf = torch.full((n + 16,), 2.0, device=DEV)
+    dx, cs = [torch.empty_like(y) for _ in range(2)], [torch.empty(C, device=DEV) for _ in range(2)]
+    F.relu_backward_colsum(dy, y, dx[0], cs[0])
+    F.relu_backward_colsum(dy, y, dx[1], cs[1], clear=buf[4 + off:4 + off + n])
+    assert torch.equal(dx[0], dx[1]) and torch.allclose(cs[0], cs[1], atol=1e-3 * P ** 0.5, rtol=0)
+    assert (buf[4 + off:4 + off + n] == 0).all() and (buf[:4 + off] == 2).all() and (buf[4 + off + n:] == 2).all()
+
+
 @pytest.mark.parametrize("B,H,Cc,pad,ldy", [(64, 29, 8, 0, 8), (61, 31, 8, 1, 8), (40, 13, 120, 0, 136), (9, 61, 40, 1, 40),
                                             (3, 27, 240, 0, 240), (2, 28, 312, 0, 312), (100, 14, 88, 1, 88),
                                             (260, 27, 32, 0, 32), (24, 55, 296, 0, 296), (36, 15, 520, 0, 520)])
