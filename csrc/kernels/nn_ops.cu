@@ -369,13 +369,22 @@ __device__ __forceinline__ void channel_reduce_body(const bf16* __restrict__ x, 
 // 22.0, 25088 x 320 32.2 -> 28.7, 25600 x 144 22.8 -> 20.0, 50000 x 48 18.1 -> 15.7, 6272 x 160 12.8 -> 11.8; one block per SM
 // with eight pixels of the sums 62.1, 20.9, 28.3, 18.4, 16.4, 12.8.
 constexpr int kChannelBlocks = 2;
+// The kernels of a BatchNorm fill the SMs' registers.  Blocks of the next one that come up while the last of this are running
+// lie two to the SMs that were done first, and its own end is as ragged, so over a large tensor they wait for the end.
+// Forward and backward, us, next blocks at once / at the end: 100352 x 192 57.5 / 55.4, x 128 37.4 / 33.8, x 64 22.1 / 21.2,
+// 300000 x 32 28.1 / 26.5, 25088 x 320 29.2 / 27.7, x 192 22.1 / 21.7, 6272 x 160 12.2 / 12.3.  In a module of branches the
+// small ones lose by it, since other branches have the SMs meanwhile (32 x 14 x 14 178.4 / 181.3, 7 x 7 99.4 / 104.9).
+__device__ __forceinline__ void batchnorm_enter(long long P, int C) {
+  geeps_pdl_wait();
+  if (P * C <= 5LL << 20) geeps_pdl_trigger();
+}
 enum { MASK_NONE = 0, MASK_Y = 1, MASK_BITS = 2 };      // what the backward pass reads a ReLU mask from
 template <int MODE>
 __global__ void __launch_bounds__(256, kChannelBlocks)
 channel_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const bf16* __restrict__ y,
                       const float* __restrict__ mean_rstd, float* __restrict__ out, long long P, int C,
                       long long ldx, long long lddy, int relu, float scale) {
-  geeps_pdl_enter();
+  if (MODE == 2) geeps_pdl_enter(); else batchnorm_enter(P, C);
   channel_reduce_body<MODE>(x, dy, y, mean_rstd, out, P, C, ldx, lddy, relu, scale);
 }
 
@@ -493,7 +502,7 @@ bn_apply_fused_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const fl
                       float* __restrict__ mean_rstd, float* running_mean, float* running_var,
                       const float* __restrict__ gamma, const float* __restrict__ beta, float* zero_after, long long P,
                       int C, long long ldx, long long ldy, int relu, float inv_count, float eps, float momentum, uint8_t* bits) {
-  geeps_pdl_enter();
+  batchnorm_enter(P, C);
   bn_apply_fused_body(x, y, sums, mean_rstd, running_mean, running_var, gamma, beta, zero_after, P, C, ldx, ldy, relu,
                       inv_count, eps, momentum, bits);
 }
@@ -554,7 +563,7 @@ bn_backward_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, cons
                    bf16* __restrict__ dx, const float* __restrict__ mean_rstd, const float* __restrict__ gamma,
                    const float* __restrict__ sums, float* dgamma, float* dbeta, long long P, int C,
                    long long ldx, long long lddy, long long lddx, int relu, float grad_scale, float* zero_after) {
-  geeps_pdl_enter();
+  batchnorm_enter(P, C);
   bn_backward_body<MASK>(x, dy, y, dx, mean_rstd, gamma, sums, dgamma, dbeta, P, C, ldx, lddy, lddx, relu, grad_scale,
                          zero_after);
 }

@@ -625,6 +625,32 @@ def test_clear_covers_exactly_its_range(off, n):
     assert (buf[:4 + off] == 2).all() and (buf[4 + off + n:] == 2).all()
 
 
+@pytest.mark.parametrize("P,C", [(81920, 64), (81921, 64), (30000, 200)])
+def test_batchnorm_passes_one_after_the_other(P, C):
+    """Tensors on both sides of the size from which a pass lets the next one in only at its end: three forward and backward
+    passes back to back, the last one's results against the formulas in fp32."""
+    torch.manual_seed(P)
+    x, dy = (torch.randn(P, C, device=DEV).to(BF) for _ in range(2))
+    y, dx, bits = torch.empty_like(x), torch.empty_like(x), torch.empty(P, C // 8, dtype=torch.uint8, device=DEV)
+    g, b = 1 + 0.1 * torch.randn(C, device=DEV), 0.1 * torch.randn(C, device=DEV)
+    s, sb, mr = torch.zeros(2 * C, device=DEV), torch.zeros(2 * C, device=DEV), torch.empty(2 * C, device=DEV)
+    rm, rv, dg, db = torch.zeros(C, device=DEV), torch.ones(C, device=DEV), torch.empty(C, device=DEV), torch.empty(C, device=DEV)
+    bar = torch.zeros(8, dtype=torch.int32, device=DEV)
+    for _ in range(3):
+        F.bn_forward_fused(x, y, g, b, s, mr, rm, rv, zero_after=sb, barrier=bar[0:4], eps=1e-5, momentum=0.1, relu=True, bits=bits)
+        F.bn_backward_fused(x, dy, y, dx, mr, g, sb, dg, db, zero_after=s, barrier=bar[4:8], relu=True, bits=bits)
+    xf = x.float()
+    mean, rstd = xf.mean(0), (xf.var(0, unbiased=False) + 1e-5).rsqrt()
+    xh = (xf - mean) * rstd
+    dz = torch.where(y > 0, dy.float(), torch.zeros((), device=DEV))
+    # results are rounded to bf16 once: 2^-8 of a value, of which half is the bound
+    assert ((y.float() - torch.relu(xh * g + b)).norm() / y.float().norm()).item() < 2.0 ** -8
+    want = g * rstd * (dz - dz.mean(0) - xh * (dz * xh).mean(0))
+    assert ((dx.float() - want).norm() / want.norm()).item() < 2.0 ** -8
+    # sums of P terms of fp32 in some order: sqrt(P) 2^-24 of the terms' norm each way
+    assert (dg - (dz * xh).sum(0)).abs().max().item() < 1e-4 * P ** 0.5 and (db - dz.sum(0)).abs().max().item() < 1e-4 * P ** 0.5
+
+
 @pytest.mark.parametrize("off,n", [(0, 1), (1, 2), (3, 4), (2, 1023), (0, 614400), (1, 5_000_001)])
 @pytest.mark.parametrize("P,C", [(3, 8), (5000, 384), (11000, 384)])
 def test_relu_backward_clears_a_range_on_the_way(off, n, P, C):
