@@ -52,7 +52,8 @@ __device__ __forceinline__ void geeps_pdl_wait() { asm volatile("griddepcontrol.
 // The blocks of the next kernel may start, as far as there is room for them, once every block has called this (or left).
 // Called before the wait of its own kernel has returned it would let a third kernel in; all kernels call it after.
 // Where it stands: in the tensor-core kernels behind the last load of a block, whose shared memory leaves no room for
-// another block before (the pair GEMM has none: its successor comes up when it ends); in the others at the start.
+// another block before (the pair GEMM has none: its successor comes up when it ends); in the others at the start, except the
+// passes of a BatchNorm over a large tensor (batchnorm_enter).
 __device__ __forceinline__ void geeps_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void geeps_pdl_enter() { geeps_pdl_wait(); geeps_pdl_trigger(); }
 

@@ -1502,6 +1502,62 @@ maxpool_backward_smem_kernel(const bf16* __restrict__ dy, const uint8_t* __restr
     }
   }
 }
+// 3 x 3 windows at stride 2: the four pixels of a quad (even padded row and column first) lie in four windows, which a thread
+// loads once, all at a time, for 8 channels.  No shared memory to fill first, so nothing waits for a block's slowest load;
+// each pixel adds its windows in the order of the other kernels.  us, windows staged in shared memory / so: 256 x 13 x 13 x 256
+// 21.1 / 9.6 (the bytes 4.5), 100 x 13 x 13 x 256 11.4 / 5.4, 8 x 13 x 13 x 256 7.9 / 3.0, 32 x 14 x 14 x 576 15.9 / 4.2, 32 x
+// 56 x 56 x 64 15.2 / 6.4.
+__global__ void __launch_bounds__(256)
+maxpool3s2_backward_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ argmax, bf16* __restrict__ dx,
+                           const GeepsPoolGeom g, int accumulate, unsigned quads_h, unsigned quads_w, unsigned total) {
+  geeps_pdl_enter();
+  const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
+  if (item >= total) return;
+  const unsigned cv = (unsigned)g.C >> 3;
+  const unsigned q = item / cv, row = q / quads_w, b = row / quads_h;
+  const int c = (int)(item - q * cv) * 8;
+  const int wr = (g.pad >> 1) + (int)(row - b * quads_h), wc = (g.pad >> 1) + (int)(q - row * quads_w);   // last windows of the quad
+  uint4 d[2][2];
+  uint2 k[2][2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int oh = wr - 1 + r, ow = wc - 1 + s;
+      d[r][s] = make_uint4(0, 0, 0, 0);
+      k[r][s] = make_uint2(0xffffffffu, 0xffffffffu);      // no element of a window
+      if (oh >= 0 && oh < g.OH && ow >= 0 && ow < g.OW) {
+        const long long opix = ((long long)b * g.OH + oh) * g.OW + ow;
+        d[r][s] = *reinterpret_cast<const uint4*>(dy + opix * g.ldy + c);
+        k[r][s] = *reinterpret_cast<const uint2*>(argmax + opix * g.C + c);
+      }
+    }
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int ih = 2 * wr + u - g.pad, iw = 2 * wc + v - g.pad;
+      if (ih < 0 || ih >= g.H || iw < 0 || iw >= g.W) continue;
+      __nv_bfloat162 acc[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j] = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+      for (int r = u; r < 2; ++r)           // an odd row is the middle of one window, an even one the last and first of two
+#pragma unroll
+        for (int s = v; s < 2; ++s) {
+          const int kh = u ? 1 : 2 - 2 * r, kw = v ? 1 : 2 - 2 * s;
+          pool_bwd_accum(acc, k[r][s], d[r][s], (uint32_t)(kh * 3 + kw));
+        }
+      bf16* dst = dx + (((long long)b * g.H + ih) * g.W + iw) * g.ldx + c;
+      if (accumulate) {
+        const uint4 old = *reinterpret_cast<const uint4*>(dst);
+        const uint32_t ov[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] = __hadd2(acc[j], *reinterpret_cast<const __nv_bfloat162*>(&ov[j]));
+      }
+      *reinterpret_cast<uint4*>(dst) = pool_bwd_pack(acc);
+    }
+}
 
 // Caffe average pooling: divisor is the window area clipped to the padded extent.
 __device__ __forceinline__ int avg_area(int o, int stride, int pad, int K, int size) {
@@ -2216,7 +2272,16 @@ int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolG
 int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const GeepsPoolGeom* g, int accumulate,
                            void* stream) {
   if (g->C % 8 || g->ldx % 8 || g->ldy % 8) return (int)cudaErrorInvalidValue;
-  // overlapping windows: stage the covering output rows in shared memory when they fit
+  if (g->K == 3 && g->stride == 2 && g->pad >= 0 && g->H > 0 && g->W > 0) {
+    const long long qh = ((g->H + g->pad - 1) >> 1) - (g->pad >> 1) + 1, qw = ((g->W + g->pad - 1) >> 1) - (g->pad >> 1) + 1;
+    const long long total = g->B * qh * qw * (g->C / 8);
+    if (total > 0 && total < (1LL << 31)) {
+      geeps_launch_plain(maxpool3s2_backward_kernel, (int)((total + 255) / 256), 256, 0, (cudaStream_t)stream, (const bf16*)dy,
+          (const uint8_t*)argmax, (bf16*)dx, *g, accumulate, (unsigned)qh, (unsigned)qw, (unsigned)total);
+      return CK();
+    }
+  }
+  // other overlapping windows: stage the covering output rows in shared memory when they fit
   const int rows_per_block = g->stride > 1 ? 2 * g->stride : 2;
   const int max_oh = (rows_per_block + g->K - 2) / g->stride + 1;
   const size_t smem = (size_t)max_oh * g->OW * g->C * 3;

@@ -625,6 +625,31 @@ def test_clear_covers_exactly_its_range(off, n):
     assert (buf[:4 + off] == 2).all() and (buf[4 + off + n:] == 2).all()
 
 
+@pytest.mark.parametrize("B,H,W,C,pad,extra", [(1, 3, 4, 8, 0, 0), (2, 4, 3, 8, 0, 8), (3, 13, 13, 256, 0, 0), (2, 14, 9, 24, 1, 16), (2, 5, 12, 40, 2, 0),
+                                               (1, 3, 3, 8, 1, 0), (5, 57, 30, 136, 0, 8)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_maxpool_backward_by_quads(B, H, W, C, pad, extra, accumulate):
+    """3 x 3 windows at stride 2, even and odd sizes and pads, pitched tensors: the sums of bf16 in the order of the windows."""
+    torch.manual_seed(H * C)
+    x = torch.randn(B, H, W, C + extra, device=DEV).to(BF)[..., :C]
+    g = F.pool_geom((B, H, W, C), 3, 2, pad, C + extra, C + extra)
+    y = torch.empty(B, g.OH, g.OW, C + extra, dtype=BF, device=DEV)[..., :C]
+    arg = torch.empty(B, g.OH, g.OW, C, dtype=torch.uint8, device=DEV)
+    F.maxpool_forward(x, y, arg, g)
+    dy = torch.randn(B, g.OH, g.OW, C + extra, device=DEV).to(BF)[..., :C]
+    wide = torch.randn(B, H, W, C + extra, device=DEV).to(BF)
+    before = wide.clone()
+    F.maxpool_backward(dy, arg, wide[..., :C], g, accumulate=accumulate)
+    acc = torch.zeros(B, H + 2 * pad + 4, W + 2 * pad + 4, C, dtype=BF, device=DEV)       # padded image; windows may end past it
+    for kh in (2, 1, 0):
+        for kw in (2, 1, 0):
+            view = acc[:, kh:kh + 2 * g.OH:2, kw:kw + 2 * g.OW:2]
+            view += torch.where(arg == kh * 3 + kw, dy, torch.zeros_like(dy))
+    want = acc[:, pad:pad + H, pad:pad + W]
+    assert torch.equal(wide[..., :C], want + before[..., :C] if accumulate else want)
+    assert torch.equal(wide[..., C:], before[..., C:])
+
+
 @pytest.mark.parametrize("P,C", [(81920, 64), (81921, 64), (30000, 200)])
 def test_batchnorm_passes_one_after_the_other(P, C):
     """Tensors on both sides of the size from which a pass lets the next one in only at its end: three forward and backward
