@@ -102,7 +102,9 @@ int geeps_lrn_maxpool_forward(const void* x, void* p, void* argmax, const GeepsP
                               float beta, float k, void* stream);
 int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax, void* dx, const GeepsPoolGeom* g,
                                int size, float alpha, float beta, float k, int relu_mask, float* colsum, void* stream);
-int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream);
+// relu_mask: a window whose maximum is not above zero gets code 255, so the backward pass hands its gradient to nobody:
+// the mask of a ReLU that x is the output of
+int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, int relu_mask, void* stream);
 int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const GeepsPoolGeom* g, int accumulate,
                            void* stream);
 // launch shape of a reduction over P pixels of C channels (host arithmetic only): channel shares, pixel shares, threads a

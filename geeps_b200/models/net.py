@@ -202,7 +202,8 @@ class Net:
         self.loss_layer.setup(s, device)
         self.device = device
         # conv + ReLU followed by LRN: the LRN backward already reads the ReLU output, so it applies the ReLU
-        # mask to the gradient it hands down and the convolution skips its own masking pass
+        # mask to the gradient it hands down and the convolution skips its own masking pass; a max pooling knows the mask from
+        # its own maxima
         for a, b in zip(self.layers, self.layers[1:]):
             if isinstance(a, Conv2d) and a.relu and isinstance(b, (LRN, LRNMaxPool)):
                 a.dy_is_masked, b.mask_relu_input = True, True
@@ -210,6 +211,8 @@ class Net:
                     # the same pass also sums the masked gradient per channel: the convolution's bias gradient
                     b.bias_grad = torch.zeros(b.C, device=device)
                     a.bias_grad_src = b.bias_grad
+            elif isinstance(a, Conv2d) and a.relu and isinstance(b, Pool) and b.kind == "max":
+                a.dy_is_masked, b.mask_relu_input = True, True
         return s
 
     def num_params(self, valid_only=True):

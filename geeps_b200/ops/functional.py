@@ -386,8 +386,10 @@ def pool_geom(x_shape, k: int, stride: int, pad: int, ldx: int, ldy: int, ceil_m
     return g
 
 
-def maxpool_forward(x, y, argmax, g: PoolGeom) -> None:
-    launch(lib().geeps_maxpool_forward, "maxpool_forward", ptr(x), ptr(y), ptr(argmax), C.byref(g), stream_ptr())
+def maxpool_forward(x, y, argmax, g: PoolGeom, relu_mask: bool = False) -> None:
+    """relu_mask: x is the output of a ReLU, whose mask maxpool_backward() then applies as well: windows without a positive
+    value name no element (code 255)."""
+    launch(lib().geeps_maxpool_forward, "maxpool_forward", ptr(x), ptr(y), ptr(argmax), C.byref(g), int(relu_mask), stream_ptr())
 
 
 def maxpool_backward(dy, argmax, dx, g: PoolGeom, accumulate=False) -> None:

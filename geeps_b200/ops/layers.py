@@ -633,6 +633,7 @@ class Pool(Layer):
     def __init__(self, kind, k, stride, pad=0, ceil_mode=True):
         super().__init__()
         self.kind, self.k, self.stride, self.pad, self.ceil_mode = kind, k, stride, pad, ceil_mode
+        self.mask_relu_input = False    # set by Net when the producer's ReLU backward is folded into this layer's
 
     def setup(self, in_shape, device):
         B, H, W, C = in_shape
@@ -659,7 +660,7 @@ class Pool(Layer):
             self.y = torch.empty(self.out_shape, dtype=BF, device=self.device)
         self.g.ldx = x.stride(-2) if x.dim() >= 2 else self.g.C
         if self.kind == "max":
-            F.maxpool_forward(x, self.y, self.argmax, self.g)
+            F.maxpool_forward(x, self.y, self.argmax, self.g, relu_mask=self.mask_relu_input)
         else:
             F.avgpool_forward(x, self.y, self.g)
         return self.y

@@ -650,6 +650,26 @@ def test_maxpool_backward_by_quads(B, H, W, C, pad, extra, accumulate):
     assert torch.equal(wide[..., C:], before[..., C:])
 
 
+@pytest.mark.parametrize("K,stride,pad", [(3, 2, 0), (3, 2, 1), (2, 2, 0), (3, 1, 1), (15, 7, 0)])
+def test_maxpool_applies_the_mask_of_a_relu(K, stride, pad):
+    """Windows that are all zeros or negative hand their gradient to nobody: the masked gradient of the plain passes, bit for bit."""
+    torch.manual_seed(K)
+    B, H, C = 3, 29, 40
+    x = torch.relu(torch.randn(B, H, H, C, device=DEV) - 1.2).to(BF)
+    x[0, :20, :20] = 0
+    x[1, 3, 4] = -1.0                                                # not from a ReLU: masked by sign all the same
+    g = F.pool_geom((B, H, H, C), K, stride, pad, C, C)
+    y, ym, dy = (torch.randn(B, g.OH, g.OW, C, device=DEV).to(BF) for _ in range(3))
+    arg, argm = (torch.empty(B, g.OH, g.OW, C, dtype=torch.uint8, device=DEV) for _ in range(2))
+    dx, dxm = torch.empty_like(x), torch.empty_like(x)
+    F.maxpool_forward(x, y, arg, g)
+    F.maxpool_backward(dy, arg, dx, g)
+    F.maxpool_forward(x, ym, argm, g, relu_mask=True)
+    F.maxpool_backward(dy, argm, dxm, g)
+    assert torch.equal(y, ym) and (argm == 255).any() and torch.equal(argm[argm != 255], arg[argm != 255])
+    assert torch.equal(dxm, torch.where(x > 0, dx, torch.zeros_like(dx)))
+
+
 @pytest.mark.parametrize("P,C", [(81920, 64), (81921, 64), (30000, 200)])
 def test_batchnorm_passes_one_after_the_other(P, C):
     """Tensors on both sides of the size from which a pass lets the next one in only at its end: three forward and backward
