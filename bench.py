@@ -112,6 +112,13 @@ def pcie_links() -> list:
         return []
 
 
+def push_times(bg: dict, tables: int) -> dict:
+    """Device time of the parameter pushes, from the sampled ones; null where a run has no samples."""
+    n = bg["device_push_samples"]
+    return {"device_push_ms_per_step": bg["device_push_ms"] / n * tables if n else None,
+            "device_push_gb_per_s": bg["device_push_gb_per_s"] if n else None, "device_push_samples": n}
+
+
 def reference_arm(args) -> None:
     """The reference is a C++ library (SCons + ZeroMQ/boost/tbb/glog/gflags/cblas) with no Python
     package, and its Caffe application (the only program in it that trains AlexNet) is an empty submodule: the
@@ -400,9 +407,7 @@ def main() -> None:
                 ("e2e_fp32_input" if e2e_other and e2e_other.get("input_dtype") == "fp32" else "e2e_other_input"): e2e_other,
                 "e2e_uint8_input": e2e_u8,
                 "diag": diag,
-                "ps": {"device_push_ms_per_step": stats["bgthread"]["device_push_ms"] / max(1, stats["bgthread"]["device_push_samples"]) * len(mod.tables),
-                       "device_push_gb_per_s": stats["bgthread"]["device_push_gb_per_s"],
-                       "device_push_samples": stats["bgthread"]["device_push_samples"]},
+                "ps": push_times(stats["bgthread"], len(mod.tables)),
                 "gpu_launches": launches + runtime_launches, "final_loss": last_loss,
             }
             print(json.dumps(out))

@@ -137,11 +137,13 @@ struct Fabric {
   void* timeline_origin = nullptr;
   std::vector<TimelineRec> timeline_recs;
   void* push_done_event = nullptr;
-  // Device time of the latest pushes of every eighth clock: a ring of event pairs around the reduce + apply + publish
-  // kernel on the comm stream, summed by GetStats() over the pairs that have completed (device_push_ms / device_push_gb_per_s).
+  // Device time of the latest sampled pushes (a table's first ones that the host enqueues, then every seventh): a ring of event
+  // pairs around the reduce + apply + publish kernel on the comm stream, summed by GetStats() over the pairs that have
+  // completed (device_push_ms / device_push_gb_per_s).
   struct PushTiming { void* begin = nullptr; void* end = nullptr; size_t table_bytes = 0; bool armed = false; };
   std::vector<PushTiming> push_timing;
   size_t push_timing_next = 0;
+  std::vector<unsigned long long> host_pushes;   // by table: pushes enqueued by the host, the initial one and captured ones left out
   std::vector<void*> table_events;
   // one worker: what a table's freshness wait needs is its latest push on the comm stream, an event
   struct Applied { void* event = nullptr; int clock = -1; };

@@ -277,3 +277,34 @@ def test_push_mirrors_a_status_block_that_is_not_zero(rows):
     L.check(lib().geeps_ps_push_apply(C.byref(p), 0, stream_ptr()), "push_apply")
     torch.cuda.synchronize()
     assert mirror.tolist() == status.tolist() and mirror[0].item() == 2 and mirror[2].item() == rows - 1
+
+
+@pytest.mark.parametrize("clocks", [1, 3, 40])
+def test_push_times_are_sampled_per_table(clocks):
+    """Host-run clocks, without the initial one: a table's first sixteen pushes are timed, then every seventh; each table has its own count,
+    so a second one that is as old has as many."""
+    dev = torch.device("cuda:0")
+    cfg = GeePsConfig(device=DEVICE_CUDA, cuda_device=0, transport=TRANSPORT_NVLINK, tcp_base_port=29300 + clocks, num_tables=2)
+    with torch.cuda.stream(torch.cuda.Stream(device=dev)):
+        g = GeePs(0, cfg)
+        rows, tables = list(range(64)), 2
+        ops = []
+        for t in range(tables):
+            r = g.virtual_read(t, rows, 0); u = g.virtual_pre_update(t, rows)
+            ops.append((r, u, g.virtual_post_read(r), g.virtual_update(u)))
+        g.virtual_clock()
+        g.finish_virtual_iteration()
+        for r, u, pr, up in ops:
+            g.pre_update(u).zero_(); g.update(up)
+        g.clock(); g.start_iterations()
+        assert g.get_stats()["bgthread"]["device_push_samples"] == 0
+        for _ in range(clocks):
+            for r, u, pr, up in ops:
+                g.read(r); b = g.pre_update(u); g.post_read(pr); b.fill_(1.0); g.update(up)
+            g.clock()
+        torch.cuda.synchronize()
+        bg = g.get_stats()["bgthread"]
+        assert bg["device_push_samples"] == tables * (min(clocks, 16) + max(0, clocks - 16) // 7)
+        assert bg["device_push_ms"] > 0 and bg["device_push_gb_per_s"] > 0
+        assert bg["device_push_bytes"] == bg["device_push_samples"] * 64 * 512
+        g.close()

@@ -171,3 +171,14 @@ def test_bench_clock_sampler_reads_a_fake_nvidia_smi(tmp_path, monkeypatch):
     s2.wait_first_sample(0.2)
     assert s2.stop()["sm_mhz"] is None
     assert bench.pcie_links() == []
+
+
+def test_bench_push_times_without_samples_are_null():
+    import os
+    import sys
+    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    import bench
+    none = bench.push_times({"device_push_ms": 0.0, "device_push_gb_per_s": 0.0, "device_push_samples": 0}, 8)
+    assert none == {"device_push_ms_per_step": None, "device_push_gb_per_s": None, "device_push_samples": 0}
+    some = bench.push_times({"device_push_ms": 6.0, "device_push_gb_per_s": 5000.0, "device_push_samples": 12}, 4)
+    assert some == {"device_push_ms_per_step": 2.0, "device_push_gb_per_s": 5000.0, "device_push_samples": 12}
