@@ -640,6 +640,7 @@ double geeps_conv_box_us(const GeepsConvTcParams* p) {
   return takes_pairs(b) ? b.pair : b.one;
 }
 double geeps_conv_box_wgrad_us(const GeepsConvTcParams* p) { return plan_wgrad_box(p, geeps_sm_count()).us; }
+int geeps_conv_box_wgrad_slices(const GeepsConvTcParams* p) { return plan_wgrad_box(p, geeps_sm_count()).split; }
 int geeps_conv_box_pairs(const GeepsConvTcParams* p) {
   return p->mode != MODE_WGRAD && p->stride <= 1 && geeps_conv_tc_supported(p) && takes_pairs(plan_box(p, 1, 1, geeps_sm_count())) ? 1 : 0;
 }

@@ -353,6 +353,8 @@ extern "C" {
 // 53 x 53, 40 -> 208 at batch 68 60 / 144; 46 x 46, 88 -> 224 at batch 84 105 / 203; 28 x 28, 136 -> 104, 5 x 5 at batch 41 44 / 80;
 // 41 x 41, 104 -> 88 at batch 90 60 / 97.  The kernel taken so is 3.8 % slower than the faster one in the geometric mean, by the
 // rule above alone 5.5 %.
+// Slices are added to dW in the order in which they come: one, or two on zeros, give the same bits in every call, more do not.  A
+// gradient that the rule above repeats bit for bit stays with its kernel (7 x 8 x 8, 72 -> 136: one slice there, seven here).
 int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p) {
   if (!halo_mode()) return 0;
   if (!geeps_conv_tc_supported(p)) return 0;
@@ -364,6 +366,8 @@ int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p) {
                     (p->KW >= 5 || (p->KW >= 3 && d.m_tiles == 1 && d.cchunks == 1));
   if (p->KW < 3 || p->cg < 32 || p->og < 32 || (p->x_pitch % 64 == 0 && p->cg % 64 == 0 && p->y_pitch % 64 == 0 && p->og % 64 == 0))
     return here ? 1 : 0;
+  const bool repeats_here = d.split <= 2, repeats_box = geeps_conv_box_wgrad_slices(p) <= 2;
+  if (repeats_here != repeats_box && here == repeats_here) return here ? 1 : 0;
   const double waves = (double)(((long long)d.m_tiles * d.cchunks * d.passes * d.split + sms - 1) / sms);
   const double us = 6.1 + waves * (3.76 + (double)((d.n_blocks + d.split - 1) / d.split) * (0.349 + 0.654 * d.kpos / 128.0));
   return us < (here ? 1.1 : 0.85) * geeps_conv_box_wgrad_us(p) ? 1 : 0;

@@ -163,3 +163,35 @@ def test_short_forward_tiles_keep_two_pairs_of_store_slabs():
         two += pairs == 2
         one += pairs == 1
     assert two > 50 and one > 50
+
+
+def test_weight_gradients_that_repeat_bit_for_bit_keep_their_kernel():
+    """Rows off 128-byte lines, where expected times choose the kernel: a gradient in one slice, or in two on zeros, has the
+    same bits in every call, and is not sent to a kernel that adds up more slices."""
+    lib = L.lib()
+
+    def plans(B, H, cg, og, k):
+        p, _, _ = _params(2, B, H, H, cg, og, k, k // 2)
+        info = L.HaloPlanInfo()
+        ok = lib.geeps_conv_wgrad_halo_plan(C.byref(p), C.byref(info))
+        return ok, info, lib.geeps_conv_box_wgrad_slices(C.byref(p))
+
+    for layer, slices in (((7, 8, 72, 136, 3), 7), ((2, 13, 368, 352, 3), 4), ((1, 19, 80, 288, 3), 5)):
+        ok, info, box = plans(*layer)
+        assert ok and info.split == slices and box == 1 and not info.routed, layer
+    routed = kept = 0
+    for B, H, cg, og, k in itertools.product((1, 2, 4, 7, 16, 40, 100, 256), (5, 8, 13, 19, 28, 53), (32, 40, 72, 80, 168, 368),
+                                             (40, 88, 136, 208, 352), (3, 5)):
+        ok, info, box = plans(B, H, cg, og, k)
+        if not ok:
+            continue
+        routed += info.routed
+        tail = cg - (cg + 63) // 64 * 64 + 64
+        lines_rule = tail >= 32 and info.util >= 0.6 and info.n_blocks >= 4 * 148 and (k >= 5 or (info.m_tiles == 1 and cg <= 64))
+        if box <= 2 < info.split and not lines_rule:
+            assert not info.routed, (B, H, cg, og, k)
+            kept += 1
+        if info.split <= 2 < box and lines_rule:
+            assert info.routed, (B, H, cg, og, k)
+            kept += 1
+    assert routed > 200 and kept > 50

@@ -548,6 +548,20 @@ def test_weight_gradients_off_128_byte_lines_agree_on_both_kernels(B, H, cg, og,
     assert _rel(out[0], out[1].double()) < 2 * (B * H * H) ** 0.5 * 2.0 ** -24
 
 
+@pytest.mark.parametrize("B,H,cg,og", [(7, 8, 72, 136), (2, 13, 368, 352), (1, 19, 80, 288)])
+def test_small_weight_gradients_off_128_byte_lines_repeat_bit_for_bit(B, H, cg, og):
+    """Layers whose gradient is written in one piece: the same bits in every call."""
+    from geeps_b200.ops import functional as F
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(cg)
+    x = torch.randn(B, H, H, cg, device=dev, generator=gen).to(BF)
+    dy = torch.randn(B, H, H, og, device=dev, generator=gen).to(BF)
+    out = [torch.full((og, 9 * cg), 3.0, device=dev) for _ in range(30)]
+    for o in out:
+        F.conv_tc(F.CONV_WGRAD, x, dy, o, 3, 1)
+    assert all(torch.equal(o, out[0]) for o in out)
+
+
 @pytest.mark.parametrize("B,H,cin,cout,k,groups,masked", [(64, 27, 96, 256, 5, 2, False), (64, 27, 96, 256, 5, 2, True), (50, 13, 128, 96, 3, 2, False),
                                                           (20, 13, 64, 200, 3, 1, False), (1, 7, 32, 48, 3, 2, True), (2, 8, 16, 8, 1, 1, False)])
 def test_layer_gradient_is_cleared_once(B, H, cin, cout, k, groups, masked):
