@@ -2173,14 +2173,18 @@ int geeps_relu_backward_2d(const void* dy, const void* y, void* dx, long long P,
                                                                                  (bf16*)dx, P, C, lddy, ldy, lddx);
   return CK();
 }
+int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* colsum, long long P, int C,
+                               long long lddy, long long ldy, long long lddx, void* stream) {
+  return geeps_relu_backward_colsum_clear(dy, y, dx, colsum, P, C, lddy, ldy, lddx, nullptr, 0, stream);
+}
 // Zeros to the clear_n values at `clear` as well: on the way in a short pass, where a launch for them in front of each group's
 // weight gradient costs more than its bytes (backward passes of layers, us, a launch each / so: 1000 x 48 from 80 channels
 // 15.5 / 13.7, two groups 1922 x 96 from 128 31.2 / 27.2, 6100 x 232 from 88 32.0 / 29.8, 22275 x 176 from 40 49.9 / 46.8).
 // After a long pass they keep a launch, one for all groups: the blocks of a weight gradient that follows it directly come up
 // in the order in which its blocks leave, on other SMs than the tiles they share lie well on (44800 x 264 from 144, 5 x 5
 // 295.5 us, 306.3 without the launch; 93600 x 352 from 88 632, 650; though 43264 x 384 from 256 145.8, 143.2).
-int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* colsum, long long P, int C,
-                               long long lddy, long long ldy, long long lddx, float* clear, long long clear_n, void* stream) {
+int geeps_relu_backward_colsum_clear(const void* dy, const void* y, void* dx, float* colsum, long long P, int C,
+                                     long long lddy, long long ldy, long long lddx, float* clear, long long clear_n, void* stream) {
   if (C % 8 || lddy % 8 || ldy % 8 || lddx % 8 || C > 8192 || clear_n < 0 || (clear_n > 0 && !clear)) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   geeps_clear_f32(colsum, C, st);
@@ -2270,11 +2274,17 @@ int geeps_lrn_backward(const void* x, const void* y, const void* rscale, const v
   return CK();
 }
 
-int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, int relu_mask, void* stream) {
+static int maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, int relu_mask, void* stream) {
   if (g->C % 8 || g->ldx % 8 || g->ldy % 8 || g->K * g->K > 255) return (int)cudaErrorInvalidValue;
   geeps_launch_plain(maxpool_forward_kernel, g->B * g->OH, pool_block(g->C / 8), 0, (cudaStream_t)stream, (const bf16*)x, (bf16*)y,
                                                                                         (uint8_t*)argmax, *g, relu_mask);
   return CK();
+}
+int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream) {
+  return maxpool_forward(x, y, argmax, g, 0, stream);
+}
+int geeps_maxpool_forward_relu(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream) {
+  return maxpool_forward(x, y, argmax, g, 1, stream);
 }
 int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const GeepsPoolGeom* g, int accumulate,
                            void* stream) {

@@ -67,7 +67,10 @@ int geeps_bn_backward_fused_bits(const void* x, const void* dy, const void* y, c
 // out[c] (+)= scale * sum_p x[p][c]
 // dx = y > 0 ? dy : 0 and colsum[c] = sum over the P pixels of dx (C % 8 == 0, C <= 8192), one pass
 int geeps_relu_backward_colsum(const void* dy, const void* y, void* dx, float* colsum, long long P, int C,
-                               long long lddy, long long ldy, long long lddx, float* clear, long long clear_n, void* stream);
+                               long long lddy, long long ldy, long long lddx, void* stream);
+// ... and zeros to the clear_n values at `clear`
+int geeps_relu_backward_colsum_clear(const void* dy, const void* y, void* dx, float* colsum, long long P, int C,
+                                     long long lddy, long long ldy, long long lddx, float* clear, long long clear_n, void* stream);
 int geeps_colsum(const void* x, float* out, long long P, int C, long long ldx, float scale, int zero_first,
                  void* stream);
 int geeps_relu_backward(const void* dy, const void* y, void* dx, long long n, void* stream);
@@ -102,9 +105,10 @@ int geeps_lrn_maxpool_forward(const void* x, void* p, void* argmax, const GeepsP
                               float beta, float k, void* stream);
 int geeps_lrn_maxpool_backward(const void* x, const void* dp, const void* argmax, void* dx, const GeepsPoolGeom* g,
                                int size, float alpha, float beta, float k, int relu_mask, float* colsum, void* stream);
-// relu_mask: a window whose maximum is not above zero gets code 255, so the backward pass hands its gradient to nobody:
-// the mask of a ReLU that x is the output of
-int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, int relu_mask, void* stream);
+int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream);
+// ... where a window whose maximum is not above zero gets code 255, so the backward pass hands its gradient to nobody: the
+// mask of a ReLU that x is the output of
+int geeps_maxpool_forward_relu(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream);
 int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const GeepsPoolGeom* g, int accumulate,
                            void* stream);
 // launch shape of a reduction over P pixels of C channels (host arithmetic only): channel shares, pixel shares, threads a

@@ -276,9 +276,12 @@ def relu_backward_colsum(dy2d, y2d, dx2d, colsum_out, clear: torch.Tensor | None
     P, Cc = dy2d.shape
     assert colsum_out.dtype == torch.float32 and colsum_out.numel() == Cc and colsum_out.is_contiguous()
     assert clear is None or clear.dtype == torch.float32 and clear.is_contiguous()
-    launch(lib().geeps_relu_backward_colsum, "relu_backward_colsum", ptr(dy2d), ptr(y2d), ptr(dx2d), ptr(colsum_out),
-           C.c_longlong(P), Cc, C.c_longlong(_ld(dy2d)), C.c_longlong(_ld(y2d)), C.c_longlong(_ld(dx2d)),
-           ptr(clear), C.c_longlong(0 if clear is None else clear.numel()), stream_ptr())
+    args = (ptr(dy2d), ptr(y2d), ptr(dx2d), ptr(colsum_out), C.c_longlong(P), Cc, C.c_longlong(_ld(dy2d)), C.c_longlong(_ld(y2d)),
+            C.c_longlong(_ld(dx2d)))
+    if clear is None:
+        launch(lib().geeps_relu_backward_colsum, "relu_backward_colsum", *args, stream_ptr())
+    else:
+        launch(lib().geeps_relu_backward_colsum_clear, "relu_backward_colsum", *args, ptr(clear), C.c_longlong(clear.numel()), stream_ptr())
 
 
 def stream_order(src_stream, dst_stream, event) -> None:
@@ -389,7 +392,8 @@ def pool_geom(x_shape, k: int, stride: int, pad: int, ldx: int, ldy: int, ceil_m
 def maxpool_forward(x, y, argmax, g: PoolGeom, relu_mask: bool = False) -> None:
     """relu_mask: x is the output of a ReLU, whose mask maxpool_backward() then applies as well: windows without a positive
     value name no element (code 255)."""
-    launch(lib().geeps_maxpool_forward, "maxpool_forward", ptr(x), ptr(y), ptr(argmax), C.byref(g), int(relu_mask), stream_ptr())
+    fn = lib().geeps_maxpool_forward_relu if relu_mask else lib().geeps_maxpool_forward
+    launch(fn, "maxpool_forward", ptr(x), ptr(y), ptr(argmax), C.byref(g), stream_ptr())
 
 
 def maxpool_backward(dy, argmax, dx, g: PoolGeom, accumulate=False) -> None:

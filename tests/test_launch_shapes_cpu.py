@@ -2,6 +2,7 @@
 import ctypes as C
 import itertools
 import re
+import subprocess
 
 import pytest
 
@@ -69,3 +70,17 @@ def test_channel_kernels_keep_to_registers_at_their_launch_bounds():
         pytest.skip("no compiler output here: the library was built elsewhere")
     assert len(found) >= 6
     assert [f for f in found if f[2] != "0"] == []
+
+
+def test_exported_calls_keep_their_arguments(tmp_path):
+    """A call that gets an option gets a name: programs that hold the C signatures, by the header or by a loaded symbol, go on as
+    they are (an argument in front of the stream would take the stream for an option)."""
+    src = tmp_path / "calls.cpp"
+    src.write_text("""
+#include "nn_ops.h"
+using P = const void*; using V = void*; using L = long long;
+int (*pool)(P x, V y, V argmax, const GeepsPoolGeom* g, V stream) = geeps_maxpool_forward;
+int (*relu)(P dy, P y, V dx, float* colsum, L n, int c, L lddy, L ldy, L lddx, V stream) = geeps_relu_backward_colsum;
+""")
+    r = subprocess.run(["g++", "-std=c++17", "-fsyntax-only", f"-I{_native.CSRC / 'kernels'}", str(src)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
