@@ -44,6 +44,21 @@ __device__ __forceinline__ float max8(const float (&w)[8]) {
   return fmaxf(fmaxf(fmaxf(w[0], w[1]), fmaxf(w[2], w[3])), fmaxf(fmaxf(w[4], w[5]), fmaxf(w[6], w[7])));
 }
 
+__device__ __forceinline__ float max4(const float2 (&w)[4]) {
+  return fmaxf(fmaxf(fmaxf(w[0].x, w[0].y), fmaxf(w[1].x, w[1].y)), fmaxf(fmaxf(w[2].x, w[2].y), fmaxf(w[3].x, w[3].y)));
+}
+// NaN where a window is
+__device__ __forceinline__ float max4_nan(const float2 (&w)[4]) {
+  auto larger = [](float a, float b) {
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(b));
+    return a;
+  };
+  return larger(larger(larger(w[0].x, w[0].y), larger(w[1].x, w[1].y)), larger(larger(w[2].x, w[2].y), larger(w[3].x, w[3].y)));
+}
+// The sum of all twelve squares under the windows of eight channels (w: windows of 5, edge: the last two squares), two
+// additions away, bounds every window; only where it is too large for the polynomials does the largest have to be found.
+__device__ __forceinline__ float squares12(const float2 (&w)[4], float2 edge) { return (w[0].x + w[2].y) + (edge.x + edge.y); }
+
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
@@ -160,8 +175,9 @@ lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uin
     const int nrows = r_hi - r_lo;
     if constexpr (HALF == 2) {
       // Pairs of channels: half the fp32 instructions, and a halo of one word per side instead of two.  Three items are
-      // loaded before the first is computed: with one, half of the time went on waiting for it (256 x 55 x 55 x 96: 96 us;
-      // two 84, three 82, four spill).
+      // loaded before the first is computed: with one, half of the time went on waiting for it (256 x 55 x 55 x 96: 94 us,
+      // three 79).  Polynomial or exact power in a branch each: the polynomial first and the exact power over it spills at the
+      // 64 registers of two blocks per SM and takes 80 us, 103 instead of 94 where half of the vectors are beyond the range.
       constexpr int U = 3;
       for (ItemWalk it(tid, nt, W, cv); it.r < nrows;) {
         uint32_t before[U], after[U];
@@ -189,11 +205,11 @@ lrn_maxpool_forward_kernel(const bf16* __restrict__ x, bf16* __restrict__ p, uin
 #pragma unroll
           for (int k = 0; k < 6; ++k) t[k] = mul2(v[k], v[k]);
           window5(t, ws);
+          if (squares12(ws, t[5]) <= cf.w_max || max4(ws) <= cf.w_max) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            o[k] = mul2(v[k + 1], fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.p3), both(cf.p2)), both(cf.p1)), both(cf.p0)));
-          // the sum of all twelve squares bounds every window's
-          if (!((ws[0].x + ws[2].y) + (t[5].x + t[5].y) <= cf.w_max)) {
+            for (int k = 0; k < 4; ++k)
+              o[k] = mul2(v[k + 1], fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.p3), both(cf.p2)), both(cf.p1)), both(cf.p0)));
+          } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
               o[k] = make_float2(v[k + 1].x * __powf(cf.k * fmaf(cf.es, ws[k].x, 1.f), -cf.beta),
@@ -378,9 +394,7 @@ lrn_maxpool_backward_lanes_kernel(const bf16* __restrict__ x, const bf16* __rest
       av[j] = make_uint4(0u, 0u, 0u, 0u);
       rv[j] = make_uint4(0u, 0u, 0u, 0u);
       if (hit[j] != 0u) {
-        const float top = fmaxf(fmaxf(fmaxf(ws[0].x, ws[0].y), fmaxf(ws[1].x, ws[1].y)),
-                                fmaxf(fmaxf(ws[2].x, ws[2].y), fmaxf(ws[3].x, ws[3].y)));
-        if (top <= cf.w_max) {
+        if (max4(ws) <= cf.w_max) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             a[k] = mul2(dy[j][k], fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.p3), both(cf.p2)), both(cf.p1)), both(cf.p0)));
@@ -453,12 +467,15 @@ lrn_maxpool_backward_lanes_kernel(const bf16* __restrict__ x, const bf16* __rest
 // a vector of their neighbours for the halo channels and store nothing, so 30 of 32 lanes work at every channel count.
 // The window codes are spread to 16-bit numbers between 0.5 and 2; one packed comparison then is a mask.  The polynomials
 // are evaluated without a branch around them (a pixel beyond their range is done again, exactly), so the arithmetic of
-// neighbouring pixels overlaps.  Sums over windows and channels are those of the lanes kernel above, in its order: the
-// results have the same bits.
+// neighbouring pixels overlaps.  Sums over windows and channels, and the choice between polynomial and exact power, are those
+// of the lanes kernel above, in its order: the results have the same bits (but for vectors with a NaN, which take the exact
+// path here).
 // Bound by instruction issue (64 % of the slots, half-rate integer pipe 62 %) at 16 warps per SM: 256 x 55 x 55 x 96
-// 170 us (lanes kernel) -> 138, 256 x 27 x 27 x 256 110 -> 95, 64 x 55 x 55 x 264 150 -> 98.  Three blocks per SM spill: 165 us;
-// two pixels at a time spill too: 147; fp32 without the register pairs: 151; without the last four of the savings named at
-// the lines below (codes expanded at use, packed sign test, merged halo words, match test only beyond the range): 153.
+// 170 us (lanes kernel) -> 132, 256 x 27 x 27 x 256 109 -> 90, 64 x 55 x 55 x 264 150 -> 98; with all vectors beyond the range
+// 240 -> 228, 150 -> 154, with half of them 205 -> 195, 133 -> 132 (the exact path by the sum of the squares alone, not the largest window:
+// 237, 159; in a branch of its own beside the polynomials: 216, 146 and 204, 137).  Three blocks per SM spill: 165 us; two pixels at a
+// time spill too: 147; fp32 without the register pairs: 151; without the last four of the savings named at the lines below
+// (codes expanded at use, packed sign test, merged halo words, match test only beyond the range): 153.
 
 // c + the two bf16 of w (a mixed-precision sum needs no conversion in front of it)
 __device__ __forceinline__ float2 add_bf16(float2 c, uint32_t w) {
@@ -586,15 +603,15 @@ lrn_maxpool_backward_quad_kernel(const bf16* __restrict__ x, const bf16* __restr
 #pragma unroll
         for (int k = 0; k < 4; ++k) t[k + 1] = mul2(v[k], v[k]);
         window5(t, ws);
+        const bool beyond = !(squares12(ws, t[5]) <= cf.w_max) && !(max4_nan(ws) <= cf.w_max);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           a[k] = mul2(dy[k], fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.p3), both(cf.p2)), both(cf.p1)), both(cf.p0)));
           rt[k] = mul2(mul2(dy[k], v[k]),
                        fma2(ws[k], fma2(ws[k], fma2(ws[k], both(cf.q3), both(cf.q2)), both(cf.q1)), both(cf.q0)));
         }
-        // the sum of all twelve squares bounds every window's
-        if (!((ws[0].x + ws[2].y) + (t[5].x + t[5].y) <= cf.w_max)) {
-          uint32_t hit = 0u;                      // a vector without a gradient has none here either (no 0 x inf)
+        if (beyond) {
+          uint32_t hit = 0u;                      // a vector without a gradient has none here either (no 0 x inf, no 0 x NaN)
 #pragma unroll
           for (int j = 2 * r; j < 4; ++j) {
             if ((j & 1) == 0 && c == 1) continue;

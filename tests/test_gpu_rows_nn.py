@@ -714,11 +714,12 @@ def test_relu_backward_clears_a_range_on_the_way(off, n, P, C):
 @pytest.mark.parametrize("B,H,Cc,pad,ldy", [(64, 29, 8, 0, 8), (61, 31, 8, 1, 8), (40, 13, 120, 0, 136), (9, 61, 40, 1, 40),
                                             (3, 27, 240, 0, 240), (2, 28, 312, 0, 312), (100, 14, 88, 1, 88),
                                             (260, 27, 32, 0, 32), (24, 55, 296, 0, 296), (36, 15, 520, 0, 520)])
-@pytest.mark.parametrize("alpha", [1e-4, 0.5])
+@pytest.mark.parametrize("alpha", [1e-4, 0.01, 0.5])
 def test_lrn_maxpool_backward_by_quads_matches_small_batches(B, H, Cc, pad, ldy, alpha):
     """A batch large enough for the quad kernel (one step a warp and several, ends of rows and images inside a warp,
     one vector a pixel, vector counts without a common factor with 30) against single images, which the other kernels take:
-    the same bits in the range of the polynomials, and each within two roundings of bf16 beyond it."""
+    the same bits, in the range of the polynomials, beyond it, and on the vectors between whose largest window is inside while
+    the sum of all their squares is not."""
     torch.manual_seed(B * Cc)
     size, beta, kk = 5, 0.75, 1.0
     x = (torch.randn(B, H, H, Cc, device=DEV) * 3).clamp_min(-0.5).to(BF)        # some negative inputs: masked by sign
@@ -733,15 +734,39 @@ def test_lrn_maxpool_backward_by_quads_matches_small_batches(B, H, Cc, pad, ldy,
     for b in range(B):
         F.lrn_maxpool_backward(x[b:b + 1], dp[b:b + 1], arg[b:b + 1], ref, one, size, alpha, beta, kk, relu_mask=True, colsum=part)
         total += part
-        if alpha < 1e-2:
-            assert torch.equal(dx[b:b + 1], ref), b
-        else:
-            assert (dx[b:b + 1].double() - ref.double()).norm() <= 2.0 ** -8 * ref.double().norm(), b
-    # n additions, each rounded by at most 2^-24 of the sum of magnitudes, with random signs: four deviations; beyond the
-    # polynomials' range the two kernels may also take different paths, 4e-4 of every value apart
+        assert torch.equal(dx[b:b + 1], ref), b
+    # n additions, each rounded by at most 2^-24 of the sum of magnitudes, with random signs: four deviations
     mag = dx.double().abs().sum((0, 1, 2))
-    bound = (4 * 2.0 ** -24 * (B * H * H) ** 0.5 + (4e-4 if alpha > 1e-2 else 0.0)) * mag
+    bound = 4 * 2.0 ** -24 * (B * H * H) ** 0.5 * mag
     assert ((cs.double() - total).abs() <= bound).all()
+
+
+def test_lrn_maxpool_backward_by_quads_with_infinities_and_nans():
+    """What an infinity or a NaN spoils by quads and in single images: the same places, and the same bits beside an infinity."""
+    torch.manual_seed(3)
+    B, H, Cc = 40, 13, 120
+    x = torch.randn(B, H, H, Cc, device=DEV).to(BF)
+    flat = x.view(-1)
+    at = torch.randperm(flat.numel(), device=DEV)[:3000]
+    flat[at[:1500]] = float("inf")
+    g = F.pool_geom(x.shape, 3, 2, 0, Cc, Cc)
+    one = F.pool_geom(x[:1].shape, 3, 2, 0, Cc, Cc)
+    arg = torch.randint(0, 9, (B, g.OH, g.OW, Cc), device=DEV, dtype=torch.uint8)
+    arg[:, ::2] = 4                                    # rows of pixels that no window points at
+    dp = torch.randn(B, g.OH, g.OW, Cc, device=DEV).to(BF)
+    dx, ref = torch.empty_like(x), torch.empty_like(x)
+    for nans in (False, True):
+        if nans:
+            flat[at[1500:]] = float("nan")
+        F.lrn_maxpool_backward(x, dp, arg, dx, g, 5, 1e-4, 0.75, 1.0)
+        for b in range(B):
+            F.lrn_maxpool_backward(x[b:b + 1], dp[b:b + 1], arg[b:b + 1], ref[b:b + 1], one, 5, 1e-4, 0.75, 1.0)
+        bad = ref.isnan()
+        assert bad.any() and not bad.all() and torch.equal(dx.isnan(), bad)
+        if nans:      # a vector with a NaN takes the exact power by quads, the polynomial (4e-4) otherwise; two roundings to bf16
+            assert torch.allclose(dx[~bad].float(), ref[~bad].float(), rtol=2.0 ** -7, atol=1e-3)
+        else:
+            assert torch.equal(dx[~bad], ref[~bad])
 
 
 @pytest.mark.parametrize("B,H,W,Cc,pad,ldx,ldy", [(33, 15, 14, 96, 1, 96, 112), (40, 8, 9, 256, 0, 272, 256), (65, 5, 7, 304, 2, 304, 304),
