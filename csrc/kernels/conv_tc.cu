@@ -533,7 +533,7 @@ BoxPlan plan_box(const GeepsConvTcParams* p, int s, int n_cls, int sms) {
     b.pair = tiles_us(fwd ? kFwdPair : kDgradPair, ((b.m_tiles + 1) / 2 * b.n_tiles + sms / 2 - 1) / (sms / 2), b.kt, b.bn, mis);
   return b;
 }
-// How a weight gradient is cut.  us: as tiles_us, fitted to 391 products of both kernels (here half of them within 14 %).
+// How a weight gradient is cut.  us: as tiles_us, fitted to 1300 products of both kernels (here half of them within 9 %).
 struct WgradPlan { int bw, bh, bnb, kt, m_tiles, per, n_tiles, split; double us; };      // per: panels (tap, chunk) per tile
 WgradPlan plan_wgrad_box(const GeepsConvTcParams* p, int sms) {
   WgradPlan g;
@@ -572,9 +572,11 @@ WgradPlan plan_wgrad_box(const GeepsConvTcParams* p, int sms) {
     split = (g.kt + per_k - 1) / per_k;      // every k-slice non-empty
   }
   g.split = split;
-  const bool mis_x = p->x_pitch % 64 != 0 || p->cg % 64 != 0, mis_y = p->y_pitch % 64 != 0 || p->og % 64 != 0;
+  // rows off 16-, 32- and 64-channel boundaries (32-byte sectors, half lines, lines)
+  auto off = [](long long v, double by16, double by32, double by64) { return v % 16 ? by16 : v % 32 ? by32 : v % 64 ? by64 : 0.0; };
   const double waves = (double)((tiles * split + sms - 1) / sms), kt = (g.kt + split - 1) / split;
-  g.us = 5.46 + waves * (0.841 * g.per + kt * (0.332 + (mis_y ? 0.092 : 0.) + (mis_x ? 0.042 * g.per : 0.)));
+  g.us = 5.95 + waves * (0.43 * g.per + kt * (0.28 + off(p->y_pitch | p->og, 0.119, 0.053, 0.031) +
+                                              g.per * (0.009 + off(p->x_pitch | p->cg, 0.061, 0.021, 0.011))));
   return g;
 }
 bool takes_pairs(const BoxPlan& b) { return b.pair >= 0 && b.pair < 0.97 * b.one; }

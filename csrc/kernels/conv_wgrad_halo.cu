@@ -348,11 +348,12 @@ extern "C" {
 // 0.087 here when the line was drawn and 0.074 now; Inception 5 x 5 0.054 -> 0.050 ms); 3-tap rows only when the layer is one item wide (one block
 // of output channels, one chunk of input channels: AlexNet conv1 0.120 -> 0.112 ms) - wider 3 x 3 layers are faster
 // on the box kernel, which covers four (tap, chunk) panels per MMA whatever the filter's shape.
-// Rows of X or dY that are no whole 128-byte lines cost the box kernel more, which loads them once per tap.  There the expected
-// times of both kernels decide (each fitted to 391 products; this one half within 4 %), unless they are close.  us, here / box:
-// 53 x 53, 40 -> 208 at batch 68 60 / 144; 46 x 46, 88 -> 224 at batch 84 105 / 203; 28 x 28, 136 -> 104, 5 x 5 at batch 41 44 / 80;
-// 41 x 41, 104 -> 88 at batch 90 60 / 97.  The kernel taken so is 3.8 % slower than the faster one in the geometric mean, by the
-// rule above alone 5.5 %.
+// Rows of X or dY that are no whole 128-byte lines cost the box kernel more, which loads them once per tap, above all where they do not
+// begin on 32-byte sectors either.  There the expected times of both kernels decide (each fitted to 1300 products with filters of
+// 3 x 3 to 7 x 7; this one half within 4 %), unless they are close.  us, here / box: 53 x 53, 40 -> 208 at batch 68 60 / 144; 46 x 46, 88
+// -> 224 at batch 84 105 / 203; 28 x 28, 136 -> 104, 5 x 5 at batch 41 44 / 80; 31 x 31, 40 -> 176, 6 x 6 at batch 48 66 / 157; but 17 x 17,
+// 416 -> 336, 7 x 7 at batch 94 463 / 349.  The kernel taken so is 3.0 % slower than the faster one in the geometric mean, by the rule
+// above alone 6.6 %, and on one product of 1300 more than 3 % slower than the one of that rule.
 // Slices are added to dW in the order in which they come: one, or two on zeros, give the same bits in every call, more do not.  A
 // gradient that the rule above repeats bit for bit stays with its kernel (7 x 8 x 8, 72 -> 136: one slice there, seven here).
 int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p) {
@@ -364,13 +365,15 @@ int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p) {
   const int tail = p->cg - (d.cchunks - 1) * 64, sms = geeps_sm_count();
   const bool here = tail >= 32 && wp.util >= 0.6 && d.n_blocks >= 4 * sms &&
                     (p->KW >= 5 || (p->KW >= 3 && d.m_tiles == 1 && d.cchunks == 1));
-  if (p->KW < 3 || p->cg < 32 || p->og < 32 || (p->x_pitch % 64 == 0 && p->cg % 64 == 0 && p->y_pitch % 64 == 0 && p->og % 64 == 0))
+  if (p->KW < 3 || p->KW > 7 || p->cg < 32 || p->og < 32 ||
+      (p->x_pitch % 64 == 0 && p->cg % 64 == 0 && p->y_pitch % 64 == 0 && p->og % 64 == 0))
     return here ? 1 : 0;
   const bool repeats_here = d.split <= 2, repeats_box = geeps_conv_box_wgrad_slices(p) <= 2;
   if (repeats_here != repeats_box && here == repeats_here) return here ? 1 : 0;
-  const double waves = (double)(((long long)d.m_tiles * d.cchunks * d.passes * d.split + sms - 1) / sms);
-  const double us = 6.1 + waves * (3.76 + (double)((d.n_blocks + d.split - 1) / d.split) * (0.349 + 0.654 * d.kpos / 128.0));
-  return us < (here ? 1.1 : 0.85) * geeps_conv_box_wgrad_us(p) ? 1 : 0;
+  const double waves = (double)(((long long)d.m_tiles * d.cchunks * d.passes * d.split + sms - 1) / sms), cols = d.TY * d.KW;
+  const double us = 5.9 + waves * (0.66 * cols + (double)((d.n_blocks + d.split - 1) / d.split) *
+                                                     (0.344 + d.kpos / 128.0 * (0.34 + 0.062 * cols)));
+  return us < (here ? 1.3 : 0.85) * geeps_conv_box_wgrad_us(p) ? 1 : 0;
 }
 
 int geeps_conv_wgrad_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {

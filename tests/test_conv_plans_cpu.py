@@ -195,3 +195,24 @@ def test_weight_gradients_that_repeat_bit_for_bit_keep_their_kernel():
             assert info.routed, (B, H, cg, og, k)
             kept += 1
     assert routed > 200 and kept > 50
+
+
+@pytest.mark.parametrize("B,H,cg,og,k,pad,there", [
+    # us, filter-row kernel / box kernel
+    (1, 12, 344, 400, 5, 0, False),               # 11.5 / 8.2
+    (94, 17, 416, 336, 7, 3, False),              # 463 / 349
+    (20, 29, 288, 416, 6, 3, False),              # 273 / 213
+    (104, 29, 240, 80, 4, 2, False),              # 99 / 80
+    (10, 7, 288, 264, 7, 3, False),               # 21.7 / 17.4
+    (48, 31, 40, 176, 6, 3, True),                # 66 / 157
+    (72, 46, 32, 80, 4, 2, True),                 # 37 / 48
+    (68, 53, 40, 208, 3, 1, True),                # 60 / 144
+    (41, 28, 136, 104, 5, 2, True)])              # 44 / 80
+def test_weight_gradients_off_128_byte_lines_go_to_the_faster_kernel(B, H, cg, og, k, pad, there):
+    p, _, _ = _params(2, B, H, H, cg, og, k, pad)
+    assert bool(L.lib().geeps_conv_wgrad_halo_applicable(C.byref(p))) == there
+
+
+def test_weight_gradients_of_filters_that_were_not_timed_go_by_the_rule_for_whole_lines():
+    p, _, _ = _params(2, 2, 40, 40, 40, 176, 8, 4)         # few blocks: the box kernel's by that rule
+    assert not L.lib().geeps_conv_wgrad_halo_applicable(C.byref(p))
