@@ -2030,6 +2030,8 @@ static SlotGrid apply_grid(long long P, int C) {
   g.smem = ((size_t)(C / 8) + g.grid.x - 1) / g.grid.x * 8 * 4 * sizeof(float);      // four constants per channel
   return g;
 }
+// ReLU mask with column sums
+static SlotGrid relu_colsum_grid(long long P, int C) { return slot_grid(P, C, 4, 4, 1); }
 
 int geeps_bn_forward(const void* x, void* y, const float* gamma, const float* beta, float* sums,
                      float* mean_rstd, float* running_mean, float* running_var, long long P, int C,
@@ -2191,7 +2193,7 @@ int geeps_relu_backward_colsum_clear(const void* dy, const void* y, void* dx, fl
   const bool apart = P * C > (1LL << 22);
   float* const along = apart ? nullptr : clear;
   const long long along_n = apart ? 0 : clear_n;
-  const SlotGrid rg = slot_grid(P, C, 4, 4, 1);
+  const SlotGrid rg = relu_colsum_grid(P, C);
   geeps_launch_plain(relu_backward_colsum_kernel, rg.grid, rg.threads, rg.smem, st,
       (const bf16*)dy, (const bf16*)y, (bf16*)dx, colsum, P, C, lddy, ldy, lddx, along, along_n, (int)clear_head(along, along_n));
   if (apart && clear_n > 0) geeps_clear_f32(clear, clear_n, st);
@@ -2317,8 +2319,10 @@ int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const G
       (const bf16*)dy, (const uint8_t*)argmax, (bf16*)dx, *g, accumulate);
   return CK();
 }
-int geeps_channel_blocks(long long P, int C, int* out) {
-  const SlotGrid g = slot_grid(P, C, 4, 4, 2);
+int geeps_channel_blocks(long long P, int C, int* out) { return geeps_channel_pass_blocks(0, P, C, out); }
+int geeps_channel_pass_blocks(int pass, long long P, int C, int* out) {
+  if (pass < 0 || pass > 3) return (int)cudaErrorInvalidValue;
+  const SlotGrid g = pass == 3 ? relu_colsum_grid(P, C) : pass == 2 ? apply_grid(P, C) : reduce_grid(pass == 1 ? 2 : 0, P, C);
   out[0] = (int)g.grid.x; out[1] = (int)g.grid.y; out[2] = g.threads; out[3] = (int)g.smem;
   return 0;
 }

@@ -111,9 +111,11 @@ int geeps_maxpool_forward(const void* x, void* y, void* argmax, const GeepsPoolG
 int geeps_maxpool_forward_relu(const void* x, void* y, void* argmax, const GeepsPoolGeom* g, void* stream);
 int geeps_maxpool_backward(const void* dy, const void* argmax, void* dx, const GeepsPoolGeom* g, int accumulate,
                            void* stream);
-// launch shape of a reduction over P pixels of C channels (host arithmetic only): channel shares, pixel shares, threads a
-// block, bytes of shared memory
+// launch shape of the sums of a BatchNorm over P pixels of C channels (host arithmetic only): channel shares, pixel shares,
+// threads a block, bytes of shared memory
 int geeps_channel_blocks(long long P, int C, int* out);
+// ... and of a pass: 0 those sums, 1 column sums, 2 a BatchNorm's element-wise pass, 3 ReLU mask with column sums
+int geeps_channel_pass_blocks(int pass, long long P, int C, int* out);
 // launch shape of the average pooling kernels (host arithmetic only): grid x, y, block x (vectors), y (pixels), z (rows);
 // group: at most three windows per direction cover a pixel
 int geeps_avgpool_blocks(int C, int width, long long rows, int group, int* out);

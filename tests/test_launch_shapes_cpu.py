@@ -34,21 +34,35 @@ def test_average_pooling_of_nothing_and_of_very_wide_rows():
     assert list(out) == [3, 65535, 256, 1, 1]                        # the second grid dimension has 16 bits
 
 
-def test_channel_blocks_cover_the_matrix_and_spread_few_pixels():
+@pytest.mark.parametrize("which,per_sm,floats", [(0, 2, 2), (1, 2, 1), (2, 2, 0), (3, 4, 1)])
+def test_channel_blocks_cover_the_matrix_and_spread_few_pixels(which, per_sm, floats):
+    """The grids that the passes launch; floats: per channel and pixel row in shared memory."""
     for P, Cc in itertools.product((1, 3, 8, 32, 49, 100, 392, 1568, 20000, 100352, 1000000),
                                    (8, 24, 64, 192, 576, 1000, 1024, 1032, 1288, 1536, 2040, 2048, 2056, 4096, 8192)):
         out = (C.c_int * 4)()
-        L.lib().geeps_channel_blocks(C.c_longlong(P), Cc, out)
+        assert L.lib().geeps_channel_pass_blocks(which, C.c_longlong(P), Cc, out) == 0
         cols, blocks, threads, smem = out
         cv = Cc // 8
         cvb = -(-cv // cols)                          # slots of a block, as the kernels compute them
         rows = threads // cvb
         assert threads % 32 == 0 and threads <= 256 and rows >= 1 and (cols - 1) * cvb < cv
-        assert smem == rows * cvb * 8 * 2 * 4 <= 32 * 1024
-        assert cols * blocks <= 148 * 4
+        # sums of the pixel rows, or four constants a channel
+        assert smem == (rows * cvb * 8 * floats * 4 if floats else cvb * 8 * 4 * 4) and smem <= 32 * 1024
+        assert cols * blocks <= 148 * per_sm
+        one = 148 // cols
+        assert which == 3 or blocks <= one or blocks >= 2 * one, (P, Cc, list(out))      # no SM with two where others have one
         assert rows * cv >= 0.75 * cols * threads, (P, Cc, list(out))         # threads with a slot
         # few pixels: an eighth of the SMs at least, or a block for every batch of rows
         assert cols * blocks >= min(148 // 8, cols * -(-P // rows)), (P, Cc, list(out))
+        if which == 0:
+            same = (C.c_int * 4)()
+            L.lib().geeps_channel_blocks(C.c_longlong(P), Cc, same)
+            assert list(same) == list(out)
+
+
+def test_channel_blocks_of_an_unknown_pass_are_refused():
+    out = (C.c_int * 4)()
+    assert L.lib().geeps_channel_pass_blocks(4, C.c_longlong(1), 8, out) != 0 and L.lib().geeps_channel_pass_blocks(-1, C.c_longlong(1), 8, out) != 0
 
 
 def test_lrn_backward_lanes_fit_the_channels():
