@@ -643,6 +643,10 @@ double geeps_conv_box_us(const GeepsConvTcParams* p) {
 }
 double geeps_conv_box_wgrad_us(const GeepsConvTcParams* p) { return plan_wgrad_box(p, geeps_sm_count()).us; }
 int geeps_conv_box_wgrad_slices(const GeepsConvTcParams* p) { return plan_wgrad_box(p, geeps_sm_count()).split; }
+long long geeps_conv_box_wgrad_steps(const GeepsConvTcParams* p) {
+  const WgradPlan g = plan_wgrad_box(p, geeps_sm_count());
+  return (long long)((g.kt + g.split - 1) / g.split) * ((g.bw * g.bh * g.bnb + 15) / 16);
+}
 int geeps_conv_box_pairs(const GeepsConvTcParams* p) {
   return p->mode != MODE_WGRAD && p->stride <= 1 && geeps_conv_tc_supported(p) && takes_pairs(plan_box(p, 1, 1, geeps_sm_count())) ? 1 : 0;
 }

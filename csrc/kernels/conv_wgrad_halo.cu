@@ -352,10 +352,14 @@ extern "C" {
 // begin on 32-byte sectors either.  There the expected times of both kernels decide (each fitted to 1300 products with filters of
 // 3 x 3 to 7 x 7; this one half within 4 %), unless they are close.  us, here / box: 53 x 53, 40 -> 208 at batch 68 60 / 144; 46 x 46, 88
 // -> 224 at batch 84 105 / 203; 28 x 28, 136 -> 104, 5 x 5 at batch 41 44 / 80; 31 x 31, 40 -> 176, 6 x 6 at batch 48 66 / 157; but 17 x 17,
-// 416 -> 336, 7 x 7 at batch 94 463 / 349.  The kernel taken so is 3.0 % slower than the faster one in the geometric mean, by the rule
+// 416 -> 336, 7 x 7 at batch 94 463 / 349.  The kernel taken so is 4.1 % slower than the faster one in the geometric mean, by the rule
 // above alone 6.6 %, and on one product of 1300 more than 3 % slower than the one of that rule.
 // Slices are added to dW in the order in which they come: one, or two on zeros, give the same bits in every call, more do not.  A
 // gradient that the rule above repeats bit for bit stays with its kernel (7 x 8 x 8, 72 -> 136: one slice there, seven here).
+// The tensor cores cut off what a step of 16 positions adds to a partial sum, so an error grows with the steps of a slice (of which
+// the positions beside the image need their share here): one that is longer than that rule's kernel has is not taken.  Error
+// against 64 bits here / there: 15 x 15, 264 -> 344, 7 x 7 at batch 45, 1260 steps / 636, 1.5e-5 / 1.0e-5; 41 x 41, 80 -> 296, 7 x 7 at
+// batch 21 5.8e-6 / 1.3e-5.
 int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p) {
   if (!halo_mode()) return 0;
   if (!geeps_conv_tc_supported(p)) return 0;
@@ -370,10 +374,12 @@ int geeps_conv_wgrad_halo_applicable(const GeepsConvTcParams* p) {
     return here ? 1 : 0;
   const bool repeats_here = d.split <= 2, repeats_box = geeps_conv_box_wgrad_slices(p) <= 2;
   if (repeats_here != repeats_box && here == repeats_here) return here ? 1 : 0;
+  const int blocks = (d.n_blocks + d.split - 1) / d.split;
   const double waves = (double)(((long long)d.m_tiles * d.cchunks * d.passes * d.split + sms - 1) / sms), cols = d.TY * d.KW;
-  const double us = 5.9 + waves * (0.66 * cols + (double)((d.n_blocks + d.split - 1) / d.split) *
-                                                     (0.344 + d.kpos / 128.0 * (0.34 + 0.062 * cols)));
-  return us < (here ? 1.3 : 0.85) * geeps_conv_box_wgrad_us(p) ? 1 : 0;
+  const double us = 5.9 + waves * (0.66 * cols + blocks * (0.344 + d.kpos / 128.0 * (0.34 + 0.062 * cols)));
+  const long long longer = (long long)blocks * (d.kpos / 16) - geeps_conv_box_wgrad_steps(p);
+  if (us < (here ? 1.3 : 0.85) * geeps_conv_box_wgrad_us(p)) return here || longer <= 0 ? 1 : 0;
+  return here && longer < 0 ? 1 : 0;
 }
 
 int geeps_conv_wgrad_halo_plan(const GeepsConvTcParams* p, GeepsHaloPlanInfo* out) {

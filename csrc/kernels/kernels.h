@@ -177,7 +177,8 @@ int geeps_conv_tc_supported(const GeepsConvTcParams* p);
 // (a negative split_k on a forward / data-gradient call keeps the call on the box kernel, -2 on its single CTAs).
 double geeps_conv_box_us(const GeepsConvTcParams* p);          // expected time of the box kernel, stride 1 (host arithmetic)
 double geeps_conv_box_wgrad_us(const GeepsConvTcParams* p);
-int geeps_conv_box_wgrad_slices(const GeepsConvTcParams* p);   // slices of the positions that the box kernel adds up
+int geeps_conv_box_wgrad_slices(const GeepsConvTcParams* p);   // slices of the positions that the box kernel adds up ...
+long long geeps_conv_box_wgrad_steps(const GeepsConvTcParams* p);      // ... and products that follow one another in a slice
 int geeps_conv_box_pairs(const GeepsConvTcParams* p);          // 1 if the box kernel runs p on CTA pairs
 int geeps_conv_halo_applicable(const GeepsConvTcParams* p);
 int geeps_conv_halo(const GeepsConvTcParams* p, void* stream);

@@ -207,6 +207,7 @@ def test_weight_gradients_that_repeat_bit_for_bit_keep_their_kernel():
     (48, 31, 40, 176, 6, 3, True),                # 66 / 157
     (72, 46, 32, 80, 4, 2, True),                 # 37 / 48
     (68, 53, 40, 208, 3, 1, True),                # 60 / 144
+    (45, 15, 264, 344, 7, 3, False),              # the faster one by its sums of 1260 steps instead of 636
     (41, 28, 136, 104, 5, 2, True)])              # 44 / 80
 def test_weight_gradients_off_128_byte_lines_go_to_the_faster_kernel(B, H, cg, og, k, pad, there):
     p, _, _ = _params(2, B, H, H, cg, og, k, pad)
@@ -216,3 +217,23 @@ def test_weight_gradients_off_128_byte_lines_go_to_the_faster_kernel(B, H, cg, o
 def test_weight_gradients_of_filters_that_were_not_timed_go_by_the_rule_for_whole_lines():
     p, _, _ = _params(2, 2, 40, 40, 40, 176, 8, 4)         # few blocks: the box kernel's by that rule
     assert not L.lib().geeps_conv_wgrad_halo_applicable(C.byref(p))
+
+
+def test_weight_gradients_go_to_no_kernel_with_longer_sums():
+    """What each step of 16 positions adds is cut off at the partial sum: off 128-byte lines the expected times choose a kernel
+    only if its slices have no more steps than those of the rule for whole lines."""
+    lib = L.lib()
+    lib.geeps_conv_box_wgrad_steps.restype = C.c_longlong
+    moved = 0
+    for B, H, cg, og, k in itertools.product((1, 3, 12, 45, 68, 200), (8, 15, 28, 41, 53), (32, 40, 80, 104, 264, 344), (40, 112, 208, 344), (3, 4, 5, 7)):
+        p, _, _ = _params(2, B, H, H, cg, og, k, k // 2)
+        info = L.HaloPlanInfo()
+        if not lib.geeps_conv_wgrad_halo_plan(C.byref(p), C.byref(info)):
+            continue
+        tail = cg - (cg + 63) // 64 * 64 + 64
+        rule = tail >= 32 and info.util >= 0.6 and info.n_blocks >= 4 * 148 and (k >= 5 or (info.m_tiles == 1 and cg <= 64))
+        here, box = -(-info.n_blocks // info.split) * info.positions // 16, lib.geeps_conv_box_wgrad_steps(C.byref(p))
+        if bool(info.routed) != rule:
+            assert (here <= box) if info.routed else (box <= here), (B, H, cg, og, k)
+            moved += 1
+    assert moved > 50

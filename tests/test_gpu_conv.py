@@ -465,7 +465,9 @@ def test_8_bit_sources_on_any_byte_take_the_fast_kernel():
     ("fwd", 19, 18, 6, 328, 360, 2, 1, 0),
     ("dgrad", 26, 30, 23, 80, 136, 2, 1, 0),      # more pairs than fit at once
     ("dgrad", 26, 27, 26, 72, 72, 3, 0, 0), ("dgrad", 11, 29, 27, 72, 208, 3, 1, 16), ("dgrad", 17, 17, 30, 72, 72, 5, 0, 0),
-    ("dgrad", 24, 20, 21, 248, 136, 3, 1, 0)])    # 256 columns: two panels of the weights in each half
+    ("dgrad", 24, 20, 21, 248, 136, 3, 1, 0),     # 256 columns: two panels of the weights in each half
+    ("fwd", 32, 17, 17, 384, 256, 5, 2, 0),       # whole 128-byte lines
+    ("fwd", 37, 17, 17, 384, 384, 5, 2, 0), ("dgrad", 37, 17, 17, 256, 384, 5, 2, 0)])
 def test_box_convolution_on_cta_pairs_gives_the_bits_of_single_ctas(mode, B, H, W, cg, og, k, pad, wide):
     """Two neighbouring pixel boxes by one product of 256 rows: the same terms in the same order, so the same bits as one CTA per
     box; nothing outside the result is written."""
@@ -529,23 +531,41 @@ def test_layers_off_128_byte_lines_agree_on_both_kernels(B, H, cg, og, k):
     assert routed
 
 
-@pytest.mark.parametrize("B,H,cg,og,k", [(68, 53, 40, 208, 3), (41, 28, 136, 104, 5), (5, 26, 280, 200, 5), (37, 27, 168, 368, 3), (20, 47, 104, 112, 5),
-                                         (40, 28, 136, 72, 3), (95, 33, 64, 360, 5)])
-def test_weight_gradients_off_128_byte_lines_agree_on_both_kernels(B, H, cg, og, k):
-    """Layers that the expected times send to the filter-row kernel (and one that they keep off it), as conv_tc() runs them and on the
-    box kernel: the same products, summed in fp32 in other slices."""
+@pytest.mark.parametrize("B,H,cg,og,k,there", [
+    (68, 53, 40, 208, 3, True), (41, 28, 136, 104, 5, True),
+    (14, 24, 136, 152, 5, True),               # a last chunk of 8 channels, few blocks
+    (9, 11, 200, 280, 5, True),                # ... and half of the positions beside the image
+    (21, 41, 80, 296, 7, True),                # a last chunk of 16
+    (95, 33, 64, 360, 5, True), (45, 15, 264, 344, 7, False),
+    (5, 26, 280, 200, 5, False), (37, 27, 168, 368, 3, False), (20, 47, 104, 112, 5, False), (40, 28, 136, 72, 3, False)])
+def test_weight_gradients_off_128_byte_lines_agree_on_both_kernels(B, H, cg, og, k, there):
+    """Layers that the expected times send to the filter-row kernel and such that they keep off it, as conv_tc() runs them and on
+    both kernels by name: the same products, summed in fp32 in other slices."""
+    import ctypes
+    from geeps_b200.ops import _lib as L
     from geeps_b200.ops import functional as F
     dev = torch.device("cuda:0")
     gen = torch.Generator(device=dev).manual_seed(H * cg)
-    ld = (k * k * cg + 7) // 8 * 8 + 8
+    kd, pad = k * k * cg, k // 2
+    ld = (kd + 7) // 8 * 8 + 8
     x = torch.randn(B, H, H, cg, device=dev, generator=gen).to(BF)
     dy = torch.randn(B, H, H, og, device=dev, generator=gen).to(BF)
-    out = [torch.full((og, ld), 3.0, device=dev) for _ in range(2)]
-    for o, split_k in zip(out, (0, -1)):
-        F.conv_tc(F.CONV_WGRAD, x, dy, o, k, k // 2, split_k=split_k)
-        assert (o[:, k * k * cg:] == 0).all()
-    # n additions of terms of norm one, each rounded by 2^-24 of a partial sum of norm at most sqrt(n): sqrt(n) 2^-24 of the result's
-    assert _rel(out[0], out[1].double()) < 2 * (B * H * H) ** 0.5 * 2.0 ** -24
+    out = [torch.full((og, ld), 3.0, device=dev) for _ in range(3)]
+    p = F.conv_tc_params(F.CONV_WGRAD, x, dy, out[0], k, pad)
+    assert bool(L.lib().geeps_conv_wgrad_halo_applicable(ctypes.byref(p))) == there
+    F.conv_tc(F.CONV_WGRAD, x, dy, out[0], k, pad)
+    F.conv_tc(F.CONV_WGRAD, x, dy, out[1], k, pad, split_k=-1)
+    p.w = out[2].data_ptr()
+    L.check(L.lib().geeps_conv_wgrad_halo(ctypes.byref(p), L.stream_ptr()), "conv_wgrad_halo")
+    x64 = torch.nn.functional.pad(x.double(), (0, 0, pad, pad, pad, pad))
+    d64 = dy.double().view(-1, og)
+    ref = torch.cat([d64.t() @ x64[:, i:i + H, j:j + H].reshape(-1, cg) for i in range(k) for j in range(k)], 1)
+    for o in out:
+        assert (o[:, kd:] == 0).all()
+        # One slice at most: a step adds 16 of n positions, so the partial sum behind step j of J = n / 16 has a norm of sqrt(j / J) of the
+        # result's, and the tensor cores cut off less than 2^-23 of it: 2 / 3 J 2^-23 in all (steps that hold fewer positions of
+        # the image, util of them, are as many more).
+        assert _rel(o[:, :kd], ref) < 2 / 3 * (B * H * H / 16 / 0.45) * 2.0 ** -23
 
 
 @pytest.mark.parametrize("B,H,cg,og", [(7, 8, 72, 136), (2, 13, 368, 352), (1, 19, 80, 288)])
