@@ -713,7 +713,7 @@ def test_relu_backward_clears_a_range_on_the_way(off, n, P, C):
 
 @pytest.mark.parametrize("B,H,Cc,pad,ldy", [(64, 29, 8, 0, 8), (61, 31, 8, 1, 8), (40, 13, 120, 0, 136), (9, 61, 40, 1, 40),
                                             (3, 27, 240, 0, 240), (2, 28, 312, 0, 312), (100, 14, 88, 1, 88),
-                                            (260, 27, 32, 0, 32), (24, 55, 296, 0, 296), (36, 15, 520, 0, 520)])
+                                            (260, 27, 32, 0, 32), (40, 24, 296, 0, 296), (36, 15, 520, 0, 520)])
 @pytest.mark.parametrize("alpha", [1e-4, 0.01, 0.5])
 def test_lrn_maxpool_backward_by_quads_matches_small_batches(B, H, Cc, pad, ldy, alpha):
     """A batch large enough for the quad kernel (one step a warp and several, ends of rows and images inside a warp,
@@ -724,7 +724,8 @@ def test_lrn_maxpool_backward_by_quads_matches_small_batches(B, H, Cc, pad, ldy,
     size, beta, kk = 5, 0.75, 1.0
     x = (torch.randn(B, H, H, Cc, device=DEV) * 3).clamp_min(-0.5).to(BF)        # some negative inputs: masked by sign
     g = F.pool_geom(x.shape, 3, 2, pad, Cc, ldy)
-    assert B * ((H + pad + 1) // 2) ** 2 * Cc // 8 >= 96 * torch.cuda.get_device_properties(0).multi_processor_count
+    vectors, line = ((H + pad + 1) // 2) ** 2 * Cc // 8, 96 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert B * vectors >= line > vectors
     arg = torch.randint(0, 9, (B, g.OH, g.OW, Cc), device=DEV, dtype=torch.uint8)
     dp = torch.randn(B, g.OH, g.OW, ldy, device=DEV).to(BF)
     dx, cs = torch.empty_like(x), torch.empty(Cc, device=DEV)

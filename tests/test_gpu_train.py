@@ -32,6 +32,51 @@ def tiny_net():
     return Net("tiny", Input(cpad=8), layers)
 
 
+def test_max_pooling_takes_the_relu_mask_from_the_convolution_in_front():
+    """A Net folds the ReLU's backward pass into the max pooling behind it: the gradients of the same layers with a mask of
+    their own.  Whole numbers, so every sum is exact."""
+    torch.manual_seed(1)
+    dev = torch.device("cuda:0")
+    make = lambda: [Conv2d("c1", 24, 3, pad=1, relu=True, need_dx=False), Pool("max", 3, 2), Conv2d("c2", 32, 3, pad=1, groups=2, relu=True),
+                    Pool("max", 2, 2)]                                                                              # noqa: E731
+    net = Net("n", Input(cpad=8), make() + [Linear("f", 16, fp32_out=True)])
+    net.setup((6, 3, 15, 15), dev)
+    folded, apart, shape = net.layers[:4], make(), (6, 15, 15, 8)
+    for layer in apart:
+        shape = layer.setup(shape, dev)
+    for a, b in zip(folded, apart):
+        if isinstance(a, Conv2d):
+            assert a.dy_is_masked and not b.dy_is_masked
+            for spec in a.param_specs():
+                name = spec.name.split(".")[-1]
+                w = torch.randint(-1, 2, spec.shape, device=dev).float()
+                for layer in (a, b):
+                    if name == "weight":
+                        layer.p16[name] = w.to(torch.bfloat16)
+                    else:
+                        layer.p32[name] = w
+                    layer.g32[name] = torch.full(spec.shape, 5.0, device=dev)
+        else:
+            assert a.mask_relu_input and not b.mask_relu_input
+    x = torch.randint(-1, 2, (6, 15, 15, 8), device=dev).to(torch.bfloat16)
+    outs = []
+    for layers in (folded, apart):
+        h = x
+        for layer in layers:
+            h = layer.forward(h).view(layer.out_shape)
+        outs.append(h.clone())
+    assert torch.equal(*outs) and (outs[0] == 0).any()
+    dy = torch.randint(-1, 2, outs[0].shape, device=dev).to(torch.bfloat16)
+    for layers in (folded, apart):
+        d = dy
+        for layer in reversed(layers):
+            d = layer.backward(d)
+    for a, b in zip(folded, apart):
+        if isinstance(a, Conv2d):
+            assert a.g32["weight"].any() and torch.equal(a.g32["weight"], b.g32["weight"]) and torch.equal(a.g32["bias"], b.g32["bias"])
+            assert not a.need_dx or torch.equal(a.dx, b.dx)
+
+
 @pytest.mark.parametrize("transport", [TRANSPORT_NVLINK, TRANSPORT_TCP])
 def test_tiny_net_gradients_match_torch(transport):
     torch.manual_seed(0)
