@@ -1697,9 +1697,10 @@ avgpool_backward_kernel(const bf16* __restrict__ dy, bf16* __restrict__ dx, cons
 // sums), backward multiplies pairs; captured chain, us,
 // forward and backward: 32 x 14 x 14 x 576 on the kernels above 10.0, 14.8, this 6.6, 6.6 (two rows a thread 6.2, 8.1, one 7.9,
 // 8.9; unpacked single products 7.5, 10.6);
-// 100 x 32 x 32 x 96 23.8, 34.9, now 13.4, 13.6.
+// 100 x 32 x 32 x 96 23.8, 34.9, now 13.4, 13.6.  Backward by one row a thread spills at five blocks per SM (2 x 28 x 28 x 320 2.86,
+// at four 2.75, 512 x 5 x 5 x 24 2.62, 2.50), forward it does not.
 template <bool BWD, int R>
-__global__ void __launch_bounds__(256, R == 1 ? 5 : 2)
+__global__ void __launch_bounds__(256, R > 1 ? 2 : BWD ? 4 : 5)
 avgpool3_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int H, int W, int OH, int OW, int cv, long long ldi,
                 long long ldo, int off, int blocks_h, int total, int accumulate) {
   geeps_pdl_enter();
