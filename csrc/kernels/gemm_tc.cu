@@ -549,7 +549,7 @@ TileChoice choose_tiles(const GeepsGemmParams* p, int unit, int kt, int sms, boo
       const int per = (kt + cs - 1) / cs;
       if (cs > 1 && (per < 4 || (long long)(cs - 1) * per >= kt)) continue;    // every slice needs k tiles
       // SMs that whole clusters find in GPCs of different sizes: 33 clusters of four and 15 of eight are resident on 148 SMs
-      const long long slots = cs <= 2 ? sms : cs == 4 ? sms * 8 / 9 : sms * 5 / 6 / 8 * 8;
+      const long long slots = cs <= 2 ? sms : cs == 4 ? sms * 9 / 10 / 4 * 4 : sms * 5 / 6 / 8 * 8;
       const long long rounds = (tiles * cs + slots - 1) / slots;
       // a k step of a slice has its price even for a few rows (4 x 1024, K = 21841: 21.5 us on 64 x 4, 16 on 128 x 8)
       double cost = rounds * (per * ((cs > 1 && a_rows < 32 ? 32.0 : a_rows) + bn) * 128.0 + kTileOver);
