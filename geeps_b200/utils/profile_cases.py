@@ -12,6 +12,8 @@ once and launches the kernel of interest three times.
   lrn_pool    LRN fused with the 3x3 stride-2 max pooling after it, forward + backward (256 x 55 x 55 x 96)
   pull_gemm   fused pull + GEMM on an fc6-shaped layer (4 local shards)
   conv_fwd / conv_dgrad / conv_wgrad   implicit-GEMM convolution, conv3 shape (256 x 13 x 13, 256 -> 384, 3x3)
+  conv_pair   box convolution on CTA pairs, a forward pass off 128-byte lines (9 x 38 x 38, 376 -> 256, 3 x 3)
+  input_u8    8-bit source images cropped and normalised into the network's input layout (256 x 256 x 256 -> 227 x 227)
   conv1_fwd   AlexNet conv1 after space-to-depth (256 x 57 x 57 x 64 (48 + 16 zero) -> 96, 3x3, no padding);
               routed to the halo-tile kernel, like conv2_fwd / conv2_dgrad (GEEPS_HALO_CONV=0: the box kernel)
   conv2_fwd / conv2_dgrad   one group of AlexNet conv2 (256 x 27 x 27, 48 of 96 -> 128 of 256 channels, 5x5)
@@ -112,14 +114,21 @@ def main():
         out = torch.zeros(M, N, dtype=torch.float32, device=dev)
         for _ in range(4):
             F.pull_gemm(x, [t.data_ptr() for t in parts], [s * (N // shards) for s in range(shards)], out, ldw=K)
-    elif case in ("conv_fwd", "conv_dgrad", "conv_wgrad"):
-        B, H, cin, cout, k, pad = 256, 13, 256, 384, 3, 1
+    elif case == "input_u8":
+        from ..ops.layers import Input
+        layer = Input(s2d=4, s2d_k=11, cpad=64, mean=(104.0, 117.0, 123.0), scale=1.0 / 58.0)
+        layer.setup((256, 3, 227, 227), dev)
+        images = torch.randint(0, 256, (256, 3, 256, 256), device=dev, dtype=torch.uint8)
+        for _ in range(4):
+            layer.forward(images)
+    elif case in ("conv_fwd", "conv_dgrad", "conv_wgrad", "conv_pair"):
+        B, H, cin, cout, k, pad = (9, 38, 376, 256, 3, 1) if case == "conv_pair" else (256, 13, 256, 384, 3, 1)
         x = (torch.randn(B, H, H, cin, device=dev) * 0.5).to(BF)
         y = (torch.randn(B, H, H, cout, device=dev) * 0.5).to(BF)
         w = (torch.randn(cout, k * k * cin, device=dev) * 0.02).to(BF)
         dw = torch.empty(cout, k * k * cin, device=dev)
         for _ in range(4):
-            if case == "conv_fwd":
+            if case in ("conv_fwd", "conv_pair"):
                 F.conv_tc(F.CONV_FWD, x, y, w, k, pad, relu=True)
             elif case == "conv_dgrad":
                 F.conv_tc(F.CONV_DGRAD, x, y, w, k, pad)
