@@ -492,7 +492,10 @@ struct BoxPlan {
 // Times (us, captured chain) of 364 forward and 364 data-gradient products with 7 x 7 to 56 x 56 pixels, 32 to 384 channels,
 // 3 x 3 and 5 x 5 taps, as launch + waves * (tile + k-tiles * (k-tile + width * per column)); half of the fits lie within
 // 13 % of the measurement.  Rows of activations or weights that do not begin on 128-byte lines cost a k-tile more, above all
-// where one CTA loads the whole weight tile: 24 x 24 x 296 -> 240 at batch 197 219 us on single CTAs, 151 on pairs.
+// where one CTA loads the whole weight tile.  us, single CTAs / pairs: 34 x 23 x 23, 248 -> 256, data gradient 44.3 / 29.0; 9 x 38 x 38, 376 ->
+// 256 39.4 / 27.7; 62 x 34 x 34, 216 -> 144, 5 x 5 236 / 172.  Sixty drawn layers that the rule sends to pairs: off the lines 0.84 of the
+// time on single CTAs (0.65 to 1.04), on them 0.985 (0.83 to 1.04), nearly all 5 x 5; AlexNet's conv3 - conv5 and the Inception layers
+// stay on single CTAs.
 struct KernelCost { double launch, tile, tile_col, kt, kt_col, kt_mis, kt_mis_col; };
 constexpr KernelCost kFwdOne = {4.09, 1.52, 0.146, 0.143, 0.028, 0., 0.062}, kFwdPair = {4.98, 1.19, 0.326, 0.152, 0.021, 0.012, 0.028},
                      kDgradOne = {3.47, 1.73, 0., 0.182, 0.033, 0., 0.044}, kDgradPair = {5.22, 0., 0.603, 0.208, 0.019, 0.023, 0.008};

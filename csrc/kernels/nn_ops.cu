@@ -2087,7 +2087,9 @@ static SlotGrid bn_coop_grid(long long P, int C) {
 static bool bn_coop_enabled() {
   static int v = -1;
   // off by default: with at most one block per SM and a grid barrier the single launch is slower than two full-width
-  // launches (Inception-BN-22K 5.84 against 5.65 ms per step, small net 1.96 against 1.95 ms)
+  // launches (Inception-BN-22K 5.84 against 5.65 ms per step, small net 1.96 against 1.95 ms).  The batches of the two launches serve
+  // it too, though the backward form by the mask bits spills 16 bytes with them: 25088 x 192 forward 14.0 -> 11.3, backward 16.6 ->
+  // 15.2 us, 6272 x 160 8.4 -> 7.6, 9.7 -> 9.4, 49 x 1024 11.2 -> 10.8, 11.3 -> 11.4
   if (v < 0) { const char* e = getenv("GEEPS_BN_COOP"); v = e ? atoi(e) : 0; }
   return v != 0;
 }
